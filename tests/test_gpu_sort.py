@@ -93,3 +93,33 @@ def test_sort_empty_and_bad_args(sdlib):
     assert st == sdlib._abi.SD_ERR_CAPACITY  # scratch too small
     st = sdlib.lib().sd_sort_pairs(None, None, None, None, 16, 33, None, 0, None)
     assert st == sdlib._abi.SD_ERR_INVALID_ARG
+
+
+@pytest.mark.parametrize("items", [8, 16])
+@pytest.mark.parametrize("n", [32 * 4096 - 1, 32 * 4096, 32 * 4096 + 1, 33 * 4096, 64 * 4096 + 17, 700 * 2048 + 5])
+@pytest.mark.parametrize("kind", ["random", "padded"])
+def test_sort_look_back_groups(sdlib, items, n, kind):
+    """Sizes around the look-back's groups of 32 tiles (2,048 or 4,096 keys),
+    digits of 8, 9 and 10 bits, random keys and runs of one padding word, and
+    key buffers off 16-byte alignment."""
+    import torch
+    rng = np.random.default_rng(n)
+    before = sdlib._abi.tune_get("sort_items")
+    sdlib._abi.tune_set("sort_items", items)
+    try:
+        for bits in (8, 18, 20, 32):
+            keys = rng.integers(0, 1 << bits, n, dtype=np.uint64).astype(np.uint32)
+            if kind == "padded":
+                keys[rng.random(n) < 0.75] = (1 << bits) - 1
+            dev = torch.device("cuda:0")
+            buf = [torch.zeros(n + 1, dtype=torch.int32, device=dev)[1:] for _ in range(4)]
+            buf[0].copy_(torch.from_numpy(keys.view(np.int32)))
+            buf[1].copy_(torch.arange(n, dtype=torch.int32))
+            scratch = torch.zeros(sdlib.SpatialPartition.sort_scratch_bytes(n, bits), dtype=torch.uint8, device=dev)
+            sdlib.SpatialPartition.sort_pairs(*buf, n, bits, scratch)
+            assert sdlib.SpatialPartition.sort_status(scratch) == 0
+            order = np.argsort(keys, kind="stable")
+            assert np.array_equal(buf[1].cpu().numpy(), order.astype(np.int32))
+            assert np.array_equal(buf[0].cpu().numpy().view(np.uint32), keys[order])
+    finally:
+        sdlib._abi.tune_set("sort_items", before)
