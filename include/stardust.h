@@ -106,8 +106,9 @@ typedef struct sd_stats {
      * re-sorts incrementally when at most knob "resort_max" changed, else it
      * runs the radix passes); 0 when the knob is 0 */
     uint64_t moved_keys;
-    /* kernels one step launches (the kernel nodes of the captured step
-     * graph; 0 before the first step) */
+    /* kernels one step launches (the kernel nodes per step of the graph the
+     * last sd_engine_step call launched; 0 before the first step).  Sphere
+     * scenes: calls of four or more steps run fewer kernels per step */
     uint64_t step_kernels;
     /* sphere scenes with contact lists (knob "skin_um"), since prepare:
      * steps that built the lists (a scan over the window widened by the
@@ -505,7 +506,8 @@ sd_status sd_engine_load_checkpoint(sd_engine* h, const char* path);
  *                   without clumps or meshes also 6 (40) or 8 (32 registers, more spills)
  *   "contact_block" threads per block of the per-sphere contact kernels: 64, 128 or 256
  *                   (default)
- *   "fix_blocks"    blocks per SM of the in-place reorder's fixed grid: 2, 4 or 8 (default)
+ *   "fix_blocks"    blocks per SM of the in-place reorder's fixed grid: 2, 4 or 8 (default);
+ *                   calls of four or more steps: 1 below 8, else 2
  *   "hull_blocks"   convex-hull scenes: resident 128-thread blocks per SM the GJK kernel is
  *                   compiled for: 3 (168 registers) or 4 (128, the default)
  *   "lbvh_rebuild"  convex-hull scenes: steps between full LBVH builds (1..4096, default 16);

@@ -37,10 +37,9 @@
 
 #include "sd_common.cuh"
 #include "sd_internal.h"
+#include "sd_reorder.cuh"
 
 namespace sd {
-
-constexpr uint32_t kIdMask = 0x7fffffffu;
 
 __device__ __forceinline__ int32_t axis_cell(float x, float lo, float cell, int32_t n) {
     float t = (x - lo) / cell;
@@ -1049,19 +1048,6 @@ dem_contact_column_kernel(DemParams p, uint32_t n, const float4* __restrict__ po
     if (staged && !use_tile && threadIdx.x == 0) mbar_wait_bounded(&s_bar, 0);
 }
 
-// Rotation matrix (row-major) of a unit quaternion (s, x, y, z).
-__device__ __forceinline__ void quat_rot(float qs, float qx, float qy, float qz, float* R) {
-    R[0] = 1.0f - 2.0f * (qy * qy + qz * qz);
-    R[1] = 2.0f * (qx * qy - qs * qz);
-    R[2] = 2.0f * (qx * qz + qs * qy);
-    R[3] = 2.0f * (qx * qy + qs * qz);
-    R[4] = 1.0f - 2.0f * (qx * qx + qz * qz);
-    R[5] = 2.0f * (qy * qz - qs * qx);
-    R[6] = 2.0f * (qx * qz - qs * qy);
-    R[7] = 2.0f * (qy * qz + qs * qx);
-    R[8] = 1.0f - 2.0f * (qx * qx + qy * qy);
-}
-
 // A rigid body's step (replaces computeForcesAndTorquesCUDA +
 // advectParticlesCUDA + updateSphereDataCUDA, physics_update.cu:26-310):
 // gather the body's sphere forces and torques in sphere-id order (the
@@ -1239,37 +1225,6 @@ __global__ void dem_keys_kernel(DemParams p, uint32_t n, const float4* __restric
     vals[i] = i;
 }
 
-constexpr int kReorderThreads = 256;
-
-// Writes cell_start for the cells block [b0, b1) owns, (s_keys[0],
-// s_keys[cnt]] (the first block starts at cell 0, the last ends at ncells),
-// by binary search over the block's sorted keys s_keys[1..cnt] in shared
-// memory, so that every cell's lower bound is written exactly once.  Cells
-// at or before the block's first key take b0 and cells after its last key
-// (only the last block has them: the tail up to ncells) take b1 without a
-// search -- an empty region past the last sphere can be tens of thousands
-// of cells, all in that one block.
-__device__ __forceinline__ void block_cell_starts(const uint32_t* s_keys, uint32_t b0, uint32_t b1, uint32_t n,
-                                                  uint32_t ncells, uint32_t* __restrict__ cell_start) {
-    const int64_t lo = b0 == 0 ? -1 : (int64_t)s_keys[0];
-    const int64_t hi = b1 == n ? (int64_t)ncells : min((int64_t)s_keys[b1 - b0], (int64_t)ncells);
-    const uint32_t cnt = b1 - b0;
-    const int64_t kfirst = cnt ? (int64_t)s_keys[1] : hi, klast = cnt ? (int64_t)s_keys[cnt] : lo;
-    for (int64_t c = lo + 1 + threadIdx.x; c <= hi; c += blockDim.x) {
-        if (c <= kfirst || c > klast) {
-            cell_start[c] = c <= kfirst ? b0 : b1;
-            continue;
-        }
-        uint32_t a = 0, z = cnt;  // first index in [0, cnt) with key >= c, else cnt
-        while (a < z) {
-            uint32_t m = (a + z) >> 1;
-            if ((int64_t)s_keys[m + 1] < c) a = m + 1;
-            else z = m;
-        }
-        cell_start[c] = b0 + a;
-    }
-}
-
 // Gather the next state into sorted order and write cell_start.
 __global__ void __launch_bounds__(kReorderThreads)
 dem_reorder_kernel(uint32_t n, uint32_t ncells, const uint32_t* __restrict__ keys,
@@ -1302,233 +1257,77 @@ dem_reorder_kernel(uint32_t n, uint32_t ncells, const uint32_t* __restrict__ key
     block_cell_starts(s_keys, b0, b1, n, ncells, cell_start);
 }
 
-// The order the incremental re-sort found: the new keys, and the M moved
-// entries in (key, slot) order with their sorted positions and, per moved
-// slot in ascending order, slot - rank.
+// The in-place reorder (sd_reorder.cuh) as two kernels, with the lists the
+// plan kernel wrote: rv.scratch[1] = M moved entries, [3] = T positions in
+// their intervals.
 struct ResortView {
-    const uint32_t* keys_new;
     const uint32_t* pos;
     const uint32_t* q;
     const unsigned long long* list;
-    const uint32_t* scratch;  // [1] = M, [3] = T
+    const uint32_t* scratch;
     uint32_t mmax;
-    const uint32_t* iv_lo;    // per moved entry: first position of the interval its move shifts
-    const uint32_t* iv_pre;   // exclusive prefix sums of the intervals' lengths (T = iv_pre[M])
+    const uint32_t* iv_lo;
+    const uint32_t* iv_pre;
 };
 
-// First index in [0, m) of ascending a with a[i] >= x (m if none).
-__device__ __forceinline__ uint32_t lower_idx(const uint32_t* a, uint32_t m, uint32_t x) {
-    uint32_t lo = 0, hi = m;
-    while (lo < hi) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (a[mid] < x) lo = mid + 1;
-        else hi = mid;
-    }
-    return lo;
-}
-
-// First index in [0, m) of ascending a with a[i] > x (m if none).
-__device__ __forceinline__ uint32_t upper_idx(const uint32_t* a, uint32_t m, uint32_t x) {
-    uint32_t lo = 0, hi = m;
-    while (lo < hi) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (a[mid] <= x) lo = mid + 1;
-        else hi = mid;
-    }
-    return lo;
-}
-
-// Copies the re-sort's positions and slot - rank lists (M <= kResortMaxCap)
-// into the block's shared memory; every thread calls it.
-__device__ __forceinline__ void load_resort_lists(const ResortView& rv, uint32_t M, uint32_t* s_pos, uint32_t* s_q) {
-    for (uint32_t i = threadIdx.x; i < M; i += blockDim.x) {
-        s_pos[i] = rv.pos[i];
-        s_q[i] = rv.q[i];
-    }
-    __syncthreads();
-}
-
-// Source slot and key of sorted position k: a moved entry where one was
-// placed (returns true), else the unmoved slot of rank u = k - (moved
-// entries placed before k), which is u + #{moved slots s_j with s_j - j <=
-// u}.  An unmoved slot's new key is its previous one.
-template <bool KEY>
-__device__ __forceinline__ bool sorted_entry(uint32_t k, uint32_t M, const uint32_t* s_pos, const uint32_t* s_q,
-                                             const ResortView& rv, uint32_t n, uint32_t& src, uint32_t& key) {
-    const uint32_t lo = lower_idx(s_pos, M, k);
-    if (lo < M && s_pos[lo] == k) {
-        const unsigned long long c = rv.list[lo];
-        src = (uint32_t)c;
-        if (KEY) key = (uint32_t)(c >> 32);
-        return true;
-    }
-    const uint32_t u = k - lo;
-    src = u + upper_idx(s_q, M, u);
-    if (KEY) key = src < n ? rv.keys_new[src] : 0u;
-    return false;
-}
-
-// The contact lists the in-place reorder moves with the state (all null
-// when the step uses none): per slot count, build position and kVlCap rows
-// of neighbour ids, and same-sized buffers for the gathered entries.
-struct ListView {
-    uint32_t* cnt;
-    float4* ref;
-    uint32_t* nbr;
-    uint32_t* cnt_t;
-    float4* ref_t;
-    uint32_t* nbr_t;
+struct FixLists {
+    uint32_t pos[kResortMaxCap], q[kResortMaxCap], iv_lo[kResortMaxCap], iv_pre[kResortMaxCap];
 };
 
-// The in-place reorder of a step whose next state stays where the contact
-// kernel wrote it (S, the *_n buffers, in the previous slot order).  Sorted
-// position k needs the entry of slot src(k); where src(k) == k -- every
-// slot but those shifted by the moved keys -- nothing moves.  Only
-// positions between a moved entry's old slot and its new position can
-// change hands, so with the re-sort's order the kernels visit those
-// intervals (T positions in all; a position in several is visited by each,
-// writing the same values) rather than all n, unless T is above n / 4.
-// Phase 1 gathers the positions that change hands into the free buffer T
-// (the step's input state, no longer read) and, with the re-sort's order,
-// shifts the cell table: cell_start[c] counts the entries with key < c, so
-// an entry moving from key a to key b takes one from the cells (a, b] when
-// b > a and adds one to (b, a] when b < a (atomic adds: several entries may
-// share cells).  Phase 2 copies the gathered entries back and records
-// their keys; for the radix passes' order (more moves than the re-sort
-// takes) every position is visited and the cell table is rebuilt as the
-// plain reorder does.  Both kernels run on a fixed grid (grid-stride).
-
-// Position visited by work item t: in interval mode the position of item t
-// among the intervals' concatenation, else t itself.
-__device__ __forceinline__ uint32_t visit_position(uint32_t t, bool iv, uint32_t M, const uint32_t* s_ivlo,
-                                                   const uint32_t* s_ivpre) {
-    if (!iv) return t;
-    const uint32_t r = upper_idx(s_ivpre, M, t) - 1u;  // s_ivpre[0] = 0 <= t
-    return s_ivlo[r] + (t - s_ivpre[r]);
-}
-
-// Loads the re-sort's lists (and the intervals when iv) into shared memory.
-__device__ __forceinline__ void load_fix_lists(const ResortView& rv, uint32_t M, bool iv, uint32_t* s_pos,
-                                               uint32_t* s_q, uint32_t* s_ivlo, uint32_t* s_ivpre) {
+// The re-sort's lists (and the intervals when iv) in shared memory.
+__device__ __forceinline__ MovedLists load_fix_lists(const ResortView& rv, uint32_t M, bool iv, FixLists& s) {
     for (uint32_t i = threadIdx.x; i < M; i += blockDim.x) {
-        s_pos[i] = rv.pos[i];
-        s_q[i] = rv.q[i];
+        s.pos[i] = rv.pos[i];
+        s.q[i] = rv.q[i];
         if (iv) {
-            s_ivlo[i] = rv.iv_lo[i];
-            s_ivpre[i] = rv.iv_pre[i];
+            s.iv_lo[i] = rv.iv_lo[i];
+            s.iv_pre[i] = rv.iv_pre[i];
         }
     }
     __syncthreads();
+    return MovedLists{M, rv.list, s.pos, s.q, s.iv_lo, s.iv_pre};
 }
 
 __global__ void __launch_bounds__(kReorderThreads)
-dem_fix_gather_kernel(uint32_t n, uint32_t ncells, const uint32_t* __restrict__ vals,
-                      const float4* __restrict__ s_pos4, const float4* __restrict__ s_vel,
-                      const float4* __restrict__ s_omg, float4* __restrict__ t_pos, float4* __restrict__ t_vel,
-                      float4* __restrict__ t_omg, uint32_t* __restrict__ cell_start,
-                      const uint32_t* __restrict__ keys_prev, ResortView rv, ListView lv) {
-    __shared__ uint32_t s_pos[kResortMaxCap], s_q[kResortMaxCap], s_ivlo[kResortMaxCap], s_ivpre[kResortMaxCap];
+dem_fix_gather_kernel(uint32_t n, uint32_t ncells, const uint32_t* __restrict__ vals, FixState f,
+                      uint32_t* __restrict__ cell_start, ResortView rv) {
+    __shared__ FixLists s;
     const uint32_t M = rv.scratch[1];
-    const bool inc = M <= rv.mmax;
-    const uint32_t T = inc ? (M ? rv.scratch[3] : 0u) : n;
-    const bool iv = inc && T <= n / 4;
+    if (M > rv.mmax) {
+        fix_gather_all(n, vals, f);
+        return;
+    }
+    const uint32_t T = M ? rv.scratch[3] : 0u;
+    const bool iv = T <= n / 4;
     const uint32_t total = iv ? T : n;
     // a block with neither positions nor a moved entry (cell shifts) to take
-    if (blockIdx.x * kReorderThreads >= total && !(inc && blockIdx.x < M)) return;
-    if (inc) load_fix_lists(rv, M, iv, s_pos, s_q, s_ivlo, s_ivpre);
-    for (uint32_t t = blockIdx.x * kReorderThreads + threadIdx.x; t < total; t += gridDim.x * kReorderThreads) {
-        const uint32_t k = visit_position(t, iv, M, s_ivlo, s_ivpre);
-        if (k >= n) continue;
-        uint32_t src, key;
-        if (inc) sorted_entry<false>(k, M, s_pos, s_q, rv, n, src, key);
-        else src = vals[k];
-        if (src != k && src < n) {
-            t_pos[k] = s_pos4[src];
-            t_vel[k] = s_vel[src];
-            t_omg[k] = s_omg[src];
-            if (lv.cnt) {
-                const uint32_t c = lv.cnt[src];
-                lv.cnt_t[k] = c;
-                lv.ref_t[k] = lv.ref[src];
-                for (uint32_t q = 0; q < min(c, kVlCap); ++q) lv.nbr_t[(size_t)q * n + k] = lv.nbr[(size_t)q * n + src];
-            }
-        }
-    }
-    if (!inc) return;
+    if (blockIdx.x * kReorderThreads >= total && blockIdx.x >= M) return;
+    const MovedLists ml = load_fix_lists(rv, M, iv, s);
+    fix_gather_moved(blockIdx.x * kReorderThreads + threadIdx.x, n, total, iv, ml, f);
     for (uint32_t r = blockIdx.x; r < M; r += gridDim.x) {  // one moved entry per block
         const unsigned long long c = rv.list[r];
         const uint32_t b = min((uint32_t)(c >> 32), ncells), slot = (uint32_t)c;
-        const uint32_t a = slot < n ? min(keys_prev[slot], ncells) : b;
-        const uint32_t lo = min(a, b) + 1, hi = max(a, b);  // cells [lo, hi]
-        const uint32_t d = b > a ? 0xffffffffu : 1u;          // -1 or +1
-        for (uint32_t cc = lo + threadIdx.x; cc <= hi; cc += kReorderThreads) atomicAdd(&cell_start[cc], d);
+        shift_cells(slot < n ? min(f.keys_prev[slot], ncells) : b, b, cell_start);
     }
 }
 
 __global__ void __launch_bounds__(kReorderThreads)
 dem_fix_place_kernel(uint32_t n, uint32_t ncells, const uint32_t* __restrict__ keys,
-                     const uint32_t* __restrict__ vals, const float4* __restrict__ t_pos,
-                     const float4* __restrict__ t_vel, const float4* __restrict__ t_omg, float4* __restrict__ s_pos4,
-                     float4* __restrict__ s_vel, float4* __restrict__ s_omg, uint32_t* __restrict__ cell_start,
-                     uint32_t* __restrict__ slot_of, uint32_t* __restrict__ keys_prev, ResortView rv,
-                     bool slot_all, ListView lv) {
+                     const uint32_t* __restrict__ vals, FixState f, uint32_t* __restrict__ cell_start,
+                     ResortView rv) {
+    __shared__ FixLists s;
     __shared__ uint32_t s_keys[kReorderThreads + 1];
-    __shared__ uint32_t s_pos[kResortMaxCap], s_q[kResortMaxCap], s_ivlo[kResortMaxCap], s_ivpre[kResortMaxCap];
     const uint32_t M = rv.scratch[1];
-    const bool inc = M <= rv.mmax;
-    const uint32_t T = inc ? (M ? rv.scratch[3] : 0u) : n;
-    const bool iv = inc && T <= n / 4;
-    // the radix order: chunks of kReorderThreads consecutive positions per
-    // block iteration, so that each chunk rebuilds its part of the cell table
-    const uint32_t total = inc ? (iv ? T : n) : (n + kReorderThreads - 1) / kReorderThreads * kReorderThreads;
-    if (blockIdx.x * kReorderThreads >= total) return;  // no positions for this block
-    if (inc) load_fix_lists(rv, M, iv, s_pos, s_q, s_ivlo, s_ivpre);
-    for (uint32_t t0 = blockIdx.x * kReorderThreads; t0 < total; t0 += gridDim.x * kReorderThreads) {
-        const uint32_t t = t0 + threadIdx.x;
-        const uint32_t k = t < total ? visit_position(t, iv, M, s_ivlo, s_ivpre) : n;
-        if (k < n) {
-            uint32_t src, key = 0;
-            bool write = true;
-            if (inc) {
-                // a position that keeps its unmoved entry keeps its key too:
-                // nothing to write there
-                const bool moved = sorted_entry<false>(k, M, s_pos, s_q, rv, n, src, key);
-                if (src == k && !moved) write = false;
-                else key = moved ? (uint32_t)(rv.list[lower_idx(s_pos, M, k)] >> 32)
-                                 : (src < n ? rv.keys_new[src] : 0u);
-            } else {
-                src = vals[k];
-                key = keys[k];
-            }
-            if (write) {
-                if (src != k && src < n) {
-                    s_pos4[k] = t_pos[k];
-                    s_vel[k] = t_vel[k];
-                    const float4 o = t_omg[k];
-                    s_omg[k] = o;
-                    const uint32_t idb = __float_as_uint(o.w);
-                    if (slot_of && (slot_all || (idb & kClumpFlag)) && (idb & kIdMask) < n)
-                        slot_of[idb & kIdMask] = k;
-                    if (lv.cnt) {
-                        const uint32_t c = lv.cnt_t[k];
-                        lv.cnt[k] = c;
-                        lv.ref[k] = lv.ref_t[k];
-                        for (uint32_t q = 0; q < min(c, kVlCap); ++q)
-                            lv.nbr[(size_t)q * n + k] = lv.nbr_t[(size_t)q * n + k];
-                    }
-                }
-                keys_prev[k] = key;
-            }
-            if (!inc) s_keys[threadIdx.x + 1] = key;
-        }
-        if (!inc) {  // uniform: the radix order rebuilds the cell table chunk by chunk
-            const uint32_t b0 = t0, b1 = min(t0 + kReorderThreads, n);
-            if (threadIdx.x == 0) s_keys[0] = b0 == 0 ? 0u : keys[b0 - 1];
-            __syncthreads();
-            block_cell_starts(s_keys, b0, b1, n, ncells, cell_start);
-            __syncthreads();
-        }
+    if (M > rv.mmax) {
+        fix_place_all(n, ncells, keys, vals, f, cell_start, s_keys);
+        return;
     }
+    const uint32_t T = M ? rv.scratch[3] : 0u;
+    const bool iv = T <= n / 4;
+    const uint32_t total = iv ? T : n;
+    if (blockIdx.x * kReorderThreads >= total) return;  // no positions for this block
+    const MovedLists ml = load_fix_lists(rv, M, iv, s);
+    fix_place_moved(blockIdx.x * kReorderThreads + threadIdx.x, n, total, iv, ml, f);
 }
 
 __global__ void dem_pairs_kernel(DemParams p, uint32_t n, const float4* __restrict__ pos,
@@ -1661,37 +1460,8 @@ __global__ void dem_energy_kernel(uint32_t n, const float4* __restrict__ pos, co
     }
 }
 
-// The mesh pose of the next step: q <- normalize(dq (x) q) (Hamilton
-// product), then the rotation matrix of q (the expression of the rigid
-// bodies).
 __global__ void mesh_advance_kernel(float* __restrict__ S, int advance) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    float qs = S[16], qx = S[17], qy = S[18], qz = S[19];
-    if (advance) {
-        const float ds = S[20], dx = S[21], dy = S[22], dz = S[23];
-        const float ns = ds * qs - ((dx * qx + dy * qy) + dz * qz);
-        const float nx = (ds * qx + qs * dx) + (dy * qz - dz * qy);
-        const float ny = (ds * qy + qs * dy) + (dz * qx - dx * qz);
-        const float nz = (ds * qz + qs * dz) + (dx * qy - dy * qx);
-        const float nrm = sqrtf((ns * ns + nx * nx) + (ny * ny + nz * nz));
-        qs = ns / nrm;
-        qx = nx / nrm;
-        qy = ny / nrm;
-        qz = nz / nrm;
-        S[16] = qs;
-        S[17] = qx;
-        S[18] = qy;
-        S[19] = qz;
-    }
-    S[0] = 1.0f - 2.0f * (qy * qy + qz * qz);
-    S[1] = 2.0f * (qx * qy - qs * qz);
-    S[2] = 2.0f * (qx * qz + qs * qy);
-    S[3] = 2.0f * (qx * qy + qs * qz);
-    S[4] = 1.0f - 2.0f * (qx * qx + qz * qz);
-    S[5] = 2.0f * (qy * qz - qs * qx);
-    S[6] = 2.0f * (qx * qz - qs * qy);
-    S[7] = 2.0f * (qy * qz + qs * qx);
-    S[8] = 1.0f - 2.0f * (qx * qx + qy * qy);
+    if (threadIdx.x == 0 && blockIdx.x == 0) mesh_pose(S, advance != 0);
 }
 
 static inline unsigned grid_for(uint32_t n, unsigned threads) { return (n + threads - 1) / threads; }
@@ -1973,6 +1743,14 @@ static unsigned fix_grid(uint32_t n) {
     return g < cap ? g : cap;
 }
 
+// The step's in-place reorder: the next state stays in the *_n buffers, the
+// step's input state is free.
+static FixState fix_state(const DemBuffers& b) {
+    return FixState{b.pos_n, b.vel_n, b.omg_n, b.pos, b.vel, b.omg, b.keys_prev, b.keys, b.slot_of, slot_all_of(b),
+                    dem_step_skin(b) ? ListView{b.vl_cnt, b.vl_ref, b.vl_nbr, b.vl_cnt_t, b.vl_ref_t, b.vl_nbr_t}
+                                     : ListView{}};
+}
+
 // One whole step.  With the incremental re-sort (dem_step_swaps): contact +
 // integrate (which lists the slots whose key changed), the re-sort's plan,
 // the radix fallback (histogram + passes, returning at once when the plan
@@ -2008,17 +1786,24 @@ cudaError_t dem_step_async(const DemParams& p, DemBuffers& b, bool record, cudaS
     // sorted in place: the next state stays in the *_n buffers
     const uint32_t* k = b.sorted_in_tmp ? b.keys_tmp : b.keys;
     const uint32_t* v = b.sorted_in_tmp ? b.vals_tmp : b.vals;
-    const ResortView rv{b.keys, b.rs_pos, b.rs_q, b.rs_list, b.rs_scratch, b.rs_max, b.rs_iv_lo, b.rs_iv_pre};
-    const ListView lv = skin ? ListView{b.vl_cnt, b.vl_ref, b.vl_nbr, b.vl_cnt_t, b.vl_ref_t, b.vl_nbr_t}
-                             : ListView{};
+    const ResortView rv{b.rs_pos, b.rs_q, b.rs_list, b.rs_scratch, b.rs_max, b.rs_iv_lo, b.rs_iv_pre};
+    const FixState f = fix_state(b);
     const unsigned grid = fix_grid(b.n);
-    dem_fix_gather_kernel<<<grid, kReorderThreads, 0, st>>>(b.n, b.ncells, v, b.pos_n, b.vel_n, b.omg_n, b.pos,
-                                                            b.vel, b.omg, b.cell_start, b.keys_prev, rv, lv);
-    dem_fix_place_kernel<<<grid, kReorderThreads, 0, st>>>(b.n, b.ncells, k, v, b.pos, b.vel, b.omg, b.pos_n,
-                                                           b.vel_n, b.omg_n, b.cell_start, b.slot_of, b.keys_prev,
-                                                           rv, slot_all_of(b), lv);
+    dem_fix_gather_kernel<<<grid, kReorderThreads, 0, st>>>(b.n, b.ncells, v, f, b.cell_start, rv);
+    dem_fix_place_kernel<<<grid, kReorderThreads, 0, st>>>(b.n, b.ncells, k, v, f, b.cell_start, rv);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     return mesh_advance_async(b.mesh, 1, st);
+}
+
+cudaError_t dem_step_fused_async(const DemParams& p, DemBuffers& b, bool record, cudaStream_t st) {
+    if (b.n == 0) return cudaSuccess;
+    const SortPlan plan = sort_plan(dem_key_bits(b.ncells));
+    const bool skin = dem_step_skin(b);
+    const MoveSink ms{b.keys_prev, b.rs_list, b.rs_scratch, b.rs_max};
+    cudaError_t e = launch_contact(p, b, record, plan, nullptr, st, skin, ms);
+    if (e != cudaSuccess) return e;
+    return resort_step_async(b, plan, g_fix_blocks >= 8 ? 2 : 1, skin ? b.vl_flags : nullptr, fix_state(b).lv,
+                             slot_all_of(b), st);
 }
 
 bool dem_step_skin(const DemBuffers& b) {

@@ -93,13 +93,18 @@ sd_status dev_alloc(sd_engine* h, T** p, size_t count) {
     return SD_OK;
 }
 
+void drop_graphs(sd_engine* h) {
+    for (auto& kind : h->graphs)
+        for (cudaGraphExec_t& g : kind) {
+            if (g) cudaGraphExecDestroy(g);
+            g = nullptr;
+        }
+    h->graph_valid = false;
+}
+
 void release_device(sd_engine* h) {
     hull_release(h);
-    if (h->graph) cudaGraphExecDestroy(h->graph);
-    if (h->graph_alt) cudaGraphExecDestroy(h->graph_alt);
-    h->graph = nullptr;
-    h->graph_alt = nullptr;
-    h->graph_valid = false;
+    drop_graphs(h);
     for (void* p : h->allocations) cudaFree(p);
     h->allocations.clear();
     h->B = sd::DemBuffers{};
@@ -596,17 +601,11 @@ static sd_status force_list_build(sd_engine* h) {
     return SD_OK;
 }
 
+// Prepares the step graphs for time step dt under the current knobs; each is
+// captured when a step first needs it (step_graph).
 sd_status build_graph(sd_engine* h, float dt) {
-    if (h->graph) {
-        cudaGraphExecDestroy(h->graph);
-        h->graph = nullptr;
-    }
-    if (h->graph_alt) {
-        cudaGraphExecDestroy(h->graph_alt);
-        h->graph_alt = nullptr;
-    }
+    drop_graphs(h);
     h->P.dt = dt;
-    bool record = (h->cfg.flags & SD_FLAG_RECORD) != 0;
     if (h->B.mesh.ntri && h->mesh.dt != dt) {
         // the rotation of one step, in double: angle omega dt about the axis
         const double half = 0.5 * (double)h->mesh.omega * (double)dt;
@@ -623,33 +622,48 @@ sd_status build_graph(sd_engine* h, float dt) {
     }
     h->graph_swaps = sd::dem_step_swaps(h->B);
     h->graph_parity = 0;
-    // with swaps: the graph on the current buffers, then the one on the
-    // swapped buffers (the state after one step); the second swap restores B
-    for (int par = 0; par < (h->graph_swaps ? 2 : 1); ++par) {
-        cudaGraph_t g = nullptr;
-        SD_CUDA(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-        cudaError_t e2 = sd::dem_step_async(h->P, h->B, record, h->stream);
-        cudaError_t e3 = cudaStreamEndCapture(h->stream, &g);
-        if (h->graph_swaps) swap_state(h->B);
-        if (e2 != cudaSuccess) {
-            if (g) cudaGraphDestroy(g);
-            if (h->graph_swaps && par == 0) swap_state(h->B);
-            return cuda_fail(h, e2, "capturing the step");
-        }
-        if (e3 != cudaSuccess) {
-            if (h->graph_swaps && par == 0) swap_state(h->B);
-            return cuda_fail(h, e3, "cudaStreamEndCapture");
-        }
-        cudaError_t e4 = cudaGraphInstantiate(par == 0 ? &h->graph : &h->graph_alt, g, 0);
-        h->graph_kernels = graph_kernel_nodes(g);
-        cudaGraphDestroy(g);
-        if (e4 != cudaSuccess) {
-            if (h->graph_swaps && par == 0) swap_state(h->B);
-            return cuda_fail(h, e4, "cudaGraphInstantiate");
-        }
-    }
     h->graph_dt = dt;
     h->graph_valid = true;
+    return SD_OK;
+}
+
+// Steps that one launch of a graph of the kind runs.
+static int32_t steps_of(StepGraph kind) { return kind == kRunGraph ? kRunSteps : 1; }
+
+// The graph of the kind on the current buffers, captured at its first use.
+// A step that leaves the next state in the *_n buffers swaps them, so every
+// kind has one graph per assignment (graph_parity); a run has an even number
+// of steps and leaves the assignment as it was.
+sd_status step_graph(sd_engine* h, StepGraph kind, cudaGraphExec_t* out) {
+    cudaGraphExec_t& exec = h->graphs[kind][h->graph_parity];
+    if (!exec) {
+        const bool record = (h->cfg.flags & SD_FLAG_RECORD) != 0;
+        cudaGraph_t g = nullptr;
+        SD_CUDA(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
+        cudaError_t e = cudaSuccess;
+        int32_t done = 0;
+        for (; done < steps_of(kind) && e == cudaSuccess; ++done) {
+            e = kind == kStepGraph ? sd::dem_step_async(h->P, h->B, record, h->stream)
+                                   : sd::dem_step_fused_async(h->P, h->B, record, h->stream);
+            if (h->graph_swaps) swap_state(h->B);
+        }
+        if (h->graph_swaps && (done & 1)) swap_state(h->B);  // the buffers as they were
+        const cudaError_t e2 = cudaStreamEndCapture(h->stream, &g);
+        if (e != cudaSuccess) {
+            if (g) cudaGraphDestroy(g);
+            return cuda_fail(h, e, "capturing the step");
+        }
+        if (e2 != cudaSuccess) return cuda_fail(h, e2, "cudaStreamEndCapture");
+        const cudaError_t e3 = cudaGraphInstantiate(&exec, g, 0);
+        h->graph_nodes[kind] = graph_kernel_nodes(g) / (uint32_t)steps_of(kind);
+        cudaGraphDestroy(g);
+        if (e3 != cudaSuccess) {
+            exec = nullptr;
+            return cuda_fail(h, e3, "cudaGraphInstantiate");
+        }
+    }
+    h->graph_kernels = h->graph_nodes[kind];
+    *out = exec;
     return SD_OK;
 }
 
@@ -1366,15 +1380,23 @@ sd_status sd_engine_step(sd_engine* h, float dt, int32_t n_steps) {
         // the first step of a list graph builds them again
         if ((s = force_list_build(h))) return s;
     }
-    for (int32_t i = 0; i < n_steps; ++i) {
-        SD_CUDA(h, cudaGraphLaunch(h->graph_parity ? h->graph_alt : h->graph, h->stream));
-        if (h->graph_swaps) {  // the next state was sorted in place in the *_n buffers
+    // A run of steps follows each contact stage with one kernel, several
+    // steps to a graph; a call of a few steps keeps the graph of separate
+    // kernels (whose nodes step_kernels counts and a profiler can tell apart).
+    const bool run = h->graph_swaps && n_steps >= kRunMin;
+    for (int32_t i = 0; i < n_steps;) {
+        const StepGraph kind = !run ? kStepGraph : (n_steps - i >= kRunSteps ? kRunGraph : kFusedGraph);
+        cudaGraphExec_t g = nullptr;
+        if ((s = step_graph(h, kind, &g))) return s;
+        SD_CUDA(h, cudaGraphLaunch(g, h->stream));
+        if (h->graph_swaps && kind != kRunGraph) {  // the next state was sorted in place in the *_n buffers
             swap_state(h->B);
             h->graph_parity ^= 1;
         }
+        i += steps_of(kind);
+        h->steps += (uint64_t)steps_of(kind);
     }
     if (n_steps > 0 && !h->hull_mode()) h->keys_current = true;  // every step ends with a sort + reorder
-    h->steps += (uint64_t)n_steps;
     return SD_OK;
 }
 

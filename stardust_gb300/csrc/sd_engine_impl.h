@@ -47,6 +47,12 @@ struct HullScene {
     uint32_t graph_kernels = 0;                   // kernel nodes of one step's graph
 };
 
+// The step as a graph of separate kernels; the step with one kernel after its
+// contact stage; kRunSteps (even) of those.
+enum StepGraph { kStepGraph, kFusedGraph, kRunGraph, kStepGraphs };
+constexpr int32_t kRunSteps = 8;
+constexpr int32_t kRunMin = 4;  // steps of a call from which it runs fused steps
+
 struct sd_engine {
     sd_config cfg{};
     std::string err;
@@ -89,16 +95,16 @@ struct sd_engine {
     std::vector<void*> allocations;
     double* d_energy = nullptr;
     float4* d_tmp = nullptr;
-    cudaGraphExec_t graph = nullptr;
-    // when the step leaves the next state in the *_n buffers (graph_swaps),
-    // a second graph captured on the swapped buffers alternates with the
-    // first; graph_parity names the one whose input is the current state
-    cudaGraphExec_t graph_alt = nullptr;
+    // step graphs by kind.  When the step leaves the next state in the *_n
+    // buffers (graph_swaps), each kind has a graph per assignment of the
+    // buffers; graph_parity names the one whose input is the current state
+    cudaGraphExec_t graphs[kStepGraphs][2] = {};
+    uint32_t graph_nodes[kStepGraphs] = {};  // kernel nodes per step
     bool graph_swaps = false;
     int graph_parity = 0;
     float graph_dt = 0.0f;
     bool graph_valid = false;
-    uint32_t graph_kernels = 0;  // kernel nodes of the step graph
+    uint32_t graph_kernels = 0;  // kernel nodes per step of the graph launched last
     uint64_t steps = 0;
     bool need_resort = false;
     // the sorted key arrays hold the cell key of every slot's sphere (true

@@ -299,7 +299,8 @@ struct DemBuffers {
     uint32_t* rs_q;                 // per moved slot (ascending): slot - rank
     uint32_t* rs_iv_lo;             // per moved entry: first position its move shifts
     uint32_t* rs_iv_pre;            // exclusive prefix sums of those intervals' lengths (M + 1 entries)
-    uint32_t* rs_scratch;           // [0] moved count, [1] M of the step, [3] total interval length
+    uint32_t* rs_scratch;           // [0] moved count, [1] M of the step, [3] total interval length,
+                                    // [4] and [5] the one-kernel re-sort's grid barrier
     uint32_t rs_max;                // most moved entries re-sorted incrementally (power of two, or 0)
     // contact partner lists (scenes without clumps): per slot a count, zero
     // between steps, and kNbrCap partner slots; null when not allocated
@@ -332,6 +333,21 @@ constexpr uint32_t kResortMaxCap = 1024;  // largest rs_max (two sorted lists in
 uint64_t resort_scratch_words(uint32_t n);
 // vl_flags (may be null): the skin lists' flags, [0] <- [1], [1] <- 0
 cudaError_t resort_plan_async(const DemBuffers& b, cudaStream_t st, uint32_t* vl_flags = nullptr);
+// The contact lists the in-place reorder moves with the state (all null when
+// the step uses none): per slot count, build position and kVlCap rows of
+// neighbour ids, and same-sized buffers for the gathered entries.
+struct ListView {
+    uint32_t* cnt;
+    float4* ref;
+    uint32_t* nbr;
+    uint32_t* cnt_t;
+    float4* ref_t;
+    uint32_t* nbr_t;
+};
+// the plan, the radix fallback, the in-place reorder and the mesh's pose as
+// one cooperative launch of at most per_sm blocks per SM
+cudaError_t resort_step_async(const DemBuffers& b, const SortPlan& plan, int per_sm, uint32_t* vl_flags,
+                              const ListView& lv, bool slot_all, cudaStream_t st);
 void dem_set_resort_max(uint32_t m);
 uint32_t dem_resort_max();
 void dem_set_pair_lists(int on);
@@ -359,6 +375,9 @@ cudaError_t dem_sort_reorder_async(const DemParams& p, DemBuffers& b, cudaStream
 cudaError_t dem_contact_integrate_async(const DemParams& p, DemBuffers& b, bool record,
                                         cudaStream_t st);
 cudaError_t dem_step_async(const DemParams& p, DemBuffers& b, bool record, cudaStream_t st);
+// the same step with all that follows the contact stage in one kernel
+// (dem_step_swaps must hold; the caller swaps as after dem_step_async)
+cudaError_t dem_step_fused_async(const DemParams& p, DemBuffers& b, bool record, cudaStream_t st);
 void dem_set_contact_mode(int mode);
 int dem_contact_mode();
 cudaError_t dem_pairs_async(const DemParams& p, DemBuffers& b, cudaStream_t st);

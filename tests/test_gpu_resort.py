@@ -120,3 +120,43 @@ def test_step_kernel_count(sdlib):
     finally:
         _abi.tune_set("resort_max", old)
     assert counts[0] >= 4 and counts[1024] == counts[0] + 3
+
+
+@pytest.mark.parametrize("n,resort_max,moved,items", [(30_000, 1024, 2, 16), (30_000, 1024, 200, 16),
+                                                      (30_000, 1024, 700, 16), (30_000, 512, 9000, 16),
+                                                      (30_000, 512, 9000, 8), (300, 1024, 20, 16), (300, 8, 200, 16),
+                                                      (257, 1024, 100, 8), (150_000, 1024, 300, 16)])
+def test_runs_of_steps_bit_exact(sdlib, orc, n, resort_max, moved, items):
+    """Calls of several steps (one kernel after each contact stage, several
+    steps to a graph): 0 to 9,000 changed keys per step, on both sides of the
+    re-sort's limit, calls of 3, 8, 5, 13 and 1 steps one after the other."""
+    from stardust_gb300 import _abi
+    knobs = {"resort_max": resort_max, "sort_items": items}
+    old = {k: _abi.tune_get(k) for k in knobs}
+    try:
+        for k, v in knobs.items():
+            _abi.tune_set(k, v)
+        pos, vel, cfg, dt = moving_scene(n, moved, seed=11)
+        eng = sdlib.DEMEngine(cfg)
+        eng.add_spheres(pos, vel)
+        eng.prepare()
+        kernels = []
+        for steps in (3, 8, 5, 13, 1):
+            eng.step(dt, steps)
+            kernels.append(eng.stats()["step_kernels"])
+        eng.sync()
+        assert kernels[1] < kernels[0] and kernels[1] == kernels[2] == kernels[3] and kernels[4] == kernels[0]
+        assert eng.stats()["device_errors"] == 0
+        assert eng.stats()["steps"] == 30
+        p = orc.params_checked(cfg, pos[:, 3], dt, eng.params())
+        op, ov, ow = orc.run(p, pos, vel, orc.with_ids(np.zeros_like(pos), np.arange(n)), 30)
+        assert np.array_equal(bits(eng.positions()), bits(orc.unsort(op, ow)))
+        assert np.array_equal(bits(eng.velocities()), bits(orc.unsort(ov, ow)))
+        assert np.array_equal(bits(eng.omegas())[:, :3], bits(orc.unsort(ow, ow))[:, :3])
+        sp, sv, sw, _, cs = orc.prepare(p, eng.positions(), eng.velocities(),
+                                        orc.with_ids(eng.omegas(), np.arange(n)))
+        assert np.array_equal(eng.pairs(), orc.contact_pairs(p, sp, sw, cs))
+        eng.close()
+    finally:
+        for k, v in old.items():
+            _abi.tune_set(k, v)
