@@ -412,6 +412,8 @@ __device__ __forceinline__ void mesh_contacts(const DemParams& p, const MeshView
     }
 }
 
+constexpr uint32_t kListUnroll = 2;  // list entries whose loads are in flight together
+
 // Listed neighbour k of slot i: its slot this step and position, and
 // whether it is in contact (|x_i - x_j| < r_i + r_j, centres apart).
 template <class SRC>
@@ -507,46 +509,76 @@ __device__ __forceinline__ uint32_t particle_step(const DemParams& p, uint32_t n
             scan = false;
         } else if (sk_cnt <= kVlCap) {
             // the listed neighbours in contact, applied by ascending slot (the
-            // scan's order).  A first pass finds them and whether list order
-            // already ascends -- the usual case: the list was written in scan
-            // order and few slots cross between builds; otherwise each is
-            // picked as the smallest slot above the last one applied.
+            // scan's order).  List order nearly always ascends (it was written
+            // in scan order and few slots cross between builds), so contacts
+            // are applied as they are found; when a slot turns out to be below
+            // one already applied, all start again, each picked as the
+            // smallest slot above the last one applied.  kListUnroll entries
+            // at a time: their chains of dependent loads (id, slot, position)
+            // overlap.
             const uint32_t c = sk_cnt;
-            uint32_t m = 0, last = 0;
+            uint32_t next = 0, found = 0;  // slots below next are applied
             bool asc = true;
-            for (uint32_t k = 0; k < c; ++k) {
-                uint32_t s;
-                float4 pa;
-                if (listed_hit(sk, n, i, k, src, pi, ri, s, pa)) {
-                    if (m && s < last) asc = false;
-                    last = s;
-                    ++m;
+            for (uint32_t k0 = 0; k0 < c && asc; k0 += kListUnroll) {
+                uint32_t sl[kListUnroll];
+                float4 pa[kListUnroll];
+#pragma unroll
+                for (uint32_t u = 0; u < kListUnroll; ++u)
+                    sl[u] = k0 + u < c ? sk->nbr[(size_t)(k0 + u) * n + i] : 0xffffffffu;
+#pragma unroll
+                for (uint32_t u = 0; u < kListUnroll; ++u) sl[u] = sl[u] < n ? sk->slot_of[sl[u]] : 0xffffffffu;
+#pragma unroll
+                for (uint32_t u = 0; u < kListUnroll; ++u) pa[u] = src.load(sl[u] < n ? sl[u] : i);
+                uint32_t hits = 0;
+#pragma unroll
+                for (uint32_t u = 0; u < kListUnroll; ++u) {  // (the sphere itself has distance 0)
+                    const float da = dist2(pi.x - pa[u].x, pi.y - pa[u].y, pi.z - pa[u].z);
+                    const float ra = ri + pa[u].w;
+                    if (da < ra * ra && da != 0.0f) hits |= 1u << u;
+                }
+                while (hits) {
+                    const uint32_t h = (uint32_t)__ffs(hits) - 1u;
+                    hits &= hits - 1u;
+                    uint32_t best = sl[0];
+                    float4 pb = pa[0];
+#pragma unroll
+                    for (uint32_t u = 1; u < kListUnroll; ++u)
+                        if (h == u) {
+                            best = sl[u];
+                            pb = pa[u];
+                        }
+                    if (best < next) {
+                        asc = false;
+                        break;
+                    }
+                    next = best + 1u;
+                    ++found;
+                    const float ax = pi.x - pb.x, ay = pi.y - pb.y, az = pi.z - pb.z;
+                    pair_contact(p, ax, ay, az, dist2(ax, ay, az), ri + pb.w, pb.w, ri, mi, vi, wi, vel, omg, best, f, t);
                 }
             }
-            uint32_t lo = 0, k0 = 0;  // slots below lo are applied; asc: entries below k0 too
-            for (uint32_t r = 0; r < m; ++r) {
-                uint32_t best = 0xffffffffu;
-                float4 pb = make_float4(0.f, 0.f, 0.f, 0.f);
-                for (uint32_t k = asc ? k0 : 0u; k < c; ++k) {
-                    uint32_t s;
-                    float4 pa;
-                    if (listed_hit(sk, n, i, k, src, pi, ri, s, pa) && s >= lo && s < best) {
-                        best = s;
-                        pb = pa;
-                        if (asc) {  // list order ascends: the next hit is the next to apply
-                            k0 = k + 1u;
-                            break;
+            if (!asc) {
+                f = t = make_float3(0.f, 0.f, 0.f);
+                found = 0;
+                for (uint32_t lo = 0;;) {
+                    uint32_t best = 0xffffffffu;
+                    float4 pb = make_float4(0.f, 0.f, 0.f, 0.f);
+                    for (uint32_t k = 0; k < c; ++k) {
+                        uint32_t s;
+                        float4 pa;
+                        if (listed_hit(sk, n, i, k, src, pi, ri, s, pa) && s >= lo && s < best) {
+                            best = s;
+                            pb = pa;
                         }
                     }
+                    if (best >= n) break;
+                    const float ax = pi.x - pb.x, ay = pi.y - pb.y, az = pi.z - pb.z;
+                    ++found;
+                    pair_contact(p, ax, ay, az, dist2(ax, ay, az), ri + pb.w, pb.w, ri, mi, vi, wi, vel, omg, best, f, t);
+                    lo = best + 1u;
                 }
-                if (best >= n) break;  // not reached: m hits were found above
-                const float ax = pi.x - pb.x, ay = pi.y - pb.y, az = pi.z - pb.z;
-                const float da = dist2(ax, ay, az);
-                const float ra = ri + pb.w;
-                ++contacts;
-                pair_contact(p, ax, ay, az, da, ra, pb.w, ri, mi, vi, wi, vel, omg, best, f, t);
-                lo = best + 1u;
             }
+            contacts += found;
             scan = false;
         }
         // else: an overflowed list -- the scan below
@@ -881,13 +913,18 @@ dem_contact_integrate_kernel(DemParams p, uint32_t n, const float4* __restrict__
     if (RECORD) count_contacts(status, contacts);
 }
 
-// The single-scene free-sphere step over contact lists (knob skin_um): one
-// thread per slot, the listed neighbours between builds, the widened scan
-// at a build.  Its own kernel so that the registers are capped for the
-// listed steps' occupancy (they are bound by load latency): MINB resident
-// blocks of 256 per SM (4: 64 registers; 5: 48, with spills in the build
-// scan; 6: 40; 8: 32; knob "listed_blocks", default 5).  It never builds radix histograms (the lists
-// run only with the incremental re-sort).
+// The step over contact lists (knob skin_um): one thread per slot, the listed
+// neighbours between builds, the widened scan at a build.  Its own kernel so
+// that the registers are capped for the listed steps' occupancy: MINB
+// resident blocks of 256 per SM (4: 64 registers; 5: 48, with spills; 6: 40;
+// 8: 32; knob "listed_blocks", default 5).  It never builds radix histograms
+// (the lists run only with the incremental re-sort).
+// Bound by load latency where spheres have few neighbours (1,048,576 falling:
+// 31 us, 4.1 TB/s of its 124 B a sphere), by the contacts' instructions in a
+// bed (199,999 spheres, 4.5 contacts each: 54 -> 33 us a step when the listed
+// neighbours were taken two at a time in one pass instead of one at a time in
+// two).  Four or eight at a time spill (falling 2648 and 3410 us for 40 steps
+// against 2499).
 template <bool RECORD, int MINB, bool BATCHED, bool CLUMPS = false, bool MESH = false>
 __global__ void __launch_bounds__(256, MINB)
 dem_contact_listed_kernel(DemParams p, uint32_t n, const float4* __restrict__ pos, const float4* __restrict__ vel,
@@ -1591,9 +1628,8 @@ int dem_contact_block() { return g_contact_block; }
 void dem_set_fix_blocks(int b) { g_fix_blocks = b; }
 int dem_fix_blocks() { return g_fix_blocks; }
 
-// resident blocks per SM the listed kernel is compiled for: 4 or 5.  Five
-// (48 registers, spills only in the build scan) measured 0.0632 ms per
-// step at 1,048,576 spheres against 0.0668 ms with four (64 registers)
+// resident 256-thread blocks per SM the listed kernel is compiled for (knob
+// "listed_blocks"; kListedSmall for what the default does)
 static int g_listed_blocks = 5;
 void dem_set_listed_blocks(int b) { g_listed_blocks = (b == 5 || b == 6 || b == 8) ? b : 4; }
 int dem_listed_blocks() { return g_listed_blocks; }
@@ -1601,6 +1637,19 @@ int dem_pair_lists() { return g_pair_lists; }
 
 void dem_set_contact_mode(int mode) { g_contact_mode = mode == 0 ? 0 : 1; }
 int dem_contact_mode() { return g_contact_mode; }
+
+// Threads per block of the listed kernel, whatever the knob "contact_block"
+// (no thread of it needs another warp): small blocks free their place early
+// and leave no thin last wave.  Against blocks of 256: 40 steps of 1,048,576
+// falling spheres 2519 -> 2448 us, 20 steps of the drum 966 -> 901.
+constexpr unsigned kListedThreads = 64;
+// Up to this many spheres the default register budget is that of four
+// 256-thread blocks per SM instead of five: their state (124 B a sphere)
+// stays in L2, so fewer warps cover its latency, and the contacts no longer
+// spill.  40 steps, four / five: 600,000 falling spheres 1563 / 1595 us, 700,000
+// in a bed 4033 / 4140, 300,000 in a bed 2020 / 2283; 1,048,576 falling 2554 /
+// 2472.  Scenes with clumps or a mesh always take four (the drum 874 / 907).
+constexpr uint32_t kListedSmall = 800000;
 
 template <bool RECORD>
 static void launch_contact_t(const DemParams& p, DemBuffers& b, uint32_t spec, uint32_t* ghist, cudaStream_t st,
@@ -1615,44 +1664,46 @@ static void launch_contact_t(const DemParams& p, DemBuffers& b, uint32_t spec, u
     // the re-sort step needs no slot identity (its radix fallback writes it)
     uint32_t* const vals = ms.list ? nullptr : b.vals;
     if (skin) {  // one scene or a batch, contact lists (clumps and meshes: one scene)
+        const int blocks = g_listed_blocks == 5 && b.n <= kListedSmall ? 4 : g_listed_blocks;
+        const unsigned lgrid = grid_for(b.n, kListedThreads);
         const float thr = 0.45f * b.vl_skin;
         const SkinLists sk{b.vl_cnt, b.vl_nbr, b.vl_ref, b.vl_flags, b.vl_flags + 1, b.slot_of, b.vl_skin, thr * thr};
         const Batch bt{b.scenes, b.scene_first, b.nscenes};
         if (b.nscenes > 1) {
-            if (g_listed_blocks == 5)
-                dem_contact_listed_kernel<RECORD, 5, true><<<grid, cb, 0, st>>>(
+            if (blocks == 5)
+                dem_contact_listed_kernel<RECORD, 5, true><<<lgrid, kListedThreads, 0, st>>>(
                     p, b.n, b.pos, b.vel, b.omg, b.cell_start, b.pos_n, b.vel_n, b.omg_n, b.keys, vals, f, t,
                     b.dev_status, sk, ms, bt);
             else
-                dem_contact_listed_kernel<RECORD, 4, true><<<grid, cb, 0, st>>>(
+                dem_contact_listed_kernel<RECORD, 4, true><<<lgrid, kListedThreads, 0, st>>>(
                     p, b.n, b.pos, b.vel, b.omg, b.cell_start, b.pos_n, b.vel_n, b.omg_n, b.keys, vals, f, t,
                     b.dev_status, sk, ms, bt);
         } else if (b.nb && b.mesh.ntri) {
-            dem_contact_listed_kernel<RECORD, 5, false, true, true><<<grid, cb, 0, st>>>(
+            dem_contact_listed_kernel<RECORD, 4, false, true, true><<<lgrid, kListedThreads, 0, st>>>(
                 p, b.n, b.pos, b.vel, b.omg, b.cell_start, b.pos_n, b.vel_n, b.omg_n, b.keys, vals, f, t,
                 b.dev_status, sk, ms, Batch{}, cc, b.mesh);
         } else if (b.nb) {
-            dem_contact_listed_kernel<RECORD, 5, false, true, false><<<grid, cb, 0, st>>>(
+            dem_contact_listed_kernel<RECORD, 4, false, true, false><<<lgrid, kListedThreads, 0, st>>>(
                 p, b.n, b.pos, b.vel, b.omg, b.cell_start, b.pos_n, b.vel_n, b.omg_n, b.keys, vals, f, t,
                 b.dev_status, sk, ms, Batch{}, cc);
         } else if (b.mesh.ntri) {
-            dem_contact_listed_kernel<RECORD, 5, false, false, true><<<grid, cb, 0, st>>>(
+            dem_contact_listed_kernel<RECORD, 4, false, false, true><<<lgrid, kListedThreads, 0, st>>>(
                 p, b.n, b.pos, b.vel, b.omg, b.cell_start, b.pos_n, b.vel_n, b.omg_n, b.keys, vals, f, t,
                 b.dev_status, sk, ms, Batch{}, ClumpCtx{}, b.mesh);
-        } else if (g_listed_blocks == 6) {
-            dem_contact_listed_kernel<RECORD, 6, false><<<grid, cb, 0, st>>>(
+        } else if (blocks == 6) {
+            dem_contact_listed_kernel<RECORD, 6, false><<<lgrid, kListedThreads, 0, st>>>(
                 p, b.n, b.pos, b.vel, b.omg, b.cell_start, b.pos_n, b.vel_n, b.omg_n, b.keys, vals, f, t,
                 b.dev_status, sk, ms, Batch{});
-        } else if (g_listed_blocks == 8) {
-            dem_contact_listed_kernel<RECORD, 8, false><<<grid, cb, 0, st>>>(
+        } else if (blocks == 8) {
+            dem_contact_listed_kernel<RECORD, 8, false><<<lgrid, kListedThreads, 0, st>>>(
                 p, b.n, b.pos, b.vel, b.omg, b.cell_start, b.pos_n, b.vel_n, b.omg_n, b.keys, vals, f, t,
                 b.dev_status, sk, ms, Batch{});
-        } else if (g_listed_blocks == 5) {
-            dem_contact_listed_kernel<RECORD, 5, false><<<grid, cb, 0, st>>>(
+        } else if (blocks == 5) {
+            dem_contact_listed_kernel<RECORD, 5, false><<<lgrid, kListedThreads, 0, st>>>(
                 p, b.n, b.pos, b.vel, b.omg, b.cell_start, b.pos_n, b.vel_n, b.omg_n, b.keys, vals, f, t,
                 b.dev_status, sk, ms, Batch{});
         } else {
-            dem_contact_listed_kernel<RECORD, 4, false><<<grid, cb, 0, st>>>(
+            dem_contact_listed_kernel<RECORD, 4, false><<<lgrid, kListedThreads, 0, st>>>(
                 p, b.n, b.pos, b.vel, b.omg, b.cell_start, b.pos_n, b.vel_n, b.omg_n, b.keys, vals, f, t,
                 b.dev_status, sk, ms, Batch{});
         }

@@ -156,3 +156,36 @@ def test_coincident_spheres_are_listed(sdlib, orc):
         eng.close()
     finally:
         _abi.tune_set("skin_um", old)
+
+
+@pytest.mark.parametrize("squeeze,skin", [(1.0, 300), (0.9, 300), (0.8, 800), (0.72, 1500), (0.62, 1500)])
+def test_listed_contacts_in_scan_order(sdlib, orc, squeeze, skin):
+    """Lists of 0 to more than kVlCap entries, odd and even counts, spheres
+    fast enough to change cells between builds (so that slots cross and a
+    list no longer ascends), in one call of several steps: bit-exact."""
+    from stardust_gb300 import _abi, scenes
+    old = _abi.tune_get("skin_um")
+    try:
+        _abi.tune_set("skin_um", skin)
+        n = 3001
+        pos, vel, cfg, dt, _ = scenes.settling_rsa(n, box=scenes.scaled_box(n), seed=5)
+        pos, vel = pos.copy(), vel.copy()
+        pos[:, :3] *= np.float32(squeeze)
+        rng = np.random.default_rng(8)
+        vel[:, :3] = rng.uniform(-3.0, 3.0, (n, 3))
+        eng = sdlib.DEMEngine(cfg)
+        eng.add_spheres(pos, vel)
+        eng.prepare()
+        steps = 21
+        eng.step(dt, steps)
+        eng.sync()
+        st = eng.stats()
+        assert st["device_errors"] == 0 and st["listed_steps"] > 0
+        p = orc.params_checked(cfg, pos[:, 3], dt, eng.params())
+        op, ov, ow = orc.run(p, pos, vel, orc.with_ids(np.zeros_like(pos), np.arange(n)), steps)
+        for got, want in ((eng.positions(), op), (eng.velocities(), ov)):
+            assert np.array_equal(got.view(np.uint32), orc.unsort(want, ow).view(np.uint32))
+        assert np.array_equal(eng.omegas().view(np.uint32)[:, :3], orc.unsort(ow, ow).view(np.uint32)[:, :3])
+        eng.close()
+    finally:
+        _abi.tune_set("skin_um", old)
