@@ -101,3 +101,23 @@ def test_candidate_pairs_overflow_counts_all(sdlib, orc):
     a, b = orc.ref_candidate_pairs(ko, vo, ocount)
     assert pairs[2] == len(a) > 100
     assert np.array_equal(pairs[0], a[:100]) and np.array_equal(pairs[1], b[:100])
+
+
+@pytest.mark.parametrize("n,cell,size,one_cell", [(227, 0.25, 0.0, False), (228, 0.25, 0.0, False), (256, 0.125, 0.12, False),
+                                                  (257, 0.125, 0.12, False), (2048, 1 / 32, 0.0, False),
+                                                  (2049, 1 / 32, 0.0, False), (700, 0.5, 0.01, True),
+                                                  (70_001, 1 / 32, 0.02, False)])
+def test_hash_tiles_and_runs(sdlib, orc, n, cell, size, one_cell):
+    """Entry counts around the pair kernel's tiles of 2,048 (size 0: one
+    entry per sphere), blocks of 256 spheres, every sphere in one run longer
+    than a block, more than 32 tiles behind the last."""
+    rng = np.random.default_rng(n)
+    pos = np.zeros((n, 4), np.float32)
+    pos[:, :3] = rng.uniform(0, 0.4 if one_cell else 1, (n, 3))
+    sizes = np.full(n, size, np.float32)
+    built, sorted_, pairs = gpu_pipeline(sdlib, pos, sizes, cell, cap=400_000 if one_cell else None)
+    oc, osp, ocount = orc.ref_hash_build(pos, sizes, cell)
+    assert built[2] == ocount and np.array_equal(built[0], oc) and np.array_equal(built[1], osp)
+    ko, vo = orc.radix_sort_pairs(oc, osp, 32)
+    a, b = orc.ref_candidate_pairs(ko, vo, ocount)
+    assert pairs[2] == len(a) and np.array_equal(pairs[0], a) and np.array_equal(pairs[1], b)
