@@ -14,11 +14,26 @@
 // shared memory as-is.
 //
 // Every GEMM is M = 128 rows (one row per thread of a 128-thread CTA, which
-// is also the TMEM lane), N in {16, 64}, K in {16, 64, 128}, issued by one
-// thread as K/16 tcgen05.mma instructions of kind::f16 and completed through
-// tcgen05.commit on an mbarrier.  Weight gradients are GEMMs over the samples
-// (K = the 128 rows of a tile) and accumulate in tensor memory across the
-// tiles a CTA processes; per-CTA partial sums are reduced in a fixed order.
+// is also the TMEM lane), N in {16, 32, 64, 80}, K in {16, 64, 128}, issued by
+// one thread as K/16 tcgen05.mma instructions of kind::f16 and completed
+// through tcgen05.commit on an mbarrier.  Weight gradients are GEMMs over the
+// samples (K = the 128 rows of a tile) and accumulate in tensor memory across
+// the tiles a CTA processes; per-CTA partial sums are reduced in a fixed order.
+//
+// The weight gradients read the tile's activations where the forward and
+// backward GEMMs left them: the core matrices (8 rows of 16 bytes) of a
+// K-major 128 x K operand are, with rows and columns exchanged, those of an
+// MN-major K x 128 one, so the descriptors alone transpose.  Column sums (the
+// bias gradients) come out of the same GEMMs: behind every 8-row group of X,
+// H1 and H2 lies one core matrix of ones.  Rows and columns of a product that
+// nobody reads hold whatever lies behind an operand.
+//
+// Measured (GB300): 100,003 rows, an Adam step 110 + 10 + 3.5 us (gradient,
+// reduction, packing) -> 27 + 7 us, the forward pass 24 -> 14.  The gradient
+// was bound by 2-byte shared-memory stores and by building transposed copies
+// (18 us per tile, one CTA per SM); now a tile's chain of five dependent GEMM
+// steps and their 16-byte-store epilogues, on two CTAs per SM, whose inputs
+// for the next tile load behind it.
 //
 // No counterpart in the reference: the learned warm start is new.
 #include "sd_common.cuh"
@@ -62,9 +77,10 @@ __device__ __forceinline__ uint64_t sdesc(uint32_t addr, uint32_t lbo, uint32_t 
            (1ull << 46);
 }
 
-// Instruction descriptor, kind::f16: D FP32, A and B BF16, both K-major.
-__host__ __device__ constexpr uint32_t idesc(uint32_t M, uint32_t N) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
+// Instruction descriptor, kind::f16: D FP32, A and B BF16, both K-major (or
+// both MN-major).
+__host__ __device__ constexpr uint32_t idesc(uint32_t M, uint32_t N, bool mn_major = false) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | (mn_major ? 3u << 15 : 0u) | ((N >> 3) << 17) | ((M >> 4) << 24);
 }
 
 __device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t id, uint32_t acc) {
@@ -131,46 +147,78 @@ __device__ __forceinline__ uint16_t bf16_bits(float x) {
 }
 __device__ __forceinline__ float bf16_val(uint16_t b) { return __bfloat162float(__ushort_as_bfloat16(b)); }
 
-__device__ __forceinline__ void st_bf16(uint8_t* base, uint32_t off, float x) {
-    *reinterpret_cast<uint16_t*>(base + off) = bf16_bits(x);
-}
-__device__ __forceinline__ float ld_bf16(const uint8_t* base, uint32_t off) {
-    return bf16_val(*reinterpret_cast<const uint16_t*>(base + off));
-}
-
-// D (tmem columns at d) [+]= A (128 x K, K-major) * B (N x K, K-major)^T.
-__device__ __forceinline__ void gemm_issue(uint32_t d, const uint8_t* A, const uint8_t* B, uint32_t N, uint32_t K,
-                                           bool accumulate) {
-    const uint32_t sboA = (K >> 3) * 128u, sboB = sboA;
-    const uint32_t id = idesc(kRows, N);
-    for (uint32_t s = 0; s < K / 16; ++s) {
-        const uint64_t a = sdesc(saddr(A) + s * 256u, 128u, sboA);
-        const uint64_t b = sdesc(saddr(B) + s * 256u, 128u, sboB);
-        mma_f16(d, a, b, id, (accumulate || s > 0) ? 1u : 0u);
-    }
+// Eight values as BF16, the first in the low half of the first word.
+__device__ __forceinline__ uint4 pack8(const float* v) {
+    uint32_t w[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        w[k] = (uint32_t)bf16_bits(v[2 * k]) | ((uint32_t)bf16_bits(v[2 * k + 1]) << 16);
+    return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// One GEMM step: thread 0 issues and commits, everyone waits for the commit.
-// Returns false (and flags) if the wait gave up.
-__device__ __forceinline__ bool gemm_sync(uint32_t d, const uint8_t* A, const uint8_t* B, uint32_t N, uint32_t K,
-                                          bool accumulate, uint64_t* bar, uint32_t& phase, uint32_t* status) {
+// Byte offset of columns 8c .. 8c + 7 of row r of an operand whose 8-row
+// groups are `group` bytes apart: one row of a core matrix.
+__device__ __forceinline__ uint32_t cm_row(uint32_t r, uint32_t c, uint32_t group) {
+    return (r >> 3) * group + c * 128u + (r & 7u) * 16u;
+}
+
+// Sixteen columns of a row, as two stores.
+__device__ __forceinline__ void st_row16(uint8_t* base, uint32_t r, uint32_t c0, uint32_t group, const float* v) {
+    *reinterpret_cast<uint4*>(base + cm_row(r, c0 >> 3, group)) = pack8(v);
+    *reinterpret_cast<uint4*>(base + cm_row(r, (c0 >> 3) + 1, group)) = pack8(v + 8);
+}
+
+// D (tmem columns at d) = A (128 x K, K-major, 8-row groups group_a bytes
+// apart) * B (N x K, K-major, packed)^T.
+__device__ __forceinline__ void gemm_issue(uint32_t d, const uint8_t* A, uint32_t group_a, const uint8_t* B, uint32_t N,
+                                           uint32_t K) {
+    const uint32_t id = idesc(kRows, N), group_b = (K >> 3) * 128u;
+    for (uint32_t s = 0; s < K / 16; ++s)
+        mma_f16(d, sdesc(saddr(A) + s * 256u, 128u, group_a), sdesc(saddr(B) + s * 256u, 128u, group_b), id,
+                s > 0 ? 1u : 0u);
+}
+
+// D (tmem columns at d) [+]= A^T B over the tile's 128 rows, A and B stored as
+// above: with K the rows, MN-major operands whose 8-element blocks along M or
+// N are 128 bytes apart and along K a group apart.  (For MN-major operands
+// without swizzle the descriptor's leading offset is the K one.)
+__device__ __forceinline__ void gemm_rows_issue(uint32_t d, const uint8_t* A, uint32_t group_a, const uint8_t* B,
+                                                uint32_t group_b, uint32_t N, bool accumulate) {
+    const uint32_t id = idesc(kRows, N, true);
+    for (uint32_t s = 0; s < kRows / 16; ++s)
+        mma_f16(d, sdesc(saddr(A) + s * 2u * group_a, group_a, 128u), sdesc(saddr(B) + s * 2u * group_b, group_b, 128u),
+                id, (accumulate || s > 0) ? 1u : 0u);
+}
+
+// Makes every thread's shared-memory writes and tensor-memory reads visible
+// to MMAs that thread 0 issues next.
+__device__ __forceinline__ void gemm_ready() {
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (threadIdx.x == 0) {
-        gemm_issue(d, A, B, N, K, accumulate);
-        mma_commit(bar);
-    }
+}
+
+// Waits for thread 0's last commit.  Returns false (and flags) if the wait
+// gave up: one verdict for the whole CTA.
+__device__ __forceinline__ bool gemm_wait(uint64_t* bar, uint32_t& phase, uint32_t* status) {
     const bool mine = mbar_wait(bar, phase);
-    const bool ok = __syncthreads_and(mine) != 0;  // one verdict for the whole CTA
-    if (ok) {
-        phase ^= 1u;
-    } else {
-        atomicOr(status, kErrWaitTimeout);
-    }
+    const bool ok = __syncthreads_and(mine) != 0;
+    if (ok) phase ^= 1u;
+    else atomicOr(status, kErrWaitTimeout);
     tc_fence_after();
     return ok;
+}
+
+// One GEMM step: thread 0 issues and commits, everyone waits for the commit.
+__device__ __forceinline__ bool gemm_sync(uint32_t d, const uint8_t* A, uint32_t group_a, const uint8_t* B, uint32_t N,
+                                          uint32_t K, uint64_t* bar, uint32_t& phase, uint32_t* status) {
+    gemm_ready();
+    if (threadIdx.x == 0) {
+        gemm_issue(d, A, group_a, B, N, K);
+        mma_commit(bar);
+    }
+    return gemm_wait(bar, phase, status);
 }
 
 // After a wait gave up: wait once more (bounded) for the MMAs in flight
@@ -189,13 +237,68 @@ __device__ __forceinline__ void copy_img(uint8_t* dst, const uint8_t* src, uint3
     for (uint32_t i = threadIdx.x; i < bytes / 16; i += blockDim.x) d[i] = s[i];
 }
 
+// 8-row groups of the operands a CTA builds: 2 or 8 core matrices, and one of
+// ones where a weight gradient takes column sums.
+constexpr uint32_t kGroup16 = 2 * 128, kGroup64 = 8 * 128, kGroup16p = 3 * 128, kGroup64p = 9 * 128;
+constexpr uint32_t kGroups = kRows / 8;
+
+// Sixteen inputs of a row (zeros when not live); vec: feat is 16-byte aligned.
+__device__ __forceinline__ void load_row16(const float* __restrict__ feat, uint64_t e, bool live, float* v,
+                                           bool vec = true) {
+    if (!vec) {
+#pragma unroll
+        for (int k = 0; k < kIn; ++k) v[k] = live ? __ldg(feat + 16 * e + k) : 0.0f;
+        return;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float4 f = live ? __ldg(reinterpret_cast<const float4*>(feat) + 4 * e + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[4 * k] = f.x;
+        v[4 * k + 1] = f.y;
+        v[4 * k + 2] = f.z;
+        v[4 * k + 3] = f.w;
+    }
+}
+
+// relu(accumulator + bias) of this thread's row, 64 columns, as the next
+// layer's operand.
+__device__ __forceinline__ void relu_row64(uint32_t taddr, const float* bias, uint8_t* h, uint32_t group, uint32_t row) {
+#pragma unroll
+    for (int c = 0; c < kHid; c += 16) {
+        float v[16];
+        tmem_ld16(taddr + c, v);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) v[k] = fmaxf(v[k] + bias[c + k], 0.0f);
+        st_row16(h, row, c, group, v);
+    }
+}
+
+// The accumulator where the activation (bf16, this thread's row) is positive,
+// else 0, as an operand.
+__device__ __forceinline__ void mask_row64(uint32_t taddr, const uint8_t* h, uint32_t group_h, uint8_t* dz, uint32_t row) {
+#pragma unroll
+    for (int c = 0; c < kHid; c += 16) {
+        float v[16];
+        tmem_ld16(taddr + c, v);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const uint4 a = *reinterpret_cast<const uint4*>(h + cm_row(row, (c >> 3) + q, group_h));
+            const uint32_t w[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                if (!(bf16_val((uint16_t)(w[k >> 1] >> (16 * (k & 1)))) > 0.0f)) v[8 * q + k] = 0.0f;
+        }
+        st_row16(dz, row, c, kGroup64, v);
+    }
+}
+
 struct InferSmem {
     alignas(1024) uint8_t w1[kHid * kIn * 2];
     alignas(1024) uint8_t w2[kHid * kHid * 2];
     alignas(1024) uint8_t w3[kOut * kHid * 2];
-    alignas(1024) uint8_t x[kRows * kIn * 2];
-    alignas(1024) uint8_t h1[kRows * kHid * 2];
-    alignas(1024) uint8_t h2[kRows * kHid * 2];
+    alignas(1024) uint8_t x[kGroups * kGroup16];
+    alignas(1024) uint8_t h1[kGroups * kGroup64];
+    alignas(1024) uint8_t h2[kGroups * kGroup64];
     float b[kHid + kHid + kOut];
     uint64_t bar;
     uint32_t tmem;
@@ -234,33 +337,19 @@ __global__ void __launch_bounds__(kRows) mlp_forward_kernel(const uint8_t* __res
     const uint32_t lane_base = (warp * 32u) << 16;
     uint32_t phase = 0;
     bool ok = true;
+    float x[kIn];
+    load_row16(feat, (uint64_t)blockIdx.x * kRows + tid, (uint64_t)blockIdx.x * kRows + tid < rows, x);
     for (uint64_t t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
-        const uint64_t e = t * kRows + tid;
+        const uint64_t e = t * kRows + tid, e2 = e + (uint64_t)gridDim.x * kRows;
         const bool live = e < rows;
-        float f7 = 0.f, skip[3] = {0.f, 0.f, 0.f};
-        // layer 1 operand: this thread's row of inputs
-        for (int k = 0; k < kIn; ++k) {
-            const float v = live ? feat[16 * e + k] : 0.0f;
-            if (k == 7) f7 = v;
-            if (k >= 8 && k < 11) skip[k - 8] = v;
-            st_bf16(S.x, cm_off(tid, k, kIn), v);
-        }
-        if (!(ok = gemm_sync(tm + 0, S.x, S.w1, kHid, kIn, false, &S.bar, phase, status))) break;
-        for (int c = 0; c < kHid; c += 16) {
-            float v[16];
-            tmem_ld16(tm + lane_base + c, v);
-#pragma unroll
-            for (int k = 0; k < 16; ++k) st_bf16(S.h1, cm_off(tid, c + k, kHid), fmaxf(v[k] + S.b[c + k], 0.0f));
-        }
-        if (!(ok = gemm_sync(tm + 64, S.h1, S.w2, kHid, kHid, false, &S.bar, phase, status))) break;
-        for (int c = 0; c < kHid; c += 16) {
-            float v[16];
-            tmem_ld16(tm + lane_base + 64 + c, v);
-#pragma unroll
-            for (int k = 0; k < 16; ++k)
-                st_bf16(S.h2, cm_off(tid, c + k, kHid), fmaxf(v[k] + S.b[kHid + c + k], 0.0f));
-        }
-        if (!(ok = gemm_sync(tm + 128, S.h2, S.w3, kOut, kHid, false, &S.bar, phase, status))) break;
+        const float f7 = x[7], skip[3] = {x[8], x[9], x[10]};
+        st_row16(S.x, tid, 0, kGroup16, x);
+        load_row16(feat, e2, e2 < rows, x);  // the next tile's, in flight behind this one's
+        if (!(ok = gemm_sync(tm + 0, S.x, kGroup16, S.w1, kHid, kIn, &S.bar, phase, status))) break;
+        relu_row64(tm + lane_base, S.b, S.h1, kGroup64, tid);
+        if (!(ok = gemm_sync(tm + 64, S.h1, kGroup64, S.w2, kHid, kHid, &S.bar, phase, status))) break;
+        relu_row64(tm + lane_base + 64, S.b + kHid, S.h2, kGroup64, tid);
+        if (!(ok = gemm_sync(tm + 128, S.h2, kGroup64, S.w3, kOut, kHid, &S.bar, phase, status))) break;
         float y[16];
         tmem_ld16(tm + lane_base + 128, y);
         if (live) {
@@ -271,9 +360,7 @@ __global__ void __launch_bounds__(kRows) mlp_forward_kernel(const uint8_t* __res
             else
                 out[e] = make_float4(y0, y1, y2, 0.f);
         }
-        tc_fence_before();
-        __syncthreads();  // the tile's operands are reused by the next tile
-        tc_fence_after();
+        // the next tile's first GEMM step orders these reads before its MMAs
     }
     if (!ok) drain(&S.bar, phase);
     tc_fence_before();
@@ -281,55 +368,56 @@ __global__ void __launch_bounds__(kRows) mlp_forward_kernel(const uint8_t* __res
     if (warp == 0) tmem_dealloc(tm, 256);
 }
 
+// The operands first: a weight gradient's MMAs may read up to 1.1 KB behind
+// one (products that nobody reads).
 struct TrainSmem {
+    alignas(1024) uint8_t x[kGroups * kGroup16p];
+    alignas(1024) uint8_t h1[kGroups * kGroup64p];
+    alignas(1024) uint8_t h2[kGroups * kGroup64p];
+    alignas(1024) uint8_t dz2[kGroups * kGroup64];
+    alignas(1024) uint8_t dz1[kGroups * kGroup64];
+    alignas(1024) uint8_t dy[kGroups * kGroup16];
     alignas(1024) uint8_t w1[kHid * kIn * 2];
     alignas(1024) uint8_t w2[kHid * kHid * 2];
     alignas(1024) uint8_t w3[kOut * kHid * 2];
     alignas(1024) uint8_t w2t[kHid * kHid * 2];
     alignas(1024) uint8_t w3t[kHid * kOut * 2];
-    alignas(1024) uint8_t x[kRows * kIn * 2];
-    alignas(1024) uint8_t h1[kRows * kHid * 2];
-    alignas(1024) uint8_t h2[kRows * kHid * 2];
-    alignas(1024) uint8_t dy[kRows * kOut * 2];
-    alignas(1024) uint8_t dz2[kRows * kHid * 2];
-    alignas(1024) uint8_t dz1[kRows * kHid * 2];
-    // transposed operands of the weight gradients: A = 128 x 128 (rows 64..127
-    // are the zero block that follows), B = up to 64 x 128
-    alignas(1024) uint8_t at[kHid * kRows * 2];
-    alignas(1024) uint8_t zero[kHid * kRows * 2];
-    alignas(1024) uint8_t bt[kHid * kRows * 2];
     float b[kHid + kHid + kOut];
-    float gb[kHid + kHid + kOut];
     uint64_t bar;
     uint32_t tmem;
 };
 
 // Forward + backward of the cosine loss 1 - y.t/|y| (mean over valid rows)
-// for the tiles of this CTA; per-CTA gradient partials to part[cta][6288].
-// tgt rows: (tx, ty, tz, valid).
+// for the tiles of this CTA; per-CTA gradient partials to part[cta][6288]
+// (none from a CTA without tiles).  tgt rows: (tx, ty, tz, valid).
 __global__ void __launch_bounds__(kRows) mlp_train_kernel(const uint8_t* __restrict__ img,
                                                          const float* __restrict__ params,
                                                          const float* __restrict__ feat, const float4* __restrict__ tgt,
                                                          uint32_t n, float inv_batch, float* __restrict__ part,
                                                          uint32_t* __restrict__ status,
-                                                         const uint32_t* __restrict__ d_count) {
+                                                         const uint32_t* __restrict__ d_count, bool vec) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
     TrainSmem& S = *reinterpret_cast<TrainSmem*>(aligned_smem(smem_raw));
     const uint32_t tid = threadIdx.x, warp = tid >> 5;
     if (d_count) n = min(n, *d_count);  // rows: the step's entry count, read on the device
     const uint32_t tiles = (n + kRows - 1) / kRows;
+    if (blockIdx.x >= tiles) return;
     copy_img(S.w1, img + kImgW1, sizeof S.w1);
     copy_img(S.w2, img + kImgW2, sizeof S.w2);
     copy_img(S.w3, img + kImgW3, sizeof S.w3);
     copy_img(S.w2t, img + kImgW2T, sizeof S.w2t);
     copy_img(S.w3t, img + kImgW3T, sizeof S.w3t);
-    for (uint32_t i = tid; i < sizeof S.zero / 16; i += kRows) reinterpret_cast<uint4*>(S.zero)[i] = make_uint4(0, 0, 0, 0);
+    {
+        const uint4 ones = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);  // bf16 1.0
+        *reinterpret_cast<uint4*>(S.x + cm_row(tid, 2, kGroup16p)) = ones;
+        *reinterpret_cast<uint4*>(S.h1 + cm_row(tid, 8, kGroup64p)) = ones;
+        *reinterpret_cast<uint4*>(S.h2 + cm_row(tid, 8, kGroup64p)) = ones;
+    }
     for (uint32_t i = tid; i < kHid; i += kRows) {
         S.b[i] = params[kB1 + i];
         S.b[kHid + i] = params[kB2 + i];
     }
     if (tid < kOut) S.b[2 * kHid + tid] = params[kB3 + tid];
-    for (uint32_t i = tid; i < 2 * kHid + kOut; i += kRows) S.gb[i] = 0.0f;
     if (warp == 0) tmem_alloc(&S.tmem, 256);
     if (tid == 0) mbar_init1(&S.bar);
     tc_fence_before();
@@ -337,172 +425,143 @@ __global__ void __launch_bounds__(kRows) mlp_train_kernel(const uint8_t* __restr
     tc_fence_after();
     const uint32_t tm = S.tmem;
     const uint32_t lane_base = (warp * 32u) << 16;
-    // tensor-memory columns: forward and activation gradients reuse [0, 144);
-    // the weight gradients accumulate over tiles in [144, 240)
-    const uint32_t cL1 = 0, cL2 = 64, cL3 = 128, cG3 = 144, cG2 = 160, cG1 = 224;
+    // tensor-memory columns: forward and activation gradients reuse [0, 128);
+    // the weight gradients accumulate over tiles in [128, 256)
+    const uint32_t cA = 0, cB = 64, cG3 = 128, cG2 = 144, cG1 = 224;
     uint32_t phase = 0;
-    bool ok = true;
-    bool first = true;
-    for (uint32_t t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
-        const uint32_t e = t * kRows + tid;
-        const bool live = e < n;
-        float skip[3] = {0.f, 0.f, 0.f};
-        for (int k = 0; k < kIn; ++k) {
-            const float v = live ? feat[16 * (size_t)e + k] : 0.0f;
-            if (k >= 8 && k < 11) skip[k - 8] = v;
-            st_bf16(S.x, cm_off(tid, k, kIn), v);
-        }
-        ok = gemm_sync(tm + cL1, S.x, S.w1, kHid, kIn, false, &S.bar, phase, status);
-        if (!ok) break;
-        for (int c = 0; c < kHid; c += 16) {
-            float v[16];
-            tmem_ld16(tm + lane_base + cL1 + c, v);
-#pragma unroll
-            for (int k = 0; k < 16; ++k) st_bf16(S.h1, cm_off(tid, c + k, kHid), fmaxf(v[k] + S.b[c + k], 0.0f));
-        }
-        ok = gemm_sync(tm + cL2, S.h1, S.w2, kHid, kHid, false, &S.bar, phase, status);
-        if (!ok) break;
-        for (int c = 0; c < kHid; c += 16) {
-            float v[16];
-            tmem_ld16(tm + lane_base + cL2 + c, v);
-#pragma unroll
-            for (int k = 0; k < 16; ++k)
-                st_bf16(S.h2, cm_off(tid, c + k, kHid), fmaxf(v[k] + S.b[kHid + c + k], 0.0f));
-        }
-        ok = gemm_sync(tm + cL3, S.h2, S.w3, kOut, kHid, false, &S.bar, phase, status);
-        if (!ok) break;
+    bool ok = true, first = true;
+    uint32_t e = blockIdx.x * kRows + tid;
+    float x[kIn];
+    load_row16(feat, e, e < n, x, vec);
+    float4 g = e < n ? tgt[e] : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+        // the last tile's weight gradients have read the operands
+        if (!first && !(ok = gemm_wait(&S.bar, phase, status))) break;
+        const float skip[3] = {x[8], x[9], x[10]};
+        const float4 target = g;
+        st_row16(S.x, tid, 0, kGroup16p, x);
+        e += gridDim.x * kRows;  // the next tile's rows, in flight behind this one's
+        load_row16(feat, e, e < n, x, vec);
+        g = e < n ? tgt[e] : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (!(ok = gemm_sync(tm + cA, S.x, kGroup16p, S.w1, kHid, kIn, &S.bar, phase, status))) break;
+        relu_row64(tm + lane_base + cA, S.b, S.h1, kGroup64p, tid);
+        if (!(ok = gemm_sync(tm + cB, S.h1, kGroup64p, S.w2, kHid, kHid, &S.bar, phase, status))) break;
+        relu_row64(tm + lane_base + cB, S.b + kHid, S.h2, kGroup64p, tid);
+        if (!(ok = gemm_sync(tm + cA, S.h2, kGroup64p, S.w3, kOut, kHid, &S.bar, phase, status))) break;
         {
             float y[16];
-            tmem_ld16(tm + lane_base + cL3, y);
-            const float4 g = live ? tgt[e] : make_float4(0.f, 0.f, 0.f, 0.f);
-            float d[3] = {0.f, 0.f, 0.f};
-            if (g.w != 0.0f) {
+            tmem_ld16(tm + lane_base + cA, y);
+            float d[16] = {};
+            if (target.w != 0.0f) {
                 const float y0 = (y[0] + S.b[2 * kHid]) + skip[0], y1 = (y[1] + S.b[2 * kHid + 1]) + skip[1],
                             y2 = (y[2] + S.b[2 * kHid + 2]) + skip[2];
                 const float nn = sqrtf(((y0 * y0 + y1 * y1) + y2 * y2) + 1e-8f);
-                const float c = ((y0 * g.x + y1 * g.y) + y2 * g.z) / nn;
+                const float c = ((y0 * target.x + y1 * target.y) + y2 * target.z) / nn;
                 const float s = -inv_batch / nn;
-                d[0] = s * (g.x - c * y0 / nn);
-                d[1] = s * (g.y - c * y1 / nn);
-                d[2] = s * (g.z - c * y2 / nn);
+                d[0] = s * (target.x - c * y0 / nn);
+                d[1] = s * (target.y - c * y1 / nn);
+                d[2] = s * (target.z - c * y2 / nn);
             }
-            for (int k = 0; k < kOut; ++k) st_bf16(S.dy, cm_off(tid, k, kOut), k < 3 ? d[k] : 0.0f);
+            st_row16(S.dy, tid, 0, kGroup16, d);
         }
-        // dH2 = dY W3  (B = W3^T, N 64 x K 16)
-        ok = gemm_sync(tm + cL1, S.dy, S.w3t, kHid, kOut, false, &S.bar, phase, status);
-        if (!ok) break;
-        for (int c = 0; c < kHid; c += 16) {
-            float v[16];
-            tmem_ld16(tm + lane_base + cL1 + c, v);
-#pragma unroll
-            for (int k = 0; k < 16; ++k) {
-                const uint32_t o = cm_off(tid, c + k, kHid);
-                st_bf16(S.dz2, o, ld_bf16(S.h2, o) > 0.0f ? v[k] : 0.0f);
-            }
+        // dH2 = dY W3  (B = W3^T, N 64 x K 16), then dH1 = dZ2 W2
+        if (!(ok = gemm_sync(tm + cB, S.dy, kGroup16, S.w3t, kHid, kOut, &S.bar, phase, status))) break;
+        mask_row64(tm + lane_base + cB, S.h2, kGroup64p, S.dz2, tid);
+        if (!(ok = gemm_sync(tm + cA, S.dz2, kGroup64, S.w2t, kHid, kHid, &S.bar, phase, status))) break;
+        mask_row64(tm + lane_base + cA, S.h1, kGroup64p, S.dz1, tid);
+        // weight gradients, K = the tile's rows: dW3^T (j, o) = H2^T dY with
+        // row 64 (of ones) the sums of dY; dW2 (k, j) = dZ2^T H1 and dW1 (j,
+        // i) = dZ1^T X, each with the sums in the column behind.  Nobody
+        // waits before the next tile.
+        gemm_ready();
+        if (tid == 0) {
+            gemm_rows_issue(tm + cG3, S.h2, kGroup64p, S.dy, kGroup16, kOut, !first);
+            gemm_rows_issue(tm + cG2, S.dz2, kGroup64, S.h1, kGroup64p, kHid + 16, !first);
+            gemm_rows_issue(tm + cG1, S.dz1, kGroup64, S.x, kGroup16p, kIn + 16, !first);
+            mma_commit(&S.bar);
         }
-        // dH1 = dZ2 W2  (B = W2^T)
-        ok = gemm_sync(tm + cL2, S.dz2, S.w2t, kHid, kHid, false, &S.bar, phase, status);
-        if (!ok) break;
-        for (int c = 0; c < kHid; c += 16) {
-            float v[16];
-            tmem_ld16(tm + lane_base + cL2 + c, v);
-#pragma unroll
-            for (int k = 0; k < 16; ++k) {
-                const uint32_t o = cm_off(tid, c + k, kHid);
-                st_bf16(S.dz1, o, ld_bf16(S.h1, o) > 0.0f ? v[k] : 0.0f);
-            }
-        }
-        __syncthreads();
-        // bias gradients: column sums over the tile's rows, fixed order
-        if (tid < kHid) {
-            float a1 = 0.f, a2 = 0.f;
-            for (uint32_t m = 0; m < kRows; ++m) {
-                a1 += ld_bf16(S.dz1, cm_off(m, tid, kHid));
-                a2 += ld_bf16(S.dz2, cm_off(m, tid, kHid));
-            }
-            S.gb[tid] += a1;
-            S.gb[kHid + tid] += a2;
-        } else if (tid < kHid + 3) {
-            const uint32_t o = tid - kHid;
-            float a3 = 0.f;
-            for (uint32_t m = 0; m < kRows; ++m) a3 += ld_bf16(S.dy, cm_off(m, o, kOut));
-            S.gb[2 * kHid + o] += a3;
-        }
-        // weight gradients, K = the tile's rows.  dW3^T (j, o) = H2^T dY
-        for (int j = 0; j < kHid; ++j) {
-            const uint16_t hv = *reinterpret_cast<const uint16_t*>(S.h2 + cm_off(tid, j, kHid));
-            *reinterpret_cast<uint16_t*>(S.at + cm_off(j, tid, kRows)) = hv;
-        }
-        for (int o = 0; o < kOut; ++o) {
-            const uint16_t dv = *reinterpret_cast<const uint16_t*>(S.dy + cm_off(tid, o, kOut));
-            *reinterpret_cast<uint16_t*>(S.bt + cm_off(o, tid, kRows)) = dv;
-        }
-        ok = gemm_sync(tm + cG3, S.at, S.bt, kOut, kRows, !first, &S.bar, phase, status);
-        if (!ok) break;
-        // dW2 (k, j) = dZ2^T H1
-        for (int j = 0; j < kHid; ++j) {
-            const uint16_t a = *reinterpret_cast<const uint16_t*>(S.dz2 + cm_off(tid, j, kHid));
-            const uint16_t b = *reinterpret_cast<const uint16_t*>(S.h1 + cm_off(tid, j, kHid));
-            *reinterpret_cast<uint16_t*>(S.at + cm_off(j, tid, kRows)) = a;
-            *reinterpret_cast<uint16_t*>(S.bt + cm_off(j, tid, kRows)) = b;
-        }
-        ok = gemm_sync(tm + cG2, S.at, S.bt, kHid, kRows, !first, &S.bar, phase, status);
-        if (!ok) break;
-        // dW1 (j, i) = dZ1^T X
-        for (int j = 0; j < kHid; ++j) {
-            const uint16_t a = *reinterpret_cast<const uint16_t*>(S.dz1 + cm_off(tid, j, kHid));
-            *reinterpret_cast<uint16_t*>(S.at + cm_off(j, tid, kRows)) = a;
-        }
-        for (int i = 0; i < kIn; ++i) {
-            const uint16_t b = *reinterpret_cast<const uint16_t*>(S.x + cm_off(tid, i, kIn));
-            *reinterpret_cast<uint16_t*>(S.bt + cm_off(i, tid, kRows)) = b;
-        }
-        ok = gemm_sync(tm + cG1, S.at, S.bt, kIn, kRows, !first, &S.bar, phase, status);
         first = false;
     }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
+    if (ok) ok = gemm_wait(&S.bar, phase, status);
     float* P = part + (size_t)blockIdx.x * kParams;
-    if (ok && !first) {
+    if (ok) {
+        float v[16];
         if (warp < 2) {  // lanes 0..63 hold the 64 rows of every weight gradient
             const uint32_t r = tid;
-            float v[16];
             tmem_ld16(tm + lane_base + cG3, v);  // dW3^T row j = r
 #pragma unroll
             for (int o = 0; o < kOut; ++o) P[kW3 + o * kHid + r] = o < 3 ? v[o] : 0.0f;
+#pragma unroll
             for (int c = 0; c < kHid; c += 16) {
                 tmem_ld16(tm + lane_base + cG2 + c, v);
 #pragma unroll
-                for (int k = 0; k < 16; ++k) P[kW2 + r * kHid + c + k] = v[k];
+                for (int k = 0; k < 16; k += 4)
+                    *reinterpret_cast<float4*>(P + kW2 + r * kHid + c + k) = make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]);
             }
+            tmem_ld16(tm + lane_base + cG2 + kHid, v);
+            P[kB2 + r] = v[0];
             tmem_ld16(tm + lane_base + cG1, v);
 #pragma unroll
-            for (int i = 0; i < kIn; ++i) P[kW1 + r * kIn + i] = v[i];
+            for (int k = 0; k < 16; k += 4)
+                *reinterpret_cast<float4*>(P + kW1 + r * kIn + k) = make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]);
+            tmem_ld16(tm + lane_base + cG1 + kIn, v);
+            P[kB1 + r] = v[0];
+        } else if (warp == 2) {  // lane 64: the row of ones
+            tmem_ld16(tm + lane_base + cG3, v);
+            if (tid == 64)
+#pragma unroll
+                for (int o = 0; o < kOut; ++o) P[kB3 + o] = o < 3 ? v[o] : 0.0f;
         }
-        for (uint32_t i = tid; i < kHid; i += kRows) {
-            P[kB1 + i] = S.gb[i];
-            P[kB2 + i] = S.gb[kHid + i];
-        }
-        if (tid < kOut) P[kB3 + tid] = tid < 3 ? S.gb[2 * kHid + tid] : 0.0f;
     } else {
         for (uint32_t i = tid; i < kParams; i += kRows) P[i] = 0.0f;
+        drain(&S.bar, phase);
     }
-    if (!ok) drain(&S.bar, phase);
     tc_fence_before();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tm, 256);
 }
 
-// grad[p] = sum over CTAs of part[c][p], in CTA order; then (adam != 0) an
-// Adam step on the master parameters (W3, b3 rows 3..15 stay zero).
-__global__ void mlp_reduce_kernel(const float* __restrict__ part, uint32_t nparts, float* __restrict__ grad,
-                                  float* __restrict__ params, float* __restrict__ m1, float* __restrict__ m2,
-                                  int adam, float lr, float c1, float c2) {
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= (uint32_t)kParams) return;
+// BF16 operand images of parameter p: W1, W2, W3 and the transposes W2^T, W3^T.
+__device__ __forceinline__ void pack_param(uint32_t p, float x, uint8_t* __restrict__ img) {
+    const uint16_t b = bf16_bits(x);
+    auto put = [&](uint32_t at) { *reinterpret_cast<uint16_t*>(img + at) = b; };
+    if (p < (uint32_t)kB1) {  // W1 [n][k]
+        put(kImgW1 + cm_off(p / kIn, p % kIn, kIn));
+    } else if (p >= (uint32_t)kW2 && p < (uint32_t)kB2) {  // W2 [n][k] and W2^T [n = k_in][k = k_out]
+        const uint32_t r = (p - kW2) / kHid, k = (p - kW2) % kHid;
+        put(kImgW2 + cm_off(r, k, kHid));
+        put(kImgW2T + cm_off(k, r, kHid));
+    } else if (p >= (uint32_t)kW3 && p < (uint32_t)kB3) {  // W3 [o][j] and W3^T [j][o]
+        const uint32_t o = (p - kW3) / kHid, j = (p - kW3) % kHid;
+        put(kImgW3 + cm_off(o, j, kHid));
+        put(kImgW3T + cm_off(j, o, kOut));
+    }
+}
+
+// grad[p] = sum over CTAs of part[c][p] in a fixed order: kSlices sums of
+// every kSlices-th CTA, then those in order (one thread a parameter, CTA after
+// CTA, took 10 us of load latency at 148 CTAs).  Then (adam != 0) an Adam step on the
+// master parameters and their operand images (W3, b3 rows 3..15 stay zero).
+// CTAs past the rows' tiles wrote no part.
+constexpr int kSlices = 32;
+__global__ void __launch_bounds__(32 * kSlices)
+mlp_reduce_kernel(const float* __restrict__ part, uint32_t nparts, uint32_t n, const uint32_t* __restrict__ d_count,
+                  float* __restrict__ grad, float* __restrict__ params, float* __restrict__ m1,
+                  float* __restrict__ m2, uint8_t* __restrict__ img, int adam, float lr, float c1, float c2) {
+    __shared__ float s[kSlices][32];
+    const uint32_t lane = threadIdx.x & 31u, slice = threadIdx.x >> 5, p = blockIdx.x * 32 + lane;
+    if (d_count) n = min(n, *d_count);
+    nparts = min(nparts, (n + kRows - 1) / kRows);
     float g = 0.0f;
-    for (uint32_t c = 0; c < nparts; ++c) g += part[(size_t)c * kParams + p];
+    if (p < (uint32_t)kParams)
+#pragma unroll 8
+        for (uint32_t c = slice; c < nparts; c += kSlices) g += part[(size_t)c * kParams + p];
+    s[slice][lane] = g;
+    __syncthreads();
+    if (slice != 0 || p >= (uint32_t)kParams) return;
+    g = 0.0f;
+#pragma unroll
+    for (int k = 0; k < kSlices; ++k) g += s[k][lane];
     const bool dead = (p >= (uint32_t)kW3 && p < (uint32_t)kB3 && (p - kW3) / kHid >= 3) || (p >= (uint32_t)kB3 + 3);
     if (dead) g = 0.0f;
     if (grad) grad[p] = g;
@@ -511,33 +570,19 @@ __global__ void mlp_reduce_kernel(const float* __restrict__ part, uint32_t npart
     const float b = 0.999f * m2[p] + 0.001f * (g * g);
     m1[p] = a;
     m2[p] = b;
-    params[p] -= lr * (a * c1) / (sqrtf(b * c2) + 1e-8f);
+    const float x = params[p] - lr * (a * c1) / (sqrtf(b * c2) + 1e-8f);
+    params[p] = x;
+    pack_param(p, x, img);
 }
 
-// BF16 operand images of W1, W2, W3 and the transposes W2^T, W3^T.
 __global__ void mlp_pack_kernel(const float* __restrict__ params, uint8_t* __restrict__ img) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < (uint32_t)(kHid * kIn)) {  // W1 [n][k]
-        const uint32_t r = i / kIn, k = i % kIn;
-        *reinterpret_cast<uint16_t*>(img + kImgW1 + cm_off(r, k, kIn)) = bf16_bits(params[kW1 + i]);
-    }
-    if (i < (uint32_t)(kHid * kHid)) {  // W2 [n][k] and W2^T [n=k_in][k=k_out]
-        const uint32_t r = i / kHid, k = i % kHid;
-        const uint16_t b = bf16_bits(params[kW2 + i]);
-        *reinterpret_cast<uint16_t*>(img + kImgW2 + cm_off(r, k, kHid)) = b;
-        *reinterpret_cast<uint16_t*>(img + kImgW2T + cm_off(k, r, kHid)) = b;
-    }
-    if (i < (uint32_t)(kOut * kHid)) {  // W3 [o][j] and W3^T [j][o]
-        const uint32_t o = i / kHid, j = i % kHid;
-        const uint16_t b = bf16_bits(params[kW3 + i]);
-        *reinterpret_cast<uint16_t*>(img + kImgW3 + cm_off(o, j, kHid)) = b;
-        *reinterpret_cast<uint16_t*>(img + kImgW3T + cm_off(j, o, kOut)) = b;
-    }
+    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p < (uint32_t)kParams) pack_param(p, params[p], img);
 }
 
 inline uint32_t grid_for(uint64_t n, int threads) { return (uint32_t)((n + threads - 1) / threads); }
 
-constexpr uint32_t kMaxTrainCtas = 148;
+constexpr uint32_t kMaxTrainCtas = 304;  // two per SM (operands and accumulators fit twice)
 
 }  // namespace
 
@@ -577,7 +622,7 @@ cudaError_t mlp_set_params_async(MlpState& s, const float* host_params, cudaStre
     if (e == cudaSuccess) e = cudaMemsetAsync(s.m1, 0, 8ull * kParams, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(s.img, 0, kImgBytes, st);
     if (e != cudaSuccess) return e;
-    mlp_pack_kernel<<<grid_for(kHid * kHid, 256), 256, 0, st>>>(s.params, s.img);
+    mlp_pack_kernel<<<grid_for(kParams, 256), 256, 0, st>>>(s.params, s.img);
     return cudaGetLastError();
 }
 
@@ -604,12 +649,12 @@ cudaError_t mlp_train_async(MlpState& s, const float* feat, const float4* tgt, u
     const uint32_t ctas = tiles < kMaxTrainCtas ? tiles : kMaxTrainCtas;
     const float inv = n_valid ? 1.0f / (float)n_valid : 0.0f;
     mlp_train_kernel<<<ctas, kRows, sizeof(TrainSmem) + 1024, st>>>(s.img, s.params, feat, tgt, n, inv, s.part,
-                                                                     s.status, d_count);
+                                                                     s.status, d_count,
+                                                                     (reinterpret_cast<uintptr_t>(feat) & 15u) == 0);
     const float c1 = update ? (float)(1.0 / (1.0 - std::pow(0.9, (double)adam_step))) : 0.f;
     const float c2 = update ? (float)(1.0 / (1.0 - std::pow(0.999, (double)adam_step))) : 0.f;
-    mlp_reduce_kernel<<<grid_for(kParams, 256), 256, 0, st>>>(s.part, ctas, s.grad, s.params, s.m1, s.m2,
-                                                              update ? 1 : 0, lr, c1, c2);
-    if (update) mlp_pack_kernel<<<grid_for(kHid * kHid, 256), 256, 0, st>>>(s.params, s.img);
+    mlp_reduce_kernel<<<grid_for(kParams, 32), 32 * kSlices, 0, st>>>(s.part, ctas, n, d_count, s.grad, s.params, s.m1,
+                                                                      s.m2, s.img, update ? 1 : 0, lr, c1, c2);
     return cudaGetLastError();
 }
 

@@ -198,3 +198,29 @@ def test_online_learned_seed_beats_its_untrained_baseline(sdlib):
     assert per["online"] < per["previous"] and per["plain"] / per["online"] > 2.0
     for eng in engines.values():
         eng.close()
+
+
+@pytest.mark.parametrize("n,shift", [(1, 0), (127, 0), (129, 1), (304 * 128 - 1, 0), (304 * 128 + 1, 2),
+                                     (2 * 304 * 128 + 77, 0)])
+def test_mlp_gradients_over_tiles(sdlib, orc, n, shift):
+    """Rows around one tile of 128 and around one tile for each of the 304
+    CTAs, the inputs 16-byte aligned or not: gradient elements within 2^-6 of
+    their sums of |terms|, as in test_mlp_gradients_match_oracle."""
+    import torch
+    eng = tiny_engine(sdlib)
+    rng = np.random.default_rng(n)
+    X, T = random_batch(rng, n)
+    p = eng.mlp_params()
+    p[:-16] += rng.normal(size=p.size - 16).astype(np.float32) * 0.05
+    P = orc.mlp_unpack(p)
+    P["W3"][3:] = 0
+    p = orc.mlp_pack(P)
+    eng.set_mlp_params(p)
+    feat = torch.zeros(16 * n + shift, device="cuda")[shift:].reshape(n, 16)
+    feat.copy_(torch.from_numpy(X))
+    g = eng.mlp_train(feat, torch.from_numpy(T).cuda(), 0)
+    _, _, gr, ga = orc.mlp_forward_backward(p, X, T, with_abs=True)
+    G, R, A = orc.mlp_unpack(g), orc.mlp_unpack(gr), orc.mlp_unpack(ga)
+    for k in ("W1", "b1", "W2", "b2", "W3", "b3"):
+        assert np.all(np.abs(G[k] - R[k]) <= 2.0 ** -6 * A[k] + 1e-12), k
+    eng.close()
