@@ -436,8 +436,8 @@ sd_status sd_sap_process_collisions(uint64_t n, const float* d_pos4, const float
 sd_status sd_lbvh_scratch_bytes(uint64_t n, uint64_t pair_cap, uint64_t* bytes);
 /* Every pair (i < j) of overlapping closed boxes, ascending u64
  * (i << 32 | j).  d_count[0] = number of pairs (written up to cap),
- * d_count[1] = device error bits (SD_DEVERR_PAIR_OVERFLOW when the partner
- * lists exceeded 2 * cap entries). */
+ * d_count[1] = device error bits (SD_DEVERR_PAIR_OVERFLOW when there are
+ * more than cap pairs). */
 sd_status sd_lbvh_pairs(uint64_t n, const float* d_lo4, const float* d_hi4, uint64_t* d_pairs, uint64_t cap,
                         uint32_t* d_count, void* d_scratch, uint64_t scratch_bytes, void* stream);
 /* The reference's 30-bit Morton code of each box centroid relative to the

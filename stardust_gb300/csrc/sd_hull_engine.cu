@@ -633,22 +633,12 @@ sd_status sd_lbvh_pairs(uint64_t n, const float* d_lo4, const float* d_hi4, uint
     sd::lbvh_carve(p, (uint32_t)n, &t);
     p += al(sd::lbvh_scratch_bytes((uint32_t)n));
     uint32_t* off = reinterpret_cast<uint32_t*>(p);
-    p += al(4 * (n + 1));
-    uint32_t* pos = reinterpret_cast<uint32_t*>(p);
-    p += al(4 * (n + 1));
-    uint32_t* partners = reinterpret_cast<uint32_t*>(p);
-    p += al(4 * (2 * cap + 1));
-    uint32_t* self = reinterpret_cast<uint32_t*>(p);
     const float4* lo = reinterpret_cast<const float4*>(d_lo4);
     const float4* hi = reinterpret_cast<const float4*>(d_hi4);
     cudaError_t e = cudaMemsetAsync(t.status, 0, 16, st);
     if (e == cudaSuccess) e = sd::lbvh_build_async(t, lo, hi, st);
-    if (e == cudaSuccess) e = sd::lbvh_partners_async(t, off, partners, self, 2 * cap, st);
     if (e == cudaSuccess)
-        e = sd::lbvh_unique_pairs_async(t, off, partners, 2 * cap, pos, reinterpret_cast<unsigned long long*>(d_pairs),
-                                        cap, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d_count, pos + n, 4, cudaMemcpyDeviceToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d_count + 1, t.status, 4, cudaMemcpyDeviceToDevice, st);
+        e = sd::lbvh_unique_pairs_async(t, off, reinterpret_cast<unsigned long long*>(d_pairs), cap, d_count, st);
     if (e != cudaSuccess) return sd_cuda_fail(nullptr, e, "sd_lbvh_pairs");
     return SD_OK;
 }

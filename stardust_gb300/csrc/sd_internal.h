@@ -36,8 +36,6 @@ void sort_set_items(int items);
 int sort_items();
 uint32_t* sort_hist_ptr(uint32_t* scratch);  // global digit histograms, pass q at q * plan.stride (2048 words)
 cudaError_t sort_clear_async(uint32_t n, const SortPlan& plan, uint32_t* scratch, cudaStream_t st);
-cudaError_t sort_histogram_async(const uint32_t* keys, uint32_t n, const SortPlan& plan, uint32_t* scratch,
-                                 cudaStream_t st);
 // skip (may be null): the passes return at once when skip[1] <= skip_max
 // (the incremental re-sort has written the result)
 // The radix fallback of the incremental re-sort: when skip[1] > skip_max,
@@ -51,10 +49,12 @@ cudaError_t sort_fallback_async(uint32_t* keys, uint32_t* vals, uint32_t* keys_t
                                 const uint32_t* skip, uint32_t skip_max);
 cudaError_t sort_passes_async(uint32_t* keys, uint32_t* vals, uint32_t* keys_tmp, uint32_t* vals_tmp,
                               uint32_t n, const SortPlan& plan, uint32_t* scratch, cudaStream_t st,
-                              bool* in_tmp, const uint32_t* skip = nullptr, uint32_t skip_max = 0);
+                              bool* in_tmp, const uint32_t* skip = nullptr, uint32_t skip_max = 0,
+                              const uint32_t* d_n = nullptr);
+// d_n (may be null): a device word, the number of keys when it is below n
 cudaError_t sort_pairs_async(uint32_t* keys, uint32_t* vals, uint32_t* keys_tmp, uint32_t* vals_tmp,
                              uint32_t n, int key_bits, uint32_t* scratch, cudaStream_t st,
-                             bool* in_tmp);
+                             bool* in_tmp, const uint32_t* d_n = nullptr);
 
 // ---- reference-compatible spatial hash (sd_hash_ref.cu)
 cudaError_t ref_hash_build_async(uint32_t n, float cell_dim, uint32_t* cells, uint32_t* spheres,
@@ -88,7 +88,7 @@ struct Lbvh {
     uint32_t* scan_scratch;
     uint32_t* status;                    // device error bits
 };
-constexpr int kLbvhFirst = 16;
+constexpr int kLbvhFirst = 32;
 uint64_t lbvh_scratch_bytes(uint32_t n);
 void lbvh_carve(void* scratch, uint32_t n, Lbvh* t);
 cudaError_t lbvh_morton_async(Lbvh& t, const float4* lo, const float4* hi, cudaStream_t st);
@@ -102,14 +102,10 @@ int lbvh_rebuild_every();
 // per box id: partners at [off[id], off[id+1]) ascending, self[] = id; off has n+1
 cudaError_t lbvh_partners_async(Lbvh& t, uint32_t* off, uint32_t* partners, uint32_t* self, uint64_t cap,
                                 cudaStream_t st);
-// ascending unique pairs (i < j) of any per-box partner lists (CSR, partners
-// ascending per box); counts n, pos n+1 (pos[n] = count), scan scratch
-cudaError_t csr_unique_pairs_async(uint32_t n, const uint32_t* off, const uint32_t* partners, uint64_t partners_cap,
-                                   uint32_t* counts, uint32_t* scan_scratch, uint32_t* pos, unsigned long long* out,
-                                   uint64_t cap, cudaStream_t st);
-// ascending unique pairs (i < j) from the partner lists; pos has n+1 (pos[n] = count)
-cudaError_t lbvh_unique_pairs_async(Lbvh& t, const uint32_t* off, const uint32_t* partners, uint64_t partners_cap,
-                                    uint32_t* pos, unsigned long long* out, uint64_t cap, cudaStream_t st);
+// ascending unique pairs (i < j); off: scratch of n + 1 words; d_count2[0] =
+// pairs (0 when they exceed cap: nothing is written then), [1] = error bits
+cudaError_t lbvh_unique_pairs_async(Lbvh& t, uint32_t* off, unsigned long long* out, uint64_t cap, uint32_t* d_count2,
+                                    cudaStream_t st);
 
 // ---- sweep and prune (sd_sap.cu)
 uint64_t sap_scratch_bytes(uint64_t n, uint64_t pair_cap);

@@ -13,12 +13,14 @@
 //      between equal codes broken by the leaf index;
 //   5. refit in ONE launch: every leaf climbs towards the root and the
 //      second thread to reach a node (atomic visit counter) writes its box;
-//   6. per-leaf stack traversal, in two passes (count, then write after an
-//      exclusive scan) so every body gets a compact, deterministic partner
-//      list, sorted by partner id in the writing thread.
+//   6. stack traversal, a few lanes to a leaf: they take as many nodes off the
+//      leaf's stack at a time.  Partner lists (both ways, per body, a count
+//      pass and a write pass) or the unique pairs (each found once, from the
+//      leaf that comes first along the curve; sd_pairs.cuh).
 // The pair set is the exact set of overlapping closed boxes, independent of
 // the tree's shape.
 #include "sd_common.cuh"
+#include "sd_pairs.cuh"
 
 #include <utility>
 
@@ -29,6 +31,7 @@ namespace {
 constexpr int kLbvhThreads = 256;
 constexpr uint32_t kLeaf = 0x80000000u;
 constexpr int kStack = 64;  // Karras tree depth <= 32 code bits + 32 index bits
+static_assert(kLbvhFirst >= (int)kPairKeep, "the sink keeps its partners in Lbvh::first");
 
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 8;
@@ -117,12 +120,17 @@ __global__ void bounds_partial_kernel(const float4* __restrict__ lo, const float
     if (threadIdx.x < 6) part[6 * blockIdx.x + threadIdx.x] = s[threadIdx.x][0];
 }
 
+// One warp per bound (a thread per bound that reads the partials one after
+// the other took 20 us).
 __global__ void bounds_final_kernel(const float* __restrict__ part, uint32_t nb, float* __restrict__ bounds) {
-    if (threadIdx.x >= 6) return;
-    const int k = threadIdx.x;
+    const uint32_t k = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     float m = k < 3 ? INFINITY : -INFINITY;
-    for (uint32_t b = 0; b < nb; ++b) m = k < 3 ? fminf(m, part[6 * b + k]) : fmaxf(m, part[6 * b + k]);
-    bounds[k] = m;
+    for (uint32_t b = lane; b < nb; b += 32) m = k < 3 ? fminf(m, part[6 * b + k]) : fmaxf(m, part[6 * b + k]);
+    for (int o = 16; o > 0; o >>= 1) {
+        const float x = __shfl_xor_sync(0xffffffffu, m, o);
+        m = k < 3 ? fminf(m, x) : fmaxf(m, x);
+    }
+    if (lane == 0) bounds[k] = m;
 }
 
 // --------------------------------------------------------------- Morton
@@ -198,6 +206,11 @@ __global__ void build_kernel(const uint32_t* __restrict__ keys, int n, int2* __r
 
 __device__ __forceinline__ float4 ldcg4(const float4* p) { return __ldcg(p); }
 
+// Orders a node's box before the arrival that announces it, and the sibling's
+// arrival before the reads of its box (release and acquire are enough here;
+// __threadfence is sequentially consistent and slower).
+__device__ __forceinline__ void fence_acq_rel() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+
 // A child reference is a leaf below n or an internal node below n - 1.
 __device__ __forceinline__ bool child_ok(int c, int n) {
     return (c & kLeaf) ? (c & ~kLeaf) < n : (c >= 0 && c < n - 1);
@@ -205,9 +218,13 @@ __device__ __forceinline__ bool child_ok(int c, int n) {
 
 // Bottom-up boxes: the last of a node's two children to finish computes
 // the node's box and writes the node's record -- both children's boxes,
-// each lower corner's w lane holding the child reference -- which the
-// traversal reads in one 64-byte piece instead of the children's indices
-// and then their boxes.
+// each lower corner's w lane holding the child reference and each upper
+// corner's the last leaf below that child -- which the traversal reads in one
+// 64-byte piece instead of the children's indices and then their boxes.
+// A chain of about 24 levels at 2.7 us each (fence, atomic, two boxes from
+// L2): 64 us at 300,001 leaves.  Joining the nodes that lie within a block's
+// 512 leaves in shared memory takes nothing off it (66 us): the paths along
+// the blocks' edges are as deep.
 __global__ void refit_kernel(int n, const uint32_t* __restrict__ vals, const float4* __restrict__ lo,
                              const float4* __restrict__ hi, float4* leaf_lo, float4* leaf_hi, float4* node_lo,
                              float4* node_hi, const int2* __restrict__ children, const int32_t* __restrict__ parent,
@@ -217,167 +234,179 @@ __global__ void refit_kernel(int n, const uint32_t* __restrict__ vals, const flo
     const uint32_t id = vals[k];
     leaf_lo[k] = lo[id];
     leaf_hi[k] = hi[id];
-    __threadfence();
+    fence_acq_rel();
     int p = n > 1 ? parent[(n - 1) + k] : -1;
     for (int level = 0; p >= 0; ++level) {
         if (level > 2 * kStack || p >= n - 1) {  // a malformed tree: report, never loop or stray
             atomicOr(status, kErrBadInput);
             return;
         }
-        if (atomicAdd(&visit[p], 1u) == 0u) return;  // the sibling subtree is not done yet
-        __threadfence();
         const int2 c = children[p];
+        const int up = parent[p];
+        if (atomicAdd(&visit[p], 1u) == 0u) return;  // the sibling subtree is not done yet
+        fence_acq_rel();
         if (!child_ok(c.x, n) || !child_ok(c.y, n)) {
             atomicOr(status, kErrBadInput);
             return;
         }
+        const int l = c.x & ~kLeaf, r = c.y & ~kLeaf;
         float4 a0, a1, b0, b1;
-        if (c.x & kLeaf) { a0 = ldcg4(leaf_lo + (c.x & ~kLeaf)); a1 = ldcg4(leaf_hi + (c.x & ~kLeaf)); }
-        else { a0 = ldcg4(node_lo + c.x); a1 = ldcg4(node_hi + c.x); }
-        if (c.y & kLeaf) { b0 = ldcg4(leaf_lo + (c.y & ~kLeaf)); b1 = ldcg4(leaf_hi + (c.y & ~kLeaf)); }
-        else { b0 = ldcg4(node_lo + c.y); b1 = ldcg4(node_hi + c.y); }
+        if (c.x & kLeaf) { a0 = ldcg4(leaf_lo + l); a1 = ldcg4(leaf_hi + l); }
+        else { a0 = ldcg4(node_lo + l); a1 = ldcg4(node_hi + l); }
+        if (c.y & kLeaf) { b0 = ldcg4(leaf_lo + r); b1 = ldcg4(leaf_hi + r); }
+        else { b0 = ldcg4(node_lo + r); b1 = ldcg4(node_hi + r); }
+        // a left child's last leaf is the index in its own reference (the split)
+        const float end_a = __int_as_float(l), end_b = (c.y & kLeaf) ? __int_as_float(r) : b1.w;
         node_lo[p] = make_float4(fminf(a0.x, b0.x), fminf(a0.y, b0.y), fminf(a0.z, b0.z), 0.f);
-        node_hi[p] = make_float4(fmaxf(a1.x, b1.x), fmaxf(a1.y, b1.y), fmaxf(a1.z, b1.z), 0.f);
+        node_hi[p] = make_float4(fmaxf(a1.x, b1.x), fmaxf(a1.y, b1.y), fmaxf(a1.z, b1.z), end_b);
         rec[4 * (size_t)p + 0] = make_float4(a0.x, a0.y, a0.z, __int_as_float(c.x));
-        rec[4 * (size_t)p + 1] = a1;
+        rec[4 * (size_t)p + 1] = make_float4(a1.x, a1.y, a1.z, end_a);
         rec[4 * (size_t)p + 2] = make_float4(b0.x, b0.y, b0.z, __int_as_float(c.y));
-        rec[4 * (size_t)p + 3] = b1;
-        __threadfence();
-        p = parent[p];
+        rec[4 * (size_t)p + 3] = make_float4(b1.x, b1.y, b1.z, end_b);
+        fence_acq_rel();
+        p = up;
     }
 }
 
-// Traversal of leaf k (sorted position) against the tree.  WRITE == false:
-// count[id] = number of partners, and the first kLbvhFirst partners found
-// into first[k * kLbvhFirst ...].  WRITE == true: partners of body id at
-// [off[id], off[id+1]), ascending, and self[] of each entry -- sorted from
-// first[] when the counting pass kept them all, else found by a second
-// traversal.
-template <bool WRITE>
-__global__ void query_kernel(int n, const uint32_t* __restrict__ vals, const float4* __restrict__ leaf_lo,
-                             const float4* __restrict__ leaf_hi, const float4* __restrict__ rec,
-                             uint32_t* __restrict__ count, const uint32_t* __restrict__ off,
-                             uint32_t* __restrict__ partners, uint32_t* __restrict__ self, uint64_t cap,
-                             uint32_t* __restrict__ first, uint32_t* __restrict__ status) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    const uint32_t id = vals[k];
+// What a traversal does with the pairs it finds.
+enum QueryMode {
+    kCount,    // count[id], and the first kLbvhFirst partners into first[k * kLbvhFirst ...]
+    kWrite,    // partners of body id at [off[id], off[id + 1]), ascending, and self[] of each entry
+    kPairs,    // each pair once, into the sink
+    kRefill    // each pair once, for the sink's boxes that have more than it kept
+};
+
+constexpr int kQueryThreads = 128;
+
+struct QueryOut {
+    uint32_t* count;
+    const uint32_t* off;
+    uint32_t* partners;
+    uint32_t* self;
+    uint64_t cap;
+    uint32_t* first;
+};
+
+// G lanes walk the tree for one leaf: each takes a node off the leaf's stack,
+// reads its record and tests both children's boxes; the lanes' finds are
+// pushed or listed together, in lane order.  A walk is some 60 visits, each a
+// load that depends on the one before when a thread makes it alone; down the
+// tree only one or two nodes are open, near the leaves many.
+// Latency bounds it: 300,001 boxes' pairs 110 us with two lanes (one lane and
+// both directions of every pair, twice: 2 x 100 us).  One warp walking for 32
+// neighbouring leaves under their common box took seven times as long: where
+// the curve jumps, that box covers much of the domain.
+template <int MODE, int G>
+__global__ void __launch_bounds__(kQueryThreads)
+query_kernel(int n, const uint32_t* __restrict__ vals, const float4* __restrict__ leaf_lo,
+             const float4* __restrict__ leaf_hi, const float4* __restrict__ rec, QueryOut q, PairSink sink,
+             uint32_t* __restrict__ status) {
+    constexpr bool kUnique = MODE == kPairs || MODE == kRefill;
+    constexpr int kLeaves = kQueryThreads / G, kDepth = kStack + 2 * G;
+    __shared__ int s_stack[kDepth][kLeaves];
+    const uint32_t lane = threadIdx.x & 31u, sub = threadIdx.x % G, group = lane & ~(uint32_t)(G - 1);
+    const uint32_t below = (1u << sub) - 1u;
+    const int at = threadIdx.x / G, k = (int)blockIdx.x * kLeaves + at;
+    if (MODE == kRefill && !sink_refill(sink)) return;
+    bool walk = k < n;
+    const uint32_t id = walk ? vals[k] : 0u;
     uint32_t c = 0;
-    const uint32_t base = WRITE ? off[id] : 0u;
-    const uint32_t lim = WRITE ? off[id + 1] : 0u;
-    if constexpr (WRITE) {
-      if (lim - base <= (uint32_t)kLbvhFirst) {
-        if ((uint64_t)lim > cap) {
+    const uint32_t base = MODE == kWrite && walk ? q.off[id] : 0u, lim = MODE == kWrite && walk ? q.off[id + 1] : 0u;
+    if constexpr (MODE == kWrite) {
+        if (walk && (uint64_t)lim > q.cap) {
             atomicOr(status, kErrPairOverflow);
-            return;
-        }
-        // the partners the counting pass kept: sorted in registers (a
-        // network over kLbvhFirst values; ids are distinct, so the order
-        // is the ascending one)
-        uint32_t v[kLbvhFirst];
-#pragma unroll
-        for (int i = 0; i < kLbvhFirst; ++i) v[i] = (uint32_t)i < lim - base ? first[(size_t)k * kLbvhFirst + i] : 0xffffffffu;
-#pragma unroll
-        for (int a = 0; a < kLbvhFirst; ++a)
-#pragma unroll
-            for (int b = (a & 1); b + 1 < kLbvhFirst; b += 2)
-                if (v[b] > v[b + 1]) {
-                    const uint32_t t = v[b];
-                    v[b] = v[b + 1];
-                    v[b + 1] = t;
-                }
-#pragma unroll
-        for (int i = 0; i < kLbvhFirst; ++i)
-            if ((uint32_t)i < lim - base) {
-                partners[base + i] = v[i];
-                self[base + i] = id;
+            walk = false;
+        } else if (walk && lim - base <= (uint32_t)kLbvhFirst) {
+            // the partners the counting pass kept, each lane placing its share
+            // by counting the smaller ones (ids are distinct)
+            const uint32_t m = lim - base;
+            const uint32_t* list = q.first + (size_t)k * kLbvhFirst;
+            for (uint32_t i = sub; i < m; i += G) {
+                const uint32_t v = list[i];
+                uint32_t r = 0;
+                for (uint32_t j = 0; j < m; ++j) r += list[j] < v;
+                q.partners[base + r] = v;
+                q.self[base + i] = id;
             }
-        return;
-      }
+            walk = false;
+        }
     }
-    const float4 qlo = leaf_lo[k], qhi = leaf_hi[k];
-    if (n > 1) {
-        int stack[kStack];
-        int sp = 0;
-        stack[sp++] = 0;
-        while (sp > 0) {
-            const int node = stack[--sp];
-            // the node's record: both children's boxes and references
-            const float4 r0 = rec[4 * (size_t)node + 0], r1 = rec[4 * (size_t)node + 1];
-            const float4 r2 = rec[4 * (size_t)node + 2], r3 = rec[4 * (size_t)node + 3];
-            const int cx = __float_as_int(r0.w), cy = __float_as_int(r2.w);
-            if (!child_ok(cx, n) || !child_ok(cy, n)) {
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 qlo = walk ? leaf_lo[k] : zero, qhi = walk ? leaf_hi[k] : zero;
+    int sp = walk && n > 1 ? 1 : 0;
+    if (sp && sub == 0) s_stack[0][at] = 0;
+    __syncwarp();
+    for (int trips = 0; __any_sync(0xffffffffu, sp > 0); ++trips) {
+        if (trips > 2 * n + 64) {  // more visits than a tree has nodes: malformed, never loop
+            if (lane == 0) atomicOr(status, kErrBadInput);
+            break;
+        }
+        // G nodes while their children fit, else one: the stack then grows by
+        // one entry a level at most
+        const int m = sp <= kStack - 2 * G ? min(sp, G) : 1;
+        const bool mine = (int)sub < m;
+        const int node = mine ? s_stack[sp - 1 - (int)sub][at] : 0;
+        sp -= m;
+        __syncwarp();
+        float4 r[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) r[u] = mine ? __ldg(&rec[4 * (size_t)node + u]) : zero;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const float4 blo = r[2 * h], bhi = r[2 * h + 1];
+            const int x = __float_as_int(blo.w), j = x & ~kLeaf;
+            bool go = mine;
+            if (go && !child_ok(x, n)) {
                 atomicOr(status, kErrBadInput);
-                continue;
+                go = false;
             }
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int x = h ? cy : cx;
-                const float4 blo = h ? r2 : r0, bhi = h ? r3 : r1;
-                if (x & kLeaf) {
-                    const int j = x & ~kLeaf;
-                    if (j == k || !box_overlap(qlo, qhi, blo, bhi)) continue;
-                    if constexpr (WRITE) {
-                        const uint32_t e = base + c;
-                        if (e < lim && (uint64_t)e < cap) partners[e] = vals[j];
-                    } else if (c < (uint32_t)kLbvhFirst) {
-                        first[(size_t)k * kLbvhFirst + c] = vals[j];
-                    }
-                    ++c;
-                } else if (box_overlap(qlo, qhi, blo, bhi)) {
-                    if (sp < kStack) stack[sp++] = x;
-                    else atomicOr(status, kErrPairOverflow);
+            // (pairs once: only leaves behind this one)
+            go = go && box_overlap(qlo, qhi, blo, bhi) && (!kUnique || __float_as_int(bhi.w) > k);
+            const bool leaf = go && (x & kLeaf) && j != k, inner = go && !(x & kLeaf);
+            const uint32_t mi = (__ballot_sync(0xffffffffu, inner) >> group) & ((1u << G) - 1u);
+            if (inner) {
+                const int to = sp + __popc(mi & below);
+                if (to < kDepth) s_stack[to][at] = x;
+                else atomicOr(status, kErrPairOverflow);
+            }
+            sp = min(sp + __popc(mi), kDepth);
+            if constexpr (kUnique) {
+                if (leaf) {
+                    if (MODE == kPairs) sink_pair(sink, id, vals[j]);
+                    else sink_pair_again(sink, id, vals[j]);
                 }
+            } else {
+                const uint32_t ml = (__ballot_sync(0xffffffffu, leaf) >> group) & ((1u << G) - 1u);
+                if (leaf) {
+                    const uint32_t to = c + (uint32_t)__popc(ml & below);
+                    if (MODE == kCount) {
+                        if (to < (uint32_t)kLbvhFirst) q.first[(size_t)k * kLbvhFirst + to] = vals[j];
+                    } else if (base + to < lim) {
+                        q.partners[base + to] = vals[j];
+                    }
+                }
+                c += (uint32_t)__popc(ml);
             }
         }
+        __syncwarp();
     }
-    if constexpr (!WRITE) {
-        count[id] = c;
-    } else {
-        if ((uint64_t)lim > cap) {
-            atomicOr(status, kErrPairOverflow);
-            return;
-        }
+    if constexpr (MODE == kCount) {
+        if (walk && sub == 0) q.count[id] = c;
+    }
+    if constexpr (MODE == kWrite) {
+        __syncwarp();  // (the group's lanes wrote the list)
+        if (!walk || sub != 0) return;
         // sort the body's partner list ascending (insertion sort: lists are short)
         for (uint32_t e = base + 1; e < lim; ++e) {
-            const uint32_t x = partners[e];
+            const uint32_t x = q.partners[e];
             uint32_t m = e;
-            while (m > base && partners[m - 1] > x) {
-                partners[m] = partners[m - 1];
+            while (m > base && q.partners[m - 1] > x) {
+                q.partners[m] = q.partners[m - 1];
                 --m;
             }
-            partners[m] = x;
+            q.partners[m] = x;
         }
-        for (uint32_t e = base; e < lim; ++e) self[e] = id;
-    }
-}
-
-// Unique pairs (i < j) of the partner lists, ascending u64.
-__global__ void upper_count_kernel(uint32_t n, const uint32_t* __restrict__ off, const uint32_t* __restrict__ partners,
-                                   uint32_t* __restrict__ cnt, uint64_t partners_cap) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    uint32_t c = 0;
-    if ((uint64_t)off[n] > partners_cap) {  // overflowed lists are reported, not read
-        cnt[i] = 0;
-        return;
-    }
-    for (uint32_t e = off[i]; e < off[i + 1]; ++e) c += partners[e] > i;
-    cnt[i] = c;
-}
-
-__global__ void upper_write_kernel(uint32_t n, const uint32_t* __restrict__ off, const uint32_t* __restrict__ partners,
-                                   const uint32_t* __restrict__ pos, unsigned long long* __restrict__ out,
-                                   uint64_t cap, uint64_t partners_cap) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || (uint64_t)off[n] > partners_cap) return;
-    uint32_t w = pos[i];
-    for (uint32_t e = off[i]; e < off[i + 1]; ++e) {
-        const uint32_t j = partners[e];
-        if (j > i) {
-            if (w < cap) out[w] = ((unsigned long long)i << 32) | j;
-            ++w;
-        }
+        for (uint32_t e = base; e < lim; ++e) q.self[e] = id;
     }
 }
 
@@ -456,7 +485,7 @@ cudaError_t lbvh_morton_async(Lbvh& t, const float4* lo, const float4* hi, cudaS
     if (n == 0) return cudaSuccess;
     const uint32_t nb = bounds_blocks(n);
     bounds_partial_kernel<<<nb, kLbvhThreads, 0, st>>>(lo, hi, n, t.bound_part);
-    bounds_final_kernel<<<1, 32, 0, st>>>(t.bound_part, nb, t.bounds);
+    bounds_final_kernel<<<1, 6 * 32, 0, st>>>(t.bound_part, nb, t.bounds);
     morton_kernel<<<grid_for(n, kLbvhThreads), kLbvhThreads, 0, st>>>(lo, hi, n, t.bounds, t.keys, t.vals);
     return cudaGetLastError();
 }
@@ -499,34 +528,51 @@ static int g_lbvh_rebuild = 16;
 void lbvh_set_rebuild_every(int k) { g_lbvh_rebuild = k < 1 ? 1 : k; }
 int lbvh_rebuild_every() { return g_lbvh_rebuild; }
 
+// Below this many leaves four lanes walk for one (too few leaves to fill the
+// chip with two: 20,000 boxes 186 us the pairs against 198, 32,768 hulls 3144
+// us ten steps against 3278), from it two (100,000 boxes 232 against 238,
+// 300,001 315 against 336, 2,000,000 1184 against 1425).  One lane is behind
+// everywhere (215 us, 249, 367, 1476), and eight too (3202 us the hulls).
+constexpr uint32_t kWideLeaves = 1u << 16;
+
+template <int MODE>
+static void launch_query(const Lbvh& t, const QueryOut& q, const PairSink& sink, cudaStream_t st) {
+    const int n = (int)t.n;
+    const auto go = [&](auto kernel, int lanes) {
+        kernel<<<grid_for(t.n, kQueryThreads / lanes), kQueryThreads, 0, st>>>(n, t.svals, t.leaf_lo, t.leaf_hi, t.rec, q,
+                                                                              sink, t.status);
+    };
+    if (t.n < kWideLeaves) go(query_kernel<MODE, 4>, 4);
+    else go(query_kernel<MODE, 2>, 2);
+}
+
 cudaError_t lbvh_partners_async(Lbvh& t, uint32_t* off, uint32_t* partners, uint32_t* self, uint64_t cap,
                                 cudaStream_t st) {
     const uint32_t n = t.n;
     if (n == 0) return cudaMemsetAsync(off, 0, 4, st);
-    query_kernel<false><<<grid_for(n, kLbvhThreads), kLbvhThreads, 0, st>>>(
-        (int)n, t.svals, t.leaf_lo, t.leaf_hi, t.rec, t.counts, nullptr, nullptr, nullptr, 0, t.first, t.status);
+    const QueryOut q{t.counts, off, partners, self, cap, t.first};
+    launch_query<kCount>(t, q, PairSink{}, st);
     cudaError_t e = scan_exclusive_async(t.counts, off, n, t.scan_scratch, st);
     if (e != cudaSuccess) return e;
-    query_kernel<true><<<grid_for(n, kLbvhThreads), kLbvhThreads, 0, st>>>(
-        (int)n, t.svals, t.leaf_lo, t.leaf_hi, t.rec, nullptr, off, partners, self, cap, t.first, t.status);
+    launch_query<kWrite>(t, q, PairSink{}, st);
     return cudaGetLastError();
 }
 
-cudaError_t csr_unique_pairs_async(uint32_t n, const uint32_t* off, const uint32_t* partners, uint64_t partners_cap,
-                                   uint32_t* counts, uint32_t* scan_scratch, uint32_t* pos, unsigned long long* out,
-                                   uint64_t cap, cudaStream_t st) {
-    if (n == 0) return cudaMemsetAsync(pos, 0, 4, st);
-    upper_count_kernel<<<grid_for(n, kLbvhThreads), kLbvhThreads, 0, st>>>(n, off, partners, counts, partners_cap);
-    cudaError_t e = scan_exclusive_async(counts, pos, n, scan_scratch, st);
-    if (e != cudaSuccess) return e;
-    upper_write_kernel<<<grid_for(n, kLbvhThreads), kLbvhThreads, 0, st>>>(n, off, partners, pos, out, cap,
-                                                                           partners_cap);
-    return cudaGetLastError();
-}
-
-cudaError_t lbvh_unique_pairs_async(Lbvh& t, const uint32_t* off, const uint32_t* partners, uint64_t partners_cap,
-                                    uint32_t* pos, unsigned long long* out, uint64_t cap, cudaStream_t st) {
-    return csr_unique_pairs_async(t.n, off, partners, partners_cap, t.counts, t.scan_scratch, pos, out, cap, st);
+cudaError_t lbvh_unique_pairs_async(Lbvh& t, uint32_t* off, unsigned long long* out, uint64_t cap, uint32_t* d_count2,
+                                    cudaStream_t st) {
+    const uint32_t n = t.n;
+    cudaError_t e;
+    if (n == 0) return cudaMemsetAsync(d_count2, 0, 8, st);
+    // t.keys: the codes are used up, the cursors take their place
+    const PairSink sink{t.counts, t.first, t.status + 1, off, t.keys, out, n, cap};
+    if ((e = cudaMemsetAsync(t.counts, 0, 4 * (size_t)n, st)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(t.keys, 0, 4 * (size_t)n, st)) != cudaSuccess) return e;
+    launch_query<kPairs>(t, QueryOut{}, sink, st);
+    if ((e = scan_exclusive_async(t.counts, off, n, t.scan_scratch, st)) != cudaSuccess) return e;
+    launch_query<kRefill>(t, QueryOut{}, sink, st);
+    pairs_write_kernel<<<grid_for(n, kLbvhThreads), kLbvhThreads, 0, st>>>(sink, d_count2, t.status);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    return cudaMemcpyAsync(d_count2 + 1, t.status, 4, cudaMemcpyDeviceToDevice, st);
 }
 
 }  // namespace sd

@@ -17,18 +17,24 @@
 //  * sap_pairs: an exact broad phase -- every pair of overlapping closed
 //    boxes -- by sorting the lower x extents (order-preserving float keys,
 //    so negative coordinates sort correctly) and sweeping each box forward
-//    while the next lower x is within its upper x, then per-box partner
-//    lists (sorted) and the ascending unique pair list.  The sweep is binned
-//    like the reference's grid prototype (src/engine/testSAP.cu:341-438,
-//    objects mapped to y-z cells, one x sweep per cell): a y-z grid of
-//    columns at least as wide as the largest box, each box entered in the
-//    (at most 2 x 2) columns it touches, entries stably sorted by column so
-//    that each column keeps the x order, and each entry swept forward
-//    inside its column only.  A pair sharing several columns is reported in
-//    the column of its overlap's lower y-z corner, so every pair is found
-//    once, by the same tests as the unbinned sweep: the same pair set.
+//    while the next lower x is within its upper x.  The sweep is binned like
+//    the reference's grid prototype (src/engine/testSAP.cu:341-438, objects
+//    mapped to y-z cells, one x sweep per cell): a y-z grid of columns at
+//    least as wide as the largest box, each box entered in the (at most 2 x 2)
+//    columns it touches, entries stably sorted by column so that each column
+//    keeps the x order, and each entry swept forward inside its column only.
+//    A pair sharing several columns is reported in the column of its overlap's
+//    lower y-z corner, so every pair is found once, by the same tests as the
+//    unbinned sweep: the same pair set, listed by sd_pairs.cuh.
+//    Measured, 2,000,000 boxes of one size (0.9 entries swept per test that
+//    passes x): 612 us in all; sweep 219 (dependent loads: key, index, box),
+//    seven radix passes 175, gather into x order 45, entries 42, list 29 + 18,
+//    bounds 19, scans 30.  It was 1174: four entries for every box whether used
+//    or not, boxes of 48 bytes gathered through two indices, and the sweep
+//    twice, once to count.
 #include "sd_common.cuh"
 #include "sd_engine_impl.h"
+#include "sd_pairs.cuh"
 
 namespace sd {
 
@@ -97,38 +103,11 @@ __global__ void sweep_ref_kernel(uint32_t n, const float* __restrict__ upperx, c
     for (int k = 0; k < kRefPadding / 4; ++k) out[k] = make_int4(row[4 * k], row[4 * k + 1], row[4 * k + 2], row[4 * k + 3]);
 }
 
-__global__ void gather_sorted_kernel(uint32_t n, const uint32_t* __restrict__ svals, const float4* __restrict__ lo,
-                                     const float4* __restrict__ hi, float4* __restrict__ slo, float4* __restrict__ shi) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    const uint32_t i = svals[k];
-    slo[k] = lo[i];
-    shi[k] = hi[i];
-}
-
-__global__ void sort_segments_kernel(uint32_t n, const uint32_t* __restrict__ off, uint32_t* __restrict__ partners,
-                                     uint64_t cap) {
-    const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= n) return;
-    const uint32_t base = off[b], lim = off[b + 1];
-    if ((uint64_t)lim > cap) return;
-    for (uint32_t e = base + 1; e < lim; ++e) {
-        const uint32_t x = partners[e];
-        uint32_t m = e;
-        while (m > base && partners[m - 1] > x) {
-            partners[m] = partners[m - 1];
-            --m;
-        }
-        partners[m] = x;
-    }
-}
-
 inline size_t al256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // ---- the column grid of the binned sweep
-constexpr uint32_t kColSentinel = 0xffffu;  // an unused entry (columns are < 255 * 255)
-constexpr int kMaxCols = 255;               // per axis
-constexpr int kSlots = 4;                   // entries per box: at most 2 x 2 columns
+constexpr int kMaxCols = 255;  // per axis
+constexpr int kSlots = 4;      // most entries per box: 2 x 2 columns
 
 struct SapGrid {
     float y0, z0, inv;  // column of v: floor((v - v0) * inv), clamped
@@ -145,41 +124,82 @@ __device__ __forceinline__ float key_float(uint32_t k) {
 }
 
 // Bounds of the boxes in y and z and their largest y or z extent, as
-// ordered keys (minima stored complemented, so every word is a maximum;
-// the words start at 0).  NaN coordinates are skipped.
-__global__ void sap_bounds_kernel(uint32_t n, const float4* __restrict__ lo, const float4* __restrict__ hi,
-                                  uint32_t* __restrict__ w) {
-    uint32_t m[5] = {0u, 0u, 0u, 0u, 0u};
+// ordered keys (minima stored complemented, so every word is a maximum; the
+// words start at 0), and the sum and number of the extents.  NaN coordinates
+// are skipped.  Also the sort keys of the lower x extents.
+struct SapBounds {
+    uint32_t w[5], count;
+    double sum;
+};
+
+constexpr int kBoundBlocks = 152 * 4;
+
+__global__ void __launch_bounds__(kSapThreads)
+sap_bounds_kernel(uint32_t n, const float4* __restrict__ lo, const float4* __restrict__ hi, SapBounds* __restrict__ out,
+                  uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
+    __shared__ uint32_t s_w[5], s_count;
+    __shared__ double s_sum;
+    if (threadIdx.x < 5) s_w[threadIdx.x] = 0u;
+    if (threadIdx.x == 0) {
+        s_count = 0u;
+        s_sum = 0.0;
+    }
+    __syncthreads();
+    uint32_t m[5] = {0u, 0u, 0u, 0u, 0u}, count = 0;
+    float sum = 0.0f;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float4 a = lo[i], b = hi[i];
+        keys[i] = float_key(a.x);
+        vals[i] = i;
         const float ly = fminf(a.y, b.y), hy = fmaxf(a.y, b.y), lz = fminf(a.z, b.z), hz = fmaxf(a.z, b.z);
         const float ey = hy - ly, ez = hz - lz;
         if (ly == ly) {
             m[0] = max(m[0], ~float_key(ly));
             m[1] = max(m[1], float_key(hy));
         }
-        if (ey == ey) m[4] = max(m[4], float_key(ey));
         if (lz == lz) {
             m[2] = max(m[2], ~float_key(lz));
             m[3] = max(m[3], float_key(hz));
         }
+        if (ey == ey) m[4] = max(m[4], float_key(ey));
         if (ez == ez) m[4] = max(m[4], float_key(ez));
+        if (ey + ez < INFINITY) {
+            sum += ey + ez;
+            count += 2;
+        }
     }
 #pragma unroll
     for (int k = 0; k < 5; ++k) {
         const uint32_t r = __reduce_max_sync(0xffffffffu, m[k]);
-        if ((threadIdx.x & 31) == 0 && r) atomicMax(&w[k], r);
+        if (lane_id() == 0 && r) atomicMax(&s_w[k], r);
+    }
+    const uint32_t c = __reduce_add_sync(0xffffffffu, count);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane_id() == 0 && c) {
+        atomicAdd(&s_count, c);
+        atomicAdd(&s_sum, (double)sum);
+    }
+    __syncthreads();
+    if (threadIdx.x < 5 && s_w[threadIdx.x]) atomicMax(&out->w[threadIdx.x], s_w[threadIdx.x]);
+    if (threadIdx.x == 0 && s_count) {
+        atomicAdd(&out->count, s_count);
+        atomicAdd(&out->sum, s_sum);
     }
 }
 
 // Columns at least 1.0001 x the largest extent wide (so a box spans at most
-// two columns per axis, rounding included) and at most kMaxCols per axis.
-__global__ void sap_grid_kernel(const uint32_t* __restrict__ w, SapGrid* __restrict__ g) {
+// two columns per axis, rounding included), twice the mean extent (boxes of
+// one size then take 2.25 entries each instead of 4, for as many tests), and
+// at most kMaxCols per axis.  The width never changes the pairs.
+__device__ __forceinline__ SapGrid sap_grid(const SapBounds& b) {
     SapGrid r{0.0f, 0.0f, 0.0f, 1, 1};
-    if (w[0] && w[1] && w[2] && w[3]) {
-        const float y0 = key_float(~w[0]), y1 = key_float(w[1]), z0 = key_float(~w[2]), z1 = key_float(w[3]);
-        const float ext = w[4] ? key_float(w[4]) : 0.0f;
-        const float c = fmaxf(fmaxf(ext * 1.0001f, (y1 - y0) / (float)kMaxCols), (z1 - z0) / (float)kMaxCols);
+    if (b.w[0] && b.w[1] && b.w[2] && b.w[3]) {
+        const float y0 = key_float(~b.w[0]), y1 = key_float(b.w[1]), z0 = key_float(~b.w[2]), z1 = key_float(b.w[3]);
+        const float ext = b.w[4] ? key_float(b.w[4]) : 0.0f;
+        const float mean = b.count ? (float)(b.sum / b.count) : 0.0f;
+        float c = fmaxf(fmaxf(ext * 1.0001f, (y1 - y0) / (float)kMaxCols), (z1 - z0) / (float)kMaxCols);
+        if (mean > 0.0f) c = fmaxf(c, 2.0f * mean);
         if (c > 0.0f && c < INFINITY) {
             r.y0 = y0;
             r.z0 = z0;
@@ -188,77 +208,79 @@ __global__ void sap_grid_kernel(const uint32_t* __restrict__ w, SapGrid* __restr
             r.gz = min(kMaxCols, max(1, (int)fminf((z1 - z0) * r.inv, 1e6f) + 1));
         }
     }
-    *g = r;
+    return r;
 }
 
-// Per x-sorted box k: its columns (y-major) in entries 4k .. 4k+3, unused
-// entries keyed kColSentinel; values are k.
-__global__ void sap_entries_kernel(uint32_t n, const float4* __restrict__ slo, const float4* __restrict__ shi,
-                                   const SapGrid* __restrict__ grid, uint32_t* __restrict__ keys,
-                                   uint32_t* __restrict__ vals, uint32_t* __restrict__ status) {
+// Columns of a box, y-major.
+struct SapSpan {
+    int y0, y1, z0, z1;
+};
+__device__ __forceinline__ SapSpan sap_span(const SapGrid& g, float4 a, float4 b) {
+    return SapSpan{sap_col(fminf(a.y, b.y), g.y0, g.inv, g.gy), sap_col(fmaxf(a.y, b.y), g.y0, g.inv, g.gy),
+                   sap_col(fminf(a.z, b.z), g.z0, g.inv, g.gz), sap_col(fmaxf(a.z, b.z), g.z0, g.inv, g.gz)};
+}
+
+// The boxes in x order, 32 bytes each with the id in the lower corner's w
+// lane, and the number of columns each touches.
+__global__ void sap_gather_kernel(uint32_t n, const uint32_t* __restrict__ svals, const float4* __restrict__ lo,
+                                  const float4* __restrict__ hi, const SapBounds* __restrict__ bounds,
+                                  float4* __restrict__ box, uint32_t* __restrict__ count, uint32_t* __restrict__ status) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
-    const SapGrid g = *grid;
-    const float4 a = slo[k], b = shi[k];
-    const int y0 = sap_col(fminf(a.y, b.y), g.y0, g.inv, g.gy), y1 = sap_col(fmaxf(a.y, b.y), g.y0, g.inv, g.gy);
-    const int z0 = sap_col(fminf(a.z, b.z), g.z0, g.inv, g.gz), z1 = sap_col(fmaxf(a.z, b.z), g.z0, g.inv, g.gz);
-    if (y1 - y0 > 1 || z1 - z0 > 1) atomicOr(status, kErrBadInput);  // excluded by the column width
-    int t = 0;
-    for (int y = y0; y <= y0 + 1; ++y)
-        for (int z = z0; z <= z0 + 1; ++z) {
-            const bool on = y <= y1 && z <= z1;
-            keys[(size_t)kSlots * k + t] = on ? (uint32_t)(y * g.gz + z) : kColSentinel;
-            vals[(size_t)kSlots * k + t] = k;
-            ++t;
+    const SapGrid g = sap_grid(*bounds);
+    const uint32_t id = svals[k];
+    const float4 a = lo[id], b = hi[id];
+    box[2 * (size_t)k] = make_float4(a.x, a.y, a.z, __uint_as_float(id));
+    box[2 * (size_t)k + 1] = b;
+    const SapSpan s = sap_span(g, a, b);
+    if (s.y1 - s.y0 > 1 || s.z1 - s.z0 > 1) atomicOr(status, kErrBadInput);  // excluded by the column width
+    count[k] = (uint32_t)((min(s.y1 - s.y0, 1) + 1) * (min(s.z1 - s.z0, 1) + 1));
+}
+
+__global__ void sap_entries_kernel(uint32_t n, const float4* __restrict__ box, const SapBounds* __restrict__ bounds,
+                                   const uint32_t* __restrict__ off, uint32_t* __restrict__ keys,
+                                   uint32_t* __restrict__ vals) {
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    const SapGrid g = sap_grid(*bounds);
+    const SapSpan s = sap_span(g, box[2 * (size_t)k], box[2 * (size_t)k + 1]);
+    uint32_t e = off[k];
+    for (int y = s.y0; y <= min(s.y1, s.y0 + 1); ++y)
+        for (int z = s.z0; z <= min(s.z1, s.z0 + 1); ++z) {
+            keys[e] = (uint32_t)(y * g.gz + z);
+            vals[e++] = k;
         }
 }
 
 // Forward sweep of entry p inside its column: entries m > p of the same
 // column with lower x <= upper x of p's box (x order within the column, the
 // first miss ends it), tested on y, z and x like the unbinned sweep; a pair
-// counts in the column of its overlap's lower y-z corner only.  COUNT: per
-// box, the number of partners (both sides, atomics on counts).  FILL:
-// partners written at off[box] + cursor (atomics), sorted later.
-template <bool FILL>
-__global__ void sweep_binned_kernel(uint32_t n_entries, const uint32_t* __restrict__ ckeys,
-                                    const uint32_t* __restrict__ cvals, const uint32_t* __restrict__ svals,
-                                    const float4* __restrict__ slo, const float4* __restrict__ shi,
-                                    const SapGrid* __restrict__ grid, uint32_t* __restrict__ counts,
-                                    const uint32_t* __restrict__ off, uint32_t* __restrict__ cursor,
-                                    uint32_t* __restrict__ partners, uint64_t cap, uint32_t* __restrict__ status) {
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+// counts in the column of its overlap's lower y-z corner only.  Neighbouring
+// threads sweep over the same few boxes, which stay in L1.
+template <bool REFILL>
+__global__ void sweep_binned_kernel(const uint32_t* __restrict__ d_entries, const uint32_t* __restrict__ ckeys,
+                                    const uint32_t* __restrict__ cvals, const float4* __restrict__ box,
+                                    const SapBounds* __restrict__ bounds, PairSink sink) {
+    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x, n_entries = *d_entries;
     if (p >= n_entries) return;
+    if (REFILL && !sink_refill(sink)) return;
     const uint32_t col = ckeys[p];
-    if (col == kColSentinel) return;
-    const SapGrid g = *grid;
-    const uint32_t k = cvals[p];
-    const float4 a0 = slo[k], a1 = shi[k];
+    const SapGrid g = sap_grid(*bounds);
+    const size_t k = cvals[p];
+    const float4 a0 = box[2 * k], a1 = box[2 * k + 1];
     const float ay = fminf(a0.y, a1.y), az = fminf(a0.z, a1.z);
-    const uint32_t i = svals[k];
     for (uint32_t q = p + 1; q < n_entries; ++q) {
         if (ckeys[q] != col) break;
-        const uint32_t m = cvals[q];
-        const float4 b0 = slo[m];
+        const size_t m = cvals[q];
+        const float4 b0 = box[2 * m];
         if (!(b0.x <= a1.x)) break;
-        const float4 b1 = shi[m];
+        const float4 b1 = box[2 * m + 1];
         if (!(b0.y <= a1.y && a0.y <= b1.y && b0.z <= a1.z && a0.z <= b1.z && a0.x <= b1.x)) continue;
         const int cy = sap_col(fmaxf(ay, fminf(b0.y, b1.y)), g.y0, g.inv, g.gy);
         const int cz = sap_col(fmaxf(az, fminf(b0.z, b1.z)), g.z0, g.inv, g.gz);
         if ((uint32_t)(cy * g.gz + cz) != col) continue;
-        const uint32_t j = svals[m];
-        if (!FILL) {
-            atomicAdd(&counts[i], 1u);
-            atomicAdd(&counts[j], 1u);
-        } else {
-            const uint32_t ei = off[i] + atomicAdd(&cursor[i], 1u);
-            const uint32_t ej = off[j] + atomicAdd(&cursor[j], 1u);
-            if ((uint64_t)ei < cap && (uint64_t)ej < cap) {
-                partners[ei] = j;
-                partners[ej] = i;
-            } else {
-                atomicOr(status, kErrPairOverflow);
-            }
-        }
+        if (REFILL) sink_pair_again(sink, __float_as_uint(a0.w), __float_as_uint(b0.w));
+        else sink_pair(sink, __float_as_uint(a0.w), __float_as_uint(b0.w));
     }
 }
 
@@ -273,11 +295,13 @@ __global__ void project_kernel(uint32_t n, const float4* __restrict__ lo, const 
 
 }  // namespace
 
+// (sd_sap_process_collisions takes its buffers from the same scratch.)
 uint64_t sap_scratch_bytes(uint64_t n, uint64_t pair_cap) {
     const uint64_t m = n ? n : 1;
-    return 4 * al256(4 * m) + al256(4 * sort_scratch_words(m, 32)) + 4 * al256(16 * m) + 3 * al256(4 * (m + 1)) +
-           al256(4 * scan_scratch_words((uint32_t)m + 1)) + al256(4 * (2 * pair_cap + 1)) + al256(16) +
-           4 * al256(4 * kSlots * m) + al256(4 * sort_scratch_words(kSlots * m, 16)) + al256(64);
+    (void)pair_cap;
+    return 4 * al256(4 * m) + al256(4 * sort_scratch_words(m, 32)) + al256(48 * m) + 4 * al256(4 * (m + 1)) +
+           al256(4 * scan_scratch_words((uint32_t)m + 1)) + al256(16) + 4 * al256(4 * kSlots * m) +
+           al256(4 * sort_scratch_words(kSlots * m, 16)) + al256(64) + al256(4 * kPairKeep * m);
 }
 
 cudaError_t sap_aabb_async(uint32_t n, const float4* pos, const float* radius, float4* lo, float4* hi,
@@ -318,57 +342,47 @@ cudaError_t sap_pairs_async(uint32_t n, const float4* lo, const float4* hi, void
     uint32_t* keys_tmp = (uint32_t*)take(4 * m);
     uint32_t* vals_tmp = (uint32_t*)take(4 * m);
     uint32_t* sort_scratch = (uint32_t*)take(4 * sort_scratch_words(m, 32));
-    float4* slo = (float4*)take(16 * m);
-    float4* shi = (float4*)take(16 * m);
-    take(16 * m);
-    take(16 * m);
+    float4* box = (float4*)take(48 * m);  // 32 bytes each; the rest is sd_sap_process_collisions'
     uint32_t* counts = (uint32_t*)take(4 * (m + 1));
+    uint32_t* eoff = (uint32_t*)take(4 * (m + 1));
     uint32_t* off = (uint32_t*)take(4 * (m + 1));
-    uint32_t* pos = (uint32_t*)take(4 * (m + 1));
+    uint32_t* cursor = (uint32_t*)take(4 * (m + 1));
     uint32_t* scan = (uint32_t*)take(4 * scan_scratch_words((uint32_t)m + 1));
-    uint32_t* partners = (uint32_t*)take(4 * (2 * pair_cap + 1));
     uint32_t* status = (uint32_t*)take(16);
     uint32_t* ckeys = (uint32_t*)take(4 * kSlots * m);
     uint32_t* cvals = (uint32_t*)take(4 * kSlots * m);
     uint32_t* ckeys_tmp = (uint32_t*)take(4 * kSlots * m);
     uint32_t* cvals_tmp = (uint32_t*)take(4 * kSlots * m);
     uint32_t* csort = (uint32_t*)take(4 * sort_scratch_words(kSlots * m, 16));
-    uint32_t* bounds = (uint32_t*)take(64);  // 5 words, then the grid
-    SapGrid* grid = reinterpret_cast<SapGrid*>(bounds + 8);
+    SapBounds* bounds = (SapBounds*)take(64);
+    uint32_t* keep = (uint32_t*)take(4 * kPairKeep * m);
+    static_assert(sizeof(SapBounds) <= 64, "bounds fit their scratch");
     cudaError_t e = cudaMemsetAsync(status, 0, 16, st);
     if (e != cudaSuccess) return e;
     if (n == 0) return cudaMemsetAsync(d_count2, 0, 8, st);
+    const uint32_t grid = grid_for(n, kSapThreads);
+    if ((e = cudaMemsetAsync(bounds, 0, sizeof(SapBounds), st)) != cudaSuccess) return e;
+    sap_bounds_kernel<<<std::min<uint32_t>(grid, kBoundBlocks), kSapThreads, 0, st>>>(n, lo, hi, bounds, keys, vals);
     bool in_tmp = false;
-    if ((e = sap_sort_lower_x_async(n, lo, true, keys, vals, keys_tmp, vals_tmp, sort_scratch, &in_tmp, st)) !=
-        cudaSuccess)
-        return e;
-    const uint32_t* svals = in_tmp ? vals_tmp : vals;
-    gather_sorted_kernel<<<grid_for(n, kSapThreads), kSapThreads, 0, st>>>(n, svals, lo, hi, slo, shi);
-    // the column grid, each box's entries, stably sorted by column
-    if ((e = cudaMemsetAsync(bounds, 0, 32, st)) != cudaSuccess) return e;
-    sap_bounds_kernel<<<std::min<uint32_t>(grid_for(n, kSapThreads), 152 * 8), kSapThreads, 0, st>>>(n, lo, hi,
-                                                                                                     bounds);
-    sap_grid_kernel<<<1, 1, 0, st>>>(bounds, grid);
-    sap_entries_kernel<<<grid_for(n, kSapThreads), kSapThreads, 0, st>>>(n, slo, shi, grid, ckeys, cvals, status);
+    if ((e = sort_pairs_async(keys, vals, keys_tmp, vals_tmp, n, 32, sort_scratch, st, &in_tmp)) != cudaSuccess) return e;
+    // each box's entries, stably sorted by column
+    sap_gather_kernel<<<grid, kSapThreads, 0, st>>>(n, in_tmp ? vals_tmp : vals, lo, hi, bounds, box, counts, status);
+    if ((e = scan_exclusive_async(counts, eoff, n, scan, st)) != cudaSuccess) return e;
+    sap_entries_kernel<<<grid, kSapThreads, 0, st>>>(n, box, bounds, eoff, ckeys, cvals);
     const uint32_t ne = kSlots * n;
     bool c_tmp = false;
-    if ((e = sort_pairs_async(ckeys, cvals, ckeys_tmp, cvals_tmp, ne, 16, csort, st, &c_tmp)) != cudaSuccess)
+    if ((e = sort_pairs_async(ckeys, cvals, ckeys_tmp, cvals_tmp, ne, 16, csort, st, &c_tmp, eoff + n)) != cudaSuccess)
         return e;
     const uint32_t* sk = c_tmp ? ckeys_tmp : ckeys;
     const uint32_t* sv = c_tmp ? cvals_tmp : cvals;
-    if ((e = cudaMemsetAsync(counts, 0, 4 * (m + 1), st)) != cudaSuccess) return e;
-    sweep_binned_kernel<false><<<grid_for(ne, kSapThreads), kSapThreads, 0, st>>>(
-        ne, sk, sv, svals, slo, shi, grid, counts, nullptr, nullptr, nullptr, 0, status);
+    const PairSink sink{counts, keep, status + 1, off, cursor, out, n, pair_cap};
+    if ((e = cudaMemsetAsync(counts, 0, 4 * m, st)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(cursor, 0, 4 * m, st)) != cudaSuccess) return e;
+    sweep_binned_kernel<false><<<grid_for(ne, kSapThreads), kSapThreads, 0, st>>>(eoff + n, sk, sv, box, bounds, sink);
     if ((e = scan_exclusive_async(counts, off, n, scan, st)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(counts, 0, 4 * (m + 1), st)) != cudaSuccess) return e;  // reused as cursors
-    sweep_binned_kernel<true><<<grid_for(ne, kSapThreads), kSapThreads, 0, st>>>(
-        ne, sk, sv, svals, slo, shi, grid, nullptr, off, counts, partners, 2 * pair_cap, status);
-    sort_segments_kernel<<<grid_for(n, kSapThreads), kSapThreads, 0, st>>>(n, off, partners, 2 * pair_cap);
-    uint32_t* ucount = keys;  // free again
-    if ((e = csr_unique_pairs_async(n, off, partners, 2 * pair_cap, ucount, scan, pos, out, pair_cap, st)) !=
-        cudaSuccess)
-        return e;
-    if ((e = cudaMemcpyAsync(d_count2, pos + n, 4, cudaMemcpyDeviceToDevice, st)) != cudaSuccess) return e;
+    sweep_binned_kernel<true><<<grid_for(ne, kSapThreads), kSapThreads, 0, st>>>(eoff + n, sk, sv, box, bounds, sink);
+    pairs_write_kernel<<<grid, kSapThreads, 0, st>>>(sink, d_count2, status);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
     return cudaMemcpyAsync(d_count2 + 1, status, 4, cudaMemcpyDeviceToDevice, st);
 }
 
@@ -434,9 +448,9 @@ sd_status sd_sap_process_collisions(uint64_t n, const float* d_pos4, const float
     uint32_t* keys_tmp = (uint32_t*)take(4ull * m);
     uint32_t* vals_tmp = (uint32_t*)take(4ull * m);
     uint32_t* sort_scratch = (uint32_t*)take(4ull * sd::sort_scratch_words(m, 32));
-    float4* lo = (float4*)take(16ull * m);
-    float4* hi = (float4*)take(16ull * m);
-    float* proj = (float*)take(16ull * m);
+    float4* lo = (float4*)take(48ull * m);  // lower and upper corners, then the projections
+    float4* hi = lo + m;
+    float* proj = reinterpret_cast<float*>(hi + m);
     float* upperx = proj;
     float* uppery = proj + m;
     float* lowery = proj + 2ull * m;

@@ -68,7 +68,8 @@ constexpr uint32_t tile_keys() { return kSortThreads * ITEMS; }
 
 __global__ void __launch_bounds__(kHistThreads)
 sort_histogram_kernel(const uint32_t* __restrict__ keys, uint32_t n, SortPlan plan, uint32_t* __restrict__ scratch,
-                      bool vec) {
+                      bool vec, const uint32_t* __restrict__ d_n) {
+    if (d_n) n = min(n, *d_n);
     __shared__ uint32_t hist[2048];  // pass p at p * plan.stride
     block_histograms<false>(keys, nullptr, n, plan, scratch, hist, vec);
 }
@@ -99,12 +100,15 @@ __global__ void __launch_bounds__(kSortThreads, 3)
 sort_pass_kernel(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
                  uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, uint32_t n,
                  int shift, int bits, int pass, uint32_t num_tiles, uint32_t hstride, uint32_t bins,
-                 uint32_t* __restrict__ scratch, const uint32_t* __restrict__ skip, uint32_t skip_max) {
+                 uint32_t* __restrict__ scratch, const uint32_t* __restrict__ skip, uint32_t skip_max,
+                 const uint32_t* __restrict__ d_n) {
     if (skip && skip[1] <= skip_max) return;  // the incremental re-sort wrote the result
+    if (d_n) n = min(n, *d_n);
     extern __shared__ __align__(16) uint32_t smem[];
     __shared__ uint32_t s_tile;
     if (threadIdx.x == 0) s_tile = atomicAdd(&scratch[4 + pass], 1u);
     __syncthreads();
+    if (s_tile >= (n + kSortThreads * ITEMS - 1) / (kSortThreads * ITEMS)) return;  // d_n: fewer keys than the grid's
     sort_tile<BINS, ITEMS>(smem, s_tile, keys_in, vals_in, keys_out, vals_out, n, shift, bits, pass, num_tiles, hstride,
                            bins, scratch);
 }
@@ -146,9 +150,9 @@ static int hist_blocks(uint32_t n) {
 }
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-cudaError_t sort_histogram_async(const uint32_t* keys, uint32_t n, const SortPlan& plan, uint32_t* scratch,
-                                 cudaStream_t st) {
-    sort_histogram_kernel<<<hist_blocks(n), kHistThreads, 0, st>>>(keys, n, plan, scratch, aligned16(keys));
+static cudaError_t sort_histogram_async(const uint32_t* keys, uint32_t n, const SortPlan& plan, uint32_t* scratch,
+                                        cudaStream_t st, const uint32_t* d_n) {
+    sort_histogram_kernel<<<hist_blocks(n), kHistThreads, 0, st>>>(keys, n, plan, scratch, aligned16(keys), d_n);
     return cudaGetLastError();
 }
 
@@ -156,7 +160,7 @@ template <int BINS, int ITEMS>
 static cudaError_t launch_pass(const uint32_t* ki, const uint32_t* vi, uint32_t* ko, uint32_t* vo,
                                uint32_t n, int shift, int bits, int pass, uint32_t tiles, uint32_t stride,
                                uint32_t bins, uint32_t* scratch, cudaStream_t st, const uint32_t* skip,
-                               uint32_t skip_max) {
+                               uint32_t skip_max, const uint32_t* d_n) {
     size_t sm = sort_tile_smem<BINS, ITEMS>();
     if (sm > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(sort_pass_kernel<BINS, ITEMS>,
@@ -165,7 +169,7 @@ static cudaError_t launch_pass(const uint32_t* ki, const uint32_t* vi, uint32_t*
     }
     sort_pass_kernel<BINS, ITEMS><<<tiles, kSortThreads, sm, st>>>(ki, vi, ko, vo, n, shift, bits,
                                                                    pass, tiles, stride, bins, scratch, skip,
-                                                                   skip_max);
+                                                                   skip_max, d_n);
     return cudaGetLastError();
 }
 
@@ -173,7 +177,7 @@ static cudaError_t launch_pass(const uint32_t* ki, const uint32_t* vi, uint32_t*
 // tile status cleared (sort_clear_async + a histogram producer).
 cudaError_t sort_passes_async(uint32_t* keys, uint32_t* vals, uint32_t* keys_tmp, uint32_t* vals_tmp,
                               uint32_t n, const SortPlan& plan, uint32_t* scratch, cudaStream_t st,
-                              bool* in_tmp, const uint32_t* skip, uint32_t skip_max) {
+                              bool* in_tmp, const uint32_t* skip, uint32_t skip_max, const uint32_t* d_n) {
     *in_tmp = false;
     if (n == 0) return cudaSuccess;
     const uint32_t tiles = num_tiles(n);
@@ -183,13 +187,13 @@ cudaError_t sort_passes_async(uint32_t* keys, uint32_t* vals, uint32_t* keys_tmp
         const int b = plan.bits[p], sh = plan.shift[p];
         const uint32_t sd = (uint32_t)plan.stride, ss = status_bins(plan);
         if (g_sort_items >= 16)
-            e = b > 9   ? launch_pass<1024, 16>(ki, vi, ko, vo, n, sh, b, p, tiles, sd, ss, scratch, st, skip, skip_max)
-                : b > 8 ? launch_pass<512, 16>(ki, vi, ko, vo, n, sh, b, p, tiles, sd, ss, scratch, st, skip, skip_max)
-                        : launch_pass<256, 16>(ki, vi, ko, vo, n, sh, b, p, tiles, sd, ss, scratch, st, skip, skip_max);
+            e = b > 9   ? launch_pass<1024, 16>(ki, vi, ko, vo, n, sh, b, p, tiles, sd, ss, scratch, st, skip, skip_max, d_n)
+                : b > 8 ? launch_pass<512, 16>(ki, vi, ko, vo, n, sh, b, p, tiles, sd, ss, scratch, st, skip, skip_max, d_n)
+                        : launch_pass<256, 16>(ki, vi, ko, vo, n, sh, b, p, tiles, sd, ss, scratch, st, skip, skip_max, d_n);
         else
-            e = b > 9   ? launch_pass<1024, 8>(ki, vi, ko, vo, n, sh, b, p, tiles, sd, ss, scratch, st, skip, skip_max)
-                : b > 8 ? launch_pass<512, 8>(ki, vi, ko, vo, n, sh, b, p, tiles, sd, ss, scratch, st, skip, skip_max)
-                        : launch_pass<256, 8>(ki, vi, ko, vo, n, sh, b, p, tiles, sd, ss, scratch, st, skip, skip_max);
+            e = b > 9   ? launch_pass<1024, 8>(ki, vi, ko, vo, n, sh, b, p, tiles, sd, ss, scratch, st, skip, skip_max, d_n)
+                : b > 8 ? launch_pass<512, 8>(ki, vi, ko, vo, n, sh, b, p, tiles, sd, ss, scratch, st, skip, skip_max, d_n)
+                        : launch_pass<256, 8>(ki, vi, ko, vo, n, sh, b, p, tiles, sd, ss, scratch, st, skip, skip_max, d_n);
         if (e != cudaSuccess) return e;
         uint32_t* t;
         t = ki; ki = ko; ko = t;
@@ -215,17 +219,18 @@ cudaError_t sort_fallback_async(uint32_t* keys, uint32_t* vals, uint32_t* keys_t
 }
 
 // Sorts (keys, vals) by bits [0, key_bits).  Returns via *in_tmp whether
-// the result ended in the tmp buffers (odd pass count).
+// the result ended in the tmp buffers (odd pass count).  d_n (may be null): a
+// device word, the number of keys when it is below n.
 cudaError_t sort_pairs_async(uint32_t* keys, uint32_t* vals, uint32_t* keys_tmp, uint32_t* vals_tmp,
                              uint32_t n, int key_bits, uint32_t* scratch, cudaStream_t st,
-                             bool* in_tmp) {
+                             bool* in_tmp, const uint32_t* d_n) {
     SortPlan plan = sort_plan(key_bits);
     *in_tmp = false;
     if (n == 0) return cudaSuccess;
     cudaError_t e = sort_clear_async(n, plan, scratch, st);
     if (e != cudaSuccess) return e;
-    if ((e = sort_histogram_async(keys, n, plan, scratch, st)) != cudaSuccess) return e;
-    return sort_passes_async(keys, vals, keys_tmp, vals_tmp, n, plan, scratch, st, in_tmp);
+    if ((e = sort_histogram_async(keys, n, plan, scratch, st, d_n)) != cudaSuccess) return e;
+    return sort_passes_async(keys, vals, keys_tmp, vals_tmp, n, plan, scratch, st, in_tmp, nullptr, 0, d_n);
 }
 
 int sort_num_passes(int key_bits) { return sort_plan(key_bits).passes; }

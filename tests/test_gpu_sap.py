@@ -104,3 +104,30 @@ def test_sap_pairs_binned_edge_cases(sdlib, orc, kind):
     got, cnt, err = sdlib.SweepAndPrune.pairs(torch.from_numpy(L).cuda(), torch.from_numpy(H).cuda(), len(want) + 8)
     assert err == 0 and cnt == len(want), (kind, cnt, len(want), err)
     assert np.array_equal(got.cpu().numpy().view(np.uint64), want)
+
+
+@pytest.mark.parametrize("op", ["sap", "lbvh"])
+@pytest.mark.parametrize("kind,n", [("dense", 1500), ("spanning", 3000), ("even", 65_535), ("even", 65_536)])
+def test_pair_lists_past_the_kept_partners(sdlib, orc, op, kind, n):
+    """Boxes with none to many more partners than are kept per box (16), a
+    box over the whole domain with the lowest and the highest id, and either
+    side of the tree's lane rule; a list that just fits, and one too short."""
+    import torch
+    rng = np.random.default_rng(n)
+    c = rng.uniform(-1.0, 1.0, (n, 3)).astype(np.float32)
+    h = np.full((n, 3), {"dense": 0.22, "spanning": 0.03, "even": 0.012}[kind], np.float32)
+    if kind == "spanning":
+        h[[0, n - 1]] = 3.0
+    L = np.zeros((n, 4), np.float32)
+    H = np.zeros((n, 4), np.float32)
+    L[:, :3] = c - h
+    H[:, :3] = c + h
+    want = orc.aabb_pairs(L, H)
+    lower = np.bincount((want >> np.uint64(32)).astype(np.int64), minlength=n)
+    assert (lower.max() > 16) == (kind != "even") and 16 in lower or kind != "dense"
+    pairs = sdlib.SweepAndPrune.pairs if op == "sap" else sdlib.BoundingVolumes.pairs
+    lo, hi = torch.from_numpy(L).cuda(), torch.from_numpy(H).cuda()
+    got, cnt, err = pairs(lo, hi, len(want))
+    assert err == 0 and cnt == len(want)
+    assert np.array_equal(got.cpu().numpy().view(np.uint64), want)
+    assert pairs(lo, hi, len(want) - 1)[2] == sdlib._abi.SD_DEVERR_PAIR_OVERFLOW
