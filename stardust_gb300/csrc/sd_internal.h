@@ -80,8 +80,10 @@ struct Lbvh {
     float *bounds, *bound_part;          // global box (lo xyz, hi xyz) and per-block partials
     int2* children;                      // n-1 internal nodes; bit 31 marks a leaf child
     int32_t* parent;                     // internal nodes [0, n-1), leaves [n-1, 2n-1); root -1
-    uint32_t* visit;                     // refit arrival counters
-    float4 *node_lo, *node_hi, *leaf_lo, *leaf_hi;
+    int32_t* other;                      // per internal node: the end of its leaf range that is not its index
+    uint32_t* top;                       // the nodes of more than 128 leaves (their number in bounds[6])
+    float4 *node_lo, *node_hi;           // boxes of the subtrees below top nodes; top nodes: atomic bounds
+    float4 *leaf_lo, *leaf_hi;
     uint32_t* counts;                    // per box id
     uint32_t* first;                     // per leaf: its first kLbvhFirst partners found (counting pass)
     float4* rec;                         // per internal node: both children's boxes (lo.w = child ref)

@@ -11,8 +11,8 @@
 //   3. this library's onesweep radix sort of (code, index), 30-bit keys;
 //   4. Karras (2012) binary radix tree, one thread per internal node, ties
 //      between equal codes broken by the leaf index;
-//   5. refit in ONE launch: every leaf climbs towards the root and the
-//      second thread to reach a node (atomic visit counter) writes its box;
+//   5. refit: subtrees of up to 128 leaves joined bottom-up in shared memory,
+//      their boxes raised through the nodes above by atomic maxima;
 //   6. stack traversal, a few lanes to a leaf: they take as many nodes off the
 //      leaf's stack at a time.  Partner lists (both ways, per body, a count
 //      pass and a write pass) or the unique pairs (each found once, from the
@@ -22,6 +22,7 @@
 #include "sd_common.cuh"
 #include "sd_pairs.cuh"
 
+#include <algorithm>
 #include <utility>
 
 namespace sd {
@@ -30,12 +31,16 @@ namespace {
 
 constexpr int kLbvhThreads = 256;
 constexpr uint32_t kLeaf = 0x80000000u;
+constexpr int kTreelet = 128;  // leaves of a subtree that a block's shared memory joins
 constexpr int kStack = 64;  // Karras tree depth <= 32 code bits + 32 index bits
 static_assert(kLbvhFirst >= (int)kPairKeep, "the sink keeps its partners in Lbvh::first");
 
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 8;
 constexpr uint32_t kScanTile = kScanThreads * kScanItems;
+
+// The number of top nodes, behind the global box.
+__host__ __device__ inline uint32_t* top_count(float* bounds) { return reinterpret_cast<uint32_t*>(bounds + 6); }
 
 __device__ __forceinline__ bool box_overlap(float4 alo, float4 ahi, float4 blo, float4 bhi) {
     return blo.x <= ahi.x && alo.x <= bhi.x && blo.y <= ahi.y && alo.y <= bhi.y && blo.z <= ahi.z &&
@@ -131,6 +136,7 @@ __global__ void bounds_final_kernel(const float* __restrict__ part, uint32_t nb,
         m = k < 3 ? fminf(m, x) : fmaxf(m, x);
     }
     if (lane == 0) bounds[k] = m;
+    if (threadIdx.x == 0) *top_count(bounds) = 0u;
 }
 
 // --------------------------------------------------------------- Morton
@@ -178,7 +184,8 @@ __device__ __forceinline__ int delta(const uint32_t* __restrict__ k, int n, int 
 // k-d Trees" (HPG 2012), Figure 4.  parent[] holds internal nodes at
 // [0, n-1) and leaves at [n-1, 2n-1).
 __global__ void build_kernel(const uint32_t* __restrict__ keys, int n, int2* __restrict__ children,
-                             int32_t* __restrict__ parent) {
+                             int32_t* __restrict__ parent, int32_t* __restrict__ other, float4* __restrict__ node_lo,
+                             float4* __restrict__ node_hi, uint32_t* __restrict__ top, uint32_t* __restrict__ n_top) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n - 1) return;
     const int d = (delta(keys, n, i, i + 1) - delta(keys, n, i, i - 1)) >= 0 ? 1 : -1;
@@ -200,71 +207,203 @@ __global__ void build_kernel(const uint32_t* __restrict__ keys, int n, int2* __r
     const int left = lo == g ? (int)(g | kLeaf) : g;
     const int right = hi == g + 1 ? (int)((g + 1) | kLeaf) : g + 1;
     children[i] = make_int2(left, right);
+    other[i] = j;
+    if (l >= kTreelet) {
+        top[atomicAdd(n_top, 1u)] = (uint32_t)i;
+        node_lo[i] = node_hi[i] = make_float4(0.f, 0.f, 0.f, 0.f);  // (no key yet)
+    }
+    if (i == 0) parent[0] = -1;  // the root
     parent[lo == g ? (n - 1) + g : g] = i;
     parent[hi == g + 1 ? (n - 1) + g + 1 : g + 1] = i;
 }
 
-__device__ __forceinline__ float4 ldcg4(const float4* p) { return __ldcg(p); }
-
-// Orders a node's box before the arrival that announces it, and the sibling's
-// arrival before the reads of its box (release and acquire are enough here;
-// __threadfence is sequentially consistent and slower).
-__device__ __forceinline__ void fence_acq_rel() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+__device__ __forceinline__ void red_max(uint32_t* p, uint32_t v) {
+    asm volatile("red.relaxed.gpu.global.max.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
 
 // A child reference is a leaf below n or an internal node below n - 1.
 __device__ __forceinline__ bool child_ok(int c, int n) {
     return (c & kLeaf) ? (c & ~kLeaf) < n : (c >= 0 && c < n - 1);
 }
 
-// Bottom-up boxes: the last of a node's two children to finish computes
-// the node's box and writes the node's record -- both children's boxes,
-// each lower corner's w lane holding the child reference and each upper
-// corner's the last leaf below that child -- which the traversal reads in one
-// 64-byte piece instead of the children's indices and then their boxes.
-// A chain of about 24 levels at 2.7 us each (fence, atomic, two boxes from
-// L2): 64 us at 300,001 leaves.  Joining the nodes that lie within a block's
-// 512 leaves in shared memory takes nothing off it (66 us): the paths along
-// the blocks' edges are as deep.
-__global__ void refit_kernel(int n, const uint32_t* __restrict__ vals, const float4* __restrict__ lo,
-                             const float4* __restrict__ hi, float4* leaf_lo, float4* leaf_hi, float4* node_lo,
-                             float4* node_hi, const int2* __restrict__ children, const int32_t* __restrict__ parent,
-                             uint32_t* visit, float4* __restrict__ rec, uint32_t* __restrict__ status) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+// Bottom-up boxes.  Every node gets a record -- both children's boxes, each
+// lower corner's w lane holding the child reference and each upper corner's
+// the last leaf below that child -- which the traversal reads in one 64-byte
+// piece instead of the children's indices and then their boxes.
+//
+// Treelets, the largest subtrees of at most kTreelet leaves, are joined in
+// shared memory: a block takes those whose first leaf is one of its
+// kRefitSpan, so kRefitSpan + kTreelet leaves hold them, and a node, whose
+// index is one end of its range, lies there too.  (A treelet across two blocks'
+// leaves is joined by both, to the same bits; the one with its first leaf goes
+// on with it.)  Its box then rises through the top nodes as atomic maxima,
+// which wait for nothing, and stops where it widens nothing: the box that
+// holds it there rises itself.  top_kernel writes the top nodes' records.
+//
+// The chain of dependent loads bounds it: some 9 levels in shared memory, 13
+// above at one load each.  With every level through global memory (a fence, an
+// atomic that returns, the sibling's box: 1.7 to 2.7 us each) the refit was 41.5
+// us at 32,768 leaves and 64 at 300,001; now 13.5 + 7 and 36.6 + 16.8 with cold
+// caches, and the pairs of 300,001 boxes 281 us in all against 355.  Treelets
+// of 32 and 64 leaves and spans of 192 to 448 are 0 to 5% behind; a block
+// joining only what lies within its own 512 leaves gains nothing, as the paths
+// along the blocks' edges stay as deep.
+constexpr int kRefitSpan = 512;
+constexpr int kRefitWindow = kRefitSpan + kTreelet;
+
+struct Corners {
+    float v[6];  // lower x, y, z, upper x, y, z
+};
+
+__device__ __forceinline__ Corners corners(float4 a, float4 b) { return Corners{{a.x, a.y, a.z, b.x, b.y, b.z}}; }
+
+// Ordered keys that grow as the box does (NaN: 0, no bound).
+__device__ __forceinline__ uint32_t bound_key(float x, bool lower) {
+    if (x != x) return 0u;
+    const uint32_t b = __float_as_uint(x), k = (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+    return lower ? ~k : k;
+}
+__device__ __forceinline__ float key_bound(uint32_t k, bool lower) {
+    if (lower) k = ~k;
+    return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
+}
+
+__device__ __forceinline__ void write_record(float4* __restrict__ rec, int p, int2 c, const Corners& a, const Corners& b,
+                                             int last) {
+    // a left child's last leaf is the index in its own reference (the split)
+    rec[4 * (size_t)p + 0] = make_float4(a.v[0], a.v[1], a.v[2], __int_as_float(c.x));
+    rec[4 * (size_t)p + 1] = make_float4(a.v[3], a.v[4], a.v[5], __int_as_float(c.x & ~kLeaf));
+    rec[4 * (size_t)p + 2] = make_float4(b.v[0], b.v[1], b.v[2], __int_as_float(c.y));
+    rec[4 * (size_t)p + 3] = make_float4(b.v[3], b.v[4], b.v[5], __int_as_float(last));
+}
+
+__global__ void __launch_bounds__(kRefitWindow)
+refit_kernel(int n, const uint32_t* __restrict__ vals, const float4* __restrict__ lo, const float4* __restrict__ hi,
+             float4* __restrict__ leaf_lo, float4* __restrict__ leaf_hi, float4* __restrict__ node_lo,
+             float4* __restrict__ node_hi, const int2* __restrict__ children, const int32_t* __restrict__ parent,
+             const int32_t* __restrict__ other, float4* __restrict__ rec, uint32_t* __restrict__ status) {
+    __shared__ float s_box[2][6][kRefitWindow];  // leaves, nodes
+    __shared__ int2 s_children[kRefitWindow];
+    __shared__ int s_parent[kRefitWindow], s_other[kRefitWindow];
+    __shared__ uint32_t s_visit[kRefitWindow];
+    const int t = (int)threadIdx.x, b0 = (int)blockIdx.x * kRefitSpan, k = b0 + t;
+    Corners box{};
+    int p = -1;
+    s_visit[t] = 0u;
+    if (k < n) {
+        const uint32_t id = vals[k];
+        if (n > 1) p = parent[(n - 1) + k];
+        if (k < n - 1) {
+            s_children[t] = children[k];
+            s_parent[t] = parent[k];
+            s_other[t] = other[k];
+        }
+        const float4 a = lo[id], b = hi[id];
+        if (t < kRefitSpan) {
+            leaf_lo[k] = a;
+            leaf_hi[k] = b;
+        }
+        box = corners(a, b);
+#pragma unroll
+        for (int c = 0; c < 6; ++c) s_box[0][c][t] = box.v[c];
+    }
+    __syncthreads();
     if (k >= n) return;
-    const uint32_t id = vals[k];
-    leaf_lo[k] = lo[id];
-    leaf_hi[k] = hi[id];
-    fence_acq_rel();
-    int p = n > 1 ? parent[(n - 1) + k] : -1;
-    for (int level = 0; p >= 0; ++level) {
+    int cur = -1, first = k;  // (no node yet: the leaf itself)
+    for (int level = 0;; ++level) {
+        if (p < 0) return;  // no top: the whole tree is a treelet
         if (level > 2 * kStack || p >= n - 1) {  // a malformed tree: report, never loop or stray
             atomicOr(status, kErrBadInput);
             return;
         }
-        const int2 c = children[p];
-        const int up = parent[p];
-        if (atomicAdd(&visit[p], 1u) == 0u) return;  // the sibling subtree is not done yet
-        fence_acq_rel();
-        if (!child_ok(c.x, n) || !child_ok(c.y, n)) {
+        const int q = p - b0, e = q >= 0 && q < kRefitWindow ? s_other[q] : other[p];
+        const int f = min(p, e), l = max(p, e);
+        if (l - f >= kTreelet) break;                       // what this thread holds is a treelet
+        if (f < b0 || l >= b0 + kRefitWindow) return;       // a neighbour's
+        __threadfence_block();
+        if (atomicAdd(&s_visit[q], 1u) == 0u) return;       // the sibling subtree is not done yet
+        __threadfence_block();
+        const int2 c = s_children[q];
+        const int a = (c.x & ~kLeaf) - b0, b = (c.y & ~kLeaf) - b0;
+        if (a < 0 || a >= kRefitWindow || b < 0 || b >= kRefitWindow) {
             atomicOr(status, kErrBadInput);
             return;
         }
-        const int l = c.x & ~kLeaf, r = c.y & ~kLeaf;
-        float4 a0, a1, b0, b1;
-        if (c.x & kLeaf) { a0 = ldcg4(leaf_lo + l); a1 = ldcg4(leaf_hi + l); }
-        else { a0 = ldcg4(node_lo + l); a1 = ldcg4(node_hi + l); }
-        if (c.y & kLeaf) { b0 = ldcg4(leaf_lo + r); b1 = ldcg4(leaf_hi + r); }
-        else { b0 = ldcg4(node_lo + r); b1 = ldcg4(node_hi + r); }
-        // a left child's last leaf is the index in its own reference (the split)
-        const float end_a = __int_as_float(l), end_b = (c.y & kLeaf) ? __int_as_float(r) : b1.w;
-        node_lo[p] = make_float4(fminf(a0.x, b0.x), fminf(a0.y, b0.y), fminf(a0.z, b0.z), 0.f);
-        node_hi[p] = make_float4(fmaxf(a1.x, b1.x), fmaxf(a1.y, b1.y), fmaxf(a1.z, b1.z), end_b);
-        rec[4 * (size_t)p + 0] = make_float4(a0.x, a0.y, a0.z, __int_as_float(c.x));
-        rec[4 * (size_t)p + 1] = make_float4(a1.x, a1.y, a1.z, end_a);
-        rec[4 * (size_t)p + 2] = make_float4(b0.x, b0.y, b0.z, __int_as_float(c.y));
-        rec[4 * (size_t)p + 3] = make_float4(b1.x, b1.y, b1.z, end_b);
-        fence_acq_rel();
+        Corners x, y;
+#pragma unroll
+        for (int m = 0; m < 6; ++m) {
+            x.v[m] = s_box[(c.x & kLeaf) ? 0 : 1][m][a];
+            y.v[m] = s_box[(c.y & kLeaf) ? 0 : 1][m][b];
+            box.v[m] = m < 3 ? fminf(x.v[m], y.v[m]) : fmaxf(x.v[m], y.v[m]);
+            s_box[1][m][q] = box.v[m];
+        }
+        write_record(rec, p, c, x, y, l);
+        cur = p;
+        first = f;
+        p = s_parent[q];
+    }
+    if (first < b0 || first >= b0 + kRefitSpan) return;  // a neighbour goes on with it
+    if (cur >= 0) {
+        node_lo[cur] = make_float4(box.v[0], box.v[1], box.v[2], 0.f);
+        node_hi[cur] = make_float4(box.v[3], box.v[4], box.v[5], 0.f);
+    }
+    uint32_t key[6];
+#pragma unroll
+    for (int m = 0; m < 6; ++m) key[m] = bound_key(box.v[m], m < 3);
+    for (int level = 0; p >= 0; ++level) {
+        if (level > 2 * kStack || p >= n - 1) {
+            atomicOr(status, kErrBadInput);
+            return;
+        }
+        uint32_t* const wl = reinterpret_cast<uint32_t*>(node_lo + p);
+        uint32_t* const wh = reinterpret_cast<uint32_t*>(node_hi + p);
+        const uint4 l4 = __ldcg(reinterpret_cast<const uint4*>(wl)), h4 = __ldcg(reinterpret_cast<const uint4*>(wh));
+        const int up = parent[p];
+        const uint32_t have[6] = {l4.x, l4.y, l4.z, h4.x, h4.y, h4.z};
+        bool wider = false;
+#pragma unroll
+        for (int m = 0; m < 6; ++m)
+            if (key[m] > have[m]) {
+                red_max((m < 3 ? wl : wh - 3) + m, key[m]);
+                wider = true;
+            }
+        if (!wider) return;
         p = up;
+    }
+}
+
+__global__ void top_kernel(int n, const uint32_t* __restrict__ top, const uint32_t* __restrict__ n_top,
+                           const float4* __restrict__ leaf_lo, const float4* __restrict__ leaf_hi, float4* node_lo,
+                           float4* node_hi, const int2* __restrict__ children, const int32_t* __restrict__ other,
+                           float4* __restrict__ rec, uint32_t* __restrict__ status) {
+    const uint32_t m = min(*n_top, (uint32_t)n);
+    const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
+        const int p = (int)top[i];
+        const int2 c = children[p];
+        const int e = other[p], first = min(p, e), last = max(p, e);
+        if (!child_ok(c.x, n) || !child_ok(c.y, n)) {
+            atomicOr(status, kErrBadInput);
+            continue;
+        }
+        Corners box[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int x = h ? c.y : c.x, j = x & ~kLeaf;
+            if (x & kLeaf) {
+                box[h] = corners(leaf_lo[j], leaf_hi[j]);
+                continue;
+            }
+            const float4 a = node_lo[j], b = node_hi[j];
+            box[h] = corners(a, b);
+            if ((h ? last - j : j - first) >= kTreelet) {  // a top node itself: keys, cleared for the next refit
+#pragma unroll
+                for (int w = 0; w < 6; ++w) box[h].v[w] = key_bound(__float_as_uint(box[h].v[w]), w < 3);
+                node_lo[j] = node_hi[j] = none;
+            }
+        }
+        if (p == 0) node_lo[0] = node_hi[0] = none;
+        write_record(rec, p, c, box[0], box[1], last);
     }
 }
 
@@ -439,7 +578,7 @@ uint64_t lbvh_scratch_bytes(uint32_t n) {
     b += 4 * align256(4 * m);                                      // keys, vals, keys_tmp, vals_tmp
     b += align256(4 * sort_scratch_words(m, 30));                  // sort
     b += align256(4 * 8) + align256(4 * 6 * 304);                  // bounds + partials
-    b += align256(8 * m) + align256(4 * (2 * m)) + align256(4 * m); // children, parent, visit
+    b += align256(8 * m) + align256(4 * (2 * m)) + 2 * align256(4 * m);  // children, parent, other, top
     b += 4 * align256(16 * m);                                     // node lo/hi, leaf lo/hi
     b += align256(4 * (m + 1)) + align256(4 * scan_scratch_words((uint32_t)m + 1));
     b += align256(4 * kLbvhFirst * m);                             // first partners per leaf
@@ -466,7 +605,8 @@ void lbvh_carve(void* scratch, uint32_t n, Lbvh* t) {
     t->bound_part = (float*)take(4 * 6 * 304);
     t->children = (int2*)take(8 * m);
     t->parent = (int32_t*)take(4 * 2 * m);
-    t->visit = (uint32_t*)take(4 * m);
+    t->other = (int32_t*)take(4 * m);
+    t->top = (uint32_t*)take(4 * m);
     t->node_lo = (float4*)take(16 * m);
     t->node_hi = (float4*)take(16 * m);
     t->leaf_lo = (float4*)take(16 * m);
@@ -501,26 +641,23 @@ cudaError_t lbvh_build_async(Lbvh& t, const float4* lo, const float4* hi, cudaSt
         return e;
     t.skeys = in_tmp ? t.keys_tmp : t.keys;
     t.svals = in_tmp ? t.vals_tmp : t.vals;
-    if ((e = cudaMemsetAsync(t.parent, 0xff, 4 * (2 * (size_t)n - 1), st)) != cudaSuccess) return e;
-    if (n > 1) {
-        if ((e = cudaMemsetAsync(t.visit, 0, 4 * ((size_t)n - 1), st)) != cudaSuccess) return e;
-        build_kernel<<<grid_for(n - 1, kLbvhThreads), kLbvhThreads, 0, st>>>(t.skeys, (int)n, t.children,
-                                                                              t.parent);
-    }
-    refit_kernel<<<grid_for(n, kLbvhThreads), kLbvhThreads, 0, st>>>((int)n, t.svals, lo, hi, t.leaf_lo, t.leaf_hi,
-                                                                       t.node_lo, t.node_hi, t.children, t.parent,
-                                                                       t.visit, t.rec, t.status);
-    return cudaGetLastError();
+    if (n > 1)
+        build_kernel<<<grid_for(n - 1, kLbvhThreads), kLbvhThreads, 0, st>>>(t.skeys, (int)n, t.children, t.parent, t.other,
+                                                                              t.node_lo, t.node_hi, t.top,
+                                                                              top_count(t.bounds));
+    return lbvh_refit_async(t, lo, hi, st);
 }
 
 cudaError_t lbvh_refit_async(Lbvh& t, const float4* lo, const float4* hi, cudaStream_t st) {
     const uint32_t n = t.n;
     if (n == 0) return cudaSuccess;
-    cudaError_t e;
-    if (n > 1 && (e = cudaMemsetAsync(t.visit, 0, 4 * ((size_t)n - 1), st)) != cudaSuccess) return e;
-    refit_kernel<<<grid_for(n, kLbvhThreads), kLbvhThreads, 0, st>>>((int)n, t.svals, lo, hi, t.leaf_lo, t.leaf_hi,
-                                                                       t.node_lo, t.node_hi, t.children, t.parent,
-                                                                       t.visit, t.rec, t.status);
+    refit_kernel<<<grid_for(n, kRefitSpan), kRefitWindow, 0, st>>>((int)n, t.svals, lo, hi, t.leaf_lo, t.leaf_hi, t.node_lo,
+                                                                   t.node_hi, t.children, t.parent, t.other, t.rec,
+                                                                   t.status);
+    if (n > (uint32_t)kTreelet)
+        top_kernel<<<std::min(152u, grid_for(n, kTreelet)), 128, 0, st>>>((int)n, t.top, top_count(t.bounds), t.leaf_lo,
+                                                                          t.leaf_hi, t.node_lo, t.node_hi, t.children,
+                                                                          t.other, t.rec, t.status);
     return cudaGetLastError();
 }
 

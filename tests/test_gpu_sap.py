@@ -131,3 +131,27 @@ def test_pair_lists_past_the_kept_partners(sdlib, orc, op, kind, n):
     assert err == 0 and cnt == len(want)
     assert np.array_equal(got.cpu().numpy().view(np.uint64), want)
     assert pairs(lo, hi, len(want) - 1)[2] == sdlib._abi.SD_DEVERR_PAIR_OVERFLOW
+
+
+@pytest.mark.parametrize("n", [2, 127, 128, 129, 512, 513, 640, 641, 1153, 5000])
+@pytest.mark.parametrize("spread", [1.0, 1e-3, 0.0])
+def test_tree_over_treelets(sdlib, orc, n, spread):
+    """Trees around the sizes of a treelet (128 leaves) and of a block's
+    window (512 + 128), with many equal codes, and nothing but equal codes."""
+    import torch
+    rng = np.random.default_rng(n)
+    c = (rng.uniform(-1.0, 1.0, (n, 3)) * (np.where(rng.random((n, 1)) < 0.7, spread, 1.0) if spread else 0.0)).astype(np.float32)
+    h = (rng.uniform(0.2, 1.0, (n, 3)) * (0.05 if spread == 1.0 else 2e-4)).astype(np.float32)
+    if n > 1000:
+        c += rng.integers(0, n // 50, (n, 1)).astype(np.float32) * (4.0 if spread else 0.0)
+    if spread == 0.0:
+        c[:, 0] = np.arange(n) * np.float32(3e-4)
+        c[0, 0], c[n - 1, 0] = -1e4, 1e4  # the rest share one cell of the code
+    L = np.zeros((n, 4), np.float32)
+    H = np.zeros((n, 4), np.float32)
+    L[:, :3] = c - h
+    H[:, :3] = c + h
+    want = orc.aabb_pairs(L, H)
+    got, cnt, err = sdlib.BoundingVolumes.pairs(torch.from_numpy(L).cuda(), torch.from_numpy(H).cuda(), len(want) + 1)
+    assert err == 0 and cnt == len(want)
+    assert np.array_equal(got.cpu().numpy().view(np.uint64), want)
