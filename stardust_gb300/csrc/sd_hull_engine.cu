@@ -144,7 +144,6 @@ sd_status build_hull_graphs(sd_engine* h, float dt) {
             e = sd::mlp_forward_async(S.mlp, H.feat, H.seeds, H.off + H.nb, H.cap, true, h->stream);
         if (e == cudaSuccess) e = sd::hull_narrow_async(S.P, H, h->stream);
         if (e == cudaSuccess) e = sd::hull_integrate_async(S.P, H, h->stream);
-        if (e == cudaSuccess) e = sd::hull_stats_async(H, S.stats, h->stream);
         cudaError_t e2 = cudaStreamEndCapture(h->stream, &g);
         if (e != cudaSuccess) return sd_cuda_fail(h, e, "capturing the hull step");
         if (e2 != cudaSuccess) return sd_cuda_fail(h, e2, "cudaStreamEndCapture");
@@ -215,17 +214,18 @@ sd_status hull_prepare(sd_engine* h) {
         (s = halloc(h, &H.lo, nb)) || (s = halloc(h, &H.hi, nb)) || (s = halloc(h, &H.ext, 2 * (size_t)nb)) ||
         (s = halloc(h, &H.self, cap)) || (s = halloc(h, &H.ef, cap)) || (s = halloc(h, &H.et, cap)) ||
         (s = halloc(h, &H.info, cap)) || (s = halloc(h, &H.seeds, cap)) || (s = halloc(h, &H.feat, 16 * cap)) ||
-        (s = halloc(h, &S.stats, 4)) || (s = halloc(h, &H.ucount, nb)) || (s = halloc(h, &H.upos, (size_t)nb + 1)) ||
-        (s = halloc(h, &H.ulist, cap / 2 + 1)) || (s = halloc(h, &H.uscan, sd::scan_scratch_words(nb) + 1)) ||
+        (s = halloc(h, &S.stats, 4)) || (s = halloc(h, &H.counters, sd::kHullCounters)) ||
+        (s = halloc(h, &H.ulist, cap / 2 + 1)) || (s = halloc(h, &H.open, cap / 2 + 1)) ||
         (s = halloc(h, &H.teach, cap)) || (s = halloc(h, &S.teach_flag, 4)) ||
         (s = halloc(h, &S.teach_feat, 16 * (cap / 2 + 1))) || (s = halloc(h, &S.teach_tgt, cap / 2 + 1)) ||
         (s = halloc(h, &S.teach_flags, cap)) || (s = halloc(h, &S.teach_pos, cap)) ||
         (s = halloc(h, &S.teach_scan, sd::scan_scratch_words((uint32_t)cap) + 1)) ||
         (s = halloc(h, &S.teach_total, 1)) ||
-        (s = halloc(h, &H.hit_count, 1)) || (s = halloc(h, &H.hits, cap / 2 + 1)) ||
+        (s = halloc(h, &H.hits, cap / 2 + 1)) ||
         (s = halloc(h, &H.hit_keys, cap / 2 + 1)))
         return s;
     H.teach_on = S.teach_flag;
+    H.stats = S.stats;
     for (int k = 0; k < 2; ++k)
         if ((s = halloc(h, &S.off[k], (size_t)nb + 1)) || (s = halloc(h, &S.partners[k], cap)) ||
             (s = halloc(h, &S.dir[k], cap)))
@@ -252,6 +252,7 @@ sd_status hull_prepare(sd_engine* h) {
     for (int k = 0; k < 2; ++k) HULL_CUDA(h, cudaMemsetAsync(S.off[k], 0, 4 * ((size_t)nb + 1), st));
     HULL_CUDA(h, cudaMemsetAsync(S.tree.status, 0, 16, st));
     HULL_CUDA(h, cudaMemsetAsync(S.stats, 0, 32, st));
+    HULL_CUDA(h, cudaMemsetAsync(H.counters, 0, 4 * sd::kHullCounters, st));
     HULL_CUDA(h, cudaMemsetAsync(S.mlp.status, 0, 16, st));
     {
         const uint32_t flags[4] = {0u, 0u, 1u, 0u};  // training off; the constants 0 and 1 to copy from
@@ -345,6 +346,9 @@ sd_status hull_launch_narrow(sd_engine* h) {
     H.prev_partners = S.partners[par ^ 1];
     H.prev_dir = S.dir[par ^ 1];
     H.keep_anchor = S.seed_mode == SD_GJK_SEED_LEARNED;
+    // the unique pairs are the last step's; the other counters start over
+    static_assert(sd::kUniquePairs == 0 && sd::kHullCounters == 4, "three cleared together");
+    HULL_CUDA(h, cudaMemsetAsync(H.counters + 1, 0, 3 * sizeof(uint32_t), h->stream));
     HULL_CUDA(h, sd::hull_narrow_async(S.P, H, h->stream));
     return SD_OK;
 }

@@ -155,17 +155,20 @@ struct HullBuffers {
     // previous direction (inputs 8..10, the anchor) as the next step's, so
     // the network is never fed its own outputs
     bool keep_anchor;
-    // the pairs GJK found intersecting, for the EPA kernel: count, and per
-    // hit the unique-pair index and the GJK support evaluations spent, and
-    // the support keys of the enclosing tetrahedron
-    uint32_t* hit_count;
+    // the pairs GJK found intersecting, for the EPA kernel: per hit the
+    // unique-pair index and the GJK support evaluations spent, and the support
+    // keys of the enclosing tetrahedron
     uint2* hits;
     uint4* hit_keys;
     const uint32_t *prev_off, *prev_partners;  // the previous step's lists
     const float4* prev_dir;
     float4 *force, *torque;                // optional per body totals
-    uint32_t *ucount, *upos, *ulist, *uscan;  // unique pairs: per body count, offsets (nb+1), entry list, scan scratch
+    uint32_t* ulist;                       // the entries of the unique pairs (self < partner), in no order
+    uint32_t* open;                        // those whose first GJK support does not separate them
+    uint32_t* counters;                    // kHullCounters, cleared by the step's first kernel
+    unsigned long long* stats;             // the step's statistics, likewise
 };
+constexpr int kUniquePairs = 0, kHitPairs = 1, kNextPair = 2, kOpenPairs = 3, kHullCounters = 4;
 cudaError_t hull_aabb_async(HullBuffers& H, cudaStream_t st);
 cudaError_t hull_seed_async(HullBuffers& H, uint32_t mode, cudaStream_t st);
 cudaError_t hull_narrow_async(const HullParams& p, HullBuffers& H, cudaStream_t st);
@@ -179,7 +182,6 @@ cudaError_t hull_teach_compact_async(const HullBuffers& H, const uint32_t* d_cou
                                      uint32_t* flags, uint32_t* pos, uint32_t* scan, uint32_t* d_total,
                                      cudaStream_t st);
 cudaError_t hull_integrate_async(const HullParams& p, HullBuffers& H, cudaStream_t st);
-cudaError_t hull_stats_async(HullBuffers& H, unsigned long long* out, cudaStream_t st);
 
 // ---- GJK warm-start network (sd_mlp.cu)
 struct MlpState {

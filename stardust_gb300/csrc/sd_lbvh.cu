@@ -38,6 +38,7 @@ static_assert(kLbvhFirst >= (int)kPairKeep, "the sink keeps its partners in Lbvh
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 8;
 constexpr uint32_t kScanTile = kScanThreads * kScanItems;
+constexpr uint32_t kScanDirect = 2048;  // tiles
 
 // The number of top nodes, behind the global box.
 __host__ __device__ inline uint32_t* top_count(float* bounds) { return reinterpret_cast<uint32_t*>(bounds + 6); }
@@ -78,9 +79,32 @@ __global__ void scan_partials_kernel(uint32_t* __restrict__ part, uint32_t nt, u
     if (threadIdx.x == 0) *total_out = carry;
 }
 
-__global__ void scan_apply_kernel(const uint32_t* __restrict__ in, uint32_t n, const uint32_t* __restrict__ part,
-                                  uint32_t* __restrict__ out) {
+// SUMS: part holds the tiles' sums as they are; each block adds up those
+// before its own (and the first all of them, for the total).
+template <bool SUMS>
+__global__ void __launch_bounds__(kScanThreads)
+scan_apply_kernel(const uint32_t* __restrict__ in, uint32_t n, const uint32_t* __restrict__ part,
+                  uint32_t* __restrict__ out) {
     __shared__ uint32_t ws[33];
+    uint32_t before = 0;
+    if constexpr (SUMS) {
+        __shared__ uint32_t s_sum;
+        const uint32_t nt = gridDim.x, upto = blockIdx.x == 0 ? nt : blockIdx.x;
+        if (threadIdx.x == 0) s_sum = 0u;
+        uint32_t x = 0;
+        for (uint32_t k = threadIdx.x; k < upto; k += kScanThreads) x += part[k];
+        __syncthreads();
+        x = __reduce_add_sync(0xffffffffu, x);
+        if (lane_id() == 0 && x) atomicAdd(&s_sum, x);
+        __syncthreads();
+        if (blockIdx.x == 0) {
+            if (threadIdx.x == 0) out[n] = s_sum;
+        } else {
+            before = s_sum;
+        }
+    } else {
+        before = part[blockIdx.x];
+    }
     const uint32_t base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
     uint32_t v[kScanItems];
     uint32_t s = 0;
@@ -90,11 +114,57 @@ __global__ void scan_apply_kernel(const uint32_t* __restrict__ in, uint32_t n, c
         s += v[k];
     }
     uint32_t tot;
-    uint32_t run = part[blockIdx.x] + block_exclusive_scan(s, ws, &tot);
+    uint32_t run = before + block_exclusive_scan(s, ws, &tot);
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
         if (base + k < n) out[base + k] = run;
         run += v[k];
+    }
+}
+
+// Up to kScanOne words (16-byte aligned): one block, each warp a stretch of
+// 128 x kScanRows of them, in one pass over memory.
+constexpr int kScanRows = 8;
+constexpr uint32_t kScanOne = 32 * 128 * kScanRows;
+
+__global__ void __launch_bounds__(1024) scan_one_kernel(const uint32_t* __restrict__ in, uint32_t n,
+                                                        uint32_t* __restrict__ out) {
+    __shared__ uint32_t ws[33];
+    const uint32_t base = (threadIdx.x >> 5) * (128 * kScanRows) + 4 * lane_id();
+    uint4 v[kScanRows];
+    uint32_t at[kScanRows], sum = 0;
+#pragma unroll
+    for (int r = 0; r < kScanRows; ++r) {
+        const uint32_t i = base + 128 * r;
+        if (i + 4 <= n) {
+            v[r] = *reinterpret_cast<const uint4*>(in + i);
+        } else {
+            v[r].x = i < n ? in[i] : 0u;
+            v[r].y = i + 1 < n ? in[i + 1] : 0u;
+            v[r].z = i + 2 < n ? in[i + 2] : 0u;
+            v[r].w = 0u;
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < kScanRows; ++r) {
+        const uint32_t s = v[r].x + v[r].y + v[r].z + v[r].w, inc = warp_inclusive_scan(s);
+        at[r] = sum + inc - s;
+        sum += __shfl_sync(0xffffffffu, inc, 31);
+    }
+    uint32_t total;
+    uint32_t before = block_exclusive_scan(lane_id() == 0 ? sum : 0u, ws, &total);
+    before = __shfl_sync(0xffffffffu, before, 0);
+    if (threadIdx.x == 0) out[n] = total;
+#pragma unroll
+    for (int r = 0; r < kScanRows; ++r) {
+        const uint32_t i = base + 128 * r, a = before + at[r], b = a + v[r].x, c = b + v[r].y, d = c + v[r].z;
+        if (i + 4 <= n) {
+            *reinterpret_cast<uint4*>(out + i) = make_uint4(a, b, c, d);
+        } else {
+            if (i < n) out[i] = a;
+            if (i + 1 < n) out[i + 1] = b;
+            if (i + 2 < n) out[i + 2] = c;
+        }
     }
 }
 
@@ -566,9 +636,22 @@ cudaError_t scan_exclusive_async(const uint32_t* in, uint32_t* out, uint32_t n, 
                                  cudaStream_t st) {
     const uint32_t nt = grid_for(n, kScanTile);
     if (n == 0) return cudaMemsetAsync(out, 0, 4, st);
+    // One block up to 32,768 words (5.6 us; three launches of 3 to 4 us and the
+    // gaps between them before); up to kScanDirect tiles each block of the second
+    // kernel adds up the tiles' sums before it, a launch less; beyond, that
+    // would be more reads than the words themselves.
+    const bool aligned = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0;
+    if (n <= kScanOne && aligned) {
+        scan_one_kernel<<<1, 1024, 0, st>>>(in, n, out);
+        return cudaGetLastError();
+    }
     scan_reduce_kernel<<<nt, kScanThreads, 0, st>>>(in, n, scratch);
+    if (nt <= kScanDirect) {
+        scan_apply_kernel<true><<<nt, kScanThreads, 0, st>>>(in, n, scratch, out);
+        return cudaGetLastError();
+    }
     scan_partials_kernel<<<1, 1024, 0, st>>>(scratch, nt, out + n);
-    scan_apply_kernel<<<nt, kScanThreads, 0, st>>>(in, n, scratch, out);
+    scan_apply_kernel<false><<<nt, kScanThreads, 0, st>>>(in, n, scratch, out);
     return cudaGetLastError();
 }
 

@@ -227,3 +227,42 @@ def test_hull_gjk_verdicts_match_reference_kernel(sdlib):
     got = np.array([(int(a), int(b)) in contact for a, b in g["pairs"]])
     assert np.array_equal(got, g["verdict"])
     eng.close()
+
+
+@pytest.mark.parametrize("seed_mode", [0, 2])
+@pytest.mark.parametrize("counts", [(4, 5, 7), (8, 9, 15, 16, 17), (31, 32, 33, 64), (4, 255, 100)])
+def test_hull_point_counts_bit_exact(sdlib, orc, counts, seed_mode):
+    """Hulls of fewer, as many and more points than lanes share them, and of
+    very unlike counts in one pair, some points twice (equal supports),
+    packed so that many intersect deeply."""
+    from stardust_gb300 import _abi, scenes
+    n = 300
+    _, pos, quat, vel, mass, cfg, dt = scenes.hull_box(n, seed=3, box=(0.2, 0.2, 0.2), spacing=0.0165, vmax=0.3)
+    cfg.flags = _abi.SD_FLAG_RECORD
+    rng = np.random.default_rng(4)
+    pts = []
+    for i in range(n):
+        m = counts[i % len(counts)]
+        d = rng.normal(size=(m, 3))
+        p = d / np.linalg.norm(d, axis=1, keepdims=True) * rng.uniform(0.8, 1.2, (m, 1)) * 0.01
+        if i % 3 == 0 and m > 4:
+            p[m // 2:] = p[:m - m // 2]
+        pts.append(p.astype(np.float32))
+    eng = sdlib.DEMEngine(cfg)
+    sdlib.add_hull_scene(eng, pts, pos, quat, vel, mass)
+    eng.prepare()
+    eng.set_gjk_seed(seed_mode)
+    eng.step(dt, 6)
+    H = oracle_hulls(orc, eng)
+    eng.step(dt, 1)
+    eng.sync()
+    assert eng.stats()["device_errors"] == 0
+    e = eng.hull_entries()
+    out = H.step(oracle_params(orc, cfg, dt), off=e["off"], partners=e["partners"],
+                 seeds=e["seeds"] if seed_mode else None, record=True)
+    assert (out["status"] == 1).sum() > 50
+    assert np.array_equal(e["status"], out["status"]) and np.array_equal(e["iters"], out["iters"])
+    for k, f in (("pos", _abi.SD_BODY_POSITION), ("quat", _abi.SD_BODY_QUATERNION), ("ang", _abi.SD_BODY_ANGMOM)):
+        assert np.array_equal(bits(eng.bodies(f)), bits(getattr(H, k))), k
+    assert np.array_equal(bits(eng.bodies(_abi.SD_BODY_FORCE)), bits(out["force"]))
+    eng.close()

@@ -155,3 +155,17 @@ def test_tree_over_treelets(sdlib, orc, n, spread):
     got, cnt, err = sdlib.BoundingVolumes.pairs(torch.from_numpy(L).cuda(), torch.from_numpy(H).cuda(), len(want) + 1)
     assert err == 0 and cnt == len(want)
     assert np.array_equal(got.cpu().numpy().view(np.uint64), want)
+
+
+@pytest.mark.parametrize("n", [3, 4097, 32_767, 32_768, 32_769, 4_194_304, 4_194_305])
+def test_pair_offsets_over_scan_sizes(sdlib, n):
+    """Either side of the scan's one block (32,768) and of its two launches
+    (2,048 tiles of 2,048): boxes in a row, each on the next one."""
+    import torch
+    x = torch.arange(n, dtype=torch.float32, device="cuda") * 2.0
+    L = torch.zeros((n, 4), device="cuda")
+    H = torch.ones((n, 4), device="cuda")
+    L[:, 0], H[:, 0] = x, x + 2.0
+    got, cnt, err = sdlib.SweepAndPrune.pairs(L, H, n)
+    i = torch.arange(n - 1, device="cuda")
+    assert err == 0 and cnt == n - 1 and torch.equal(got, (i << 32) | (i + 1))
