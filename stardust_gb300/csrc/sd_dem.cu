@@ -1438,6 +1438,7 @@ __global__ void dem_scatter_in_kernel(const float4* __restrict__ src, const floa
 
 // slot_of_id[id] = slot for every sphere (ids in the omega w lane).
 __global__ void dem_slot_of_id_kernel(const float4* __restrict__ omg, uint32_t* __restrict__ slot_of_id, uint32_t n) {
+    stream_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint32_t id = __float_as_uint(omg[i].w) & kIdMask;
@@ -1449,6 +1450,7 @@ __global__ void dem_slot_of_id_kernel(const float4* __restrict__ omg, uint32_t* 
 // slot side is the random one, in device memory.
 __global__ void dem_by_id_in_kernel(const float4* __restrict__ host_src, const uint32_t* __restrict__ slot_of_id,
                                     float4* __restrict__ dst, uint32_t n, bool keep_w) {
+    stream_wait();
     const uint32_t id = blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= n) return;
     const uint32_t s = slot_of_id[id];
@@ -1460,6 +1462,7 @@ __global__ void dem_by_id_in_kernel(const float4* __restrict__ host_src, const u
 
 __global__ void dem_by_id_out_kernel(const float4* __restrict__ src, const uint32_t* __restrict__ slot_of_id,
                                      float4* __restrict__ host_dst, uint32_t n) {
+    stream_wait();
     const uint32_t id = blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= n) return;
     const uint32_t s = slot_of_id[id];
@@ -1884,23 +1887,23 @@ cudaError_t dem_unsort_async(const float4* src, const float4* omg, float4* dst, 
 
 cudaError_t dem_slot_of_all_async(const float4* omg, uint32_t* slot_of, uint32_t n, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    dem_slot_of_id_kernel<<<grid_for(n, 256), 256, 0, st>>>(omg, slot_of, n);
+    launch_after(st, grid_for(n, 256), 256, 0, dem_slot_of_id_kernel, omg, slot_of, n);
     return cudaGetLastError();
 }
 
 cudaError_t dem_host_in_async(const float4* host_src, const float4* omg, float4* dst, uint32_t* slot_of_id,
                               uint32_t n, bool keep_w, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    dem_slot_of_id_kernel<<<grid_for(n, 256), 256, 0, st>>>(omg, slot_of_id, n);
-    dem_by_id_in_kernel<<<grid_for(n, 256), 256, 0, st>>>(host_src, slot_of_id, dst, n, keep_w);
+    launch_after(st, grid_for(n, 256), 256, 0, dem_slot_of_id_kernel, omg, slot_of_id, n);
+    launch_after(st, grid_for(n, 256), 256, 0, dem_by_id_in_kernel, host_src, slot_of_id, dst, n, keep_w);
     return cudaGetLastError();
 }
 
 cudaError_t dem_host_out_async(const float4* src, const float4* omg, float4* host_dst, uint32_t* slot_of_id,
                                uint32_t n, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    dem_slot_of_id_kernel<<<grid_for(n, 256), 256, 0, st>>>(omg, slot_of_id, n);
-    dem_by_id_out_kernel<<<grid_for(n, 256), 256, 0, st>>>(src, slot_of_id, host_dst, n);
+    launch_after(st, grid_for(n, 256), 256, 0, dem_slot_of_id_kernel, omg, slot_of_id, n);
+    launch_after(st, grid_for(n, 256), 256, 0, dem_by_id_out_kernel, src, slot_of_id, host_dst, n);
     return cudaGetLastError();
 }
 

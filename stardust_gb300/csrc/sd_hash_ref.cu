@@ -44,6 +44,7 @@ __global__ void __launch_bounds__(kBuildThreads)
 ref_hash_build_kernel(uint32_t n, float cell_dim, uint32_t* __restrict__ cells, uint32_t* __restrict__ spheres,
                       const float* __restrict__ sizes, const float4* __restrict__ pos4,
                       uint32_t* __restrict__ d_count) {
+    stream_wait();
     __shared__ uint32_t s_cells[9 * kBuildThreads], s_spheres[9 * kBuildThreads];
     const uint32_t first = blockIdx.x * kBuildThreads, i = first + threadIdx.x;
     uint32_t count = 0;
@@ -102,8 +103,8 @@ cudaError_t ref_hash_build_async(uint32_t n, float cell_dim, uint32_t* cells, ui
                                  cudaStream_t st) {
     cudaError_t e = cudaMemsetAsync(d_count, 0, sizeof(uint32_t), st);
     if (e != cudaSuccess || n == 0) return e;
-    ref_hash_build_kernel<<<(n + kBuildThreads - 1) / kBuildThreads, kBuildThreads, 0, st>>>(
-        n, cell_dim, cells, spheres, sizes, pos, d_count);
+    launch_after(st, (n + kBuildThreads - 1) / kBuildThreads, kBuildThreads, 0, ref_hash_build_kernel, n, cell_dim,
+                 cells, spheres, sizes, pos, d_count);
     return cudaGetLastError();
 }
 
@@ -173,6 +174,7 @@ ref_pairs_kernel(const uint32_t* __restrict__ cells, const uint32_t* __restrict_
                  const int32_t* __restrict__ body_of, uint32_t* __restrict__ pair_a,
                  uint32_t* __restrict__ pair_b, uint64_t cap, unsigned long long* __restrict__ d_npairs,
                  uint32_t* __restrict__ scratch) {
+    stream_wait();
     __shared__ uint32_t s_np[kPairTile];              // pairs of every entry
     __shared__ unsigned long long s_off[kPairTile];   // the first of them
     __shared__ unsigned long long s_part[kPairThreads / kWarp];
@@ -296,8 +298,8 @@ cudaError_t ref_candidate_pairs_async(const uint32_t* cells, const uint32_t* sph
     if (e != cudaSuccess) return e;
     if (n_entries == 0) return cudaSuccess;
     uint32_t tiles = (uint32_t)((n_entries + kPairTile - 1) / kPairTile);
-    ref_pairs_kernel<<<tiles, kPairThreads, 0, st>>>(cells, spheres, d_count, n_entries, body_of, pair_a,
-                                                     pair_b, cap, d_npairs, scratch);
+    launch_after(st, tiles, kPairThreads, 0, ref_pairs_kernel, cells, spheres, d_count, n_entries, body_of, pair_a,
+                 pair_b, cap, d_npairs, scratch);
     return cudaGetLastError();
 }
 

@@ -1134,6 +1134,7 @@ cudaError_t hull_seed_async(HullBuffers& H, uint32_t mode, cudaStream_t st) {
 // the step's count return at once.
 __global__ void hull_teach_flags_kernel(const float4* __restrict__ teach, const uint32_t* __restrict__ d_count,
                                         uint32_t cap, uint32_t* __restrict__ flags) {
+    stream_wait();
     const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= cap) return;
     const uint32_t n = min(*d_count, cap);
@@ -1144,6 +1145,7 @@ __global__ void hull_teach_gather_kernel(const float* __restrict__ feat, const f
                                          const uint32_t* __restrict__ flags, const uint32_t* __restrict__ pos,
                                          uint32_t cap, uint32_t rows_cap, float* __restrict__ feat_c,
                                          float4* __restrict__ teach_c, uint32_t* __restrict__ d_total) {
+    stream_wait();
     const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= cap) return;
     if (e == cap - 1) *d_total = min(pos[e] + flags[e], rows_cap);
@@ -1166,11 +1168,11 @@ cudaError_t hull_teach_compact_async(const HullBuffers& H, const uint32_t* d_cou
                                      cudaStream_t st) {
     const uint32_t cap = (uint32_t)H.cap;
     if (cap == 0) return cudaMemsetAsync(d_total, 0, 4, st);
-    hull_teach_flags_kernel<<<grid_for(cap, 256), 256, 0, st>>>(H.teach, d_count, cap, flags);
+    launch_after(st, grid_for(cap, 256), 256, 0, hull_teach_flags_kernel, H.teach, d_count, cap, flags);
     cudaError_t e = scan_exclusive_async(flags, pos, cap, scan, st);
     if (e != cudaSuccess) return e;
-    hull_teach_gather_kernel<<<grid_for(cap, 256), 256, 0, st>>>(H.feat, H.teach, flags, pos, cap, cap / 2 + 1,
-                                                                 feat_c, teach_c, d_total);
+    launch_after(st, grid_for(cap, 256), 256, 0, hull_teach_gather_kernel, H.feat, H.teach, flags, pos, cap,
+                 cap / 2 + 1, feat_c, teach_c, d_total);
     return cudaGetLastError();
 }
 

@@ -51,6 +51,7 @@ __device__ __forceinline__ bool box_overlap(float4 alo, float4 ahi, float4 blo, 
 // ---------------------------------------------------------------- scan
 
 __global__ void scan_reduce_kernel(const uint32_t* __restrict__ in, uint32_t n, uint32_t* __restrict__ part) {
+    stream_wait();
     __shared__ uint32_t ws[33];
     const uint32_t base = blockIdx.x * kScanTile;
     uint32_t s = 0;
@@ -66,6 +67,7 @@ __global__ void scan_reduce_kernel(const uint32_t* __restrict__ in, uint32_t n, 
 
 // One block: exclusive scan of the tile sums; part[nt] = grand total.
 __global__ void scan_partials_kernel(uint32_t* __restrict__ part, uint32_t nt, uint32_t* __restrict__ total_out) {
+    stream_wait();
     __shared__ uint32_t ws[33];
     uint32_t carry = 0;
     for (uint32_t b = 0; b < nt; b += blockDim.x) {
@@ -85,6 +87,7 @@ template <bool SUMS>
 __global__ void __launch_bounds__(kScanThreads)
 scan_apply_kernel(const uint32_t* __restrict__ in, uint32_t n, const uint32_t* __restrict__ part,
                   uint32_t* __restrict__ out) {
+    stream_wait();
     __shared__ uint32_t ws[33];
     uint32_t before = 0;
     if constexpr (SUMS) {
@@ -129,6 +132,7 @@ constexpr uint32_t kScanOne = 32 * 128 * kScanRows;
 
 __global__ void __launch_bounds__(1024) scan_one_kernel(const uint32_t* __restrict__ in, uint32_t n,
                                                         uint32_t* __restrict__ out) {
+    stream_wait();
     __shared__ uint32_t ws[33];
     const uint32_t base = (threadIdx.x >> 5) * (128 * kScanRows) + 4 * lane_id();
     uint4 v[kScanRows];
@@ -172,6 +176,7 @@ __global__ void __launch_bounds__(1024) scan_one_kernel(const uint32_t* __restri
 
 __global__ void bounds_partial_kernel(const float4* __restrict__ lo, const float4* __restrict__ hi, uint32_t n,
                                       float* __restrict__ part) {
+    stream_wait();
     __shared__ float s[6][kLbvhThreads];
     float m[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -198,6 +203,7 @@ __global__ void bounds_partial_kernel(const float4* __restrict__ lo, const float
 // One warp per bound (a thread per bound that reads the partials one after
 // the other took 20 us).
 __global__ void bounds_final_kernel(const float* __restrict__ part, uint32_t nb, float* __restrict__ bounds) {
+    stream_wait();
     const uint32_t k = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     float m = k < 3 ? INFINITY : -INFINITY;
     for (uint32_t b = lane; b < nb; b += 32) m = k < 3 ? fminf(m, part[6 * b + k]) : fmaxf(m, part[6 * b + k]);
@@ -223,6 +229,7 @@ __device__ __forceinline__ uint32_t spread10(uint32_t x) {
 __global__ void morton_kernel(const float4* __restrict__ lo, const float4* __restrict__ hi, uint32_t n,
                               const float* __restrict__ bounds, uint32_t* __restrict__ keys,
                               uint32_t* __restrict__ vals) {
+    stream_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 a = lo[i], b = hi[i];
@@ -256,6 +263,7 @@ __device__ __forceinline__ int delta(const uint32_t* __restrict__ k, int n, int 
 __global__ void build_kernel(const uint32_t* __restrict__ keys, int n, int2* __restrict__ children,
                              int32_t* __restrict__ parent, int32_t* __restrict__ other, float4* __restrict__ node_lo,
                              float4* __restrict__ node_hi, uint32_t* __restrict__ top, uint32_t* __restrict__ n_top) {
+    stream_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n - 1) return;
     const int d = (delta(keys, n, i, i + 1) - delta(keys, n, i, i - 1)) >= 0 ? 1 : -1;
@@ -352,6 +360,7 @@ refit_kernel(int n, const uint32_t* __restrict__ vals, const float4* __restrict_
              float4* __restrict__ leaf_lo, float4* __restrict__ leaf_hi, float4* __restrict__ node_lo,
              float4* __restrict__ node_hi, const int2* __restrict__ children, const int32_t* __restrict__ parent,
              const int32_t* __restrict__ other, float4* __restrict__ rec, uint32_t* __restrict__ status) {
+    stream_wait();
     __shared__ float s_box[2][6][kRefitWindow];  // leaves, nodes
     __shared__ int2 s_children[kRefitWindow];
     __shared__ int s_parent[kRefitWindow], s_other[kRefitWindow];
@@ -446,6 +455,7 @@ __global__ void top_kernel(int n, const uint32_t* __restrict__ top, const uint32
                            const float4* __restrict__ leaf_lo, const float4* __restrict__ leaf_hi, float4* node_lo,
                            float4* node_hi, const int2* __restrict__ children, const int32_t* __restrict__ other,
                            float4* __restrict__ rec, uint32_t* __restrict__ status) {
+    stream_wait();
     const uint32_t m = min(*n_top, (uint32_t)n);
     const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
@@ -510,6 +520,7 @@ __global__ void __launch_bounds__(kQueryThreads)
 query_kernel(int n, const uint32_t* __restrict__ vals, const float4* __restrict__ leaf_lo,
              const float4* __restrict__ leaf_hi, const float4* __restrict__ rec, QueryOut q, PairSink sink,
              uint32_t* __restrict__ status) {
+    stream_wait();
     constexpr bool kUnique = MODE == kPairs || MODE == kRefill;
     constexpr int kLeaves = kQueryThreads / G, kDepth = kStack + 2 * G;
     __shared__ int s_stack[kDepth][kLeaves];
@@ -642,16 +653,16 @@ cudaError_t scan_exclusive_async(const uint32_t* in, uint32_t* out, uint32_t n, 
     // would be more reads than the words themselves.
     const bool aligned = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0;
     if (n <= kScanOne && aligned) {
-        scan_one_kernel<<<1, 1024, 0, st>>>(in, n, out);
+        launch_after(st, 1, 1024, 0, scan_one_kernel, in, n, out);
         return cudaGetLastError();
     }
-    scan_reduce_kernel<<<nt, kScanThreads, 0, st>>>(in, n, scratch);
+    launch_after(st, nt, kScanThreads, 0, scan_reduce_kernel, in, n, scratch);
     if (nt <= kScanDirect) {
-        scan_apply_kernel<true><<<nt, kScanThreads, 0, st>>>(in, n, scratch, out);
+        launch_after(st, nt, kScanThreads, 0, scan_apply_kernel<true>, in, n, scratch, out);
         return cudaGetLastError();
     }
-    scan_partials_kernel<<<1, 1024, 0, st>>>(scratch, nt, out + n);
-    scan_apply_kernel<false><<<nt, kScanThreads, 0, st>>>(in, n, scratch, out);
+    launch_after(st, 1, 1024, 0, scan_partials_kernel, scratch, nt, out + n);
+    launch_after(st, nt, kScanThreads, 0, scan_apply_kernel<false>, in, n, scratch, out);
     return cudaGetLastError();
 }
 
@@ -707,9 +718,9 @@ cudaError_t lbvh_morton_async(Lbvh& t, const float4* lo, const float4* hi, cudaS
     const uint32_t n = t.n;
     if (n == 0) return cudaSuccess;
     const uint32_t nb = bounds_blocks(n);
-    bounds_partial_kernel<<<nb, kLbvhThreads, 0, st>>>(lo, hi, n, t.bound_part);
-    bounds_final_kernel<<<1, 6 * 32, 0, st>>>(t.bound_part, nb, t.bounds);
-    morton_kernel<<<grid_for(n, kLbvhThreads), kLbvhThreads, 0, st>>>(lo, hi, n, t.bounds, t.keys, t.vals);
+    launch_after(st, nb, kLbvhThreads, 0, bounds_partial_kernel, lo, hi, n, t.bound_part);
+    launch_after(st, 1, 6 * 32, 0, bounds_final_kernel, t.bound_part, nb, t.bounds);
+    launch_after(st, grid_for(n, kLbvhThreads), kLbvhThreads, 0, morton_kernel, lo, hi, n, t.bounds, t.keys, t.vals);
     return cudaGetLastError();
 }
 
@@ -725,22 +736,20 @@ cudaError_t lbvh_build_async(Lbvh& t, const float4* lo, const float4* hi, cudaSt
     t.skeys = in_tmp ? t.keys_tmp : t.keys;
     t.svals = in_tmp ? t.vals_tmp : t.vals;
     if (n > 1)
-        build_kernel<<<grid_for(n - 1, kLbvhThreads), kLbvhThreads, 0, st>>>(t.skeys, (int)n, t.children, t.parent, t.other,
-                                                                              t.node_lo, t.node_hi, t.top,
-                                                                              top_count(t.bounds));
+        launch_after(st, grid_for(n - 1, kLbvhThreads), kLbvhThreads, 0, build_kernel, t.skeys, (int)n, t.children,
+                     t.parent, t.other, t.node_lo, t.node_hi, t.top, top_count(t.bounds));
     return lbvh_refit_async(t, lo, hi, st);
 }
 
 cudaError_t lbvh_refit_async(Lbvh& t, const float4* lo, const float4* hi, cudaStream_t st) {
     const uint32_t n = t.n;
     if (n == 0) return cudaSuccess;
-    refit_kernel<<<grid_for(n, kRefitSpan), kRefitWindow, 0, st>>>((int)n, t.svals, lo, hi, t.leaf_lo, t.leaf_hi, t.node_lo,
-                                                                   t.node_hi, t.children, t.parent, t.other, t.rec,
-                                                                   t.status);
+    launch_after(st, grid_for(n, kRefitSpan), kRefitWindow, 0, refit_kernel, (int)n, t.svals, lo, hi, t.leaf_lo,
+                 t.leaf_hi, t.node_lo, t.node_hi, t.children, t.parent, t.other, t.rec, t.status);
     if (n > (uint32_t)kTreelet)
-        top_kernel<<<std::min(152u, grid_for(n, kTreelet)), 128, 0, st>>>((int)n, t.top, top_count(t.bounds), t.leaf_lo,
-                                                                          t.leaf_hi, t.node_lo, t.node_hi, t.children,
-                                                                          t.other, t.rec, t.status);
+        launch_after(st, std::min(152u, grid_for(n, kTreelet)), 128, 0, top_kernel, (int)n, t.top,
+                     top_count(t.bounds), t.leaf_lo, t.leaf_hi, t.node_lo, t.node_hi, t.children, t.other, t.rec,
+                     t.status);
     return cudaGetLastError();
 }
 
@@ -759,8 +768,8 @@ template <int MODE>
 static void launch_query(const Lbvh& t, const QueryOut& q, const PairSink& sink, cudaStream_t st) {
     const int n = (int)t.n;
     const auto go = [&](auto kernel, int lanes) {
-        kernel<<<grid_for(t.n, kQueryThreads / lanes), kQueryThreads, 0, st>>>(n, t.svals, t.leaf_lo, t.leaf_hi, t.rec, q,
-                                                                              sink, t.status);
+        launch_after(st, grid_for(t.n, kQueryThreads / lanes), kQueryThreads, 0, kernel, n, t.svals, t.leaf_lo,
+                     t.leaf_hi, t.rec, q, sink, t.status);
     };
     if (t.n < kWideLeaves) go(query_kernel<MODE, 4>, 4);
     else go(query_kernel<MODE, 2>, 2);
@@ -790,7 +799,7 @@ cudaError_t lbvh_unique_pairs_async(Lbvh& t, uint32_t* off, unsigned long long* 
     launch_query<kPairs>(t, QueryOut{}, sink, st);
     if ((e = scan_exclusive_async(t.counts, off, n, t.scan_scratch, st)) != cudaSuccess) return e;
     launch_query<kRefill>(t, QueryOut{}, sink, st);
-    pairs_write_kernel<<<grid_for(n, kLbvhThreads), kLbvhThreads, 0, st>>>(sink, d_count2, t.status);
+    launch_after(st, grid_for(n, kLbvhThreads), kLbvhThreads, 0, pairs_write_kernel, sink, d_count2, t.status);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     return cudaMemcpyAsync(d_count2 + 1, t.status, 4, cudaMemcpyDeviceToDevice, st);
 }

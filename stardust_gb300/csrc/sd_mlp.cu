@@ -314,6 +314,7 @@ __global__ void __launch_bounds__(kRows) mlp_forward_kernel(const uint8_t* __res
                                                            const float* __restrict__ feat, float4* __restrict__ out,
                                                            const uint32_t* __restrict__ d_count, uint64_t n,
                                                            uint32_t* __restrict__ status) {
+    stream_wait();
     extern __shared__ __align__(16) uint8_t smem_raw[];
     InferSmem& S = *reinterpret_cast<InferSmem*>(aligned_smem(smem_raw));
     const uint32_t tid = threadIdx.x, warp = tid >> 5;
@@ -396,6 +397,7 @@ __global__ void __launch_bounds__(kRows) mlp_train_kernel(const uint8_t* __restr
                                                          uint32_t n, float inv_batch, float* __restrict__ part,
                                                          uint32_t* __restrict__ status,
                                                          const uint32_t* __restrict__ d_count, bool vec) {
+    stream_wait();
     extern __shared__ __align__(16) uint8_t smem_raw[];
     TrainSmem& S = *reinterpret_cast<TrainSmem*>(aligned_smem(smem_raw));
     const uint32_t tid = threadIdx.x, warp = tid >> 5;
@@ -548,6 +550,7 @@ __global__ void __launch_bounds__(32 * kSlices)
 mlp_reduce_kernel(const float* __restrict__ part, uint32_t nparts, uint32_t n, const uint32_t* __restrict__ d_count,
                   float* __restrict__ grad, float* __restrict__ params, float* __restrict__ m1,
                   float* __restrict__ m2, uint8_t* __restrict__ img, int adam, float lr, float c1, float c2) {
+    stream_wait();
     __shared__ float s[kSlices][32];
     const uint32_t lane = threadIdx.x & 31u, slice = threadIdx.x >> 5, p = blockIdx.x * 32 + lane;
     if (d_count) n = min(n, *d_count);
@@ -576,6 +579,7 @@ mlp_reduce_kernel(const float* __restrict__ part, uint32_t nparts, uint32_t n, c
 }
 
 __global__ void mlp_pack_kernel(const float* __restrict__ params, uint8_t* __restrict__ img) {
+    stream_wait();
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p < (uint32_t)kParams) pack_param(p, params[p], img);
 }
@@ -622,7 +626,7 @@ cudaError_t mlp_set_params_async(MlpState& s, const float* host_params, cudaStre
     if (e == cudaSuccess) e = cudaMemsetAsync(s.m1, 0, 8ull * kParams, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(s.img, 0, kImgBytes, st);
     if (e != cudaSuccess) return e;
-    mlp_pack_kernel<<<grid_for(kParams, 256), 256, 0, st>>>(s.params, s.img);
+    launch_after(st, grid_for(kParams, 256), 256, 0, mlp_pack_kernel, s.params, s.img);
     return cudaGetLastError();
 }
 
@@ -636,9 +640,9 @@ cudaError_t mlp_forward_async(const MlpState& s, const float* feat, float4* out,
     const uint32_t grid = tiles < 304 ? tiles : 304;
     const size_t sm = sizeof(InferSmem) + 1024;
     if (seeds)
-        mlp_forward_kernel<0><<<grid, kRows, sm, st>>>(s.img, s.params, feat, out, d_count, n, s.status);
+        launch_after(st, grid, kRows, sm, mlp_forward_kernel<0>, s.img, s.params, feat, out, d_count, n, s.status);
     else
-        mlp_forward_kernel<1><<<grid, kRows, sm, st>>>(s.img, s.params, feat, out, nullptr, n, s.status);
+        launch_after(st, grid, kRows, sm, mlp_forward_kernel<1>, s.img, s.params, feat, out, nullptr, n, s.status);
     return cudaGetLastError();
 }
 
@@ -648,13 +652,12 @@ cudaError_t mlp_train_async(MlpState& s, const float* feat, const float4* tgt, u
     const uint32_t tiles = grid_for(n, kRows);
     const uint32_t ctas = tiles < kMaxTrainCtas ? tiles : kMaxTrainCtas;
     const float inv = n_valid ? 1.0f / (float)n_valid : 0.0f;
-    mlp_train_kernel<<<ctas, kRows, sizeof(TrainSmem) + 1024, st>>>(s.img, s.params, feat, tgt, n, inv, s.part,
-                                                                     s.status, d_count,
-                                                                     (reinterpret_cast<uintptr_t>(feat) & 15u) == 0);
+    launch_after(st, ctas, kRows, sizeof(TrainSmem) + 1024, mlp_train_kernel, s.img, s.params, feat, tgt, n, inv,
+                 s.part, s.status, d_count, (reinterpret_cast<uintptr_t>(feat) & 15u) == 0);
     const float c1 = update ? (float)(1.0 / (1.0 - std::pow(0.9, (double)adam_step))) : 0.f;
     const float c2 = update ? (float)(1.0 / (1.0 - std::pow(0.999, (double)adam_step))) : 0.f;
-    mlp_reduce_kernel<<<grid_for(kParams, 32), 32 * kSlices, 0, st>>>(s.part, ctas, n, d_count, s.grad, s.params, s.m1,
-                                                                      s.m2, s.img, update ? 1 : 0, lr, c1, c2);
+    launch_after(st, grid_for(kParams, 32), 32 * kSlices, 0, mlp_reduce_kernel, s.part, ctas, n, d_count, s.grad,
+                 s.params, s.m1, s.m2, s.img, update ? 1 : 0, lr, c1, c2);
     return cudaGetLastError();
 }
 

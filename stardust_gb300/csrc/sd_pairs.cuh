@@ -50,6 +50,7 @@ __device__ __forceinline__ void sink_pair_again(const PairSink& s, uint32_t a, u
 }
 
 static __global__ void pairs_write_kernel(PairSink s, uint32_t* __restrict__ d_count, uint32_t* __restrict__ status) {
+    stream_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t total = s.off[s.n];
     const bool fits = total <= s.cap;

@@ -55,6 +55,7 @@ __device__ __forceinline__ uint32_t float_key(float x) {
 
 __global__ void aabb_kernel(uint32_t n, const float4* __restrict__ pos, const float* __restrict__ radius,
                             float4* __restrict__ lo, float4* __restrict__ hi) {
+    stream_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 p = pos[i];
@@ -67,6 +68,7 @@ __global__ void aabb_kernel(uint32_t n, const float4* __restrict__ pos, const fl
 // for non-negative x) or the order-preserving image.
 __global__ void lower_x_keys_kernel(uint32_t n, const float4* __restrict__ lo, uint32_t* __restrict__ keys,
                                     uint32_t* __restrict__ vals, int ordered) {
+    stream_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     keys[i] = ordered ? float_key(lo[i].x) : __float_as_uint(lo[i].x);
@@ -76,6 +78,7 @@ __global__ void lower_x_keys_kernel(uint32_t n, const float4* __restrict__ lo, u
 __global__ void sweep_ref_kernel(uint32_t n, const float* __restrict__ upperx, const float* __restrict__ lowerx_sorted,
                                  const float* __restrict__ uppery, const float* __restrict__ lowery,
                                  const uint32_t* __restrict__ idx_sorted, int32_t* __restrict__ rows) {
+    stream_wait();
     const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
     if (tid >= n) return;
     int32_t row[kRefPadding];
@@ -137,6 +140,7 @@ constexpr int kBoundBlocks = 152 * 4;
 __global__ void __launch_bounds__(kSapThreads)
 sap_bounds_kernel(uint32_t n, const float4* __restrict__ lo, const float4* __restrict__ hi, SapBounds* __restrict__ out,
                   uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
+    stream_wait();
     __shared__ uint32_t s_w[5], s_count;
     __shared__ double s_sum;
     if (threadIdx.x < 5) s_w[threadIdx.x] = 0u;
@@ -225,6 +229,7 @@ __device__ __forceinline__ SapSpan sap_span(const SapGrid& g, float4 a, float4 b
 __global__ void sap_gather_kernel(uint32_t n, const uint32_t* __restrict__ svals, const float4* __restrict__ lo,
                                   const float4* __restrict__ hi, const SapBounds* __restrict__ bounds,
                                   float4* __restrict__ box, uint32_t* __restrict__ count, uint32_t* __restrict__ status) {
+    stream_wait();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const SapGrid g = sap_grid(*bounds);
@@ -240,6 +245,7 @@ __global__ void sap_gather_kernel(uint32_t n, const uint32_t* __restrict__ svals
 __global__ void sap_entries_kernel(uint32_t n, const float4* __restrict__ box, const SapBounds* __restrict__ bounds,
                                    const uint32_t* __restrict__ off, uint32_t* __restrict__ keys,
                                    uint32_t* __restrict__ vals) {
+    stream_wait();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const SapGrid g = sap_grid(*bounds);
@@ -261,6 +267,7 @@ template <bool REFILL>
 __global__ void sweep_binned_kernel(const uint32_t* __restrict__ d_entries, const uint32_t* __restrict__ ckeys,
                                     const uint32_t* __restrict__ cvals, const float4* __restrict__ box,
                                     const SapBounds* __restrict__ bounds, PairSink sink) {
+    stream_wait();
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x, n_entries = *d_entries;
     if (p >= n_entries) return;
     if (REFILL && !sink_refill(sink)) return;
@@ -286,6 +293,7 @@ __global__ void sweep_binned_kernel(const uint32_t* __restrict__ d_entries, cons
 
 __global__ void project_kernel(uint32_t n, const float4* __restrict__ lo, const float4* __restrict__ hi,
                                float* __restrict__ upperx, float* __restrict__ uppery, float* __restrict__ lowery) {
+    stream_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     upperx[i] = hi[i].x;
@@ -307,7 +315,7 @@ uint64_t sap_scratch_bytes(uint64_t n, uint64_t pair_cap) {
 cudaError_t sap_aabb_async(uint32_t n, const float4* pos, const float* radius, float4* lo, float4* hi,
                            cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    aabb_kernel<<<grid_for(n, kSapThreads), kSapThreads, 0, st>>>(n, pos, radius, lo, hi);
+    launch_after(st, grid_for(n, kSapThreads), kSapThreads, 0, aabb_kernel, n, pos, radius, lo, hi);
     return cudaGetLastError();
 }
 
@@ -316,15 +324,16 @@ cudaError_t sap_sort_lower_x_async(uint32_t n, const float4* lo, bool ordered, u
                                    cudaStream_t st) {
     *in_tmp = false;
     if (n == 0) return cudaSuccess;
-    lower_x_keys_kernel<<<grid_for(n, kSapThreads), kSapThreads, 0, st>>>(n, lo, keys, vals, ordered ? 1 : 0);
+    launch_after(st, grid_for(n, kSapThreads), kSapThreads, 0, lower_x_keys_kernel, n, lo, keys, vals,
+                 ordered ? 1 : 0);
     return sort_pairs_async(keys, vals, keys_tmp, vals_tmp, n, 32, sort_scratch, st, in_tmp);
 }
 
 cudaError_t sap_sweep_ref_async(uint32_t n, const float* upperx, const float* lowerx_sorted, const float* uppery,
                                 const float* lowery, const uint32_t* idx_sorted, int32_t* rows, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    sweep_ref_kernel<<<grid_for(n, kSapThreads), kSapThreads, 0, st>>>(n, upperx, lowerx_sorted, uppery, lowery,
-                                                                       idx_sorted, rows);
+    launch_after(st, grid_for(n, kSapThreads), kSapThreads, 0, sweep_ref_kernel, n, upperx, lowerx_sorted, uppery,
+                 lowery, idx_sorted, rows);
     return cudaGetLastError();
 }
 
@@ -362,13 +371,15 @@ cudaError_t sap_pairs_async(uint32_t n, const float4* lo, const float4* hi, void
     if (n == 0) return cudaMemsetAsync(d_count2, 0, 8, st);
     const uint32_t grid = grid_for(n, kSapThreads);
     if ((e = cudaMemsetAsync(bounds, 0, sizeof(SapBounds), st)) != cudaSuccess) return e;
-    sap_bounds_kernel<<<std::min<uint32_t>(grid, kBoundBlocks), kSapThreads, 0, st>>>(n, lo, hi, bounds, keys, vals);
+    launch_after(st, std::min<uint32_t>(grid, kBoundBlocks), kSapThreads, 0, sap_bounds_kernel, n, lo, hi, bounds,
+                 keys, vals);
     bool in_tmp = false;
     if ((e = sort_pairs_async(keys, vals, keys_tmp, vals_tmp, n, 32, sort_scratch, st, &in_tmp)) != cudaSuccess) return e;
     // each box's entries, stably sorted by column
-    sap_gather_kernel<<<grid, kSapThreads, 0, st>>>(n, in_tmp ? vals_tmp : vals, lo, hi, bounds, box, counts, status);
+    launch_after(st, grid, kSapThreads, 0, sap_gather_kernel, n, in_tmp ? vals_tmp : vals, lo, hi, bounds, box,
+                 counts, status);
     if ((e = scan_exclusive_async(counts, eoff, n, scan, st)) != cudaSuccess) return e;
-    sap_entries_kernel<<<grid, kSapThreads, 0, st>>>(n, box, bounds, eoff, ckeys, cvals);
+    launch_after(st, grid, kSapThreads, 0, sap_entries_kernel, n, box, bounds, eoff, ckeys, cvals);
     const uint32_t ne = kSlots * n;
     bool c_tmp = false;
     if ((e = sort_pairs_async(ckeys, cvals, ckeys_tmp, cvals_tmp, ne, 16, csort, st, &c_tmp, eoff + n)) != cudaSuccess)
@@ -378,10 +389,12 @@ cudaError_t sap_pairs_async(uint32_t n, const float4* lo, const float4* hi, void
     const PairSink sink{counts, keep, status + 1, off, cursor, out, n, pair_cap};
     if ((e = cudaMemsetAsync(counts, 0, 4 * m, st)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(cursor, 0, 4 * m, st)) != cudaSuccess) return e;
-    sweep_binned_kernel<false><<<grid_for(ne, kSapThreads), kSapThreads, 0, st>>>(eoff + n, sk, sv, box, bounds, sink);
+    launch_after(st, grid_for(ne, kSapThreads), kSapThreads, 0, sweep_binned_kernel<false>, eoff + n, sk, sv, box,
+                 bounds, sink);
     if ((e = scan_exclusive_async(counts, off, n, scan, st)) != cudaSuccess) return e;
-    sweep_binned_kernel<true><<<grid_for(ne, kSapThreads), kSapThreads, 0, st>>>(eoff + n, sk, sv, box, bounds, sink);
-    pairs_write_kernel<<<grid, kSapThreads, 0, st>>>(sink, d_count2, status);
+    launch_after(st, grid_for(ne, kSapThreads), kSapThreads, 0, sweep_binned_kernel<true>, eoff + n, sk, sv, box,
+                 bounds, sink);
+    launch_after(st, grid, kSapThreads, 0, pairs_write_kernel, sink, d_count2, status);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     return cudaMemcpyAsync(d_count2 + 1, status, 4, cudaMemcpyDeviceToDevice, st);
 }
@@ -461,7 +474,8 @@ sd_status sd_sap_process_collisions(uint64_t n, const float* d_pos4, const float
         e = sd::sap_sort_lower_x_async((uint32_t)n, lo, false, keys, vals, keys_tmp, vals_tmp, sort_scratch, &in_tmp,
                                        st);
     if (e == cudaSuccess) {
-        sd::project_kernel<<<sd::grid_for(n, sd::kSapThreads), sd::kSapThreads, 0, st>>>((uint32_t)n, lo, hi, upperx, uppery, lowery);
+        sd::launch_after(st, sd::grid_for(n, sd::kSapThreads), sd::kSapThreads, 0, sd::project_kernel, (uint32_t)n,
+                         lo, hi, upperx, uppery, lowery);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess)

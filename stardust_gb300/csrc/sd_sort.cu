@@ -69,6 +69,7 @@ constexpr uint32_t tile_keys() { return kSortThreads * ITEMS; }
 __global__ void __launch_bounds__(kHistThreads)
 sort_histogram_kernel(const uint32_t* __restrict__ keys, uint32_t n, SortPlan plan, uint32_t* __restrict__ scratch,
                       bool vec, const uint32_t* __restrict__ d_n) {
+    stream_wait();
     if (d_n) n = min(n, *d_n);
     __shared__ uint32_t hist[2048];  // pass p at p * plan.stride
     block_histograms<false>(keys, nullptr, n, plan, scratch, hist, vec);
@@ -84,6 +85,7 @@ __global__ void __launch_bounds__(kHistThreads)
 sort_hist_fallback_kernel(const uint32_t* __restrict__ keys, uint32_t* __restrict__ vals, uint32_t n,
                           SortPlan plan, uint32_t* __restrict__ scratch, const uint32_t* __restrict__ skip,
                           uint32_t skip_max, uint64_t words, bool vec) {
+    stream_wait();
     if (skip[1] <= skip_max) return;
     const uint64_t gstride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; w < words; w += gstride)
@@ -102,6 +104,7 @@ sort_pass_kernel(const uint32_t* __restrict__ keys_in, const uint32_t* __restric
                  int shift, int bits, int pass, uint32_t num_tiles, uint32_t hstride, uint32_t bins,
                  uint32_t* __restrict__ scratch, const uint32_t* __restrict__ skip, uint32_t skip_max,
                  const uint32_t* __restrict__ d_n) {
+    stream_wait();
     if (skip && skip[1] <= skip_max) return;  // the incremental re-sort wrote the result
     if (d_n) n = min(n, *d_n);
     extern __shared__ __align__(16) uint32_t smem[];
@@ -152,7 +155,8 @@ static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 
 static cudaError_t sort_histogram_async(const uint32_t* keys, uint32_t n, const SortPlan& plan, uint32_t* scratch,
                                         cudaStream_t st, const uint32_t* d_n) {
-    sort_histogram_kernel<<<hist_blocks(n), kHistThreads, 0, st>>>(keys, n, plan, scratch, aligned16(keys), d_n);
+    launch_after(st, hist_blocks(n), kHistThreads, 0, sort_histogram_kernel, keys, n, plan, scratch,
+                 aligned16(keys), d_n);
     return cudaGetLastError();
 }
 
@@ -167,9 +171,8 @@ static cudaError_t launch_pass(const uint32_t* ki, const uint32_t* vi, uint32_t*
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         if (e != cudaSuccess) return e;
     }
-    sort_pass_kernel<BINS, ITEMS><<<tiles, kSortThreads, sm, st>>>(ki, vi, ko, vo, n, shift, bits,
-                                                                   pass, tiles, stride, bins, scratch, skip,
-                                                                   skip_max, d_n);
+    launch_after(st, tiles, kSortThreads, sm, sort_pass_kernel<BINS, ITEMS>, ki, vi, ko, vo, n, shift, bits, pass,
+                 tiles, stride, bins, scratch, skip, skip_max, d_n);
     return cudaGetLastError();
 }
 
@@ -211,8 +214,8 @@ cudaError_t sort_fallback_async(uint32_t* keys, uint32_t* vals, uint32_t* keys_t
     *in_tmp = false;
     if (n == 0) return cudaSuccess;
     const uint64_t words = (uint64_t)plan.passes * status_words(num_tiles(n), status_bins(plan));
-    sort_hist_fallback_kernel<<<hist_blocks(n), kHistThreads, 0, st>>>(keys, vals, n, plan, scratch, skip, skip_max,
-                                                                       words, aligned16(keys));
+    launch_after(st, hist_blocks(n), kHistThreads, 0, sort_hist_fallback_kernel, keys, vals, n, plan, scratch, skip,
+                 skip_max, words, aligned16(keys));
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     return sort_passes_async(keys, vals, keys_tmp, vals_tmp, n, plan, scratch, st, in_tmp, skip, skip_max);

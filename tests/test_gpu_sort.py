@@ -123,3 +123,54 @@ def test_sort_look_back_groups(sdlib, items, n, kind):
             assert np.array_equal(buf[0].cpu().numpy().view(np.uint32), keys[order])
     finally:
         sdlib._abi.tune_set("sort_items", before)
+
+
+@pytest.mark.parametrize("n", [1, 4097, 300_000])
+def test_chained_launches_in_streams_and_graphs(sdlib, orc, n):
+    """Operators back to back on one stream, each on what the last one wrote,
+    with the caller's own kernels and copies between them; and the same chain
+    captured and replayed, where the launches are plain ones."""
+    import torch
+    P = sdlib.SpatialPartition
+    rng = np.random.default_rng(n)
+    host = rng.integers(0, 2 ** 32, n, dtype=np.uint32)
+    src = torch.from_numpy(host.view(np.int32)).cuda()
+    k, v, kt, vt = (torch.empty_like(src) for _ in range(4))
+    scratch = torch.zeros((P.sort_scratch_bytes(n, 32) + 3) // 4, dtype=torch.int32, device="cuda")
+    ids = torch.arange(n, dtype=torch.int32, device="cuda")
+
+    def chain():
+        k.copy_(src)
+        v.copy_(ids)
+        for _ in range(3):
+            P.sort_collision_list(k, v, kt, vt, n, scratch)
+            k.bitwise_not_()
+        P.sort_collision_list(k, v, kt, vt, n, scratch)
+
+    want_k, want_v = host, np.arange(n, dtype=np.uint32)
+    for _ in range(3):
+        want_k, want_v = orc.radix_sort_pairs(want_k, want_v, 32)
+        want_k = ~want_k
+    want_k, want_v = orc.radix_sort_pairs(want_k, want_v, 32)
+
+    def check():
+        torch.cuda.synchronize()
+        assert np.array_equal(k.cpu().numpy().view(np.uint32), want_k)
+        assert np.array_equal(v.cpu().numpy().view(np.uint32), want_v)
+
+    chain()
+    check()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        for _ in range(4):
+            chain()
+    check()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        chain()
+    for t in (k, v, kt, vt):
+        t.zero_()
+    for _ in range(3):
+        graph.replay()
+    check()
