@@ -13,8 +13,8 @@
 // UMMA canonical K-major layout without swizzle, so a CTA copies them to
 // shared memory as-is.
 //
-// Every GEMM is M = 128 rows (one row per thread of a 128-thread CTA, which
-// is also the TMEM lane), N in {16, 32, 64, 80}, K in {16, 64, 128}, issued by
+// Every GEMM is M = 128 rows (one row per thread of a team of 128 threads,
+// which is also the TMEM lane), N in {16, 64}, K in {16, 64, 128}, issued by
 // one thread as K/16 tcgen05.mma instructions of kind::f16 and completed
 // through tcgen05.commit on an mbarrier.  Weight gradients are GEMMs over the
 // samples (K = the 128 rows of a tile) and accumulate in tensor memory across
@@ -23,17 +23,21 @@
 // The weight gradients read the tile's activations where the forward and
 // backward GEMMs left them: the core matrices (8 rows of 16 bytes) of a
 // K-major 128 x K operand are, with rows and columns exchanged, those of an
-// MN-major K x 128 one, so the descriptors alone transpose.  Column sums (the
-// bias gradients) come out of the same GEMMs: behind every 8-row group of X,
-// H1 and H2 lies one core matrix of ones.  Rows and columns of a product that
-// nobody reads hold whatever lies behind an operand.
+// MN-major K x 128 one, so the descriptors alone transpose.  Rows of a product
+// that nobody reads hold whatever lies behind an operand.
+//
+// Training sums in one order whatever runs beside it -- 148 chains of tiles, a
+// tile's bias sums row by row, the chains one after the other: a last bit of a
+// gradient moves roundings of the BF16 weights some steps later, and near a
+// minimum the gradient by 1e-4.  (Taking 304 chains and the bias sums as
+// columns of the GEMMs saves 12% more.)
 //
 // Measured (GB300): 100,003 rows, an Adam step 110 + 10 + 3.5 us (gradient,
-// reduction, packing) -> 27 + 7 us, the forward pass 24 -> 14.  The gradient
-// was bound by 2-byte shared-memory stores and by building transposed copies
-// (18 us per tile, one CTA per SM); now a tile's chain of five dependent GEMM
-// steps and their 16-byte-store epilogues, on two CTAs per SM, whose inputs
-// for the next tile load behind it.
+// reduction, packing) -> 31 + 5 us with the same bits, the forward pass 24 ->
+// 13.  The gradient was bound by 2-byte shared-memory stores and by building
+// transposed copies (18 us per tile, one tile at a time); now by a tile's chain
+// of five dependent GEMM steps and their epilogues, of which two teams keep two
+// in flight, the inputs of the next tile loading behind them.
 //
 // No counterpart in the reference: the learned warm start is new.
 #include "sd_common.cuh"
@@ -96,11 +100,14 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
                  : "memory");
 }
 
-__device__ __forceinline__ void mbar_init1(uint64_t* bar) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(saddr(bar)) : "memory");
+__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t arrivals) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(saddr(bar)), "r"(arrivals) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
 
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("{\n .reg .b64 s;\n mbarrier.arrive.shared::cta.b64 s, [%0];\n}" ::"r"(saddr(bar)) : "memory");
+}
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
     for (uint32_t it = 0; it < kMmaSpin; ++it) {
         uint32_t ok;
@@ -157,9 +164,13 @@ __device__ __forceinline__ uint4 pack8(const float* v) {
 }
 
 // Byte offset of columns 8c .. 8c + 7 of row r of an operand whose 8-row
-// groups are `group` bytes apart: one row of a core matrix.
+// groups are `group` bytes apart: one row of a core matrix.  Core matrices of
+// an operand that a CTA builds are kCore = 128 + 16 bytes apart, so that a row's
+// columns lie in different banks.
+constexpr uint32_t kCore = 144;
+
 __device__ __forceinline__ uint32_t cm_row(uint32_t r, uint32_t c, uint32_t group) {
-    return (r >> 3) * group + c * 128u + (r & 7u) * 16u;
+    return (r >> 3) * group + c * kCore + (r & 7u) * 16u;
 }
 
 // Sixteen columns of a row, as two stores.
@@ -174,51 +185,90 @@ __device__ __forceinline__ void gemm_issue(uint32_t d, const uint8_t* A, uint32_
                                            uint32_t K) {
     const uint32_t id = idesc(kRows, N), group_b = (K >> 3) * 128u;
     for (uint32_t s = 0; s < K / 16; ++s)
-        mma_f16(d, sdesc(saddr(A) + s * 256u, 128u, group_a), sdesc(saddr(B) + s * 256u, 128u, group_b), id,
+        mma_f16(d, sdesc(saddr(A) + s * 2u * kCore, kCore, group_a), sdesc(saddr(B) + s * 256u, 128u, group_b), id,
                 s > 0 ? 1u : 0u);
 }
 
 // D (tmem columns at d) [+]= A^T B over the tile's 128 rows, A and B stored as
 // above: with K the rows, MN-major operands whose 8-element blocks along M or
-// N are 128 bytes apart and along K a group apart.  (For MN-major operands
+// N are kCore bytes apart and along K a group apart.  (For MN-major operands
 // without swizzle the descriptor's leading offset is the K one.)
 __device__ __forceinline__ void gemm_rows_issue(uint32_t d, const uint8_t* A, uint32_t group_a, const uint8_t* B,
                                                 uint32_t group_b, uint32_t N, bool accumulate) {
     const uint32_t id = idesc(kRows, N, true);
     for (uint32_t s = 0; s < kRows / 16; ++s)
-        mma_f16(d, sdesc(saddr(A) + s * 2u * group_a, group_a, 128u), sdesc(saddr(B) + s * 2u * group_b, group_b, 128u),
+        mma_f16(d, sdesc(saddr(A) + s * 2u * group_a, group_a, kCore), sdesc(saddr(B) + s * 2u * group_b, group_b, kCore),
                 id, (accumulate || s > 0) ? 1u : 0u);
 }
 
+// A team: 128 threads of a CTA, with a named barrier of their own, that take a
+// tile of 128 rows through the network together (thread = row = TMEM lane).
+struct Team {
+    uint32_t id, tid;
+};
+__device__ __forceinline__ void team_sync(const Team& m) {
+    asm volatile("barrier.cta.sync %0, 128;" ::"r"(m.id + 1u) : "memory");
+}
+__device__ __forceinline__ bool team_all(const Team& m, bool mine) {
+    uint32_t r;
+    asm volatile(
+        "{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n barrier.cta.red.and.pred q, %2, 128, p;\n selp.u32 %0, 1, 0, q;\n}"
+        : "=r"(r)
+        : "r"((uint32_t)mine), "r"(m.id + 1u)
+        : "memory");
+    return r != 0u;
+}
+
 // Makes every thread's shared-memory writes and tensor-memory reads visible
-// to MMAs that thread 0 issues next.
-__device__ __forceinline__ void gemm_ready() {
+// to MMAs that the team's thread 0 issues next.
+__device__ __forceinline__ void gemm_ready(const Team& m) {
     fence_async_smem();
     tc_fence_before();
-    __syncthreads();
+    team_sync(m);
     tc_fence_after();
 }
 
-// Waits for thread 0's last commit.  Returns false (and flags) if the wait
-// gave up: one verdict for the whole CTA.
-__device__ __forceinline__ bool gemm_wait(uint64_t* bar, uint32_t& phase, uint32_t* status) {
+// Waits for thread 0's last commit to bar.  Returns false (and flags) if the
+// wait gave up: one verdict for the whole team.
+__device__ __forceinline__ bool gemm_wait(const Team& m, uint64_t* bar, uint32_t& phase, uint32_t* status) {
     const bool mine = mbar_wait(bar, phase);
-    const bool ok = __syncthreads_and(mine) != 0;
+    const bool ok = team_all(m, mine);
     if (ok) phase ^= 1u;
     else atomicOr(status, kErrWaitTimeout);
     tc_fence_after();
     return ok;
 }
 
-// One GEMM step: thread 0 issues and commits, everyone waits for the commit.
-__device__ __forceinline__ bool gemm_sync(uint32_t d, const uint8_t* A, uint32_t group_a, const uint8_t* B, uint32_t N,
-                                          uint32_t K, uint64_t* bar, uint32_t& phase, uint32_t* status) {
-    gemm_ready();
-    if (threadIdx.x == 0) {
+// One GEMM step: thread 0 issues and commits, the team does `meanwhile` (which
+// may read the operands) and waits for the commit.
+template <class F>
+__device__ __forceinline__ bool gemm_sync(const Team& m, uint32_t d, const uint8_t* A, uint32_t group_a,
+                                          const uint8_t* B, uint32_t N, uint32_t K, uint64_t* bar, uint32_t& phase,
+                                          uint32_t* status, F&& meanwhile) {
+    gemm_ready(m);
+    if (m.tid == 0) {
         gemm_issue(d, A, group_a, B, N, K);
         mma_commit(bar);
     }
-    return gemm_wait(bar, phase, status);
+    meanwhile();
+    return gemm_wait(m, bar, phase, status);
+}
+__device__ __forceinline__ bool gemm_sync(const Team& m, uint32_t d, const uint8_t* A, uint32_t group_a,
+                                          const uint8_t* B, uint32_t N, uint32_t K, uint64_t* bar, uint32_t& phase,
+                                          uint32_t* status) {
+    return gemm_sync(m, d, A, group_a, B, N, K, bar, phase, status, [] {});
+}
+
+// Column c of an operand summed over the tile's rows, first to last.
+__device__ __forceinline__ float column_sum(const uint8_t* base, uint32_t c, uint32_t group) {
+    const uint8_t* p = base + (c >> 3) * kCore + (c & 7u) * 2u;
+    float a = 0.0f;
+#pragma unroll 4
+    for (uint32_t r = 0; r < kRows; r += 8)
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k)
+            a += bf16_val(*reinterpret_cast<const uint16_t*>(p + (r >> 3) * group + k * 16u));
+    return a;
 }
 
 // After a wait gave up: wait once more (bounded) for the MMAs in flight
@@ -237,9 +287,8 @@ __device__ __forceinline__ void copy_img(uint8_t* dst, const uint8_t* src, uint3
     for (uint32_t i = threadIdx.x; i < bytes / 16; i += blockDim.x) d[i] = s[i];
 }
 
-// 8-row groups of the operands a CTA builds: 2 or 8 core matrices, and one of
-// ones where a weight gradient takes column sums.
-constexpr uint32_t kGroup16 = 2 * 128, kGroup64 = 8 * 128, kGroup16p = 3 * 128, kGroup64p = 9 * 128;
+// 8-row groups of the operands a CTA builds: 2 or 8 core matrices.
+constexpr uint32_t kGroup16 = 2 * kCore, kGroup64 = 8 * kCore;
 constexpr uint32_t kGroups = kRows / 8;
 
 // Sixteen inputs of a row (zeros when not live); vec: feat is 16-byte aligned.
@@ -318,6 +367,7 @@ __global__ void __launch_bounds__(kRows) mlp_forward_kernel(const uint8_t* __res
     extern __shared__ __align__(16) uint8_t smem_raw[];
     InferSmem& S = *reinterpret_cast<InferSmem*>(aligned_smem(smem_raw));
     const uint32_t tid = threadIdx.x, warp = tid >> 5;
+    const Team team{0u, tid};
     const uint64_t rows = MODE == 0 ? min((uint64_t)*d_count, n) : n;
     const uint64_t tiles = (rows + kRows - 1) / kRows;
     if ((uint64_t)blockIdx.x >= tiles) return;
@@ -330,7 +380,7 @@ __global__ void __launch_bounds__(kRows) mlp_forward_kernel(const uint8_t* __res
     }
     if (tid < kOut) S.b[2 * kHid + tid] = params[kB3 + tid];
     if (warp == 0) tmem_alloc(&S.tmem, 256);
-    if (tid == 0) mbar_init1(&S.bar);
+    if (tid == 0) mbar_init(&S.bar, 1);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -346,11 +396,11 @@ __global__ void __launch_bounds__(kRows) mlp_forward_kernel(const uint8_t* __res
         const float f7 = x[7], skip[3] = {x[8], x[9], x[10]};
         st_row16(S.x, tid, 0, kGroup16, x);
         load_row16(feat, e2, e2 < rows, x);  // the next tile's, in flight behind this one's
-        if (!(ok = gemm_sync(tm + 0, S.x, kGroup16, S.w1, kHid, kIn, &S.bar, phase, status))) break;
+        if (!(ok = gemm_sync(team, tm + 0, S.x, kGroup16, S.w1, kHid, kIn, &S.bar, phase, status))) break;
         relu_row64(tm + lane_base, S.b, S.h1, kGroup64, tid);
-        if (!(ok = gemm_sync(tm + 64, S.h1, kGroup64, S.w2, kHid, kHid, &S.bar, phase, status))) break;
+        if (!(ok = gemm_sync(team, tm + 64, S.h1, kGroup64, S.w2, kHid, kHid, &S.bar, phase, status))) break;
         relu_row64(tm + lane_base + 64, S.b + kHid, S.h2, kGroup64, tid);
-        if (!(ok = gemm_sync(tm + 128, S.h2, kGroup64, S.w3, kOut, kHid, &S.bar, phase, status))) break;
+        if (!(ok = gemm_sync(team, tm + 128, S.h2, kGroup64, S.w3, kOut, kHid, &S.bar, phase, status))) break;
         float y[16];
         tmem_ld16(tm + lane_base + 128, y);
         if (live) {
@@ -369,38 +419,51 @@ __global__ void __launch_bounds__(kRows) mlp_forward_kernel(const uint8_t* __res
     if (warp == 0) tmem_dealloc(tm, 256);
 }
 
-// The operands first: a weight gradient's MMAs may read up to 1.1 KB behind
-// one (products that nobody reads).
-struct TrainSmem {
-    alignas(1024) uint8_t x[kGroups * kGroup16p];
-    alignas(1024) uint8_t h1[kGroups * kGroup64p];
-    alignas(1024) uint8_t h2[kGroups * kGroup64p];
+// What a team works on.  A weight gradient's MMAs may read up to 1.2 KB behind
+// an operand (products that nobody reads).
+struct TeamSmem {
+    alignas(1024) uint8_t x[kGroups * kGroup16];
+    alignas(1024) uint8_t h1[kGroups * kGroup64];
+    alignas(1024) uint8_t h2[kGroups * kGroup64];
     alignas(1024) uint8_t dz2[kGroups * kGroup64];
     alignas(1024) uint8_t dz1[kGroups * kGroup64];
     alignas(1024) uint8_t dy[kGroups * kGroup16];
+};
+struct TrainSmem {
+    TeamSmem team[2];
     alignas(1024) uint8_t w1[kHid * kIn * 2];
     alignas(1024) uint8_t w2[kHid * kHid * 2];
     alignas(1024) uint8_t w3[kOut * kHid * 2];
     alignas(1024) uint8_t w2t[kHid * kHid * 2];
     alignas(1024) uint8_t w3t[kHid * kOut * 2];
-    float b[kHid + kHid + kOut];
-    uint64_t bar;
+    float b[kHid + kHid + kOut], gb[kHid + kHid + 4];
+    // per team: its GEMM steps, its weight gradients, its bias sums
+    uint64_t step[2], grad[2], sums[2];
     uint32_t tmem;
 };
 
 // Forward + backward of the cosine loss 1 - y.t/|y| (mean over valid rows)
 // for the tiles of this CTA; per-CTA gradient partials to part[cta][6288]
 // (none from a CTA without tiles).  tgt rows: (tx, ty, tz, valid).
-__global__ void __launch_bounds__(kRows) mlp_train_kernel(const uint8_t* __restrict__ img,
-                                                         const float* __restrict__ params,
-                                                         const float* __restrict__ feat, const float4* __restrict__ tgt,
-                                                         uint32_t n, float inv_batch, float* __restrict__ part,
-                                                         uint32_t* __restrict__ status,
-                                                         const uint32_t* __restrict__ d_count, bool vec) {
+//
+// Two teams take the CTA's tiles in turn, a tile each at a time, so that one's
+// MMAs run behind the other's epilogues.  The sums keep the order of one team:
+// the weight gradients of a tile are issued once those of the tile before it
+// are complete, into the same accumulators, and the bias sums are added in
+// tile order.
+__global__ void __launch_bounds__(2 * kRows, 1) mlp_train_kernel(const uint8_t* __restrict__ img,
+                                                                const float* __restrict__ params,
+                                                                const float* __restrict__ feat,
+                                                                const float4* __restrict__ tgt, uint32_t n,
+                                                                float inv_batch, float* __restrict__ part,
+                                                                uint32_t* __restrict__ status,
+                                                                const uint32_t* __restrict__ d_count, bool vec) {
     stream_wait();
     extern __shared__ __align__(16) uint8_t smem_raw[];
     TrainSmem& S = *reinterpret_cast<TrainSmem*>(aligned_smem(smem_raw));
-    const uint32_t tid = threadIdx.x, warp = tid >> 5;
+    const uint32_t warp = threadIdx.x >> 5, me = threadIdx.x / kRows, tid = threadIdx.x % kRows;
+    const Team team{me, tid};
+    TeamSmem& T = S.team[me];
     if (d_count) n = min(n, *d_count);  // rows: the step's entry count, read on the device
     const uint32_t tiles = (n + kRows - 1) / kRows;
     if (blockIdx.x >= tiles) return;
@@ -409,47 +472,49 @@ __global__ void __launch_bounds__(kRows) mlp_train_kernel(const uint8_t* __restr
     copy_img(S.w3, img + kImgW3, sizeof S.w3);
     copy_img(S.w2t, img + kImgW2T, sizeof S.w2t);
     copy_img(S.w3t, img + kImgW3T, sizeof S.w3t);
-    {
-        const uint4 ones = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);  // bf16 1.0
-        *reinterpret_cast<uint4*>(S.x + cm_row(tid, 2, kGroup16p)) = ones;
-        *reinterpret_cast<uint4*>(S.h1 + cm_row(tid, 8, kGroup64p)) = ones;
-        *reinterpret_cast<uint4*>(S.h2 + cm_row(tid, 8, kGroup64p)) = ones;
+    if (me == 0 && tid < kHid) {
+        S.b[tid] = params[kB1 + tid];
+        S.b[kHid + tid] = params[kB2 + tid];
+        S.gb[tid] = S.gb[kHid + tid] = 0.0f;
+        if (tid < kOut) S.b[2 * kHid + tid] = params[kB3 + tid];
+        if (tid < 4) S.gb[2 * kHid + tid] = 0.0f;
     }
-    for (uint32_t i = tid; i < kHid; i += kRows) {
-        S.b[i] = params[kB1 + i];
-        S.b[kHid + i] = params[kB2 + i];
-    }
-    if (tid < kOut) S.b[2 * kHid + tid] = params[kB3 + tid];
-    if (warp == 0) tmem_alloc(&S.tmem, 256);
-    if (tid == 0) mbar_init1(&S.bar);
+    if (warp == 0) tmem_alloc(&S.tmem, 512);
+    if (threadIdx.x == 0)
+        for (int k = 0; k < 2; ++k) {
+            mbar_init(&S.step[k], 1);
+            mbar_init(&S.grad[k], 1);
+            mbar_init(&S.sums[k], kHid);
+        }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tm = S.tmem;
-    const uint32_t lane_base = (warp * 32u) << 16;
-    // tensor-memory columns: forward and activation gradients reuse [0, 128);
-    // the weight gradients accumulate over tiles in [128, 256)
-    const uint32_t cA = 0, cB = 64, cG3 = 128, cG2 = 144, cG1 = 224;
-    uint32_t phase = 0;
-    bool ok = true, first = true;
-    uint32_t e = blockIdx.x * kRows + tid;
+    const uint32_t lane_base = ((warp & 3u) * 32u) << 16;
+    // tensor-memory columns: a team's forward and activation gradients in 128
+    // of its own, the weight gradients, accumulated over tiles, in [256, 352)
+    const uint32_t cA = me * 128, cB = cA + 64, cG3 = 256, cG2 = 272, cG1 = 336;
+    uint32_t phase = 0, own = 0, other = 0;  // parities: GEMM steps, this team's gradients, the other's
+    bool ok = true;
+    const uint32_t turn = 2 * gridDim.x;  // tiles from one of this team's to the next
+    uint32_t t = blockIdx.x + me * gridDim.x, e = t * kRows + tid;
     float x[kIn];
-    load_row16(feat, e, e < n, x, vec);
-    float4 g = e < n ? tgt[e] : make_float4(0.f, 0.f, 0.f, 0.f);
-    for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
-        // the last tile's weight gradients have read the operands
-        if (!first && !(ok = gemm_wait(&S.bar, phase, status))) break;
+    load_row16(feat, e, t < tiles && e < n, x, vec);
+    float4 g = t < tiles && e < n ? tgt[e] : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (bool first = true; t < tiles; t += turn, first = false) {
+        // this team's last weight gradients have read the operands
+        if (!first && !(ok = gemm_wait(team, &S.grad[me], own, status))) break;
         const float skip[3] = {x[8], x[9], x[10]};
         const float4 target = g;
-        st_row16(S.x, tid, 0, kGroup16p, x);
-        e += gridDim.x * kRows;  // the next tile's rows, in flight behind this one's
-        load_row16(feat, e, e < n, x, vec);
-        g = e < n ? tgt[e] : make_float4(0.f, 0.f, 0.f, 0.f);
-        if (!(ok = gemm_sync(tm + cA, S.x, kGroup16p, S.w1, kHid, kIn, &S.bar, phase, status))) break;
-        relu_row64(tm + lane_base + cA, S.b, S.h1, kGroup64p, tid);
-        if (!(ok = gemm_sync(tm + cB, S.h1, kGroup64p, S.w2, kHid, kHid, &S.bar, phase, status))) break;
-        relu_row64(tm + lane_base + cB, S.b + kHid, S.h2, kGroup64p, tid);
-        if (!(ok = gemm_sync(tm + cA, S.h2, kGroup64p, S.w3, kOut, kHid, &S.bar, phase, status))) break;
+        st_row16(T.x, tid, 0, kGroup16, x);
+        e += turn * kRows;  // the next tile's rows, in flight behind this one's
+        load_row16(feat, e, t + turn < tiles && e < n, x, vec);
+        g = t + turn < tiles && e < n ? tgt[e] : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (!(ok = gemm_sync(team, tm + cA, T.x, kGroup16, S.w1, kHid, kIn, &S.step[me], phase, status))) break;
+        relu_row64(tm + lane_base + cA, S.b, T.h1, kGroup64, tid);
+        if (!(ok = gemm_sync(team, tm + cB, T.h1, kGroup64, S.w2, kHid, kHid, &S.step[me], phase, status))) break;
+        relu_row64(tm + lane_base + cB, S.b + kHid, T.h2, kGroup64, tid);
+        if (!(ok = gemm_sync(team, tm + cA, T.h2, kGroup64, S.w3, kOut, kHid, &S.step[me], phase, status))) break;
         {
             float y[16];
             tmem_ld16(tm + lane_base + cA, y);
@@ -464,32 +529,61 @@ __global__ void __launch_bounds__(kRows) mlp_train_kernel(const uint8_t* __restr
                 d[1] = s * (target.y - c * y1 / nn);
                 d[2] = s * (target.z - c * y2 / nn);
             }
-            st_row16(S.dy, tid, 0, kGroup16, d);
+            st_row16(T.dy, tid, 0, kGroup16, d);
         }
-        // dH2 = dY W3  (B = W3^T, N 64 x K 16), then dH1 = dZ2 W2
-        if (!(ok = gemm_sync(tm + cB, S.dy, kGroup16, S.w3t, kHid, kOut, &S.bar, phase, status))) break;
-        mask_row64(tm + lane_base + cB, S.h2, kGroup64p, S.dz2, tid);
-        if (!(ok = gemm_sync(tm + cA, S.dz2, kGroup64, S.w2t, kHid, kHid, &S.bar, phase, status))) break;
-        mask_row64(tm + lane_base + cA, S.h1, kGroup64p, S.dz1, tid);
-        // weight gradients, K = the tile's rows: dW3^T (j, o) = H2^T dY with
-        // row 64 (of ones) the sums of dY; dW2 (k, j) = dZ2^T H1 and dW1 (j,
-        // i) = dZ1^T X, each with the sums in the column behind.  Nobody
-        // waits before the next tile.
-        gemm_ready();
+        // dH2 = dY W3  (B = W3^T, N 64 x K 16), then dH1 = dZ2 W2; the bias
+        // gradients, sums over the rows, behind the MMAs
+        float a1 = 0.0f, a2 = 0.0f, a3 = 0.0f;
+        if (!(ok = gemm_sync(team, tm + cB, T.dy, kGroup16, S.w3t, kHid, kOut, &S.step[me], phase, status, [&] {
+                  if (tid < 3) a3 = column_sum(T.dy, tid, kGroup16);
+              })))
+            break;
+        mask_row64(tm + lane_base + cB, T.h2, kGroup64, T.dz2, tid);
+        if (!(ok = gemm_sync(team, tm + cA, T.dz2, kGroup64, S.w2t, kHid, kHid, &S.step[me], phase, status, [&] {
+                  if (tid < kHid) a2 = column_sum(T.dz2, tid, kGroup64);
+              })))
+            break;
+        mask_row64(tm + lane_base + cA, T.h1, kGroup64, T.dz1, tid);
+        // weight gradients, K = the tile's rows: dW3^T (j, o) = H2^T dY, dW2
+        // (k, j) = dZ2^T H1, dW1 (j, i) = dZ1^T X, after the tile before's.
+        // Nobody waits for them before this team's next tile.
+        gemm_ready(team);
+        const bool chained = !first || me != 0;  // (the CTA's first tile has none before it)
         if (tid == 0) {
-            gemm_rows_issue(tm + cG3, S.h2, kGroup64p, S.dy, kGroup16, kOut, !first);
-            gemm_rows_issue(tm + cG2, S.dz2, kGroup64, S.h1, kGroup64p, kHid + 16, !first);
-            gemm_rows_issue(tm + cG1, S.dz1, kGroup64, S.x, kGroup16p, kIn + 16, !first);
-            mma_commit(&S.bar);
+            if (chained && !mbar_wait(&S.grad[me ^ 1u], other)) ok = false;
+            tc_fence_after();
+            if (ok) {
+                gemm_rows_issue(tm + cG3, T.h2, kGroup64, T.dy, kGroup16, kOut, chained);
+                gemm_rows_issue(tm + cG2, T.dz2, kGroup64, T.h1, kGroup64, kHid, chained);
+                gemm_rows_issue(tm + cG1, T.dz1, kGroup64, T.x, kGroup16, kIn, chained);
+            }
+            mma_commit(&S.grad[me]);
         }
-        first = false;
+        if (tid < kHid) {
+            a1 = column_sum(T.dz1, tid, kGroup64);
+            if (chained && !mbar_wait(&S.sums[me ^ 1u], other)) ok = false;
+            S.gb[tid] += a1;
+            S.gb[kHid + tid] += a2;
+            if (tid < 3) S.gb[2 * kHid + tid] += a3;
+            mbar_arrive(&S.sums[me]);
+        }
+        if (chained) other ^= 1u;
+        if (!(ok = team_all(team, ok))) {
+            if (tid == 0) atomicOr(status, kErrWaitTimeout);
+            break;
+        }
     }
-    if (ok) ok = gemm_wait(&S.bar, phase, status);
+    const bool ran = blockIdx.x + me * gridDim.x < tiles;
+    if (ok && ran) ok = gemm_wait(team, &S.grad[me], own, status);
+    const bool mine = ok;
+    tc_fence_before();
+    ok = __syncthreads_and(ok) != 0;
+    tc_fence_after();
     float* P = part + (size_t)blockIdx.x * kParams;
     if (ok) {
-        float v[16];
-        if (warp < 2) {  // lanes 0..63 hold the 64 rows of every weight gradient
+        if (threadIdx.x < kHid) {  // lanes 0..63 hold the 64 rows of every weight gradient
             const uint32_t r = tid;
+            float v[16];
             tmem_ld16(tm + lane_base + cG3, v);  // dW3^T row j = r
 #pragma unroll
             for (int o = 0; o < kOut; ++o) P[kW3 + o * kHid + r] = o < 3 ? v[o] : 0.0f;
@@ -500,27 +594,24 @@ __global__ void __launch_bounds__(kRows) mlp_train_kernel(const uint8_t* __restr
                 for (int k = 0; k < 16; k += 4)
                     *reinterpret_cast<float4*>(P + kW2 + r * kHid + c + k) = make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]);
             }
-            tmem_ld16(tm + lane_base + cG2 + kHid, v);
-            P[kB2 + r] = v[0];
             tmem_ld16(tm + lane_base + cG1, v);
 #pragma unroll
             for (int k = 0; k < 16; k += 4)
                 *reinterpret_cast<float4*>(P + kW1 + r * kIn + k) = make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]);
-            tmem_ld16(tm + lane_base + cG1 + kIn, v);
-            P[kB1 + r] = v[0];
-        } else if (warp == 2) {  // lane 64: the row of ones
-            tmem_ld16(tm + lane_base + cG3, v);
-            if (tid == 64)
-#pragma unroll
-                for (int o = 0; o < kOut; ++o) P[kB3 + o] = o < 3 ? v[o] : 0.0f;
+            P[kB1 + r] = S.gb[r];
+            P[kB2 + r] = S.gb[kHid + r];
+            if (r < kOut) P[kB3 + r] = r < 3 ? S.gb[2 * kHid + r] : 0.0f;
         }
     } else {
-        for (uint32_t i = tid; i < kParams; i += kRows) P[i] = 0.0f;
-        drain(&S.bar, phase);
+        for (uint32_t i = threadIdx.x; i < kParams; i += 2 * kRows) P[i] = 0.0f;
+        if (!mine) {
+            drain(&S.step[me], phase);
+            drain(&S.grad[me], own);
+        }
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tm, 256);
+    if (warp == 0) tmem_dealloc(tm, 512);
 }
 
 // BF16 operand images of parameter p: W1, W2, W3 and the transposes W2^T, W3^T.
@@ -540,31 +631,30 @@ __device__ __forceinline__ void pack_param(uint32_t p, float x, uint8_t* __restr
     }
 }
 
-// grad[p] = sum over CTAs of part[c][p] in a fixed order: kSlices sums of
-// every kSlices-th CTA, then those in order (one thread a parameter, CTA after
-// CTA, took 10 us of load latency at 148 CTAs).  Then (adam != 0) an Adam step on the
-// master parameters and their operand images (W3, b3 rows 3..15 stay zero).
-// CTAs past the rows' tiles wrote no part.
-constexpr int kSlices = 32;
-__global__ void __launch_bounds__(32 * kSlices)
+// grad[p] = sum over CTAs of part[c][p] in the CTAs' order, kBatch loads in
+// flight at a time (one after the other took 10 us at 148 CTAs).  Then (adam !=
+// 0) an Adam step on the master parameters and their operand images (W3, b3
+// rows 3..15 stay zero).  CTAs past the rows' tiles wrote no part.
+constexpr int kReduceThreads = 32, kBatch = 37;
+__global__ void __launch_bounds__(kReduceThreads)
 mlp_reduce_kernel(const float* __restrict__ part, uint32_t nparts, uint32_t n, const uint32_t* __restrict__ d_count,
                   float* __restrict__ grad, float* __restrict__ params, float* __restrict__ m1,
                   float* __restrict__ m2, uint8_t* __restrict__ img, int adam, float lr, float c1, float c2) {
     stream_wait();
-    __shared__ float s[kSlices][32];
-    const uint32_t lane = threadIdx.x & 31u, slice = threadIdx.x >> 5, p = blockIdx.x * 32 + lane;
+    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= (uint32_t)kParams) return;
     if (d_count) n = min(n, *d_count);
     nparts = min(nparts, (n + kRows - 1) / kRows);
     float g = 0.0f;
-    if (p < (uint32_t)kParams)
-#pragma unroll 8
-        for (uint32_t c = slice; c < nparts; c += kSlices) g += part[(size_t)c * kParams + p];
-    s[slice][lane] = g;
-    __syncthreads();
-    if (slice != 0 || p >= (uint32_t)kParams) return;
-    g = 0.0f;
+    uint32_t c = 0;
+    for (; c + kBatch <= nparts; c += kBatch) {  // loads together, sums in the CTAs' order
+        float v[kBatch];
 #pragma unroll
-    for (int k = 0; k < kSlices; ++k) g += s[k][lane];
+        for (int k = 0; k < kBatch; ++k) v[k] = part[(size_t)(c + k) * kParams + p];
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) g += v[k];
+    }
+    for (; c < nparts; ++c) g += part[(size_t)c * kParams + p];
     const bool dead = (p >= (uint32_t)kW3 && p < (uint32_t)kB3 && (p - kW3) / kHid >= 3) || (p >= (uint32_t)kB3 + 3);
     if (dead) g = 0.0f;
     if (grad) grad[p] = g;
@@ -586,7 +676,7 @@ __global__ void mlp_pack_kernel(const float* __restrict__ params, uint8_t* __res
 
 inline uint32_t grid_for(uint64_t n, int threads) { return (uint32_t)((n + threads - 1) / threads); }
 
-constexpr uint32_t kMaxTrainCtas = 304;  // two per SM (operands and accumulators fit twice)
+constexpr uint32_t kMaxTrainCtas = 148;  // partial sums, and so the gradients' bits, go by this
 
 }  // namespace
 
@@ -652,11 +742,11 @@ cudaError_t mlp_train_async(MlpState& s, const float* feat, const float4* tgt, u
     const uint32_t tiles = grid_for(n, kRows);
     const uint32_t ctas = tiles < kMaxTrainCtas ? tiles : kMaxTrainCtas;
     const float inv = n_valid ? 1.0f / (float)n_valid : 0.0f;
-    launch_after(st, ctas, kRows, sizeof(TrainSmem) + 1024, mlp_train_kernel, s.img, s.params, feat, tgt, n, inv,
+    launch_after(st, ctas, 2 * kRows, sizeof(TrainSmem) + 1024, mlp_train_kernel, s.img, s.params, feat, tgt, n, inv,
                  s.part, s.status, d_count, (reinterpret_cast<uintptr_t>(feat) & 15u) == 0);
     const float c1 = update ? (float)(1.0 / (1.0 - std::pow(0.9, (double)adam_step))) : 0.f;
     const float c2 = update ? (float)(1.0 / (1.0 - std::pow(0.999, (double)adam_step))) : 0.f;
-    launch_after(st, grid_for(kParams, 32), 32 * kSlices, 0, mlp_reduce_kernel, s.part, ctas, n, d_count, s.grad,
+    launch_after(st, grid_for(kParams, kReduceThreads), kReduceThreads, 0, mlp_reduce_kernel, s.part, ctas, n, d_count, s.grad,
                  s.params, s.m1, s.m2, s.img, update ? 1 : 0, lr, c1, c2);
     return cudaGetLastError();
 }

@@ -200,11 +200,11 @@ def test_online_learned_seed_beats_its_untrained_baseline(sdlib):
         eng.close()
 
 
-@pytest.mark.parametrize("n,shift", [(1, 0), (127, 0), (129, 1), (304 * 128 - 1, 0), (304 * 128 + 1, 2),
-                                     (2 * 304 * 128 + 77, 0)])
+@pytest.mark.parametrize("n,shift", [(1, 0), (127, 0), (129, 1), (148 * 128 - 1, 0), (148 * 128 + 1, 2),
+                                     (2 * 148 * 128 + 1, 0), (3 * 148 * 128, 0), (4 * 148 * 128 + 77, 0)])
 def test_mlp_gradients_over_tiles(sdlib, orc, n, shift):
-    """Rows around one tile of 128 and around one tile for each of the 304
-    CTAs, the inputs 16-byte aligned or not: gradient elements within 2^-6 of
+    """Rows around one tile of 128 and around one to four tiles for each of the
+    148 CTAs' two teams, the inputs 16-byte aligned or not: gradient elements within 2^-6 of
     their sums of |terms|, as in test_mlp_gradients_match_oracle."""
     import torch
     eng = tiny_engine(sdlib)
