@@ -109,19 +109,41 @@ scan_apply_kernel(const uint32_t* __restrict__ in, uint32_t n, const uint32_t* _
         before = part[blockIdx.x];
     }
     const uint32_t base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
+    const bool vec = base + kScanItems <= n &&
+                     ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0;
     uint32_t v[kScanItems];
     uint32_t s = 0;
+    if (vec) {
 #pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-        v[k] = base + k < n ? in[base + k] : 0u;
-        s += v[k];
+        for (int k = 0; k < kScanItems; k += 4) {
+            const uint4 x = *reinterpret_cast<const uint4*>(in + base + k);
+            v[k] = x.x;
+            v[k + 1] = x.y;
+            v[k + 2] = x.z;
+            v[k + 3] = x.w;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < kScanItems; ++k) v[k] = base + k < n ? in[base + k] : 0u;
     }
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) s += v[k];
     uint32_t tot;
     uint32_t run = before + block_exclusive_scan(s, ws, &tot);
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
-        if (base + k < n) out[base + k] = run;
-        run += v[k];
+        const uint32_t x = v[k];
+        v[k] = run;
+        run += x;
+    }
+    if (vec) {
+#pragma unroll
+        for (int k = 0; k < kScanItems; k += 4)
+            *reinterpret_cast<uint4*>(out + base + k) = make_uint4(v[k], v[k + 1], v[k + 2], v[k + 3]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < kScanItems; ++k)
+            if (base + k < n) out[base + k] = v[k];
     }
 }
 
@@ -511,8 +533,9 @@ struct QueryOut {
 // pushed or listed together, in lane order.  A walk is some 60 visits, each a
 // load that depends on the one before when a thread makes it alone; down the
 // tree only one or two nodes are open, near the leaves many.
-// Latency bounds it: 300,001 boxes' pairs 110 us with two lanes (one lane and
-// both directions of every pair, twice: 2 x 100 us).  One warp walking for 32
+// Latency bounds it: 300,001 boxes' pairs 99 us with two lanes, 106 with each
+// pair handed over as it is found (one lane and both directions of every pair,
+// twice: 2 x 100 us).  One warp walking for 32
 // neighbouring leaves under their common box took seven times as long: where
 // the curve jumps, that box covers much of the domain.
 template <int MODE, int G>
@@ -524,10 +547,13 @@ query_kernel(int n, const uint32_t* __restrict__ vals, const float4* __restrict_
     constexpr bool kUnique = MODE == kPairs || MODE == kRefill;
     constexpr int kLeaves = kQueryThreads / G, kDepth = kStack + 2 * G;
     __shared__ int s_stack[kDepth][kLeaves];
+    __shared__ PairBuffer<MODE == kPairs ? 128 : 1> s_found[kQueryThreads / 32];
     const uint32_t lane = threadIdx.x & 31u, sub = threadIdx.x % G, group = lane & ~(uint32_t)(G - 1);
     const uint32_t below = (1u << sub) - 1u;
     const int at = threadIdx.x / G, k = (int)blockIdx.x * kLeaves + at;
     if (MODE == kRefill && !sink_refill(sink)) return;
+    PairBuffer<MODE == kPairs ? 128 : 1>& found = s_found[threadIdx.x >> 5];
+    if (lane == 0) found.n = 0u;
     bool walk = k < n;
     const uint32_t id = walk ? vals[k] : 0u;
     uint32_t c = 0;
@@ -592,7 +618,7 @@ query_kernel(int n, const uint32_t* __restrict__ vals, const float4* __restrict_
             sp = min(sp + __popc(mi), kDepth);
             if constexpr (kUnique) {
                 if (leaf) {
-                    if (MODE == kPairs) sink_pair(sink, id, vals[j]);
+                    if (MODE == kPairs) buffer_pair(found, sink, id, vals[j]);
                     else sink_pair_again(sink, id, vals[j]);
                 }
             } else {
@@ -610,6 +636,7 @@ query_kernel(int n, const uint32_t* __restrict__ vals, const float4* __restrict_
         }
         __syncwarp();
     }
+    if constexpr (MODE == kPairs) flush_pairs(found, sink, lane, 32u);  // (the warp met at the end of its last trip)
     if constexpr (MODE == kCount) {
         if (walk && sub == 0) q.count[id] = c;
     }

@@ -8,10 +8,10 @@
 // their finder (which returns at once when there are none) straight into the
 // list, and sorted there.  A list that does not fit is not written.
 //
-// 16 kept: 2,000,000 boxes at four to six pairs a box never search twice, and
-// the write (16 words read, the sort in registers) takes 29 us.  Lists both
-// ways from a counting and a writing search, then the upper halves counted,
-// scanned and copied, took 2.6 searches' time there.
+// 16 kept: 2,000,000 boxes of two pairs each never search twice, and the write
+// (16 words read, the sort in registers) takes 31 us.  Lists both ways from a
+// counting and a writing search, then the upper halves counted, scanned and
+// copied, took 2.6 searches' time there.
 #pragma once
 
 #include "sd_common.cuh"
@@ -37,6 +37,30 @@ __device__ __forceinline__ void sink_pair(const PairSink& s, uint32_t a, uint32_
     const uint32_t at = atomicAdd(s.count + i, 1u);
     if (at < kPairKeep) s.keep[(size_t)i * kPairKeep + at] = j;
     else if (at == kPairKeep) *s.over = 1u;
+}
+
+// Pairs found on the way, set aside in shared memory: handed over one by one,
+// each would hold its whole warp up for an atomic's way to L2 and back (a
+// place in the box's list), some ten times a warp; set aside they are handed
+// over side by side (the sweep of 2,000,000 boxes 192 -> 166 us).  Up to CAP;
+// further ones go straight to the sink.
+template <int CAP>
+struct PairBuffer {
+    uint2 pair[CAP];
+    uint32_t n;  // (zero before)
+};
+template <int CAP>
+__device__ __forceinline__ void buffer_pair(PairBuffer<CAP>& b, const PairSink& s, uint32_t i, uint32_t j) {
+    const uint32_t at = atomicAdd(&b.n, 1u);
+    if (at < (uint32_t)CAP) b.pair[at] = make_uint2(i, j);
+    else sink_pair(s, i, j);
+}
+// By `threads` threads that have met since the last buffer_pair(), this one the
+// t-th.
+template <int CAP>
+__device__ __forceinline__ void flush_pairs(const PairBuffer<CAP>& b, const PairSink& s, uint32_t t, uint32_t threads) {
+    const uint32_t n = min(b.n, (uint32_t)CAP);
+    for (uint32_t k = t; k < n; k += threads) sink_pair(s, b.pair[k].x, b.pair[k].y);
 }
 
 // Whether the second search has anything to do.

@@ -26,12 +26,11 @@
 //    A pair sharing several columns is reported in the column of its overlap's
 //    lower y-z corner, so every pair is found once, by the same tests as the
 //    unbinned sweep: the same pair set, listed by sd_pairs.cuh.
-//    Measured, 2,000,000 boxes of one size (0.9 entries swept per test that
-//    passes x): 612 us in all; sweep 219 (dependent loads: key, index, box),
-//    seven radix passes 175, gather into x order 45, entries 42, list 29 + 18,
-//    bounds 19, scans 30.  It was 1174: four entries for every box whether used
-//    or not, boxes of 48 bytes gathered through two indices, and the sweep
-//    twice, once to count.
+//    Measured, 2,000,000 boxes of one size, 2.25 entries and two pairs each:
+//    442 us in all; six radix passes 157, sweep 149, gather into x order 37, list
+//    31, entries 22, bounds 23, scans 19.  It was 1412: four entries for every
+//    box whether used or not, boxes of 48 bytes gathered through two indices,
+//    and the sweep twice, once to count.
 #include "sd_common.cuh"
 #include "sd_engine_impl.h"
 #include "sd_pairs.cuh"
@@ -133,7 +132,34 @@ __device__ __forceinline__ float key_float(uint32_t k) {
 struct SapBounds {
     uint32_t w[5], count;
     double sum;
+    uint32_t done;  // blocks that have added theirs
+    SapGrid grid;   // made by the last of them
 };
+
+// Columns at least 1.0001 x the largest extent wide (so a box spans at most
+// two columns per axis, rounding included), twice the mean extent (boxes of
+// one size then take 2.25 entries each instead of 4, for as many tests), and
+// at most kMaxCols per axis.  The width never changes the pairs.  (Made once:
+// made by every thread of the kernels that use it, its division of doubles was
+// 38 of the sweep's 230 us and 18 of the entries' 40.)
+__device__ __forceinline__ SapGrid sap_grid(const SapBounds& b) {
+    SapGrid r{0.0f, 0.0f, 0.0f, 1, 1};
+    if (b.w[0] && b.w[1] && b.w[2] && b.w[3]) {
+        const float y0 = key_float(~b.w[0]), y1 = key_float(b.w[1]), z0 = key_float(~b.w[2]), z1 = key_float(b.w[3]);
+        const float ext = b.w[4] ? key_float(b.w[4]) : 0.0f;
+        const float mean = b.count ? (float)(b.sum / b.count) : 0.0f;
+        float c = fmaxf(fmaxf(ext * 1.0001f, (y1 - y0) / (float)kMaxCols), (z1 - z0) / (float)kMaxCols);
+        if (mean > 0.0f) c = fmaxf(c, 2.0f * mean);
+        if (c > 0.0f && c < INFINITY) {
+            r.y0 = y0;
+            r.z0 = z0;
+            r.inv = 1.0f / c;
+            r.gy = min(kMaxCols, max(1, (int)fminf((y1 - y0) * r.inv, 1e6f) + 1));
+            r.gz = min(kMaxCols, max(1, (int)fminf((z1 - z0) * r.inv, 1e6f) + 1));
+        }
+    }
+    return r;
+}
 
 constexpr int kBoundBlocks = 152 * 4;
 
@@ -190,29 +216,16 @@ sap_bounds_kernel(uint32_t n, const float4* __restrict__ lo, const float4* __res
         atomicAdd(&out->count, s_count);
         atomicAdd(&out->sum, s_sum);
     }
-}
-
-// Columns at least 1.0001 x the largest extent wide (so a box spans at most
-// two columns per axis, rounding included), twice the mean extent (boxes of
-// one size then take 2.25 entries each instead of 4, for as many tests), and
-// at most kMaxCols per axis.  The width never changes the pairs.
-__device__ __forceinline__ SapGrid sap_grid(const SapBounds& b) {
-    SapGrid r{0.0f, 0.0f, 0.0f, 1, 1};
-    if (b.w[0] && b.w[1] && b.w[2] && b.w[3]) {
-        const float y0 = key_float(~b.w[0]), y1 = key_float(b.w[1]), z0 = key_float(~b.w[2]), z1 = key_float(b.w[3]);
-        const float ext = b.w[4] ? key_float(b.w[4]) : 0.0f;
-        const float mean = b.count ? (float)(b.sum / b.count) : 0.0f;
-        float c = fmaxf(fmaxf(ext * 1.0001f, (y1 - y0) / (float)kMaxCols), (z1 - z0) / (float)kMaxCols);
-        if (mean > 0.0f) c = fmaxf(c, 2.0f * mean);
-        if (c > 0.0f && c < INFINITY) {
-            r.y0 = y0;
-            r.z0 = z0;
-            r.inv = 1.0f / c;
-            r.gy = min(kMaxCols, max(1, (int)fminf((y1 - y0) * r.inv, 1e6f) + 1));
-            r.gz = min(kMaxCols, max(1, (int)fminf((z1 - z0) * r.inv, 1e6f) + 1));
-        }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(&out->done, 1u) == gridDim.x - 1) {
+        __threadfence();
+        SapBounds b{};
+        for (int k = 0; k < 5; ++k) b.w[k] = __ldcg(&out->w[k]);
+        b.count = __ldcg(&out->count);
+        b.sum = __ldcg(&out->sum);
+        out->grid = sap_grid(b);
     }
-    return r;
 }
 
 // Columns of a box, y-major.
@@ -225,35 +238,40 @@ __device__ __forceinline__ SapSpan sap_span(const SapGrid& g, float4 a, float4 b
 }
 
 // The boxes in x order, 32 bytes each with the id in the lower corner's w
-// lane, and the number of columns each touches.
+// lane and its first columns (y, z: a byte each) in the upper one's, the columns
+// each touches (first y, first z, one more in y, in z: a byte
+// each) and their number.
 __global__ void sap_gather_kernel(uint32_t n, const uint32_t* __restrict__ svals, const float4* __restrict__ lo,
                                   const float4* __restrict__ hi, const SapBounds* __restrict__ bounds,
-                                  float4* __restrict__ box, uint32_t* __restrict__ count, uint32_t* __restrict__ status) {
+                                  float4* __restrict__ box, uint32_t* __restrict__ span, uint32_t* __restrict__ count,
+                                  uint32_t* __restrict__ status) {
     stream_wait();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
-    const SapGrid g = sap_grid(*bounds);
+    const SapGrid g = bounds->grid;
     const uint32_t id = svals[k];
     const float4 a = lo[id], b = hi[id];
     box[2 * (size_t)k] = make_float4(a.x, a.y, a.z, __uint_as_float(id));
-    box[2 * (size_t)k + 1] = b;
     const SapSpan s = sap_span(g, a, b);
+    box[2 * (size_t)k + 1] = make_float4(b.x, b.y, b.z, __uint_as_float((uint32_t)s.y0 | (uint32_t)s.z0 << 8));
     if (s.y1 - s.y0 > 1 || s.z1 - s.z0 > 1) atomicOr(status, kErrBadInput);  // excluded by the column width
-    count[k] = (uint32_t)((min(s.y1 - s.y0, 1) + 1) * (min(s.z1 - s.z0, 1) + 1));
+    const uint32_t dy = (uint32_t)min(s.y1 - s.y0, 1), dz = (uint32_t)min(s.z1 - s.z0, 1);
+    span[k] = (uint32_t)s.y0 | (uint32_t)s.z0 << 8 | dy << 16 | dz << 24;
+    count[k] = (dy + 1u) * (dz + 1u);
 }
 
-__global__ void sap_entries_kernel(uint32_t n, const float4* __restrict__ box, const SapBounds* __restrict__ bounds,
+__global__ void sap_entries_kernel(uint32_t n, const uint32_t* __restrict__ span, const SapBounds* __restrict__ bounds,
                                    const uint32_t* __restrict__ off, uint32_t* __restrict__ keys,
                                    uint32_t* __restrict__ vals) {
     stream_wait();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
-    const SapGrid g = sap_grid(*bounds);
-    const SapSpan s = sap_span(g, box[2 * (size_t)k], box[2 * (size_t)k + 1]);
+    const SapGrid g = bounds->grid;
+    const uint32_t s = span[k], y0 = s & 255u, z0 = (s >> 8) & 255u;
     uint32_t e = off[k];
-    for (int y = s.y0; y <= min(s.y1, s.y0 + 1); ++y)
-        for (int z = s.z0; z <= min(s.z1, s.z0 + 1); ++z) {
-            keys[e] = (uint32_t)(y * g.gz + z);
+    for (uint32_t y = y0; y <= y0 + ((s >> 16) & 1u); ++y)
+        for (uint32_t z = z0; z <= z0 + (s >> 24); ++z) {
+            keys[e] = y * (uint32_t)g.gz + z;
             vals[e++] = k;
         }
 }
@@ -261,33 +279,81 @@ __global__ void sap_entries_kernel(uint32_t n, const float4* __restrict__ box, c
 // Forward sweep of entry p inside its column: entries m > p of the same
 // column with lower x <= upper x of p's box (x order within the column, the
 // first miss ends it), tested on y, z and x like the unbinned sweep; a pair
-// counts in the column of its overlap's lower y-z corner only.  Neighbouring
-// threads sweep over the same few boxes, which stay in L1.
+// counts in the column of its overlap's lower y-z corner only: in y and in z
+// the later of the two boxes' first columns.  A block's
+// kSweep entries and the kSweepAhead behind them are fetched once, into shared
+// memory (an entry is tested against some nine before it; fetched anew for each
+// test -- column, index, box, one load waiting for the other -- the sweep of
+// 2,000,000 boxes took 215 us, now 149: 64 the fetching, 38 the tests, 47 the
+// pairs); what lies further is fetched.  256 entries to a block; with 128, 512 or
+// a block walking over tiles, the next one's indices loaded ahead, it takes 270,
+// 165 and 162.
+constexpr int kSweep = 256, kSweepAhead = 32, kSweepTile = kSweep + kSweepAhead;
+constexpr uint32_t kSweepBlocks = 128;  // per SM: a block takes one tile of up to 5 million entries
+
 template <bool REFILL>
-__global__ void sweep_binned_kernel(const uint32_t* __restrict__ d_entries, const uint32_t* __restrict__ ckeys,
-                                    const uint32_t* __restrict__ cvals, const float4* __restrict__ box,
-                                    const SapBounds* __restrict__ bounds, PairSink sink) {
+__global__ void __launch_bounds__(kSweep)
+sweep_binned_kernel(const uint32_t* __restrict__ d_entries, const uint32_t* __restrict__ ckeys,
+                    const uint32_t* __restrict__ cvals, const float4* __restrict__ box,
+                    const SapBounds* __restrict__ bounds, PairSink sink) {
     stream_wait();
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x, n_entries = *d_entries;
-    if (p >= n_entries) return;
+    __shared__ float s_lx[kSweepTile], s_ly[kSweepTile], s_lz[kSweepTile], s_hx[kSweepTile], s_hy[kSweepTile],
+        s_hz[kSweepTile];
+    __shared__ uint32_t s_col[kSweepTile], s_id[kSweepTile], s_first[kSweepTile];
+    __shared__ PairBuffer<REFILL ? 1 : 1024> s_found;
+    const uint32_t n_entries = *d_entries;
     if (REFILL && !sink_refill(sink)) return;
-    const uint32_t col = ckeys[p];
-    const SapGrid g = sap_grid(*bounds);
-    const size_t k = cvals[p];
-    const float4 a0 = box[2 * k], a1 = box[2 * k + 1];
-    const float ay = fminf(a0.y, a1.y), az = fminf(a0.z, a1.z);
-    for (uint32_t q = p + 1; q < n_entries; ++q) {
-        if (ckeys[q] != col) break;
-        const size_t m = cvals[q];
-        const float4 b0 = box[2 * m];
-        if (!(b0.x <= a1.x)) break;
-        const float4 b1 = box[2 * m + 1];
-        if (!(b0.y <= a1.y && a0.y <= b1.y && b0.z <= a1.z && a0.z <= b1.z && a0.x <= b1.x)) continue;
-        const int cy = sap_col(fmaxf(ay, fminf(b0.y, b1.y)), g.y0, g.inv, g.gy);
-        const int cz = sap_col(fmaxf(az, fminf(b0.z, b1.z)), g.z0, g.inv, g.gz);
-        if ((uint32_t)(cy * g.gz + cz) != col) continue;
-        if (REFILL) sink_pair_again(sink, __float_as_uint(a0.w), __float_as_uint(b0.w));
-        else sink_pair(sink, __float_as_uint(a0.w), __float_as_uint(b0.w));
+    const uint32_t gz = (uint32_t)bounds->grid.gz, t = threadIdx.x;
+    for (uint32_t p0 = blockIdx.x * kSweep; p0 < n_entries; p0 += gridDim.x * kSweep) {
+        const uint32_t end = min(n_entries - p0, (uint32_t)kSweepTile);
+        if (t == 0) s_found.n = 0u;
+        for (uint32_t i = t; i < end; i += kSweep) {
+            const size_t m = cvals[p0 + i];
+            const float4 lo = box[2 * m], hi = box[2 * m + 1];
+            s_col[i] = ckeys[p0 + i];
+            s_lx[i] = lo.x;
+            s_ly[i] = lo.y;
+            s_lz[i] = lo.z;
+            s_id[i] = __float_as_uint(lo.w);
+            s_hx[i] = hi.x;
+            s_hy[i] = hi.y;
+            s_hz[i] = hi.z;
+            s_first[i] = __float_as_uint(hi.w);
+        }
+        __syncthreads();
+        if (t < end) {
+            const uint32_t col = s_col[t], id = s_id[t];
+            const float lx = s_lx[t], ly = s_ly[t], lz = s_lz[t], hx = s_hx[t], hy = s_hy[t], hz = s_hz[t];
+            const uint32_t first = s_first[t];
+            const auto found = [&](uint32_t theirs, uint32_t other) {
+                const uint32_t cy = max(first & 255u, theirs & 255u), cz = max(first >> 8, theirs >> 8);
+                if (cy * gz + cz != col) return;
+                if (REFILL) sink_pair_again(sink, id, other);
+                else buffer_pair(s_found, sink, id, other);
+            };
+            uint32_t i = t + 1;
+            for (; i < end; ++i) {
+                if (s_col[i] != col || !(s_lx[i] <= hx)) break;
+                const float bly = s_ly[i], bhy = s_hy[i];
+                if (!(bly <= hy && ly <= bhy)) continue;
+                const float blz = s_lz[i], bhz = s_hz[i];
+                if (blz <= hz && lz <= bhz && lx <= s_hx[i]) found(s_first[i], s_id[i]);
+            }
+            if (i == (uint32_t)kSweepTile)  // past what the block holds
+                for (uint32_t q = p0 + i; q < n_entries && ckeys[q] == col; ++q) {
+                    const size_t m = cvals[q];
+                    const float4 lo = box[2 * m];
+                    if (!(lo.x <= hx)) break;
+                    const float4 hi = box[2 * m + 1];
+                    if (lo.y <= hy && ly <= hi.y && lo.z <= hz && lz <= hi.z && lx <= hi.x)
+                        found(__float_as_uint(hi.w), __float_as_uint(lo.w));
+                }
+        }
+        __syncthreads();
+        if (!REFILL) {
+            flush_pairs(s_found, sink, t, kSweep);
+            if (p0 + gridDim.x * kSweep < n_entries) __syncthreads();
+        }
     }
 }
 
@@ -377,9 +443,9 @@ cudaError_t sap_pairs_async(uint32_t n, const float4* lo, const float4* hi, void
     if ((e = sort_pairs_async(keys, vals, keys_tmp, vals_tmp, n, 32, sort_scratch, st, &in_tmp)) != cudaSuccess) return e;
     // each box's entries, stably sorted by column
     launch_after(st, grid, kSapThreads, 0, sap_gather_kernel, n, in_tmp ? vals_tmp : vals, lo, hi, bounds, box,
-                 counts, status);
+                 cursor, counts, status);
     if ((e = scan_exclusive_async(counts, eoff, n, scan, st)) != cudaSuccess) return e;
-    launch_after(st, grid, kSapThreads, 0, sap_entries_kernel, n, box, bounds, eoff, ckeys, cvals);
+    launch_after(st, grid, kSapThreads, 0, sap_entries_kernel, n, cursor, bounds, eoff, ckeys, cvals);
     const uint32_t ne = kSlots * n;
     bool c_tmp = false;
     if ((e = sort_pairs_async(ckeys, cvals, ckeys_tmp, cvals_tmp, ne, 16, csort, st, &c_tmp, eoff + n)) != cudaSuccess)
@@ -389,11 +455,11 @@ cudaError_t sap_pairs_async(uint32_t n, const float4* lo, const float4* hi, void
     const PairSink sink{counts, keep, status + 1, off, cursor, out, n, pair_cap};
     if ((e = cudaMemsetAsync(counts, 0, 4 * m, st)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(cursor, 0, 4 * m, st)) != cudaSuccess) return e;
-    launch_after(st, grid_for(ne, kSapThreads), kSapThreads, 0, sweep_binned_kernel<false>, eoff + n, sk, sv, box,
-                 bounds, sink);
+    launch_after(st, std::min(grid_for(ne, kSweep), 152u * kSweepBlocks), kSweep, 0, sweep_binned_kernel<false>, eoff + n, sk, sv, box, bounds,
+                 sink);
     if ((e = scan_exclusive_async(counts, off, n, scan, st)) != cudaSuccess) return e;
-    launch_after(st, grid_for(ne, kSapThreads), kSapThreads, 0, sweep_binned_kernel<true>, eoff + n, sk, sv, box,
-                 bounds, sink);
+    launch_after(st, std::min(grid_for(ne, kSweep), 152u * 4), kSweep, 0, sweep_binned_kernel<true>, eoff + n, sk, sv,
+                 box, bounds, sink);
     launch_after(st, grid, kSapThreads, 0, pairs_write_kernel, sink, d_count2, status);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     return cudaMemcpyAsync(d_count2 + 1, status, 4, cudaMemcpyDeviceToDevice, st);

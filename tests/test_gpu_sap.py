@@ -169,3 +169,24 @@ def test_pair_offsets_over_scan_sizes(sdlib, n):
     got, cnt, err = sdlib.SweepAndPrune.pairs(L, H, n)
     i = torch.arange(n - 1, device="cuda")
     assert err == 0 and cnt == n - 1 and torch.equal(got, (i << 32) | (i + 1))
+
+
+@pytest.mark.parametrize("n,cols", [(255, 1), (256, 1), (257, 2), (700, 2), (3000, 1), (20_000, 8)])
+def test_sweep_past_a_blocks_entries(sdlib, orc, n, cols):
+    """Columns of entries around and over the 256 + 64 that a block holds, x
+    windows of some and of all of them, more pairs than a block sets aside,
+    and pairs whose boxes share two and four columns."""
+    import torch
+    rng = np.random.default_rng(n)
+    c = rng.uniform(0.0, 1.0, (n, 3)).astype(np.float32)
+    c[:, 1:] = 0.013 * rng.integers(0, cols, (n, 2)) + rng.uniform(0.0, 0.012, (n, 2))
+    h = np.full((n, 3), 0.005, np.float32)
+    h[:, 0] = 0.5 * np.where(rng.random(n) < 0.05, 0.6, 60.0 / n)
+    L = np.zeros((n, 4), np.float32)
+    H = np.zeros((n, 4), np.float32)
+    L[:, :3] = c - h
+    H[:, :3] = c + h
+    want = orc.aabb_pairs(L, H)
+    got, cnt, err = sdlib.SweepAndPrune.pairs(torch.from_numpy(L).cuda(), torch.from_numpy(H).cuda(), len(want) + 1)
+    assert err == 0 and cnt == len(want)
+    assert np.array_equal(got.cpu().numpy().view(np.uint64), want)
