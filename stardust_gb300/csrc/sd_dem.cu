@@ -1448,16 +1448,46 @@ __global__ void dem_slot_of_id_kernel(const float4* __restrict__ omg, uint32_t* 
 // Id-ordered host buffer <-> slot-ordered state, one thread per id: the
 // host side is read or written in order (one pass over the host link); the
 // slot side is the random one, in device memory.
+// CHECK: positions, looked at as they pass.  *changed (the host's memory) is set
+// when a sphere's cell key is not the one it is sorted under (null: not asked);
+// the lists' build flag when one is more than 0.45 skin from its position at the
+// last build (the steps' own check runs only after integration).  Kernels of
+// their own for the two took 8 us at 131,072 spheres, a counter's clearing and
+// copy 6 more.
+struct HostCheck {
+    DemParams p;
+    Batch bt;
+    const uint32_t* sorted_keys;
+    uint32_t* changed;
+    const float4* ref;  // null: no lists
+    float thr2;
+    uint32_t* flags;
+};
+
+template <bool CHECK>
 __global__ void dem_by_id_in_kernel(const float4* __restrict__ host_src, const uint32_t* __restrict__ slot_of_id,
-                                    float4* __restrict__ dst, uint32_t n, bool keep_w) {
+                                    float4* __restrict__ dst, uint32_t n, bool keep_w, HostCheck k) {
     stream_wait();
     const uint32_t id = blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= n) return;
-    const uint32_t s = slot_of_id[id];
-    if (s >= n) return;
-    float4 v = host_src[id];
-    if (keep_w) v.w = dst[s].w;
-    dst[s] = v;
+    const uint32_t s = id < n ? slot_of_id[id] : n;
+    bool changed = false, far = false;
+    if (s < n) {
+        float4 v = host_src[id];
+        if (keep_w) v.w = dst[s].w;
+        dst[s] = v;
+        if (CHECK && k.changed) {
+            const Grid g = k.bt.n > 1 ? grid_of_slot(k.bt.scenes, k.bt.first, k.bt.n, s) : grid_of(k.p);
+            changed = cell_key_g(g, v.x, v.y, v.z) != k.sorted_keys[s];
+        }
+        if (CHECK && k.ref) {
+            const float4 r = k.ref[s];
+            far = dist2(v.x - r.x, v.y - r.y, v.z - r.z) > k.thr2;
+        }
+    }
+    if (CHECK) {
+        if (__ballot_sync(0xffffffffu, changed) && lane_id() == 0) *(volatile uint32_t*)k.changed = 1u;
+        if (__ballot_sync(0xffffffffu, far) && lane_id() == 0) k.flags[0] = 1u;
+    }
 }
 
 __global__ void dem_by_id_out_kernel(const float4* __restrict__ src, const uint32_t* __restrict__ slot_of_id,
@@ -1891,19 +1921,35 @@ cudaError_t dem_slot_of_all_async(const float4* omg, uint32_t* slot_of, uint32_t
     return cudaGetLastError();
 }
 
-cudaError_t dem_host_in_async(const float4* host_src, const float4* omg, float4* dst, uint32_t* slot_of_id,
-                              uint32_t n, bool keep_w, cudaStream_t st) {
-    if (n == 0) return cudaSuccess;
-    launch_after(st, grid_for(n, 256), 256, 0, dem_slot_of_id_kernel, omg, slot_of_id, n);
-    launch_after(st, grid_for(n, 256), 256, 0, dem_by_id_in_kernel, host_src, slot_of_id, dst, n, keep_w);
+// The id -> slot table: kept for every sphere while the lists are on, else made
+// in tmp for this transfer (3.5 us at 131,072 spheres, and a launch).
+static const uint32_t* slot_table(const DemBuffers& b, uint32_t* tmp, cudaStream_t st) {
+    if (slot_all_of(b) && b.slot_of) return b.slot_of;
+    launch_after(st, grid_for(b.n, 256), 256, 0, dem_slot_of_id_kernel, b.omg, tmp, b.n);
+    return tmp;
+}
+
+cudaError_t dem_host_in_async(const DemParams& p, const DemBuffers& b, const float4* host_src, float4* dst, uint32_t* tmp,
+                              bool keep_w, bool position, uint32_t* changed, cudaStream_t st) {
+    if (b.n == 0) return cudaSuccess;
+    const uint32_t* table = slot_table(b, tmp, st);
+    const bool skin = b.vl_flags && b.vl_skin > 0.0f;
+    if (position && (changed || skin)) {
+        const float thr = 0.45f * b.vl_skin;
+        const HostCheck c{p, Batch{b.scenes, b.scene_first, b.nscenes}, b.keys_prev, changed, skin ? b.vl_ref : nullptr,
+                          thr * thr, b.vl_flags};
+        launch_after(st, grid_for(b.n, 256), 256, 0, dem_by_id_in_kernel<true>, host_src, table, dst, b.n, keep_w, c);
+    } else {
+        launch_after(st, grid_for(b.n, 256), 256, 0, dem_by_id_in_kernel<false>, host_src, table, dst, b.n, keep_w,
+                     HostCheck{});
+    }
     return cudaGetLastError();
 }
 
-cudaError_t dem_host_out_async(const float4* src, const float4* omg, float4* host_dst, uint32_t* slot_of_id,
-                               uint32_t n, cudaStream_t st) {
-    if (n == 0) return cudaSuccess;
-    launch_after(st, grid_for(n, 256), 256, 0, dem_slot_of_id_kernel, omg, slot_of_id, n);
-    launch_after(st, grid_for(n, 256), 256, 0, dem_by_id_out_kernel, src, slot_of_id, host_dst, n);
+cudaError_t dem_host_out_async(const DemBuffers& b, const float4* src, float4* host_dst, uint32_t* tmp,
+                               cudaStream_t st) {
+    if (b.n == 0) return cudaSuccess;
+    launch_after(st, grid_for(b.n, 256), 256, 0, dem_by_id_out_kernel, src, slot_table(b, tmp, st), host_dst, b.n);
     return cudaGetLastError();
 }
 

@@ -110,6 +110,8 @@ void release_device(sd_engine* h) {
     h->B = sd::DemBuffers{};
     h->d_energy = nullptr;
     h->d_tmp = nullptr;
+    if (h->host_word) cudaFreeHost(h->host_word);
+    h->host_word = nullptr;
     if (h->stream) cudaStreamDestroy(h->stream);
     h->stream = nullptr;
     h->prepared = false;
@@ -1520,8 +1522,7 @@ sd_status sd_engine_get_state(sd_engine* h, int32_t field, void* host_dst, size_
         // recorded by sphere id already
         SD_CUDA(h, cudaMemcpyAsync(host_dst, src, bytes, cudaMemcpyDeviceToHost, h->stream));
     } else if (float4* dev_view = static_cast<float4*>(mapped_host(host_dst))) {
-        SD_CUDA(h, sd::dem_host_out_async(src, h->B.omg, dev_view, reinterpret_cast<uint32_t*>(h->d_tmp), n,
-                                          h->stream));
+        SD_CUDA(h, sd::dem_host_out_async(h->B, src, dev_view, reinterpret_cast<uint32_t*>(h->d_tmp), h->stream));
     } else {
         SD_CUDA(h, sd::dem_unsort_async(src, h->B.omg, h->d_tmp, n, h->stream));
         SD_CUDA(h, cudaMemcpyAsync(host_dst, h->d_tmp, bytes, cudaMemcpyDeviceToHost, h->stream));
@@ -1548,19 +1549,28 @@ sd_status sd_engine_set_state(sd_engine* h, int32_t field, const void* host_src,
     float4* dst = const_cast<float4*>(field_ptr(h, field));
     // the omega array's w lane holds the slot's sphere id: keep it
     const bool keep_w = field == SD_FIELD_OMEGA;
-    if (const float4* in = static_cast<const float4*>(mapped_host(host_src))) {
-        SD_CUDA(h, sd::dem_host_in_async(in, h->B.omg, dst, reinterpret_cast<uint32_t*>(h->d_tmp), n, keep_w,
-                                         h->stream));
-    } else {
-        SD_CUDA(h, cudaMemcpyAsync(h->d_tmp, host_src, bytes, cudaMemcpyHostToDevice, h->stream));
-        SD_CUDA(h, sd::dem_scatter_in_async(h->d_tmp, h->B.omg, dst, n, keep_w, h->stream));
-    }
     // Only a position change can change cell keys.  When every sphere stays
     // in the cell it is sorted under, a stable re-sort is the identity and
-    // the cell table still holds: count the slots whose key changed, and
+    // the cell table still holds: look for slots whose key changed, and
     // re-sort before the next step only if there are any.
-    const bool check = field == SD_FIELD_POSITION && h->keys_current && !h->need_resort;
+    const bool position = field == SD_FIELD_POSITION, check = position && h->keys_current && !h->need_resort;
     uint32_t changed = 1;
+    if (const float4* in = static_cast<const float4*>(mapped_host(host_src))) {
+        if (!h->host_word) {
+            SD_CUDA(h, cudaHostAlloc(reinterpret_cast<void**>(&h->host_word), sizeof(uint32_t), cudaHostAllocMapped));
+            SD_CUDA(h, cudaHostGetDevicePointer(reinterpret_cast<void**>(&h->host_word_dev), h->host_word, 0));
+        }
+        volatile uint32_t* word = h->host_word;
+        *word = 0u;
+        SD_CUDA(h, sd::dem_host_in_async(h->P, h->B, in, dst, reinterpret_cast<uint32_t*>(h->d_tmp), keep_w, position,
+                                         check ? h->host_word_dev : nullptr, h->stream));
+        SD_CUDA(h, cudaStreamSynchronize(h->stream));
+        if (check) changed = *word;
+        if (position && changed != 0) h->need_resort = true;
+        return SD_OK;
+    }
+    SD_CUDA(h, cudaMemcpyAsync(h->d_tmp, host_src, bytes, cudaMemcpyHostToDevice, h->stream));
+    SD_CUDA(h, sd::dem_scatter_in_async(h->d_tmp, h->B.omg, dst, n, keep_w, h->stream));
     if (check) {
         uint32_t* d_changed = h->B.dev_status + 4;
         SD_CUDA(h, sd::dem_keys_changed_async(h->P, h->B, d_changed, h->stream));
@@ -1569,9 +1579,9 @@ sd_status sd_engine_set_state(sd_engine* h, int32_t field, const void* host_src,
     // new positions: the contact lists are built again at the next step if
     // a sphere left its skin (lists that are off are rebuilt when they come
     // back on)
-    if (field == SD_FIELD_POSITION) SD_CUDA(h, sd::dem_skin_check_async(h->B, h->stream));
+    if (position) SD_CUDA(h, sd::dem_skin_check_async(h->B, h->stream));
     SD_CUDA(h, cudaStreamSynchronize(h->stream));
-    if (field == SD_FIELD_POSITION && changed != 0) h->need_resort = true;
+    if (position && changed != 0) h->need_resort = true;
     return SD_OK;
 }
 

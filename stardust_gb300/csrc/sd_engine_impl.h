@@ -95,6 +95,7 @@ struct sd_engine {
     std::vector<void*> allocations;
     double* d_energy = nullptr;
     float4* d_tmp = nullptr;
+    uint32_t *host_word = nullptr, *host_word_dev = nullptr;  // a word of mapped page-locked memory
     // step graphs by kind.  When the step leaves the next state in the *_n
     // buffers (graph_swaps), each kind has a graph per assignment of the
     // buffers; graph_parity names the one whose input is the current state

@@ -383,18 +383,20 @@ int dem_contact_mode();
 cudaError_t dem_pairs_async(const DemParams& p, DemBuffers& b, cudaStream_t st);
 cudaError_t dem_unsort_async(const float4* src, const float4* omg, float4* dst, uint32_t n,
                              cudaStream_t st);
-// State fields between a host buffer in sphere-id order that the device can
-// address (mapped page-locked memory) and the slot-ordered device arrays;
-// slot_of_id (n words) receives the id -> slot table.
 // After the host wrote positions: sets the lists' build flag when a sphere
 // left 0.45 skin of its position at the last build (no-op without lists).
 cudaError_t dem_skin_check_async(const DemBuffers& b, cudaStream_t st);
 // slot_of[id] = slot of every sphere of the current state (ids in omg.w).
 cudaError_t dem_slot_of_all_async(const float4* omg, uint32_t* slot_of, uint32_t n, cudaStream_t st);
-cudaError_t dem_host_in_async(const float4* host_src, const float4* omg, float4* dst, uint32_t* slot_of_id,
-                              uint32_t n, bool keep_w, cudaStream_t st);
-cudaError_t dem_host_out_async(const float4* src, const float4* omg, float4* host_dst, uint32_t* slot_of_id,
-                               uint32_t n, cudaStream_t st);
+// State fields between a host buffer in sphere-id order that the device can
+// address (mapped page-locked memory) and the slot-ordered device arrays; tmp: n
+// words.  Positions (position) are checked against the lists' skin on the way,
+// and with `changed` (mapped too, 0 before) against the keys they are sorted
+// under: 1 when one differs.
+cudaError_t dem_host_in_async(const DemParams& p, const DemBuffers& b, const float4* host_src, float4* dst, uint32_t* tmp,
+                              bool keep_w, bool position, uint32_t* changed, cudaStream_t st);
+cudaError_t dem_host_out_async(const DemBuffers& b, const float4* src, float4* host_dst, uint32_t* tmp,
+                               cudaStream_t st);
 cudaError_t dem_scatter_in_async(const float4* src_by_id, const float4* omg, float4* dst, uint32_t n, bool keep_w,
                                  cudaStream_t st);
 cudaError_t dem_energy_async(const DemBuffers& b, double* d_out, cudaStream_t st);

@@ -189,3 +189,49 @@ def test_listed_contacts_in_scan_order(sdlib, orc, squeeze, skin):
         eng.close()
     finally:
         _abi.tune_set("skin_um", old)
+
+
+@pytest.mark.parametrize("skin,n,shift", [(0, 3001, 3e-4), (500, 3001, 1e-5), (500, 3001, 3e-4), (500, 20_000, 0.02),
+                                          (500, 1, 0.02)])
+def test_page_locked_transfers_as_staged(sdlib, skin, n, shift):
+    """States that kernels read and write in page-locked memory, checked on
+    the way against the cells and the skin, against the staged path with its
+    separate checks: positions that stay, leave their skin, change cells."""
+    import ctypes
+    import torch
+    from stardust_gb300 import _abi
+    old = _abi.tune_get("skin_um")
+    try:
+        _abi.tune_set("skin_um", skin)
+        pos, vel, cfg, dt = scene(max(n, 300), 1.2, 0.5, seed=9)
+        pos, vel = pos[:n], vel[:n]
+        got = []
+        for pinned in (False, True):
+            eng = sdlib.DEMEngine(cfg)
+            eng.add_spheres(pos, vel)
+            eng.prepare()
+            buf = [torch.empty((n, 4), pin_memory=True) if pinned else torch.empty((n, 4)) for _ in range(3)]
+
+            def move(name, f, t):
+                _abi.call(name, eng._h, f, ctypes.c_void_p(t.data_ptr()), t.numel() * 4, h=eng._h)
+
+            out = []
+            for k in range(4):
+                eng.step(dt, 3)
+                for f, t in enumerate(buf):
+                    move("sd_engine_get_state", (_abi.SD_FIELD_POSITION, _abi.SD_FIELD_VELOCITY, _abi.SD_FIELD_OMEGA)[f], t)
+                out += [t.numpy().copy() for t in buf]
+                if k % 2 == 0:
+                    buf[0][:, k % 3] += shift * (torch.arange(n) % 7 == 0)
+                move("sd_engine_set_state", _abi.SD_FIELD_POSITION, buf[0])
+                move("sd_engine_set_state", _abi.SD_FIELD_OMEGA, buf[2])
+                move("sd_engine_set_state", _abi.SD_FIELD_VELOCITY, buf[1])
+            st = eng.stats()
+            assert st["device_errors"] == 0
+            got.append((out, st["list_builds"]))
+            eng.close()
+        assert got[0][1] == got[1][1]
+        for a, b in zip(*(g[0] for g in got)):
+            assert np.array_equal(bits(a), bits(b))
+    finally:
+        _abi.tune_set("skin_um", old)
