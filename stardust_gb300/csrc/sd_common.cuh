@@ -91,21 +91,33 @@ __device__ __forceinline__ void stream_wait() {
     if (wait) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-template <class... P, class... A>
-inline void launch_after(cudaStream_t st, dim3 grid, dim3 block, size_t smem, void (*kernel)(P...), A&&... args) {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    const bool plain = cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
+// launch_chained(): also between the nodes of a graph (0.2 us less each), for
+// graphs that the engine captures for itself; launch_after() captures a plain
+// launch, as the graph is then a caller's.
+template <bool COOPERATIVE = false, class... P, class... A>
+inline void launch_chained(cudaStream_t st, dim3 grid, dim3 block, size_t smem, void (*kernel)(P...), A&&... args) {
+    cudaLaunchAttribute attr[2]{};
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeCooperative;
+    attr[1].val.cooperative = 1;
     cudaLaunchConfig_t c{};
     c.gridDim = grid;
     c.blockDim = block;
     c.dynamicSmemBytes = smem;
     c.stream = st;
-    c.attrs = &attr;
-    c.numAttrs = plain ? 0 : 1;
+    c.attrs = attr;
+    c.numAttrs = COOPERATIVE ? 2 : 1;
     cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...);  // (an error is the next cudaGetLastError's)
+}
+
+template <class... P, class... A>
+inline void launch_after(cudaStream_t st, dim3 grid, dim3 block, size_t smem, void (*kernel)(P...), A&&... args) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone)
+        launch_chained(st, grid, block, smem, kernel, std::forward<A>(args)...);
+    else
+        kernel<<<grid, block, smem, st>>>(std::forward<A>(args)...);
 }
 
 }  // namespace sd

@@ -932,7 +932,8 @@ dem_contact_listed_kernel(DemParams p, uint32_t n, const float4* __restrict__ po
                           float4* __restrict__ pos_n, float4* __restrict__ vel_n, float4* __restrict__ omg_n,
                           uint32_t* __restrict__ keys, uint32_t* __restrict__ vals, float4* __restrict__ force,
                           float4* __restrict__ torque, uint32_t* __restrict__ status, SkinLists sk, MoveSink ms,
-                          Batch bt, ClumpCtx cc = ClumpCtx{}, MeshView mesh = MeshView{}) {
+                          Batch bt, ClumpCtx cc, MeshView mesh) {
+    stream_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t contacts = 0, key = 0;
     bool has_key = false;
@@ -1237,6 +1238,7 @@ dem_body_kernel(DemParams p, uint32_t nb, float4* __restrict__ bpos, float4* __r
                 const float4* __restrict__ st, float4* __restrict__ pos_n, float4* __restrict__ vel_n,
                 float4* __restrict__ omg_n, uint32_t* __restrict__ keys, uint32_t* __restrict__ vals, uint32_t n,
                 uint32_t hist_spec, uint32_t* __restrict__ ghist, MoveSink ms, SkinLists sk) {
+    stream_wait();
     __shared__ uint32_t s_hist[kHistWords];
     if (ghist) {
         for (int q = threadIdx.x; q < kHistWords; q += blockDim.x) s_hist[q] = 0;
@@ -1704,41 +1706,41 @@ static void launch_contact_t(const DemParams& p, DemBuffers& b, uint32_t spec, u
         const Batch bt{b.scenes, b.scene_first, b.nscenes};
         if (b.nscenes > 1) {
             if (blocks == 5)
-                dem_contact_listed_kernel<RECORD, 5, true><<<lgrid, kListedThreads, 0, st>>>(
-                    p, b.n, b.pos, b.vel, b.omg, b.cell_start, b.pos_n, b.vel_n, b.omg_n, b.keys, vals, f, t,
-                    b.dev_status, sk, ms, bt);
+                launch_chained(st, lgrid, kListedThreads, 0, dem_contact_listed_kernel<RECORD, 5, true>, p, b.n,
+                               b.pos, b.vel, b.omg, b.cell_start, b.pos_n, b.vel_n, b.omg_n, b.keys, vals, f, t,
+                               b.dev_status, sk, ms, bt, ClumpCtx{}, MeshView{});
             else
-                dem_contact_listed_kernel<RECORD, 4, true><<<lgrid, kListedThreads, 0, st>>>(
-                    p, b.n, b.pos, b.vel, b.omg, b.cell_start, b.pos_n, b.vel_n, b.omg_n, b.keys, vals, f, t,
-                    b.dev_status, sk, ms, bt);
+                launch_chained(st, lgrid, kListedThreads, 0, dem_contact_listed_kernel<RECORD, 4, true>, p, b.n,
+                               b.pos, b.vel, b.omg, b.cell_start, b.pos_n, b.vel_n, b.omg_n, b.keys, vals, f, t,
+                               b.dev_status, sk, ms, bt, ClumpCtx{}, MeshView{});
         } else if (b.nb && b.mesh.ntri) {
-            dem_contact_listed_kernel<RECORD, 4, false, true, true><<<lgrid, kListedThreads, 0, st>>>(
-                p, b.n, b.pos, b.vel, b.omg, b.cell_start, b.pos_n, b.vel_n, b.omg_n, b.keys, vals, f, t,
-                b.dev_status, sk, ms, Batch{}, cc, b.mesh);
+            launch_chained(st, lgrid, kListedThreads, 0, dem_contact_listed_kernel<RECORD, 4, false, true, true>, p,
+                           b.n, b.pos, b.vel, b.omg, b.cell_start, b.pos_n, b.vel_n, b.omg_n, b.keys, vals, f, t,
+                           b.dev_status, sk, ms, Batch{}, cc, b.mesh);
         } else if (b.nb) {
-            dem_contact_listed_kernel<RECORD, 4, false, true, false><<<lgrid, kListedThreads, 0, st>>>(
-                p, b.n, b.pos, b.vel, b.omg, b.cell_start, b.pos_n, b.vel_n, b.omg_n, b.keys, vals, f, t,
-                b.dev_status, sk, ms, Batch{}, cc);
+            launch_chained(st, lgrid, kListedThreads, 0, dem_contact_listed_kernel<RECORD, 4, false, true, false>, p,
+                           b.n, b.pos, b.vel, b.omg, b.cell_start, b.pos_n, b.vel_n, b.omg_n, b.keys, vals, f, t,
+                           b.dev_status, sk, ms, Batch{}, cc, MeshView{});
         } else if (b.mesh.ntri) {
-            dem_contact_listed_kernel<RECORD, 4, false, false, true><<<lgrid, kListedThreads, 0, st>>>(
-                p, b.n, b.pos, b.vel, b.omg, b.cell_start, b.pos_n, b.vel_n, b.omg_n, b.keys, vals, f, t,
-                b.dev_status, sk, ms, Batch{}, ClumpCtx{}, b.mesh);
+            launch_chained(st, lgrid, kListedThreads, 0, dem_contact_listed_kernel<RECORD, 4, false, false, true>, p,
+                           b.n, b.pos, b.vel, b.omg, b.cell_start, b.pos_n, b.vel_n, b.omg_n, b.keys, vals, f, t,
+                           b.dev_status, sk, ms, Batch{}, ClumpCtx{}, b.mesh);
         } else if (blocks == 6) {
-            dem_contact_listed_kernel<RECORD, 6, false><<<lgrid, kListedThreads, 0, st>>>(
-                p, b.n, b.pos, b.vel, b.omg, b.cell_start, b.pos_n, b.vel_n, b.omg_n, b.keys, vals, f, t,
-                b.dev_status, sk, ms, Batch{});
+            launch_chained(st, lgrid, kListedThreads, 0, dem_contact_listed_kernel<RECORD, 6, false>, p, b.n, b.pos,
+                           b.vel, b.omg, b.cell_start, b.pos_n, b.vel_n, b.omg_n, b.keys, vals, f, t, b.dev_status,
+                           sk, ms, Batch{}, ClumpCtx{}, MeshView{});
         } else if (blocks == 8) {
-            dem_contact_listed_kernel<RECORD, 8, false><<<lgrid, kListedThreads, 0, st>>>(
-                p, b.n, b.pos, b.vel, b.omg, b.cell_start, b.pos_n, b.vel_n, b.omg_n, b.keys, vals, f, t,
-                b.dev_status, sk, ms, Batch{});
+            launch_chained(st, lgrid, kListedThreads, 0, dem_contact_listed_kernel<RECORD, 8, false>, p, b.n, b.pos,
+                           b.vel, b.omg, b.cell_start, b.pos_n, b.vel_n, b.omg_n, b.keys, vals, f, t, b.dev_status,
+                           sk, ms, Batch{}, ClumpCtx{}, MeshView{});
         } else if (blocks == 5) {
-            dem_contact_listed_kernel<RECORD, 5, false><<<lgrid, kListedThreads, 0, st>>>(
-                p, b.n, b.pos, b.vel, b.omg, b.cell_start, b.pos_n, b.vel_n, b.omg_n, b.keys, vals, f, t,
-                b.dev_status, sk, ms, Batch{});
+            launch_chained(st, lgrid, kListedThreads, 0, dem_contact_listed_kernel<RECORD, 5, false>, p, b.n, b.pos,
+                           b.vel, b.omg, b.cell_start, b.pos_n, b.vel_n, b.omg_n, b.keys, vals, f, t, b.dev_status,
+                           sk, ms, Batch{}, ClumpCtx{}, MeshView{});
         } else {
-            dem_contact_listed_kernel<RECORD, 4, false><<<lgrid, kListedThreads, 0, st>>>(
-                p, b.n, b.pos, b.vel, b.omg, b.cell_start, b.pos_n, b.vel_n, b.omg_n, b.keys, vals, f, t,
-                b.dev_status, sk, ms, Batch{});
+            launch_chained(st, lgrid, kListedThreads, 0, dem_contact_listed_kernel<RECORD, 4, false>, p, b.n, b.pos,
+                           b.vel, b.omg, b.cell_start, b.pos_n, b.vel_n, b.omg_n, b.keys, vals, f, t, b.dev_status,
+                           sk, ms, Batch{}, ClumpCtx{}, MeshView{});
         }
     } else if (b.mesh.ntri) {  // mesh walls (one scene; clumps allowed; per-slot kernel)
         if (b.nb)
@@ -1804,12 +1806,11 @@ static cudaError_t launch_contact(const DemParams& p, DemBuffers& b, bool record
         launch_contact_t<false>(p, b, spec, ghist, st, skin, ms);
     }
     if (b.nb) {
-        dem_body_kernel<<<grid_for(4u * b.nb, 128), 128, 0, st>>>(
-            p, b.nb, b.bpos, b.bvel, b.bquat, b.bomg, b.bang, b.binv, b.bfirst, b.bcount, b.r0, b.slot_of, b.pos,
-            b.omg, b.sf, b.st, b.pos_n, b.vel_n, b.omg_n, b.keys, ms.list ? nullptr : b.vals, b.n, spec, ghist, ms,
-            skin ? SkinLists{b.vl_cnt, b.vl_nbr, b.vl_ref, b.vl_flags, b.vl_flags + 1, b.slot_of, b.vl_skin,
-                             (0.45f * b.vl_skin) * (0.45f * b.vl_skin)}
-                 : SkinLists{});
+        launch_chained(st, grid_for(4u * b.nb, 128), 128, 0, dem_body_kernel, p, b.nb, b.bpos, b.bvel, b.bquat,
+                       b.bomg, b.bang, b.binv, b.bfirst, b.bcount, b.r0, b.slot_of, b.pos, b.omg, b.sf, b.st,
+                       b.pos_n, b.vel_n, b.omg_n, b.keys, ms.list ? nullptr : b.vals, b.n, spec, ghist, ms, skin ?
+                       SkinLists{b.vl_cnt, b.vl_nbr, b.vl_ref, b.vl_flags, b.vl_flags + 1, b.slot_of, b.vl_skin,
+                       (0.45f * b.vl_skin) * (0.45f * b.vl_skin)} : SkinLists{});
     }
     return cudaGetLastError();
 }

@@ -410,6 +410,7 @@ __device__ __forceinline__ bool radix_sort_grid(const StepArgs& a, uint32_t* sme
 // place and cells 2.5.  Two blocks per SM (registers of the fallback's tiles).
 template <int BINS, int ITEMS>
 __global__ void __launch_bounds__(kStepThreads, 2) resort_step_kernel(StepArgs a) {
+    stream_wait();
     extern __shared__ __align__(16) uint32_t smem[];
     __shared__ uint32_t ws[33], s_tile, s_keys[kReorderThreads + 1];
     const uint32_t M = a.scratch[0];
@@ -519,10 +520,8 @@ cudaError_t launch_step(const StepArgs& a, int per_sm, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     const uint32_t most = (uint32_t)(sms * (fit < per_sm ? fit : per_sm));
     const uint32_t want = (a.n + kStepThreads - 1) / kStepThreads;
-    StepArgs arg = a;
-    void* args[] = {&arg};
-    return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(want < most ? want : most),
-                                       dim3(kStepThreads), args, sm, st);
+    launch_chained<true>(st, want < most ? want : most, kStepThreads, sm, kernel, a);
+    return cudaGetLastError();
 }
 
 }  // namespace
