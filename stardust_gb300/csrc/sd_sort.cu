@@ -111,9 +111,14 @@ sort_pass_kernel(const uint32_t* __restrict__ keys_in, const uint32_t* __restric
     __shared__ uint32_t s_tile;
     if (threadIdx.x == 0) s_tile = atomicAdd(&scratch[4 + pass], 1u);
     __syncthreads();
-    if (s_tile >= (n + kSortThreads * ITEMS - 1) / (kSortThreads * ITEMS)) return;  // d_n: fewer keys than the grid's
-    sort_tile<BINS, ITEMS>(smem, s_tile, keys_in, vals_in, keys_out, vals_out, n, shift, bits, pass, num_tiles, hstride,
-                           bins, scratch);
+    constexpr uint32_t kTile = kSortThreads * ITEMS;
+    const uint32_t tile = s_tile;
+    if (tile < n / kTile)
+        sort_tile<BINS, ITEMS, true>(smem, tile, keys_in, vals_in, keys_out, vals_out, n, shift, bits, pass, num_tiles,
+                                     hstride, bins, scratch);
+    else if (tile < (n + kTile - 1) / kTile)  // (d_n: fewer keys than the grid's)
+        sort_tile<BINS, ITEMS>(smem, tile, keys_in, vals_in, keys_out, vals_out, n, shift, bits, pass, num_tiles, hstride,
+                               bins, scratch);
 }
 
 // Smallest tile the pass kernel is instantiated with; sizes the status area.
