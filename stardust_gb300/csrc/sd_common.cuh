@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <initializer_list>
 #include <utility>
 
 #include "../../include/stardust.h"
@@ -118,6 +119,36 @@ inline void launch_after(cudaStream_t st, dim3 grid, dim3 block, size_t smem, vo
         launch_chained(st, grid, block, smem, kernel, std::forward<A>(args)...);
     else
         kernel<<<grid, block, smem, st>>>(std::forward<A>(args)...);
+}
+
+// Up to four ranges of words set to zero by one launch of the chain (a memset
+// between two kernels ends it: 3 us each); while capturing, memsets, as before.
+struct ZeroRange {
+    void* p;
+    uint64_t words;
+};
+static __global__ void zero_kernel(ZeroRange a, ZeroRange b, ZeroRange c, ZeroRange d) {
+    stream_wait();
+    const uint64_t first = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (uint64_t)gridDim.x * blockDim.x;
+    const ZeroRange r[4] = {a, b, c, d};
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        for (uint64_t i = first; i < r[k].words; i += step) static_cast<uint32_t*>(r[k].p)[i] = 0u;
+}
+static inline cudaError_t zero_async(cudaStream_t st, ZeroRange a, ZeroRange b = {nullptr, 0}, ZeroRange c = {nullptr, 0},
+                                     ZeroRange d = {nullptr, 0}) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
+        uint64_t most = 1;
+        for (const ZeroRange& r : {a, b, c, d}) most = r.words > most ? r.words : most;
+        const uint64_t blocks = (most + 1023) / 1024;
+        launch_chained(st, (unsigned)(blocks < 608 ? blocks : 608), 256, 0, zero_kernel, a, b, c, d);
+        return cudaGetLastError();
+    }
+    for (const ZeroRange& r : {a, b, c, d})
+        if (r.words)
+            if (cudaError_t e = cudaMemsetAsync(r.p, 0, 4 * r.words, st)) return e;
+    return cudaSuccess;
 }
 
 }  // namespace sd

@@ -640,6 +640,7 @@ sd_status sd_lbvh_pairs(uint64_t n, const float* d_lo4, const float* d_hi4, uint
     const float4* lo = reinterpret_cast<const float4*>(d_lo4);
     const float4* hi = reinterpret_cast<const float4*>(d_hi4);
     cudaError_t e = cudaMemsetAsync(t.status, 0, 16, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(d_count, 0, 8, st);
     if (e == cudaSuccess) e = sd::lbvh_build_async(t, lo, hi, st);
     if (e == cudaSuccess)
         e = sd::lbvh_unique_pairs_async(t, off, reinterpret_cast<unsigned long long*>(d_pairs), cap, d_count, st);

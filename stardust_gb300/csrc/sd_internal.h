@@ -35,7 +35,7 @@ int sort_num_passes(int key_bits);
 void sort_set_items(int items);
 int sort_items();
 uint32_t* sort_hist_ptr(uint32_t* scratch);  // global digit histograms, pass q at q * plan.stride (2048 words)
-cudaError_t sort_clear_async(uint32_t n, const SortPlan& plan, uint32_t* scratch, cudaStream_t st);
+cudaError_t sort_clear_async(uint32_t n, const SortPlan& plan, uint32_t* scratch, cudaStream_t st, bool checked = false);
 // skip (may be null): the passes return at once when skip[1] <= skip_max
 // (the incremental re-sort has written the result)
 // The radix fallback of the incremental re-sort: when skip[1] > skip_max,
@@ -52,9 +52,10 @@ cudaError_t sort_passes_async(uint32_t* keys, uint32_t* vals, uint32_t* keys_tmp
                               bool* in_tmp, const uint32_t* skip = nullptr, uint32_t skip_max = 0,
                               const uint32_t* d_n = nullptr);
 // d_n (may be null): a device word, the number of keys when it is below n
+// checked: scratch is known to be good (else the clearing memset finds out).
 cudaError_t sort_pairs_async(uint32_t* keys, uint32_t* vals, uint32_t* keys_tmp, uint32_t* vals_tmp,
                              uint32_t n, int key_bits, uint32_t* scratch, cudaStream_t st,
-                             bool* in_tmp, const uint32_t* d_n = nullptr);
+                             bool* in_tmp, const uint32_t* d_n = nullptr, bool checked = false);
 
 // ---- reference-compatible spatial hash (sd_hash_ref.cu)
 cudaError_t ref_hash_build_async(uint32_t n, float cell_dim, uint32_t* cells, uint32_t* spheres,

@@ -554,6 +554,7 @@ query_kernel(int n, const uint32_t* __restrict__ vals, const float4* __restrict_
     if (MODE == kRefill && !sink_refill(sink)) return;
     PairBuffer<MODE == kPairs ? 128 : 1>& found = s_found[threadIdx.x >> 5];
     if (lane == 0) found.n = 0u;
+    if (MODE == kPairs && sub == 0 && k < n) sink.cursor[k] = 0u;
     bool walk = k < n;
     const uint32_t id = walk ? vals[k] : 0u;
     uint32_t c = 0;
@@ -757,8 +758,8 @@ cudaError_t lbvh_build_async(Lbvh& t, const float4* lo, const float4* hi, cudaSt
     if (n == 0) return cudaSuccess;
     if ((e = lbvh_morton_async(t, lo, hi, st)) != cudaSuccess) return e;
     bool in_tmp = false;
-    if ((e = sort_pairs_async(t.keys, t.vals, t.keys_tmp, t.vals_tmp, n, 30, t.sort_scratch, st, &in_tmp)) !=
-        cudaSuccess)
+    if ((e = sort_pairs_async(t.keys, t.vals, t.keys_tmp, t.vals_tmp, n, 30, t.sort_scratch, st, &in_tmp, nullptr,
+                              true)) != cudaSuccess)
         return e;
     t.skeys = in_tmp ? t.keys_tmp : t.keys;
     t.svals = in_tmp ? t.vals_tmp : t.vals;
@@ -818,17 +819,16 @@ cudaError_t lbvh_unique_pairs_async(Lbvh& t, uint32_t* off, unsigned long long* 
                                     cudaStream_t st) {
     const uint32_t n = t.n;
     cudaError_t e;
-    if (n == 0) return cudaMemsetAsync(d_count2, 0, 8, st);
-    // t.keys: the codes are used up, the cursors take their place
+    if (n == 0) return cudaSuccess;
+    // t.keys: the codes are used up, the cursors take their place (cleared by the
+    // first search, for the second)
     const PairSink sink{t.counts, t.first, t.status + 1, off, t.keys, out, n, cap};
-    if ((e = cudaMemsetAsync(t.counts, 0, 4 * (size_t)n, st)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(t.keys, 0, 4 * (size_t)n, st)) != cudaSuccess) return e;
+    if ((e = zero_async(st, {t.counts, n})) != cudaSuccess) return e;
     launch_query<kPairs>(t, QueryOut{}, sink, st);
     if ((e = scan_exclusive_async(t.counts, off, n, t.scan_scratch, st)) != cudaSuccess) return e;
     launch_query<kRefill>(t, QueryOut{}, sink, st);
     launch_after(st, grid_for(n, kLbvhThreads), kLbvhThreads, 0, pairs_write_kernel, sink, d_count2, t.status);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    return cudaMemcpyAsync(d_count2 + 1, t.status, 4, cudaMemcpyDeviceToDevice, st);
+    return cudaGetLastError();
 }
 
 }  // namespace sd

@@ -73,20 +73,23 @@ __device__ __forceinline__ void sink_pair_again(const PairSink& s, uint32_t a, u
     if (at < s.off[i + 1] && at < s.cap) s.out[at] = ((unsigned long long)i << 32) | j;
 }
 
-static __global__ void pairs_write_kernel(PairSink s, uint32_t* __restrict__ d_count, uint32_t* __restrict__ status) {
+// d_count: the pairs (0 when they do not fit) and the error bits, status's among
+// them; both zero before.
+static __global__ void pairs_write_kernel(PairSink s, uint32_t* __restrict__ d_count,
+                                          const uint32_t* __restrict__ status) {
     stream_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t total = s.off[s.n];
     const bool fits = total <= s.cap;
     if (i == 0) {
         *d_count = fits ? total : 0u;
-        if (!fits) atomicOr(status, kErrPairOverflow);
+        atomicOr(d_count + 1, *status | (fits ? 0u : kErrPairOverflow));
     }
     if (i >= s.n || !fits) return;
     const uint32_t base = s.off[i], c = s.off[i + 1] - base;
     if (c == 0) return;
     if ((uint64_t)base + c > s.cap) {  // (only where 2^32 pairs or more wrapped the total)
-        atomicOr(status, kErrPairOverflow);
+        atomicOr(d_count + 1, kErrPairOverflow);
         return;
     }
     if (c <= kPairKeep) {

@@ -260,9 +260,10 @@ __global__ void sap_gather_kernel(uint32_t n, const uint32_t* __restrict__ svals
     count[k] = (dy + 1u) * (dz + 1u);
 }
 
-__global__ void sap_entries_kernel(uint32_t n, const uint32_t* __restrict__ span, const SapBounds* __restrict__ bounds,
-                                   const uint32_t* __restrict__ off, uint32_t* __restrict__ keys,
-                                   uint32_t* __restrict__ vals) {
+// (The columns and counts are used up: span and count, cleared, are the sink's.)
+__global__ void sap_entries_kernel(uint32_t n, uint32_t* __restrict__ span, uint32_t* __restrict__ count,
+                                   const SapBounds* __restrict__ bounds, const uint32_t* __restrict__ off,
+                                   uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
     stream_wait();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
@@ -274,6 +275,8 @@ __global__ void sap_entries_kernel(uint32_t n, const uint32_t* __restrict__ span
             keys[e] = y * (uint32_t)g.gz + z;
             vals[e++] = k;
         }
+    span[k] = 0u;
+    count[k] = 0u;
 }
 
 // Forward sweep of entry p inside its column: entries m > p of the same
@@ -432,37 +435,40 @@ cudaError_t sap_pairs_async(uint32_t n, const float4* lo, const float4* hi, void
     SapBounds* bounds = (SapBounds*)take(64);
     uint32_t* keep = (uint32_t*)take(4 * kPairKeep * m);
     static_assert(sizeof(SapBounds) <= 64, "bounds fit their scratch");
-    cudaError_t e = cudaMemsetAsync(status, 0, 16, st);
-    if (e != cudaSuccess) return e;
     if (n == 0) return cudaMemsetAsync(d_count2, 0, 8, st);
+    // (the caller's two pointers by memsets, which check them; the rest by kernels)
+    cudaError_t e = cudaMemsetAsync(status, 0, 16, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(d_count2, 0, 8, st);
+    if (e == cudaSuccess) e = zero_async(st, {bounds, sizeof(SapBounds) / 4});
+    if (e != cudaSuccess) return e;
     const uint32_t grid = grid_for(n, kSapThreads);
-    if ((e = cudaMemsetAsync(bounds, 0, sizeof(SapBounds), st)) != cudaSuccess) return e;
     launch_after(st, std::min<uint32_t>(grid, kBoundBlocks), kSapThreads, 0, sap_bounds_kernel, n, lo, hi, bounds,
                  keys, vals);
     bool in_tmp = false;
-    if ((e = sort_pairs_async(keys, vals, keys_tmp, vals_tmp, n, 32, sort_scratch, st, &in_tmp)) != cudaSuccess) return e;
+    if ((e = sort_pairs_async(keys, vals, keys_tmp, vals_tmp, n, 32, sort_scratch, st, &in_tmp, nullptr, true)) !=
+        cudaSuccess)
+        return e;
     // each box's entries, stably sorted by column
     launch_after(st, grid, kSapThreads, 0, sap_gather_kernel, n, in_tmp ? vals_tmp : vals, lo, hi, bounds, box,
                  cursor, counts, status);
     if ((e = scan_exclusive_async(counts, eoff, n, scan, st)) != cudaSuccess) return e;
-    launch_after(st, grid, kSapThreads, 0, sap_entries_kernel, n, cursor, bounds, eoff, ckeys, cvals);
+    launch_after(st, grid, kSapThreads, 0, sap_entries_kernel, n, cursor, counts, bounds, eoff, ckeys,
+                 cvals);
     const uint32_t ne = kSlots * n;
     bool c_tmp = false;
-    if ((e = sort_pairs_async(ckeys, cvals, ckeys_tmp, cvals_tmp, ne, 16, csort, st, &c_tmp, eoff + n)) != cudaSuccess)
+    if ((e = sort_pairs_async(ckeys, cvals, ckeys_tmp, cvals_tmp, ne, 16, csort, st, &c_tmp, eoff + n, true)) !=
+        cudaSuccess)
         return e;
     const uint32_t* sk = c_tmp ? ckeys_tmp : ckeys;
     const uint32_t* sv = c_tmp ? cvals_tmp : cvals;
     const PairSink sink{counts, keep, status + 1, off, cursor, out, n, pair_cap};
-    if ((e = cudaMemsetAsync(counts, 0, 4 * m, st)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(cursor, 0, 4 * m, st)) != cudaSuccess) return e;
-    launch_after(st, std::min(grid_for(ne, kSweep), 152u * kSweepBlocks), kSweep, 0, sweep_binned_kernel<false>, eoff + n, sk, sv, box, bounds,
-                 sink);
+    launch_after(st, std::min(grid_for(ne, kSweep), 152u * kSweepBlocks), kSweep, 0, sweep_binned_kernel<false>,
+                 eoff + n, sk, sv, box, bounds, sink);
     if ((e = scan_exclusive_async(counts, off, n, scan, st)) != cudaSuccess) return e;
     launch_after(st, std::min(grid_for(ne, kSweep), 152u * 4), kSweep, 0, sweep_binned_kernel<true>, eoff + n, sk, sv,
                  box, bounds, sink);
     launch_after(st, grid, kSapThreads, 0, pairs_write_kernel, sink, d_count2, status);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    return cudaMemcpyAsync(d_count2 + 1, status, 4, cudaMemcpyDeviceToDevice, st);
+    return cudaGetLastError();
 }
 
 }  // namespace sd

@@ -142,10 +142,11 @@ static uint32_t num_tiles(uint32_t n) {
     return (n + t - 1) / t;
 }
 
-cudaError_t sort_clear_async(uint32_t n, const SortPlan& plan, uint32_t* scratch, cudaStream_t st) {
+cudaError_t sort_clear_async(uint32_t n, const SortPlan& plan, uint32_t* scratch, cudaStream_t st, bool checked) {
     // counters, histograms and this sort's tile status; not the status word
     size_t clear_words = kStatusOff - 4 + (size_t)plan.passes * (size_t)status_words(num_tiles(n), status_bins(plan));
-    return cudaMemsetAsync(scratch + 4, 0, clear_words * sizeof(uint32_t), st);
+    return checked ? zero_async(st, {scratch + 4, clear_words})
+                   : cudaMemsetAsync(scratch + 4, 0, clear_words * sizeof(uint32_t), st);
 }
 
 // Blocks of the histogram kernels: 8 keys per thread and loop trip at small
@@ -231,11 +232,11 @@ cudaError_t sort_fallback_async(uint32_t* keys, uint32_t* vals, uint32_t* keys_t
 // device word, the number of keys when it is below n.
 cudaError_t sort_pairs_async(uint32_t* keys, uint32_t* vals, uint32_t* keys_tmp, uint32_t* vals_tmp,
                              uint32_t n, int key_bits, uint32_t* scratch, cudaStream_t st,
-                             bool* in_tmp, const uint32_t* d_n) {
+                             bool* in_tmp, const uint32_t* d_n, bool checked) {
     SortPlan plan = sort_plan(key_bits);
     *in_tmp = false;
     if (n == 0) return cudaSuccess;
-    cudaError_t e = sort_clear_async(n, plan, scratch, st);
+    cudaError_t e = sort_clear_async(n, plan, scratch, st, checked);
     if (e != cudaSuccess) return e;
     if ((e = sort_histogram_async(keys, n, plan, scratch, st, d_n)) != cudaSuccess) return e;
     return sort_passes_async(keys, vals, keys_tmp, vals_tmp, n, plan, scratch, st, in_tmp, nullptr, 0, d_n);
