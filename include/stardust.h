@@ -509,8 +509,8 @@ sd_status sd_engine_load_checkpoint(sd_engine* h, const char* path);
  *                   128 or 256 (default); the contact-list kernel takes 64
  *   "fix_blocks"    blocks per SM of the in-place reorder's fixed grid: 2, 4 or 8 (default);
  *                   calls of four or more steps: 1 below 8, else 2
- *   "hull_blocks"   convex-hull scenes: resident 128-thread blocks per SM the GJK kernel is
- *                   compiled for: 3 (168 registers) or 4 (128, the default)
+ *   "hull_blocks"   convex-hull scenes: 128-thread blocks per SM that the GJK kernel (a
+ *                   block takes pairs as it goes) is launched with: 3 or 4 (default)
  *   "lbvh_rebuild"  convex-hull scenes: steps between full LBVH builds (1..4096, default 16);
  *                   the steps between refit the last build's tree (exact bounds, so the
  *                   same candidate pairs) */

@@ -926,17 +926,15 @@ __device__ __forceinline__ void gjk_pair(const HullBuffers& H, uint32_t u, float
 // Part 2, kGjkLanes lanes per pair left: GJK (seeded or plain).  A separated or
 // touching pair is finished here; a pair found intersecting goes to the hit
 // list for hull_epa_kernel.  Split so that GJK does not carry EPA's registers
-// and polytope.  MINB: resident blocks per SM it is compiled for (knob
-// "hull_blocks").
+// and polytope.  "hull_blocks" of its blocks per SM (109 registers, so four fit).
 // 43,500 pairs of 32,768 packed hulls, 9,600 of them intersecting: the two
 // parts 13 + 30 us a step; one thread per pair, 32 pairs of all kinds to a
 // warp, took 62 (its simplex walked through local memory, its loads served a
 // point at a time), and 219 on a training step, where a few lanes of a warp had
 // the margin to find (now 13 + 124).  Latency still bounds both: part 2's chain
-// is up to 13 supports, a training step's up to 64.  Lanes per pair, ten
-// steps: 4 in both parts 2540 us, 8 in both 2472, 4 and 8 2363.
-template <int MINB>
-__global__ void __launch_bounds__(kHullThreads, MINB) hull_gjk_kernel(HullBuffers H) {
+// is up to 13 supports, a training step's up to 64.  Lanes per pair: part 1 takes
+// 13 us with four, 16 with eight; part 2 34 and 30.
+__global__ void __launch_bounds__(kHullThreads, 4) hull_gjk_kernel(HullBuffers H) {
     // the simplex and the supports seen, per group in shared memory
     __shared__ float4 s_simplex[kHullThreads / kGjkLanes][4];
     __shared__ uint16_t s_seen[kHullThreads / kGjkLanes][kGjkMaxIt];
@@ -1179,10 +1177,7 @@ cudaError_t hull_teach_compact_async(const HullBuffers& H, const uint32_t* d_cou
 cudaError_t hull_narrow_async(const HullParams& p, HullBuffers& H, cudaStream_t st) {
     if (H.nb == 0 || H.cap == 0) return cudaSuccess;
     hull_gjk_first_kernel<<<152 * 8, kHullThreads, 0, st>>>(H);
-    if (g_hull_blocks == 3)
-        hull_gjk_kernel<3><<<152 * 3, kHullThreads, 0, st>>>(H);
-    else
-        hull_gjk_kernel<4><<<152 * 4, kHullThreads, 0, st>>>(H);
+    hull_gjk_kernel<<<152 * g_hull_blocks, kHullThreads, 0, st>>>(H);
     hull_epa_kernel<<<152 * kEpaBlocks, kEpaWarps * 32, 0, st>>>(p, H);
     return cudaGetLastError();
 }
