@@ -363,9 +363,9 @@ def bench_hulls(n_hulls: int, steps: int, warmup: int, local: int):
 # Compulsory HBM bytes of one unique hull pair in the narrow phase besides its
 # vertices: the unique-list entry, its self and partner ids (12); per body
 # position and quaternion (2 x 32) and its vertex range (2 x 8); the seed
-# (16); written for the entry and its mirror: direction, force, torque, info
-# (2 x 52).
-NARROW_BYTES_PER_PAIR = 12 + 64 + 16 + 16 + 104
+# (16); written for the entry and its mirror: direction, info (2 x 20; a hit's
+# force and torque are not counted).
+NARROW_BYTES_PER_PAIR = 12 + 64 + 16 + 16 + 40
 
 
 def narrow_roofline(eng, local: int, reps: int = 10):

@@ -33,8 +33,8 @@
 // columns of the GEMMs saves 12% more.)
 //
 // Measured (GB300): 100,003 rows, an Adam step 110 + 10 + 3.5 us (gradient,
-// reduction, packing) -> 31 + 5 us with the same bits, the forward pass 24 ->
-// 13.  The gradient was bound by 2-byte shared-memory stores and by building
+// reduction, packing) -> 30 + 5 us with the same bits, the forward pass 24 ->
+// 12.  The gradient was bound by 2-byte shared-memory stores and by building
 // transposed copies (18 us per tile, one tile at a time); now by a tile's chain
 // of five dependent GEMM steps and their epilogues, of which two teams keep two
 // in flight, the inputs of the next tile loading behind them.
@@ -43,6 +43,8 @@
 #include "sd_common.cuh"
 
 #include <cuda_bf16.h>
+
+#include <cstddef>
 
 namespace sd {
 
@@ -281,10 +283,19 @@ __device__ __forceinline__ uint8_t* aligned_smem(uint8_t* raw) {
     return raw + pad;
 }
 
-__device__ __forceinline__ void copy_img(uint8_t* dst, const uint8_t* src, uint32_t bytes) {
-    const uint4* s = reinterpret_cast<const uint4*>(src);
-    uint4* d = reinterpret_cast<uint4*>(dst);
-    for (uint32_t i = threadIdx.x; i < bytes / 16; i += blockDim.x) d[i] = s[i];
+// The first BYTES of the operand images, which shared memory holds in the same
+// order: all of a thread's loads in flight together (a loop per image took 3 us
+// of a training kernel).
+template <uint32_t BYTES, uint32_t THREADS>
+__device__ __forceinline__ void copy_images(uint8_t* dst, const uint8_t* src) {
+    constexpr uint32_t kPieces = BYTES / 16, kEach = (kPieces + THREADS - 1) / THREADS;
+    uint4 v[kEach];
+#pragma unroll
+    for (uint32_t k = 0; k < kEach; ++k)
+        if (k * THREADS + threadIdx.x < kPieces) v[k] = reinterpret_cast<const uint4*>(src)[k * THREADS + threadIdx.x];
+#pragma unroll
+    for (uint32_t k = 0; k < kEach; ++k)
+        if (k * THREADS + threadIdx.x < kPieces) reinterpret_cast<uint4*>(dst)[k * THREADS + threadIdx.x] = v[k];
 }
 
 // 8-row groups of the operands a CTA builds: 2 or 8 core matrices.
@@ -342,6 +353,7 @@ __device__ __forceinline__ void mask_row64(uint32_t taddr, const uint8_t* h, uin
 }
 
 struct InferSmem {
+    // the images W1, W2, W3, as packed
     alignas(1024) uint8_t w1[kHid * kIn * 2];
     alignas(1024) uint8_t w2[kHid * kHid * 2];
     alignas(1024) uint8_t w3[kOut * kHid * 2];
@@ -371,15 +383,15 @@ __global__ void __launch_bounds__(kRows) mlp_forward_kernel(const uint8_t* __res
     const uint64_t rows = MODE == 0 ? min((uint64_t)*d_count, n) : n;
     const uint64_t tiles = (rows + kRows - 1) / kRows;
     if ((uint64_t)blockIdx.x >= tiles) return;
-    copy_img(S.w1, img + kImgW1, sizeof S.w1);
-    copy_img(S.w2, img + kImgW2, sizeof S.w2);
-    copy_img(S.w3, img + kImgW3, sizeof S.w3);
+    float x[kIn];
+    load_row16(feat, (uint64_t)blockIdx.x * kRows + tid, (uint64_t)blockIdx.x * kRows + tid < rows, x);
+    if (warp == 0) tmem_alloc(&S.tmem, 256);
+    copy_images<kImgW2T, kRows>(S.w1, img);
     for (uint32_t i = tid; i < kHid; i += kRows) {
         S.b[i] = params[kB1 + i];
         S.b[kHid + i] = params[kB2 + i];
     }
     if (tid < kOut) S.b[2 * kHid + tid] = params[kB3 + tid];
-    if (warp == 0) tmem_alloc(&S.tmem, 256);
     if (tid == 0) mbar_init(&S.bar, 1);
     tc_fence_before();
     __syncthreads();
@@ -388,8 +400,6 @@ __global__ void __launch_bounds__(kRows) mlp_forward_kernel(const uint8_t* __res
     const uint32_t lane_base = (warp * 32u) << 16;
     uint32_t phase = 0;
     bool ok = true;
-    float x[kIn];
-    load_row16(feat, (uint64_t)blockIdx.x * kRows + tid, (uint64_t)blockIdx.x * kRows + tid < rows, x);
     for (uint64_t t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
         const uint64_t e = t * kRows + tid, e2 = e + (uint64_t)gridDim.x * kRows;
         const bool live = e < rows;
@@ -441,6 +451,13 @@ struct TrainSmem {
     uint64_t step[2], grad[2], sums[2];
     uint32_t tmem;
 };
+static_assert(offsetof(InferSmem, w2) - offsetof(InferSmem, w1) == kImgW2 &&
+                  offsetof(InferSmem, w3) - offsetof(InferSmem, w1) == kImgW3 &&
+                  offsetof(TrainSmem, w2) - offsetof(TrainSmem, w1) == kImgW2 &&
+                  offsetof(TrainSmem, w3) - offsetof(TrainSmem, w1) == kImgW3 &&
+                  offsetof(TrainSmem, w2t) - offsetof(TrainSmem, w1) == kImgW2T &&
+                  offsetof(TrainSmem, w3t) - offsetof(TrainSmem, w1) == kImgW3T && kImgW1 == 0,
+              "shared memory holds the operand images as packed");
 
 // Forward + backward of the cosine loss 1 - y.t/|y| (mean over valid rows)
 // for the tiles of this CTA; per-CTA gradient partials to part[cta][6288]
@@ -467,11 +484,13 @@ __global__ void __launch_bounds__(2 * kRows, 1) mlp_train_kernel(const uint8_t* 
     if (d_count) n = min(n, *d_count);  // rows: the step's entry count, read on the device
     const uint32_t tiles = (n + kRows - 1) / kRows;
     if (blockIdx.x >= tiles) return;
-    copy_img(S.w1, img + kImgW1, sizeof S.w1);
-    copy_img(S.w2, img + kImgW2, sizeof S.w2);
-    copy_img(S.w3, img + kImgW3, sizeof S.w3);
-    copy_img(S.w2t, img + kImgW2T, sizeof S.w2t);
-    copy_img(S.w3t, img + kImgW3T, sizeof S.w3t);
+    const uint32_t turn = 2 * gridDim.x;  // tiles from one of this team's to the next
+    uint32_t t = blockIdx.x + me * gridDim.x, e = t * kRows + tid;
+    float x[kIn];
+    load_row16(feat, e, t < tiles && e < n, x, vec);
+    float4 g = t < tiles && e < n ? tgt[e] : make_float4(0.f, 0.f, 0.f, 0.f);
+    if (warp == 0) tmem_alloc(&S.tmem, 512);
+    copy_images<kImgBytes, 2 * kRows>(S.w1, img);
     if (me == 0 && tid < kHid) {
         S.b[tid] = params[kB1 + tid];
         S.b[kHid + tid] = params[kB2 + tid];
@@ -479,7 +498,6 @@ __global__ void __launch_bounds__(2 * kRows, 1) mlp_train_kernel(const uint8_t* 
         if (tid < kOut) S.b[2 * kHid + tid] = params[kB3 + tid];
         if (tid < 4) S.gb[2 * kHid + tid] = 0.0f;
     }
-    if (warp == 0) tmem_alloc(&S.tmem, 512);
     if (threadIdx.x == 0)
         for (int k = 0; k < 2; ++k) {
             mbar_init(&S.step[k], 1);
@@ -496,11 +514,6 @@ __global__ void __launch_bounds__(2 * kRows, 1) mlp_train_kernel(const uint8_t* 
     const uint32_t cA = me * 128, cB = cA + 64, cG3 = 256, cG2 = 272, cG1 = 336;
     uint32_t phase = 0, own = 0, other = 0;  // parities: GEMM steps, this team's gradients, the other's
     bool ok = true;
-    const uint32_t turn = 2 * gridDim.x;  // tiles from one of this team's to the next
-    uint32_t t = blockIdx.x + me * gridDim.x, e = t * kRows + tid;
-    float x[kIn];
-    load_row16(feat, e, t < tiles && e < n, x, vec);
-    float4 g = t < tiles && e < n ? tgt[e] : make_float4(0.f, 0.f, 0.f, 0.f);
     for (bool first = true; t < tiles; t += turn, first = false) {
         // this team's last weight gradients have read the operands
         if (!first && !(ok = gemm_wait(team, &S.grad[me], own, status))) break;
