@@ -85,8 +85,8 @@ struct Lbvh {
     uint32_t* top;                       // the nodes of more than 128 leaves (their number in bounds[6])
     float4 *node_lo, *node_hi;           // boxes of the subtrees below top nodes; top nodes: atomic bounds
     float4 *leaf_lo, *leaf_hi;
-    uint32_t* counts;                    // per box id
-    uint32_t* first;                     // per leaf: its first kLbvhFirst partners found (counting pass)
+    uint32_t* counts;                    // per box id; the refit leaves it zero
+    uint32_t* first;                     // per box id: its first kLbvhFirst partners found (counting pass)
     float4* rec;                         // per internal node: both children's boxes (lo.w = child ref)
     uint32_t* scan_scratch;
     uint32_t* status;                    // device error bits

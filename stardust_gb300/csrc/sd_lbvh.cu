@@ -381,7 +381,8 @@ __global__ void __launch_bounds__(kRefitWindow)
 refit_kernel(int n, const uint32_t* __restrict__ vals, const float4* __restrict__ lo, const float4* __restrict__ hi,
              float4* __restrict__ leaf_lo, float4* __restrict__ leaf_hi, float4* __restrict__ node_lo,
              float4* __restrict__ node_hi, const int2* __restrict__ children, const int32_t* __restrict__ parent,
-             const int32_t* __restrict__ other, float4* __restrict__ rec, uint32_t* __restrict__ status) {
+             const int32_t* __restrict__ other, float4* __restrict__ rec, uint32_t* __restrict__ counts,
+             uint32_t* __restrict__ status) {
     stream_wait();
     __shared__ float s_box[2][6][kRefitWindow];  // leaves, nodes
     __shared__ int2 s_children[kRefitWindow];
@@ -401,6 +402,7 @@ refit_kernel(int n, const uint32_t* __restrict__ vals, const float4* __restrict_
         }
         const float4 a = lo[id], b = hi[id];
         if (t < kRefitSpan) {
+            counts[k] = 0u;  // (for the search that follows)
             leaf_lo[k] = a;
             leaf_hi[k] = b;
         }
@@ -511,7 +513,7 @@ __global__ void top_kernel(int n, const uint32_t* __restrict__ top, const uint32
 
 // What a traversal does with the pairs it finds.
 enum QueryMode {
-    kCount,    // count[id], and the first kLbvhFirst partners into first[k * kLbvhFirst ...]
+    kCount,    // each pair once: counts of both boxes (zero before), and their first kLbvhFirst partners
     kWrite,    // partners of body id at [off[id], off[id + 1]), ascending, and self[] of each entry
     kPairs,    // each pair once, into the sink
     kRefill    // each pair once, for the sink's boxes that have more than it kept
@@ -520,13 +522,23 @@ enum QueryMode {
 constexpr int kQueryThreads = 128;
 
 struct QueryOut {
-    uint32_t* count;
+    uint32_t* count;  // per box id, as first: kLbvhFirst words a box
     const uint32_t* off;
     uint32_t* partners;
     uint32_t* self;
     uint64_t cap;
     uint32_t* first;
 };
+
+// A pair for the lists of both its boxes.
+struct BothWays {
+    uint32_t *count, *first;
+};
+__device__ __forceinline__ void hand_over(const BothWays& s, uint32_t a, uint32_t b) {
+    const uint32_t i = atomicAdd(s.count + a, 1u), j = atomicAdd(s.count + b, 1u);
+    if (i < (uint32_t)kLbvhFirst) s.first[(size_t)a * kLbvhFirst + i] = b;
+    if (j < (uint32_t)kLbvhFirst) s.first[(size_t)b * kLbvhFirst + j] = a;
+}
 
 // G lanes walk the tree for one leaf: each takes a node off the leaf's stack,
 // reads its record and tests both children's boxes; the lanes' finds are
@@ -544,15 +556,16 @@ query_kernel(int n, const uint32_t* __restrict__ vals, const float4* __restrict_
              const float4* __restrict__ leaf_hi, const float4* __restrict__ rec, QueryOut q, PairSink sink,
              uint32_t* __restrict__ status) {
     stream_wait();
-    constexpr bool kUnique = MODE == kPairs || MODE == kRefill;
+    constexpr bool kUnique = MODE != kWrite;  // each pair once, from the leaf that comes first
+    constexpr bool kBuffer = MODE == kPairs || MODE == kCount;
     constexpr int kLeaves = kQueryThreads / G, kDepth = kStack + 2 * G;
     __shared__ int s_stack[kDepth][kLeaves];
-    __shared__ PairBuffer<MODE == kPairs ? 128 : 1> s_found[kQueryThreads / 32];
+    __shared__ PairBuffer<kBuffer ? 128 : 1> s_found[kQueryThreads / 32];
     const uint32_t lane = threadIdx.x & 31u, sub = threadIdx.x % G, group = lane & ~(uint32_t)(G - 1);
     const uint32_t below = (1u << sub) - 1u;
     const int at = threadIdx.x / G, k = (int)blockIdx.x * kLeaves + at;
     if (MODE == kRefill && !sink_refill(sink)) return;
-    PairBuffer<MODE == kPairs ? 128 : 1>& found = s_found[threadIdx.x >> 5];
+    PairBuffer<kBuffer ? 128 : 1>& found = s_found[threadIdx.x >> 5];
     if (lane == 0) found.n = 0u;
     if (MODE == kPairs && sub == 0 && k < n) sink.cursor[k] = 0u;
     bool walk = k < n;
@@ -567,7 +580,7 @@ query_kernel(int n, const uint32_t* __restrict__ vals, const float4* __restrict_
             // the partners the counting pass kept, each lane placing its share
             // by counting the smaller ones (ids are distinct)
             const uint32_t m = lim - base;
-            const uint32_t* list = q.first + (size_t)k * kLbvhFirst;
+            const uint32_t* list = q.first + (size_t)id * kLbvhFirst;
             for (uint32_t i = sub; i < m; i += G) {
                 const uint32_t v = list[i];
                 uint32_t r = 0;
@@ -620,17 +633,14 @@ query_kernel(int n, const uint32_t* __restrict__ vals, const float4* __restrict_
             if constexpr (kUnique) {
                 if (leaf) {
                     if (MODE == kPairs) buffer_pair(found, sink, id, vals[j]);
+                    else if (MODE == kCount) buffer_pair(found, BothWays{q.count, q.first}, id, vals[j]);
                     else sink_pair_again(sink, id, vals[j]);
                 }
             } else {
                 const uint32_t ml = (__ballot_sync(0xffffffffu, leaf) >> group) & ((1u << G) - 1u);
                 if (leaf) {
                     const uint32_t to = c + (uint32_t)__popc(ml & below);
-                    if (MODE == kCount) {
-                        if (to < (uint32_t)kLbvhFirst) q.first[(size_t)k * kLbvhFirst + to] = vals[j];
-                    } else if (base + to < lim) {
-                        q.partners[base + to] = vals[j];
-                    }
+                    if (base + to < lim) q.partners[base + to] = vals[j];
                 }
                 c += (uint32_t)__popc(ml);
             }
@@ -638,9 +648,7 @@ query_kernel(int n, const uint32_t* __restrict__ vals, const float4* __restrict_
         __syncwarp();
     }
     if constexpr (MODE == kPairs) flush_pairs(found, sink, lane, 32u);  // (the warp met at the end of its last trip)
-    if constexpr (MODE == kCount) {
-        if (walk && sub == 0) q.count[id] = c;
-    }
+    if constexpr (MODE == kCount) flush_pairs(found, BothWays{q.count, q.first}, lane, 32u);
     if constexpr (MODE == kWrite) {
         __syncwarp();  // (the group's lanes wrote the list)
         if (!walk || sub != 0) return;
@@ -773,7 +781,8 @@ cudaError_t lbvh_refit_async(Lbvh& t, const float4* lo, const float4* hi, cudaSt
     const uint32_t n = t.n;
     if (n == 0) return cudaSuccess;
     launch_after(st, grid_for(n, kRefitSpan), kRefitWindow, 0, refit_kernel, (int)n, t.svals, lo, hi, t.leaf_lo,
-                 t.leaf_hi, t.node_lo, t.node_hi, t.children, t.parent, t.other, t.rec, t.status);
+                 t.leaf_hi, t.node_lo, t.node_hi, t.children, t.parent, t.other, t.rec, t.counts,
+                 t.status);
     if (n > (uint32_t)kTreelet)
         launch_after(st, std::min(152u, grid_for(n, kTreelet)), 128, 0, top_kernel, (int)n, t.top,
                      top_count(t.bounds), t.leaf_lo, t.leaf_hi, t.node_lo, t.node_hi, t.children, t.other, t.rec,
@@ -823,7 +832,6 @@ cudaError_t lbvh_unique_pairs_async(Lbvh& t, uint32_t* off, unsigned long long* 
     // t.keys: the codes are used up, the cursors take their place (cleared by the
     // first search, for the second)
     const PairSink sink{t.counts, t.first, t.status + 1, off, t.keys, out, n, cap};
-    if ((e = zero_async(st, {t.counts, n})) != cudaSuccess) return e;
     launch_query<kPairs>(t, QueryOut{}, sink, st);
     if ((e = scan_exclusive_async(t.counts, off, n, t.scan_scratch, st)) != cudaSuccess) return e;
     launch_query<kRefill>(t, QueryOut{}, sink, st);

@@ -49,18 +49,20 @@ struct PairBuffer {
     uint2 pair[CAP];
     uint32_t n;  // (zero before)
 };
-template <int CAP>
-__device__ __forceinline__ void buffer_pair(PairBuffer<CAP>& b, const PairSink& s, uint32_t i, uint32_t j) {
+__device__ __forceinline__ void hand_over(const PairSink& s, uint32_t i, uint32_t j) { sink_pair(s, i, j); }
+
+template <int CAP, class SINK>
+__device__ __forceinline__ void buffer_pair(PairBuffer<CAP>& b, const SINK& s, uint32_t i, uint32_t j) {
     const uint32_t at = atomicAdd(&b.n, 1u);
     if (at < (uint32_t)CAP) b.pair[at] = make_uint2(i, j);
-    else sink_pair(s, i, j);
+    else hand_over(s, i, j);
 }
 // By `threads` threads that have met since the last buffer_pair(), this one the
 // t-th.
-template <int CAP>
-__device__ __forceinline__ void flush_pairs(const PairBuffer<CAP>& b, const PairSink& s, uint32_t t, uint32_t threads) {
+template <int CAP, class SINK>
+__device__ __forceinline__ void flush_pairs(const PairBuffer<CAP>& b, const SINK& s, uint32_t t, uint32_t threads) {
     const uint32_t n = min(b.n, (uint32_t)CAP);
-    for (uint32_t k = t; k < n; k += threads) sink_pair(s, b.pair[k].x, b.pair[k].y);
+    for (uint32_t k = t; k < n; k += threads) hand_over(s, b.pair[k].x, b.pair[k].y);
 }
 
 // Whether the second search has anything to do.
