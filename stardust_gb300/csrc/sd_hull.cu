@@ -26,8 +26,10 @@ namespace {
 constexpr int kHullThreads = 128;
 constexpr int kSeedThreads = 256;
 constexpr int kFirstLanes = 4, kGjkLanes = 8;  // lanes of a pair in parts 1 and 2 of the narrow phase
-// EPA's blocks per SM, all resident at once: 4 (118 registers) ten steps of
-// 32,768 hulls 2314 us, 5 (96) 2325, 6 (80, spilling) 2357, 8 (64) 2381.
+// EPA's blocks per SM (the margin's come first), all resident at once: 4 (118
+// registers) ten steps of 32,768 hulls 2314 us, 5 (96) 2325, 6 (80, spilling)
+// 2357, 8 (64) 2381.
+constexpr uint32_t kMarginBlocks = 152;
 constexpr int kEpaBlocks = 4;
 constexpr int kEpaWarps = 4;  // warps per block of the EPA kernel
 constexpr int kGjkMaxIt = 64;
@@ -826,14 +828,14 @@ __device__ __forceinline__ GjkSeed gjk_seed(const HullBuffers& H, uint32_t e) {
 
 // A pair that ends without a hit: status, direction and no force (only entries
 // with a hit are summed) for its entry e and the mirror in B's list; dA is the
-// final direction in A's frame (seed of the next step), t the training target.
-__device__ __forceinline__ void end_pair(const HullBuffers& H, uint32_t e, uint32_t em, v3 dA, bool sep, float4 t) {
+// final direction in A's frame (seed of the next step).  No training sample yet.
+__device__ __forceinline__ void end_pair(const HullBuffers& H, uint32_t e, uint32_t em, v3 dA, bool sep) {
     const float4 d4 = make_float4(dA.x, dA.y, dA.z, sep ? 1.0f : 0.0f);
     H.dir[e] = d4;
     if (em != e) H.dir[em] = d4;
     if (H.teach && *H.teach_on) {
-        H.teach[e] = t;
-        if (em != e) H.teach[em] = make_float4(0.f, 0.f, 0.f, 0.f);  // one sample per pair
+        H.teach[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (em != e) H.teach[em] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
 }
 
@@ -875,7 +877,7 @@ __global__ void __launch_bounds__(kHullThreads) hull_gjk_first_kernel(HullBuffer
             if (!open) {
                 const uint32_t em = mirror_entry(H, e, A, B, g);
                 if (g.sub == 0) {
-                    end_pair(H, e, em, sd.learned ? sd.anchor : rotT(P.A.R, d), true, make_float4(0.f, 0.f, 0.f, 0.f));
+                    end_pair(H, e, em, sd.learned ? sd.anchor : rotT(P.A.R, d), true);
                     H.info[e] = H.info[em] = (uint32_t)kSep | (1u << 8);
                 }
             }
@@ -904,15 +906,13 @@ __device__ __forceinline__ void gjk_pair(const HullBuffers& H, uint32_t u, float
     int which = 0, iters = 0;
     v3 dir;
     const int st = gjk_attempts(P, at, &S, &iters, &dir, &which, seen, g, sd.learned ? 1 : 0, sd.learned ? 1 : 0);
-    // a training step: the max-margin direction of a separated pair whose
-    // anchor failed (the cases the network's seed is tried on)
-    v3 m = mk(0.f, 0.f, 0.f);
-    const bool ok = H.teach && *H.teach_on && st == kSep && sd.learned && gjk_margin_dir(P, dir, &m, &S, g);
     const uint32_t em = mirror_entry(H, e, A, B, g);
     if (g.sub != 0) return;
-    const v3 mA = rotT(P.A.R, m);
-    end_pair(H, e, em, rotT(P.A.R, dir), st == kSep,
-             ok ? make_float4(mA.x, mA.y, mA.z, 1.0f) : make_float4(0.f, 0.f, 0.f, 0.f));
+    end_pair(H, e, em, rotT(P.A.R, dir), st == kSep);
+    // a training step: a separated pair whose anchor failed (the cases the
+    // network's seed is tried on) gets its max-margin direction beside EPA
+    if (H.teach && *H.teach_on && st == kSep && sd.learned)
+        H.margin[atomicAdd(H.counters + kMarginPairs, 1u)] = make_float4(dir.x, dir.y, dir.z, __uint_as_float(e));
     if (st == kHit) {  // EPA and the contact force in hull_epa_kernel
         const uint32_t k = atomicAdd(H.counters + kHitPairs, 1u);  // k < unique pairs <= cap / 2 + 1
         H.hits[k] = make_uint2(u, (uint32_t)iters);
@@ -931,8 +931,8 @@ __device__ __forceinline__ void gjk_pair(const HullBuffers& H, uint32_t u, float
 // parts 13 + 30 us a step; one thread per pair, 32 pairs of all kinds to a
 // warp, took 62 (its simplex walked through local memory, its loads served a
 // point at a time), and 219 on a training step, where a few lanes of a warp had
-// the margin to find (now 13 + 124).  Latency still bounds both: part 2's chain
-// is up to 13 supports, a training step's up to 64.  Lanes per pair: part 1 takes
+// the margin to find.  Latency still bounds both: part 2's chain is up to 13
+// supports.  Lanes per pair: part 1 takes
 // 13 us with four, 16 with eight; part 2 34 and 30.
 __global__ void __launch_bounds__(kHullThreads, 4) hull_gjk_kernel(HullBuffers H) {
     // the simplex and the supports seen, per group in shared memory
@@ -960,13 +960,38 @@ __global__ void __launch_bounds__(kHullThreads, 4) hull_gjk_kernel(HullBuffers H
 // force at the EPA point; A's entry and B's mirror get forces of opposite
 // sign -- exact action = reaction, no atomics.  Warps stride over the hit
 // count.
+//
+// The first kMarginBlocks blocks take a training step's separated pairs (none on
+// other steps), kGjkLanes lanes each: the max-margin direction in A's frame, a
+// chain of up to 64 supports.  As the end of GJK it took 94 us more (ten steps,
+// two of them training, 2133 us); beside EPA 2072 (76 blocks 2077, 38 2251).
 __global__ void __launch_bounds__(kEpaWarps * 32, kEpaBlocks) hull_epa_kernel(HullParams p, HullBuffers H) {
-    __shared__ EpaShared polytope[kEpaWarps];
+    __shared__ __align__(16) EpaShared polytope[kEpaWarps];
+    if (blockIdx.x < kMarginBlocks) {
+        constexpr uint32_t kGroups = kEpaWarps * 32 / kGjkLanes;
+        static_assert(sizeof polytope >= kGroups * 4 * sizeof(float4), "the groups' simplexes fit");
+        const Group<kGjkLanes> g = lane_group<kGjkLanes>();
+        const uint32_t at = threadIdx.x / kGjkLanes, n = H.counters[kMarginPairs];
+        float4* const slots = reinterpret_cast<float4*>(polytope) + 4 * at;
+        for (uint32_t k = blockIdx.x * kGroups + at; k < n; k += kMarginBlocks * kGroups) {
+            const float4 d = H.margin[k];
+            const uint32_t e = __float_as_uint(d.w);
+            HPair P;
+            make_pair(H, H.self[e], H.partners[e], &P);
+            Simplex S{slots, 0u, 0};
+            v3 m;
+            if (gjk_margin_dir(P, f3(d), &m, &S, g) && g.sub == 0) {
+                const v3 mA = rotT(P.A.R, m);
+                H.teach[e] = make_float4(mA.x, mA.y, mA.z, 1.0f);
+            }
+        }
+        return;
+    }
     EpaShared& sh = polytope[threadIdx.x >> 5];
     const uint32_t n_hits = H.counters[kHitPairs];
     const uint32_t lane = threadIdx.x & 31;
-    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < n_hits; k += nwarps) {
+    const uint32_t nwarps = ((gridDim.x - kMarginBlocks) * blockDim.x) >> 5;
+    for (uint32_t k = ((blockIdx.x - kMarginBlocks) * blockDim.x + threadIdx.x) >> 5; k < n_hits; k += nwarps) {
         const uint2 hit = H.hits[k];
         const uint32_t key = reinterpret_cast<const uint32_t*>(H.hit_keys + k)[lane & 3u];
         const uint32_t e = H.ulist[hit.x];
@@ -1178,7 +1203,7 @@ cudaError_t hull_narrow_async(const HullParams& p, HullBuffers& H, cudaStream_t 
     if (H.nb == 0 || H.cap == 0) return cudaSuccess;
     hull_gjk_first_kernel<<<152 * 8, kHullThreads, 0, st>>>(H);
     hull_gjk_kernel<<<152 * g_hull_blocks, kHullThreads, 0, st>>>(H);
-    hull_epa_kernel<<<152 * kEpaBlocks, kEpaWarps * 32, 0, st>>>(p, H);
+    hull_epa_kernel<<<kMarginBlocks + 152 * kEpaBlocks, kEpaWarps * 32, 0, st>>>(p, H);
     return cudaGetLastError();
 }
 

@@ -225,6 +225,7 @@ sd_status hull_prepare(sd_engine* h) {
         (s = halloc(h, &H.hit_keys, cap / 2 + 1)))
         return s;
     H.teach_on = S.teach_flag;
+    H.margin = S.teach_tgt;  // (filled with the targets after the step)
     H.stats = S.stats;
     for (int k = 0; k < 2; ++k)
         if ((s = halloc(h, &S.off[k], (size_t)nb + 1)) || (s = halloc(h, &S.partners[k], cap)) ||
@@ -347,8 +348,8 @@ sd_status hull_launch_narrow(sd_engine* h) {
     H.prev_dir = S.dir[par ^ 1];
     H.keep_anchor = S.seed_mode == SD_GJK_SEED_LEARNED;
     // the unique pairs are the last step's; the other counters start over
-    static_assert(sd::kUniquePairs == 0 && sd::kHullCounters == 4, "three cleared together");
-    HULL_CUDA(h, cudaMemsetAsync(H.counters + 1, 0, 3 * sizeof(uint32_t), h->stream));
+    static_assert(sd::kUniquePairs == 0, "those behind it are cleared together");
+    HULL_CUDA(h, cudaMemsetAsync(H.counters + 1, 0, (sd::kHullCounters - 1) * sizeof(uint32_t), h->stream));
     HULL_CUDA(h, sd::hull_narrow_async(S.P, H, h->stream));
     return SD_OK;
 }

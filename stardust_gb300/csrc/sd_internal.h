@@ -152,6 +152,7 @@ struct HullBuffers {
     // a separated pair in A's frame (w = 1), else w = 0
     float4* teach;
     const uint32_t* teach_on;
+    float4* margin;                        // a training step's pairs for it: direction, entry (cap / 2 + 1)
     // learned seeds: a pair whose seeded run certified separation keeps its
     // previous direction (inputs 8..10, the anchor) as the next step's, so
     // the network is never fed its own outputs
@@ -169,7 +170,7 @@ struct HullBuffers {
     uint32_t* counters;                    // kHullCounters, cleared by the step's first kernel
     unsigned long long* stats;             // the step's statistics, likewise
 };
-constexpr int kUniquePairs = 0, kHitPairs = 1, kNextPair = 2, kOpenPairs = 3, kHullCounters = 4;
+constexpr int kUniquePairs = 0, kHitPairs = 1, kNextPair = 2, kOpenPairs = 3, kMarginPairs = 4, kHullCounters = 5;
 cudaError_t hull_aabb_async(HullBuffers& H, cudaStream_t st);
 cudaError_t hull_seed_async(HullBuffers& H, uint32_t mode, cudaStream_t st);
 cudaError_t hull_narrow_async(const HullParams& p, HullBuffers& H, cudaStream_t st);
