@@ -481,24 +481,42 @@ __device__ __forceinline__ uint32_t particle_step(const DemParams& p, uint32_t n
                     const uint32_t col = g.base + (uint32_t)((X * g.ny + Y) * g.nz);
                     const uint32_t s0 = __ldg(&cell_start[col + (uint32_t)bz0]);
                     const uint32_t s1 = min(__ldg(&cell_start[col + (uint32_t)bz1 + 1]), n);
-                    for (uint32_t s = s0; s < s1; ++s) {
-                        const float4 pa = src.load(s);
-                        const float ax = pi.x - pa.x, ay = pi.y - pa.y, az = pi.z - pa.z;
-                        const float da = dist2(ax, ay, az);
-                        if (s == i) continue;  // the sphere itself; a coincident partner is listed
+                    const auto list_one = [&](uint32_t sc, const float4& pc, float dc) {
                         // a sphere of the same rigid body is never a contact: not listed
-                        if (clump_i && same_body(cc, idb, omg, s)) continue;
-                        const float rl = ri + pa.w + sk->skin;
-                        if (da < rl * rl) {
-                            if (c < kVlCap)
-                                sk->nbr[(size_t)c * n + i] =
-                                    __float_as_uint(__ldg(reinterpret_cast<const float*>(omg) + 4 * (size_t)s + 3)) &
-                                    kIdMask;
-                            ++c;
-                            const float ra = ri + pa.w;
-                            if (da < ra * ra && da != 0.0f) {  // coincident centres: no normal, no contact
-                                ++contacts;
-                                pair_contact(p, ax, ay, az, da, ra, pa.w, ri, mi, vi, wi, vel, omg, s, f, t);
+                        if (clump_i && same_body(cc, idb, omg, sc)) return;
+                        if (c < kVlCap)
+                            sk->nbr[(size_t)c * n + i] =
+                                __float_as_uint(__ldg(reinterpret_cast<const float*>(omg) + 4 * (size_t)sc + 3)) &
+                                kIdMask;
+                        ++c;
+                        const float ax = pi.x - pc.x, ay = pi.y - pc.y, az = pi.z - pc.z, rc = ri + pc.w;
+                        if (dc < rc * rc && dc != 0.0f) {  // coincident centres: no normal, no contact
+                            ++contacts;
+                            pair_contact(p, ax, ay, az, dc, rc, pc.w, ri, mi, vi, wi, vel, omg, sc, f, t);
+                        }
+                    };
+                    // (not the sphere itself; a coincident partner is listed)
+                    if constexpr (BATCHED) {  // one at a time: the scenes' state makes two spill (20 steps 2246 us, 2185)
+                        for (uint32_t s = s0; s < s1; ++s) {
+                            const float4 pa = src.load(s);
+                            const float da = dist2(pi.x - pa.x, pi.y - pa.y, pi.z - pa.z);
+                            if (s == i) continue;
+                            const float rl = ri + pa.w + sk->skin;
+                            if (da < rl * rl) list_one(s, pa, da);
+                        }
+                    } else {  // two, so that their loads overlap (a bed of 199,999 spheres, 50 steps 2015 -> 1866 us)
+                        for (uint32_t s = s0; s < s1; s += 2) {
+                            const uint32_t s2 = s + 1 < s1 ? s + 1 : s;
+                            const float4 pa = src.load(s), pb = src.load(s2);
+                            const float da = dist2(pi.x - pa.x, pi.y - pa.y, pi.z - pa.z);
+                            const float db = dist2(pi.x - pb.x, pi.y - pb.y, pi.z - pb.z);
+                            const float rla = ri + pa.w + sk->skin, rlb = ri + pb.w + sk->skin;
+                            uint32_t near = (da < rla * rla && s != i ? 1u : 0u) |
+                                            (db < rlb * rlb && s2 != i && s2 != s ? 2u : 0u);
+                            while (near) {
+                                const bool second = !(near & 1u);
+                                near &= near - 1u;
+                                list_one(second ? s2 : s, second ? pb : pa, second ? db : da);
                             }
                         }
                     }
