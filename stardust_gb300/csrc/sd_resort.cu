@@ -402,7 +402,7 @@ __device__ __forceinline__ bool radix_sort_grid(const StepArgs& a, uint32_t* sme
 // to the others would need a barrier more), gathers its share of the
 // positions, and after one grid barrier places them and shifts the cell
 // table.  A step without moved slots ends at once.
-// Measured (per step, the separate kernels before): 4,096 spheres 17.4 -> 8.8
+// Measured (per step, the separate kernels before): 4,096 spheres 17.4 -> 7.5
 // us the step; 1,048,576 falling spheres 26 -> 10 us after the contact stage
 // (50-90 moved slots, up to 85,000 positions); 256 scenes of 1.57M spheres 44
 // -> 16 us (340 moved slots); the drum 28 -> 11 us.  Bound by latency: load
