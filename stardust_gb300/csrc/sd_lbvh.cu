@@ -32,13 +32,22 @@ namespace {
 constexpr int kLbvhThreads = 256;
 constexpr uint32_t kLeaf = 0x80000000u;
 constexpr int kTreelet = 128;  // leaves of a subtree that a block's shared memory joins
-constexpr int kStack = 64;  // Karras tree depth <= 32 code bits + 32 index bits
+constexpr int kStack = 64;  // one lane's stack: at most an entry a level (tree_levels) and one more
 static_assert(kLbvhFirst >= (int)kPairKeep, "the sink keeps its partners in Lbvh::first");
 
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 8;
 constexpr uint32_t kScanTile = kScanThreads * kScanItems;
 constexpr uint32_t kScanDirect = 2048;  // tiles
+
+// Internal nodes on the longest path of a tree of n leaves, at most: the common
+// prefix grows with every one of them, through the 30 code bits and, between
+// equal codes, the bits in which two indices below n can differ (60 at 2^30).
+inline int tree_levels(uint32_t n) {
+    int bits = 0;
+    while (bits < 32 && ((uint64_t)1 << bits) < n) ++bits;
+    return 30 + bits;
+}
 
 // The number of top nodes, behind the global box.
 __host__ __device__ inline uint32_t* top_count(float* bounds) { return reinterpret_cast<uint32_t*>(bounds + 6); }
@@ -550,15 +559,25 @@ __device__ __forceinline__ void hand_over(const BothWays& s, uint32_t a, uint32_
 // twice: 2 x 100 us).  One warp walking for 32
 // neighbouring leaves under their common box took seven times as long: where
 // the curve jumps, that box covers much of the domain.
+//
+// A walk never runs out of stack.  G nodes are taken at a time only from a
+// stack of up to `batch` entries, which then has batch + G at most; one node at
+// a time adds at most an entry for every level below the node it starts from,
+// tree_levels - 1 in all: batch + G + tree_levels - 1 <= kDepth.  (A box over
+// small boxes graded toward a corner fills whatever `batch` allows and then
+// goes down 40 levels; walks among boxes of like sizes stay below it.)
+template <int G>
+constexpr int query_depth() { return kStack + 2 * G; }
+
 template <int MODE, int G>
 __global__ void __launch_bounds__(kQueryThreads)
-query_kernel(int n, const uint32_t* __restrict__ vals, const float4* __restrict__ leaf_lo,
+query_kernel(int n, int batch, const uint32_t* __restrict__ vals, const float4* __restrict__ leaf_lo,
              const float4* __restrict__ leaf_hi, const float4* __restrict__ rec, QueryOut q, PairSink sink,
              uint32_t* __restrict__ status) {
     stream_wait();
     constexpr bool kUnique = MODE != kWrite;  // each pair once, from the leaf that comes first
     constexpr bool kBuffer = MODE == kPairs || MODE == kCount;
-    constexpr int kLeaves = kQueryThreads / G, kDepth = kStack + 2 * G;
+    constexpr int kLeaves = kQueryThreads / G, kDepth = query_depth<G>();
     __shared__ int s_stack[kDepth][kLeaves];
     __shared__ PairBuffer<kBuffer ? 128 : 1> s_found[kQueryThreads / 32];
     const uint32_t lane = threadIdx.x & 31u, sub = threadIdx.x % G, group = lane & ~(uint32_t)(G - 1);
@@ -601,9 +620,7 @@ query_kernel(int n, const uint32_t* __restrict__ vals, const float4* __restrict_
             if (lane == 0) atomicOr(status, kErrBadInput);
             break;
         }
-        // G nodes while their children fit, else one: the stack then grows by
-        // one entry a level at most
-        const int m = sp <= kStack - 2 * G ? min(sp, G) : 1;
+        const int m = sp <= batch ? min(sp, G) : 1;
         const bool mine = (int)sub < m;
         const int node = mine ? s_stack[sp - 1 - (int)sub][at] : 0;
         sp -= m;
@@ -627,7 +644,7 @@ query_kernel(int n, const uint32_t* __restrict__ vals, const float4* __restrict_
             if (inner) {
                 const int to = sp + __popc(mi & below);
                 if (to < kDepth) s_stack[to][at] = x;
-                else atomicOr(status, kErrPairOverflow);
+                else atomicOr(status, kErrBadInput);  // (no tree of n leaves: see above)
             }
             sp = min(sp + __popc(mi), kDepth);
             if constexpr (kUnique) {
@@ -804,12 +821,12 @@ constexpr uint32_t kWideLeaves = 1u << 16;
 template <int MODE>
 static void launch_query(const Lbvh& t, const QueryOut& q, const PairSink& sink, cudaStream_t st) {
     const int n = (int)t.n;
-    const auto go = [&](auto kernel, int lanes) {
-        launch_after(st, grid_for(t.n, kQueryThreads / lanes), kQueryThreads, 0, kernel, n, t.svals, t.leaf_lo,
-                     t.leaf_hi, t.rec, q, sink, t.status);
+    const auto go = [&](auto kernel, int lanes, int depth) {
+        launch_after(st, grid_for(t.n, kQueryThreads / lanes), kQueryThreads, 0, kernel, n,
+                     depth - lanes - tree_levels(t.n) + 1, t.svals, t.leaf_lo, t.leaf_hi, t.rec, q, sink, t.status);
     };
-    if (t.n < kWideLeaves) go(query_kernel<MODE, 4>, 4);
-    else go(query_kernel<MODE, 2>, 2);
+    if (t.n < kWideLeaves) go(query_kernel<MODE, 4>, 4, query_depth<4>());
+    else go(query_kernel<MODE, 2>, 2, query_depth<2>());
 }
 
 cudaError_t lbvh_partners_async(Lbvh& t, uint32_t* off, uint32_t* partners, uint32_t* self, uint64_t cap,

@@ -266,3 +266,54 @@ def test_hull_point_counts_bit_exact(sdlib, orc, counts, seed_mode):
         assert np.array_equal(bits(eng.bodies(f)), bits(getattr(H, k))), k
     assert np.array_equal(bits(eng.bodies(_abi.SD_BODY_FORCE)), bits(out["force"]))
     eng.close()
+
+
+def _graded(n, seed=1):
+    """n - 1 small boxes graded toward the unit cube's corner (as many at each
+    of ten scales), whose tree is some 40 levels deep, and one over the cube."""
+    rng = np.random.default_rng(seed)
+    c = 1 - 2.0 ** (-10 * rng.random((n, 1))) * rng.random((n, 3))
+    L = np.zeros((n, 4), np.float32)
+    H = np.zeros((n, 4), np.float32)
+    L[:, :3] = c - 1e-5
+    H[:, :3] = c + 1e-5
+    L[-1, :3] = 0.0
+    H[-1, :3] = 1.0
+    return c, L, H
+
+
+@pytest.mark.parametrize("n", [3000, 20_001, 60_001, 65_536, 200_001])
+def test_lbvh_pairs_over_graded_boxes(sdlib, orc, n):
+    """A walk whose stack fills with nodes near the root and then goes down a
+    deep tree, with four lanes to a leaf and with two (from 65,536)."""
+    import torch
+    _, L, H = _graded(n)
+    want = orc.aabb_pairs(L, H)
+    assert len(want) > 0.9 * n
+    got, cnt, err = sdlib.BoundingVolumes.pairs(torch.from_numpy(L).cuda(), torch.from_numpy(H).cuda(), len(want))
+    assert err == 0 and cnt == len(want)
+    assert np.array_equal(got.cpu().numpy().view(np.uint64), want)
+
+
+def test_hull_lists_over_graded_hulls(sdlib, orc):
+    """The same walk for a hull scene's candidate lists: small cubes graded
+    toward a corner, and a rod across the box."""
+    from stardust_gb300 import scenes
+    n = 8000
+    c, _, _ = _graded(n)
+    *_, cfg, dt = scenes.hull_box(8, box=(1.0, 1.0, 1.0))
+    eng = sdlib.DEMEngine(cfg)
+    cube = 1e-5 * np.array([[x, y, z] for x in (-1, 1) for y in (-1, 1) for z in (-1, 1)], np.float32)
+    for p in c[:-1]:
+        eng.add_hull(cube, 1e-6, tuple(p), (1.0, 0.0, 0.0, 0.0))
+    eng.add_hull(np.array([[-0.5, 0.5, -0.5], [0.5, -0.5, 0.5]], np.float32), 1.0, (0.5, 0.5, 0.5), (1.0, 0.0, 0.0, 0.0))
+    eng.prepare()
+    H = oracle_hulls(orc, eng)
+    out = H.step(oracle_params(orc, cfg, dt), record=True)
+    assert np.diff(out["off"]).max() > 0.9 * n
+    eng.step(dt, 1)
+    eng.sync()
+    assert eng.stats()["device_errors"] == 0
+    e = eng.hull_entries()
+    assert np.array_equal(e["off"], out["off"]) and np.array_equal(e["partners"], out["partners"])
+    eng.close()
