@@ -504,7 +504,8 @@ sd_status sd_engine_load_checkpoint(sd_engine* h, const char* path);
  *   "listed_blocks" resident 256-thread blocks per SM the contact-list kernel is compiled
  *                   for: 4 (64 registers) or 5 (48 registers, the default; scenes of up to
  *                   800,000 spheres then take 4); single scenes without clumps or meshes also
- *                   6 (40) or 8 (32 registers, more spills); clumps or meshes: always 4
+ *                   6 (40) or 8 (32 registers, more spills); clumps or meshes: 4, but
+ *                   5 with a mesh under SD_ENGINE_SAP where spheres alone do not take 4
  *   "contact_block" threads per block of the per-sphere contact kernels without lists: 64,
  *                   128 or 256 (default); the contact-list kernel takes 64
  *   "fix_blocks"    blocks per SM of the in-place reorder's fixed grid: 2, 4 or 8 (default);

@@ -1701,7 +1701,12 @@ constexpr unsigned kListedThreads = 64;
 // stays in L2, so fewer warps cover its latency, and the contacts no longer
 // spill.  40 steps, four / five: 600,000 falling spheres 1563 / 1595 us, 700,000
 // in a bed 4033 / 4140, 300,000 in a bed 2020 / 2283; 1,048,576 falling 2554 /
-// 2472.  Scenes with clumps or a mesh always take four (the drum 874 / 907).
+// 2472.  Scenes with clumps or a mesh take four whatever their size (2,097,152
+// spheres in a drum 262 / 291 us a step, without clumps 103 / 115; 1,500,000 with
+// clumps in a box 152 / 173), except where a sweep finds the mesh's triangles
+// (SD_ENGINE_SAP): a binary search and then hundreds of boxes for a sphere, whose
+// latency the warps of five cover (the drum 1949 / 1782 us, without clumps 1766 / 1541;
+// 1,000,000 spheres 1001 / 911, 800,001 836 / 831, 400,000 712 / 743).
 constexpr uint32_t kListedSmall = 800000;
 
 template <bool RECORD>
@@ -1718,6 +1723,7 @@ static void launch_contact_t(const DemParams& p, DemBuffers& b, uint32_t spec, u
     uint32_t* const vals = ms.list ? nullptr : b.vals;
     if (skin) {  // one scene or a batch, contact lists (clumps and meshes: one scene)
         const int blocks = g_listed_blocks == 5 && b.n <= kListedSmall ? 4 : g_listed_blocks;
+        const bool sweep5 = b.mesh.sap_n && blocks != 4;  // a mesh whose triangles a sweep finds
         const unsigned lgrid = grid_for(b.n, kListedThreads);
         const float thr = 0.45f * b.vl_skin;
         const SkinLists sk{b.vl_cnt, b.vl_nbr, b.vl_ref, b.vl_flags, b.vl_flags + 1, b.slot_of, b.vl_skin, thr * thr};
@@ -1731,6 +1737,10 @@ static void launch_contact_t(const DemParams& p, DemBuffers& b, uint32_t spec, u
                 launch_chained(st, lgrid, kListedThreads, 0, dem_contact_listed_kernel<RECORD, 4, true>, p, b.n,
                                b.pos, b.vel, b.omg, b.cell_start, b.pos_n, b.vel_n, b.omg_n, b.keys, vals, f, t,
                                b.dev_status, sk, ms, bt, ClumpCtx{}, MeshView{});
+        } else if (b.nb && b.mesh.ntri && sweep5) {
+            launch_chained(st, lgrid, kListedThreads, 0, dem_contact_listed_kernel<RECORD, 5, false, true, true>, p,
+                           b.n, b.pos, b.vel, b.omg, b.cell_start, b.pos_n, b.vel_n, b.omg_n, b.keys, vals, f, t,
+                           b.dev_status, sk, ms, Batch{}, cc, b.mesh);
         } else if (b.nb && b.mesh.ntri) {
             launch_chained(st, lgrid, kListedThreads, 0, dem_contact_listed_kernel<RECORD, 4, false, true, true>, p,
                            b.n, b.pos, b.vel, b.omg, b.cell_start, b.pos_n, b.vel_n, b.omg_n, b.keys, vals, f, t,
@@ -1739,6 +1749,10 @@ static void launch_contact_t(const DemParams& p, DemBuffers& b, uint32_t spec, u
             launch_chained(st, lgrid, kListedThreads, 0, dem_contact_listed_kernel<RECORD, 4, false, true, false>, p,
                            b.n, b.pos, b.vel, b.omg, b.cell_start, b.pos_n, b.vel_n, b.omg_n, b.keys, vals, f, t,
                            b.dev_status, sk, ms, Batch{}, cc, MeshView{});
+        } else if (b.mesh.ntri && sweep5) {
+            launch_chained(st, lgrid, kListedThreads, 0, dem_contact_listed_kernel<RECORD, 5, false, false, true>, p,
+                           b.n, b.pos, b.vel, b.omg, b.cell_start, b.pos_n, b.vel_n, b.omg_n, b.keys, vals, f, t,
+                           b.dev_status, sk, ms, Batch{}, ClumpCtx{}, b.mesh);
         } else if (b.mesh.ntri) {
             launch_chained(st, lgrid, kListedThreads, 0, dem_contact_listed_kernel<RECORD, 4, false, false, true>, p,
                            b.n, b.pos, b.vel, b.omg, b.cell_start, b.pos_n, b.vel_n, b.omg_n, b.keys, vals, f, t,

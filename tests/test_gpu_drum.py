@@ -87,3 +87,46 @@ def test_drum_keeps_spheres_inside_and_drags_the_bed(sdlib):
     Lx = (v[:, 3] * ((p[:, 1] - c[1]) * v[:, 2] - (p[:, 2] - c[2]) * v[:, 1])).sum()
     assert Lx > 0
     eng.close()
+
+
+@pytest.mark.parametrize("clumps", [0, 200])
+@pytest.mark.parametrize("n", [800_000, 800_001])
+def test_large_drum_register_budgets(sdlib, n, clumps):
+    """Either side of the size from which the list kernel of a swept mesh is
+    the one of five blocks per SM: with it, with four, and with the grid's
+    candidates, the same bits."""
+    from stardust_gb300 import _abi, scenes
+    rng = np.random.default_rng(n)
+    r, radius, length = 0.002, 0.25, 0.5
+    a = 1.995 * r
+    ys = np.arange(r, 2 * radius - r, a)
+    sites = np.stack(np.meshgrid(ys, ys, np.arange(r, length - r, a), indexing="ij"), -1).reshape(-1, 3)[:, ::-1]
+    sites = sites[((sites[:, 1:] - radius) ** 2).sum(1) < (radius - 0.99 * r) ** 2][:n - 3 * clumps]
+    assert len(sites) == n - 3 * clumps
+    tris, patch = scenes.drum_mesh(radius, length, 32, 8, 2, (0.5 * length, radius, radius))
+    tet = np.array([[1, 1, 1, 0], [1, -1, -1, 0], [-1, 1, -1, 0], [-1, -1, 1, 0]]) * (0.3 * r) + (0, 0, 0, 0.5 * r)
+    pos = np.concatenate([sites[clumps:], np.full((len(sites) - clumps, 1), r)], 1).astype(np.float32)
+    vel = rng.uniform(-0.5, 0.5, pos.shape).astype(np.float32)
+    vel[:, 3] = 1e-4
+    got, old = [], _abi.tune_get("listed_blocks")
+    try:
+        for engine, blocks in ((_abi.SD_ENGINE_SAP, 5), (_abi.SD_ENGINE_SAP, 4), (_abi.SD_ENGINE_SHP, 5)):
+            _abi.tune_set("listed_blocks", blocks)
+            cfg = sdlib.EngineConfig(box_hi=(length, 2 * radius, 2 * radius), walls=0, cell=2.01 * r,
+                                     pair_capacity=1 << 22, collision_engine=engine)
+            eng = sdlib.DEMEngine(cfg)
+            for c in sites[:clumps]:
+                eng.add_clump(tet.astype(np.float32), 1e-4, tuple(c))
+            eng.add_spheres(pos, vel)
+            eng.add_mesh(tris, (0.5 * length, radius, radius), (1.0, 0.0, 0.0), 20.0, patch)
+            eng.prepare()
+            eng.step(2e-6, 5)
+            eng.sync()
+            st = eng.stats()
+            assert st["device_errors"] == 0 and st["listed_steps"] > 0
+            got.append([bits(eng.positions()), bits(eng.velocities()), bits(eng.omegas())])
+            eng.close()
+    finally:
+        _abi.tune_set("listed_blocks", old)
+    for other in got[1:]:
+        assert all(np.array_equal(x, y) for x, y in zip(got[0], other))
