@@ -234,8 +234,8 @@ sd_status hull_prepare(sd_engine* h) {
     if (h->cfg.flags & SD_FLAG_RECORD)
         if ((s = halloc(h, &H.force, nb)) || (s = halloc(h, &H.torque, nb))) return s;
     void* tm = nullptr;
-    if ((s = sd_alloc_bytes(h, &tm, sd::lbvh_scratch_bytes(nb)))) return s;
-    sd::lbvh_carve(tm, nb, &S.tree);
+    if ((s = sd_alloc_bytes(h, &tm, sd::lbvh_scratch_bytes(nb, sd::kLbvhFirst)))) return s;
+    sd::lbvh_carve(tm, nb, &S.tree, sd::kLbvhFirst);
     void* mm = nullptr;
     if ((s = sd_alloc_bytes(h, &mm, sd::mlp_state_bytes()))) return s;
     S.mlp = sd::mlp_carve(mm);
@@ -617,7 +617,8 @@ sd_status sd_lbvh_scratch_bytes(uint64_t n, uint64_t pair_cap, uint64_t* bytes) 
     if (!bytes) return sd_fail(nullptr, SD_ERR_INVALID_ARG, "bytes NULL");
     if (n >= (1ull << 30)) return sd_fail(nullptr, SD_ERR_CAPACITY, "n must be < 2^30");
     auto al = [](uint64_t x) { return (x + 255) & ~255ull; };
-    *bytes = al(sd::lbvh_scratch_bytes((uint32_t)n)) + 2 * al(4 * (n + 1)) + 2 * al(4 * (2 * pair_cap + 1));
+    (void)pair_cap;
+    *bytes = al(sd::lbvh_scratch_bytes((uint32_t)n, sd::kLbvhUnique)) + al(4 * (n + 1));
     return SD_OK;
 }
 
@@ -635,8 +636,8 @@ sd_status sd_lbvh_pairs(uint64_t n, const float* d_lo4, const float* d_hi4, uint
     auto al = [](uint64_t x) { return (x + 255) & ~255ull; };
     char* p = static_cast<char*>(d_scratch);
     sd::Lbvh t;
-    sd::lbvh_carve(p, (uint32_t)n, &t);
-    p += al(sd::lbvh_scratch_bytes((uint32_t)n));
+    sd::lbvh_carve(p, (uint32_t)n, &t, sd::kLbvhUnique);
+    p += al(sd::lbvh_scratch_bytes((uint32_t)n, sd::kLbvhUnique));
     uint32_t* off = reinterpret_cast<uint32_t*>(p);
     const float4* lo = reinterpret_cast<const float4*>(d_lo4);
     const float4* hi = reinterpret_cast<const float4*>(d_hi4);
@@ -653,11 +654,11 @@ sd_status sd_lbvh_morton(uint64_t n, const float* d_lo4, const float* d_hi4, uin
                          uint64_t scratch_bytes, void* stream) {
     if (n && (!d_lo4 || !d_hi4 || !d_codes || !d_scratch)) return sd_fail(nullptr, SD_ERR_INVALID_ARG, "NULL pointer");
     if (n >= (1ull << 30)) return sd_fail(nullptr, SD_ERR_CAPACITY, "n must be < 2^30");
-    if (scratch_bytes < sd::lbvh_scratch_bytes((uint32_t)n))
+    if (scratch_bytes < sd::lbvh_scratch_bytes((uint32_t)n, sd::kLbvhUnique))
         return sd_fail(nullptr, SD_ERR_CAPACITY, "scratch smaller than sd_lbvh_scratch_bytes");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     sd::Lbvh t;
-    sd::lbvh_carve(d_scratch, (uint32_t)n, &t);
+    sd::lbvh_carve(d_scratch, (uint32_t)n, &t, sd::kLbvhUnique);
     cudaError_t e = sd::lbvh_morton_async(t, reinterpret_cast<const float4*>(d_lo4),
                                           reinterpret_cast<const float4*>(d_hi4), st);
     if (e == cudaSuccess && n) e = cudaMemcpyAsync(d_codes, t.keys, 4 * n, cudaMemcpyDeviceToDevice, st);

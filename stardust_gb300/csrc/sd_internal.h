@@ -86,14 +86,15 @@ struct Lbvh {
     float4 *node_lo, *node_hi;           // boxes of the subtrees below top nodes; top nodes: atomic bounds
     float4 *leaf_lo, *leaf_hi;
     uint32_t* counts;                    // per box id; the refit leaves it zero
-    uint32_t* first;                     // per box id: its first kLbvhFirst partners found (counting pass)
+    uint32_t* first;                     // per box id: its first partners found (counting pass)
     float4* rec;                         // per internal node: both children's boxes (lo.w = child ref)
     uint32_t* scan_scratch;
     uint32_t* status;                    // device error bits
 };
-constexpr int kLbvhFirst = 32;
-uint64_t lbvh_scratch_bytes(uint32_t n);
-void lbvh_carve(void* scratch, uint32_t n, Lbvh* t);
+// first partners kept per box: by lbvh_partners_async, by lbvh_unique_pairs_async
+constexpr int kLbvhFirst = 32, kLbvhUnique = 16;
+uint64_t lbvh_scratch_bytes(uint32_t n, int first);
+void lbvh_carve(void* scratch, uint32_t n, Lbvh* t, int first);
 cudaError_t lbvh_morton_async(Lbvh& t, const float4* lo, const float4* hi, cudaStream_t st);
 cudaError_t lbvh_build_async(Lbvh& t, const float4* lo, const float4* hi, cudaStream_t st);
 // new boxes in the tree the last build made (its leaf order and topology):

@@ -33,7 +33,7 @@ constexpr int kLbvhThreads = 256;
 constexpr uint32_t kLeaf = 0x80000000u;
 constexpr int kTreelet = 128;  // leaves of a subtree that a block's shared memory joins
 constexpr int kStack = 64;  // one lane's stack: at most an entry a level (tree_levels) and one more
-static_assert(kLbvhFirst >= (int)kPairKeep, "the sink keeps its partners in Lbvh::first");
+static_assert(kLbvhUnique >= (int)kPairKeep, "the sink keeps its partners in Lbvh::first");
 
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 8;
@@ -719,7 +719,7 @@ cudaError_t scan_exclusive_async(const uint32_t* in, uint32_t* out, uint32_t n, 
     return cudaGetLastError();
 }
 
-uint64_t lbvh_scratch_bytes(uint32_t n) {
+uint64_t lbvh_scratch_bytes(uint32_t n, int first) {
     const uint64_t m = n ? n : 1;
     size_t b = 0;
     b += 4 * align256(4 * m);                                      // keys, vals, keys_tmp, vals_tmp
@@ -728,13 +728,13 @@ uint64_t lbvh_scratch_bytes(uint32_t n) {
     b += align256(8 * m) + align256(4 * (2 * m)) + 2 * align256(4 * m);  // children, parent, other, top
     b += 4 * align256(16 * m);                                     // node lo/hi, leaf lo/hi
     b += align256(4 * (m + 1)) + align256(4 * scan_scratch_words((uint32_t)m + 1));
-    b += align256(4 * kLbvhFirst * m);                             // first partners per leaf
+    b += align256(4 * (uint64_t)first * m);                        // first partners per box
     b += align256(64 * m);                                         // node records
     b += align256(4 * 4);                                          // status
     return b;
 }
 
-void lbvh_carve(void* scratch, uint32_t n, Lbvh* t) {
+void lbvh_carve(void* scratch, uint32_t n, Lbvh* t, int first) {
     const uint64_t m = n ? n : 1;
     char* p = static_cast<char*>(scratch);
     auto take = [&](size_t bytes) {
@@ -760,7 +760,7 @@ void lbvh_carve(void* scratch, uint32_t n, Lbvh* t) {
     t->leaf_hi = (float4*)take(16 * m);
     t->counts = (uint32_t*)take(4 * (m + 1));
     t->scan_scratch = (uint32_t*)take(4 * scan_scratch_words((uint32_t)m + 1));
-    t->first = (uint32_t*)take(4 * kLbvhFirst * m);
+    t->first = (uint32_t*)take(4 * (uint64_t)first * m);
     t->rec = (float4*)take(64 * m);
     t->status = (uint32_t*)take(16);
     t->skeys = t->keys;

@@ -372,13 +372,23 @@ __global__ void project_kernel(uint32_t n, const float4* __restrict__ lo, const 
 
 }  // namespace
 
-// (sd_sap_process_collisions takes its buffers from the same scratch.)
+// The kept partners lie over what the columns' sort is done with when the sweep
+// begins: the *_tmp arrays (two passes end where they began) and its scratch.
+static uint64_t keep_more_bytes(uint64_t m) {
+    const uint64_t over = 2 * al256(4 * kSlots * m) + al256(4 * sort_scratch_words(kSlots * m, 16));
+    return 4 * kPairKeep * m > over ? al256(4 * kPairKeep * m - over) : 0;
+}
 uint64_t sap_scratch_bytes(uint64_t n, uint64_t pair_cap) {
     const uint64_t m = n ? n : 1;
     (void)pair_cap;
-    return 4 * al256(4 * m) + al256(4 * sort_scratch_words(m, 32)) + al256(48 * m) + 4 * al256(4 * (m + 1)) +
+    return 4 * al256(4 * m) + al256(4 * sort_scratch_words(m, 32)) + al256(32 * m) + 4 * al256(4 * (m + 1)) +
            al256(4 * scan_scratch_words((uint32_t)m + 1)) + al256(16) + 4 * al256(4 * kSlots * m) +
-           al256(4 * sort_scratch_words(kSlots * m, 16)) + al256(64) + al256(4 * kPairKeep * m);
+           al256(4 * sort_scratch_words(kSlots * m, 16)) + keep_more_bytes(m) + al256(64);
+}
+// What sd_sap_process_collisions takes of it: the x sort, corners and projections.
+static uint64_t process_scratch_bytes(uint64_t n) {
+    const uint64_t m = n ? n : 1;
+    return 4 * al256(4 * m) + al256(4 * sort_scratch_words(m, 32)) + al256(48 * m);
 }
 
 cudaError_t sap_aabb_async(uint32_t n, const float4* pos, const float* radius, float4* lo, float4* hi,
@@ -420,7 +430,7 @@ cudaError_t sap_pairs_async(uint32_t n, const float4* lo, const float4* hi, void
     uint32_t* keys_tmp = (uint32_t*)take(4 * m);
     uint32_t* vals_tmp = (uint32_t*)take(4 * m);
     uint32_t* sort_scratch = (uint32_t*)take(4 * sort_scratch_words(m, 32));
-    float4* box = (float4*)take(48 * m);  // 32 bytes each; the rest is sd_sap_process_collisions'
+    float4* box = (float4*)take(32 * m);
     uint32_t* counts = (uint32_t*)take(4 * (m + 1));
     uint32_t* eoff = (uint32_t*)take(4 * (m + 1));
     uint32_t* off = (uint32_t*)take(4 * (m + 1));
@@ -432,8 +442,9 @@ cudaError_t sap_pairs_async(uint32_t n, const float4* lo, const float4* hi, void
     uint32_t* ckeys_tmp = (uint32_t*)take(4 * kSlots * m);
     uint32_t* cvals_tmp = (uint32_t*)take(4 * kSlots * m);
     uint32_t* csort = (uint32_t*)take(4 * sort_scratch_words(kSlots * m, 16));
+    take(keep_more_bytes(m));
     SapBounds* bounds = (SapBounds*)take(64);
-    uint32_t* keep = (uint32_t*)take(4 * kPairKeep * m);
+    uint32_t* keep = ckeys_tmp;  // (free when the sweep begins)
     static_assert(sizeof(SapBounds) <= 64, "bounds fit their scratch");
     if (n == 0) return cudaMemsetAsync(d_count2, 0, 8, st);
     // (the caller's two pointers by memsets, which check them; the rest by kernels)
@@ -459,14 +470,13 @@ cudaError_t sap_pairs_async(uint32_t n, const float4* lo, const float4* hi, void
     if ((e = sort_pairs_async(ckeys, cvals, ckeys_tmp, cvals_tmp, ne, 16, csort, st, &c_tmp, eoff + n, true)) !=
         cudaSuccess)
         return e;
-    const uint32_t* sk = c_tmp ? ckeys_tmp : ckeys;
-    const uint32_t* sv = c_tmp ? cvals_tmp : cvals;
+    if (c_tmp) return cudaErrorUnknown;  // (16 bits: two passes)
     const PairSink sink{counts, keep, status + 1, off, cursor, out, n, pair_cap};
     launch_after(st, std::min(grid_for(ne, kSweep), 152u * kSweepBlocks), kSweep, 0, sweep_binned_kernel<false>,
-                 eoff + n, sk, sv, box, bounds, sink);
+                 eoff + n, ckeys, cvals, box, bounds, sink);
     if ((e = scan_exclusive_async(counts, off, n, scan, st)) != cudaSuccess) return e;
-    launch_after(st, std::min(grid_for(ne, kSweep), 152u * 4), kSweep, 0, sweep_binned_kernel<true>, eoff + n, sk, sv,
-                 box, bounds, sink);
+    launch_after(st, std::min(grid_for(ne, kSweep), 152u * 4), kSweep, 0, sweep_binned_kernel<true>, eoff + n, ckeys,
+                 cvals, box, bounds, sink);
     launch_after(st, grid, kSapThreads, 0, pairs_write_kernel, sink, d_count2, status);
     return cudaGetLastError();
 }
@@ -516,7 +526,7 @@ sd_status sd_sap_process_collisions(uint64_t n, const float* d_pos4, const float
                                     void* d_scratch, uint64_t scratch_bytes, void* stream) {
     if (n && (!d_pos4 || !d_rows || !d_scratch)) return sd_fail(nullptr, SD_ERR_INVALID_ARG, "NULL pointer");
     if (n >= (1ull << 31) / 16) return sd_fail(nullptr, SD_ERR_CAPACITY, "n too large for 16-entry rows");
-    if (scratch_bytes < sd::sap_scratch_bytes(n, 0))
+    if (scratch_bytes < sd::process_scratch_bytes(n))
         return sd_fail(nullptr, SD_ERR_CAPACITY, "scratch smaller than sd_sap_scratch_bytes(n, 0)");
     if ((reinterpret_cast<uintptr_t>(d_pos4) | reinterpret_cast<uintptr_t>(d_rows)) & 15u)
         return sd_fail(nullptr, SD_ERR_INVALID_ARG, "positions and rows must be 16-byte aligned");

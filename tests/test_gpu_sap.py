@@ -190,3 +190,53 @@ def test_sweep_past_a_blocks_entries(sdlib, orc, n, cols):
     got, cnt, err = sdlib.SweepAndPrune.pairs(torch.from_numpy(L).cuda(), torch.from_numpy(H).cuda(), len(want) + 1)
     assert err == 0 and cnt == len(want)
     assert np.array_equal(got.cpu().numpy().view(np.uint64), want)
+
+
+def _workspace(op, n, cap):
+    """Bytes of the workspace that held both ways' partner lists, which a
+    program may keep: it stays enough."""
+    a = lambda x: (x + 255) // 256 * 256
+    m = max(n, 1)
+    sort = lambda k, passes: a(4 * (16 + 4 * 512 + passes * -(-k // 2048) * 512))
+    scan = a(4 * (-(-(m + 1) // 2048) + 1))
+    if op == "lbvh":
+        return (4 * a(4 * m) + sort(m, 4) + a(32) + a(24 * 304) + a(8 * m) + a(8 * m) + a(4 * m) + 4 * a(16 * m) +
+                a(4 * (m + 1)) + scan + 2 * a(64 * m) + a(16) + 2 * a(4 * (n + 1)) +
+                2 * a(4 * (2 * cap + 1)))
+    return (4 * a(4 * m) + sort(m, 4) + 4 * a(16 * m) + 3 * a(4 * (m + 1)) + scan + a(4 * (2 * cap + 1)) + a(16) +
+            4 * a(16 * m) + sort(4 * m, 2) + a(64))
+
+
+@pytest.mark.parametrize("op", ["sap", "lbvh", "process"])
+@pytest.mark.parametrize("n", [1, 300, 5000, 100_003])
+def test_workspaces_stay_enough(sdlib, orc, op, n):
+    """A workspace of the size above is taken, and nothing is written past
+    the size that the library asks for."""
+    import ctypes as C
+    import torch
+    from stardust_gb300 import _abi
+    rng = np.random.default_rng(n)
+    L, H = np.zeros((n, 4), np.float32), np.zeros((n, 4), np.float32)
+    c = rng.uniform(0.1, 0.9, (n, 3))
+    L[:, :3], H[:, :3] = c - 0.5 * n ** (-1 / 3), c + 0.5 * n ** (-1 / 3)
+    want = orc.aabb_pairs(L, H)
+    cap = 0 if op == "process" else len(want)
+    ask = C.c_uint64()
+    _abi.call("sd_lbvh_scratch_bytes" if op == "lbvh" else "sd_sap_scratch_bytes", n, cap, C.byref(ask))
+    kept = _workspace("lbvh" if op == "lbvh" else "sap", n, cap)
+    buf = torch.full((max(kept, ask.value) + 4096,), 0xA5, dtype=torch.uint8, device="cuda")
+    st = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    lo, hi = torch.from_numpy(L).cuda(), torch.from_numpy(H).cuda()
+    if op == "process":
+        pos = torch.from_numpy(np.concatenate([c, np.full((n, 1), 0.01)], 1).astype(np.float32)).cuda()
+        rows = torch.empty((n, 16), dtype=torch.int32, device="cuda")
+        _abi.call("sd_sap_process_collisions", n, pos.data_ptr(), None, rows.data_ptr(), buf.data_ptr(), kept, st)
+        assert torch.equal(rows, sdlib.SweepAndPrune.process_collisions(pos))
+    else:
+        out = torch.empty(max(cap, 1), dtype=torch.int64, device="cuda")
+        cnt = torch.zeros(2, dtype=torch.int32, device="cuda")
+        _abi.call(f"sd_{op}_pairs", n, lo.data_ptr(), hi.data_ptr(), out.data_ptr(), cap, cnt.data_ptr(), buf.data_ptr(),
+                  kept, st)
+        assert cnt.tolist() == [len(want), 0]
+        assert np.array_equal(out.cpu().numpy().view(np.uint64)[:cap], want)
+    assert (buf[ask.value:] == 0xA5).all()
