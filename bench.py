@@ -442,7 +442,7 @@ def bench_batch(n_scenes: int, steps: int, warmup: int, local: int, tune: bool):
     tuned = None
     if tune:
         from stardust_gb300 import autotune
-        tuned = autotune.tune_engine(eng, dt, reps=3)
+        tuned = autotune.tune_engine(eng, dt, reps=3, steps=1)
     ms = timed(eng, steps)
     st = eng.stats()
     eng.close()
@@ -504,7 +504,7 @@ def bench_drum(steps: int, warmup: int, local: int, tune: bool = True):
     if tune:  # the contact-list skin, timed by the mean over 24 steps (the turning wall makes builds recur)
         from stardust_gb300 import autotune
         tuned = autotune.tune_engine(eng, dt, reps=24, knobs={"skin_um": (50, 100, 200, 400, 800, 1600)},
-                                     rounds=1, label="drum", stat="mean")
+                                     rounds=1, label="drum", stat="mean", steps=1)
     flush = torch.empty(256 << 20, dtype=torch.uint8, device=f"cuda:{local}")
     st = torch.cuda.ExternalStream(eng.stream(), device=torch.device("cuda", local))
     a = [torch.cuda.Event(enable_timing=True) for _ in range(steps)]
@@ -652,7 +652,7 @@ def bench_dense_bed(pos, vel, cfg, dt, steps: int, advance: int, local: int, tun
     tuned = None
     if tune:  # the skin and the list kernel's register budget, for this contact network
         tuned = autotune.tune_engine(eng, dt, reps=3, knobs={"skin_um": (0, 50, 200, 500), "listed_blocks": (4, 5, 6)},
-                                     label=autotune.bucket_of(eng) + ":dense")
+                                     label=autotune.bucket_of(eng) + ":dense", steps=1)
     skin = _abi.tune_get("skin_um")
     eng.step(dt, 3)
     ms = statistics.mean(timed_steps(eng, dt, steps, stream, flush))
@@ -703,7 +703,7 @@ def run_ours(args, rank, world, local):
     tuned = None
     if not args.no_tune:
         from stardust_gb300 import autotune
-        tuned = autotune.tune_engine(eng, dt, reps=5)
+        tuned = autotune.tune_engine(eng, dt, reps=5, steps=1)
         log(f"autotune: {tuned}")
     # the knobs this workload is timed with (later sections tune their own)
     knobs = {k: _abi.tune_get(k) for k in ("contact_mode", "sort_items", "z_div", "resort_max", "pair_lists",

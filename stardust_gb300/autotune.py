@@ -11,7 +11,8 @@ reorder's grid.  The search is coordinate descent -- every value of one knob
 with the others held, knob after knob, two rounds -- from the current
 settings, so a knob that interacts with another is revisited once the other
 has moved.  Combinations that run the same kernels as one already timed are
-skipped.
+skipped.  Settings are timed in calls of as many steps as the program makes
+(`steps`): a call of four or more runs other kernels than calls of one.
 
 Choices are kept per size bucket: the engine's kind (one scene, or a batch
 of scenes) and its sphere count in powers of eight from 4,096.  ``apply``
@@ -55,31 +56,74 @@ def _redundant(c: dict) -> bool:
     return False
 
 
-def _time(eng, dt: float, reps: int, stream, flush, stat: str = "median") -> float:
+# The library's dispatch (sd_engine.cu, sd_dem.cu): steps of a call from which
+# it runs fused steps, and spheres up to which listed_blocks 5 takes 4.
+RUN_MIN = 4
+LISTED_SMALL = 800_000
+
+
+def _budgets(eng) -> str:
+    """Which register budgets of the list kernel the engine's scene has
+    (none: past three radix passes of cells a scene takes no lists)."""
+    if hasattr(eng, "stats") and eng.stats()["n_cells"] > 1 << 27:
+        return "none"
+    if hasattr(eng, "mesh") and len(eng.mesh()[0]):
+        return "swept mesh" if eng.config.collision_engine == _abi.SD_ENGINE_SAP else "one"
+    if getattr(eng, "n_bodies", 0):
+        return "one"
+    return "batch" if getattr(eng, "n_scenes", 0) > 1 else "spheres"
+
+
+def _kernels(c: dict, n: int, budgets: str, steps: int) -> tuple:
+    """What c makes the engine run: its knobs, less those that pick nothing
+    under the others, values that pick the same kernel as one."""
+    full = {k: c.get(k, _abi.tune_get(k)) for k in ("skin_um", "resort_max", "contact_mode")}
+    lists = full["skin_um"] > 0 and full["resort_max"] > 0 and full["contact_mode"] == 0 and budgets != "none"
+    k = dict(c)
+    if lists:
+        k.pop("contact_block", None)  # the list kernel has a block size of its own
+    else:
+        k.pop("listed_blocks", None)
+    if "listed_blocks" in k:
+        b = 4 if k["listed_blocks"] == 5 and n <= LISTED_SMALL else k["listed_blocks"]
+        if budgets == "one" or (budgets == "batch" and b != 5):
+            b = 4
+        elif budgets == "swept mesh" and b != 4:
+            b = 5
+        k["listed_blocks"] = b
+    if "fix_blocks" in k and steps >= RUN_MIN and full["resort_max"] > 0:
+        k["fix_blocks"] = 8 if k["fix_blocks"] == 8 else 4  # blocks per SM of the step kernel: two or one
+    return tuple(sorted(k.items()))
+
+
+def _time(eng, dt: float, reps: int, stream, flush, stat: str = "median", steps: int = 8) -> float:
     import torch
-    eng.step(dt, 2)  # re-capture + warm
+    for _ in range(2):  # captures the graphs such calls launch, on either assignment of the buffers
+        eng.step(dt, steps)
     eng.sync()
     ev = [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)) for _ in range(reps)]
     for a, b in ev:
         with torch.cuda.stream(stream):
             flush.fill_(1)
         a.record(stream)
-        eng.step(dt, 1)
+        eng.step(dt, steps)
         b.record(stream)
     torch.cuda.synchronize()
-    ms = sorted(a.elapsed_time(b) for a, b in ev)
+    ms = sorted(a.elapsed_time(b) / steps for a, b in ev)
     return sum(ms) / len(ms) if stat == "mean" else ms[len(ms) // 2]
 
 
 def tune_engine(eng, dt: float, reps: int = 5, knobs: dict | None = None, rounds: int = 2,
                 flush_bytes: int = 256 << 20, label: str | None = None, stat: str = "median",
-                timer=None) -> dict:
+                timer=None, steps: int = 8) -> dict:
     """Coordinate descent over `knobs` (default: the bucket kind's set) on
     the live engine; sets the best and records it for the engine's bucket
     (or under `label`, for a regime of one bucket tuned apart, e.g. a dense
-    bed).  Each setting is timed over `reps` steps by their median, or by
-    their mean (stat "mean": for scenes whose contact-list builds recur
-    within a few steps, e.g. a turning drum, so that the builds count).
+    bed).  Each setting is timed over `reps` calls of `steps` steps, as long
+    as those of the program (1 for one that steps and looks), by the median of
+    their times a step, or by the mean (stat "mean": for scenes whose
+    contact-list builds recur within a few steps, e.g. a turning drum, so that
+    the builds count).
     `timer` (tests): a function of no arguments that times the current
     settings in its place.  Returns {"bucket", "choice", "ms", "table"}:
     every timed setting."""
@@ -94,13 +138,14 @@ def tune_engine(eng, dt: float, reps: int = 5, knobs: dict | None = None, rounds
         flush = torch.empty(flush_bytes, dtype=torch.uint8, device=dev)
 
         def timer():
-            return _time(eng, dt, reps, stream, flush, stat)
+            return _time(eng, dt, reps, stream, flush, stat, steps)
     cur = {k: _abi.tune_get(k) for k in knobs}
     seen: dict[tuple, float] = {}
     table = []
+    budgets = _budgets(eng)
 
     def run(c: dict) -> float:
-        key = tuple(sorted(c.items()))
+        key = _kernels(c, eng.n, budgets, steps)
         if key not in seen:
             for k, v in c.items():
                 _abi.tune_set(k, v)

@@ -97,3 +97,78 @@ def test_coordinate_descent_finds_the_best_setting(sdlib):
         for k, v in old.items():
             _abi.tune_set(k, v)
         autotune._TABLE.pop("test:cost", None)
+
+
+class _Steps(FakeEngine):
+    def __init__(self, n, scenes=0):
+        super().__init__(n, scenes)
+        self.calls = []
+
+    def step(self, dt, k):
+        self.calls.append(k)
+
+    def sync(self):
+        pass
+
+
+def test_settings_of_the_same_kernels_are_timed_once(sdlib):
+    """With lists on, the contact kernel's block size picks nothing, and up to
+    800,000 spheres four and five blocks of the list kernel are the same."""
+    from stardust_gb300 import _abi, autotune
+    old = {k: _abi.tune_get(k) for k in autotune.SCENE_KNOBS}
+    try:
+        for n in (4096, 1 << 20):
+            for k, v in old.items():
+                _abi.tune_set(k, v)
+            rows = []
+
+            def timer():
+                rows.append({k: _abi.tune_get(k) for k in autotune.SCENE_KNOBS})
+                return float(len(rows) % 7)
+
+            autotune.tune_engine(_Steps(n), 1e-5, label="test:same", timer=timer)
+            ran = set()
+            for c in rows:
+                on = c["skin_um"] > 0 and c["contact_mode"] == 0
+                c["contact_block" if on else "listed_blocks"] = None
+                if n <= 800_000 and c["listed_blocks"] == 5:
+                    c["listed_blocks"] = 4
+                ran.add(tuple(sorted((k, str(v)) for k, v in c.items())))
+            assert len(ran) == len(rows)
+    finally:
+        for k, v in old.items():
+            _abi.tune_set(k, v)
+        autotune._TABLE.pop("test:same", None)
+
+
+def test_settings_are_timed_in_calls_of_the_programs_length(monkeypatch):
+    """A call of four or more steps runs other kernels than calls of one: the
+    timed calls are as long as those to come, runs unless told otherwise."""
+    import torch
+    from stardust_gb300 import autotune
+
+    class Event:
+        def __init__(self, enable_timing):
+            pass
+
+        def record(self, stream):
+            pass
+
+        def elapsed_time(self, other):
+            return 24.0
+
+    class Nothing:
+        def __enter__(self):
+            pass
+
+        def __exit__(self, *a):
+            pass
+
+    monkeypatch.setattr(torch.cuda, "Event", Event)
+    monkeypatch.setattr(torch.cuda, "stream", lambda s: Nothing())
+    monkeypatch.setattr(torch.cuda, "synchronize", lambda: None)
+    flush = torch.empty(1)
+    eng = _Steps(4096)
+    assert autotune._time(eng, 1e-5, 3, None, flush) == 3.0 and set(eng.calls) == {8}
+    eng = _Steps(4096)
+    assert autotune._time(eng, 1e-5, 3, None, flush, steps=1) == 24.0 and set(eng.calls) == {1}
