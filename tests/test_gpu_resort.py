@@ -160,3 +160,73 @@ def test_runs_of_steps_bit_exact(sdlib, orc, n, resort_max, moved, items):
     finally:
         for k, v in old.items():
             _abi.tune_set(k, v)
+
+
+def _state(eng):
+    eng.sync()
+    assert eng.stats()["device_errors"] == 0
+    return [bits(eng.positions()), bits(eng.velocities()), bits(eng.omegas())[:, :3]]
+
+
+@pytest.mark.parametrize("items,fix_blocks", [(8, 4), (16, 8)])
+def test_run_fallback_with_more_tiles_than_blocks(sdlib, items, fix_blocks):
+    """The step kernel's radix passes when its blocks take several tiles each
+    (one block per SM and tiles of 2,048 keys: 196 tiles for 152 blocks; two
+    and 4,096: 329 for 304), against the separate kernels of one-step calls."""
+    from stardust_gb300 import _abi
+    knobs = {"resort_max": 256, "sort_items": items, "fix_blocks": fix_blocks}
+    old = {k: _abi.tune_get(k) for k in knobs}
+    n = 400_000 if items == 8 else 1_345_000
+    try:
+        for k, v in knobs.items():
+            _abi.tune_set(k, v)
+        small, vel, cfg, dt = moving_scene(50_000, 900, seed=5)
+        copies = -(-n // len(small))  # side by side along x, in one box
+        width = float(cfg.box_hi[0])
+        pos = np.concatenate([small + np.float32([c * width, 0, 0, 0]) for c in range(copies)])[:n]
+        vel = np.concatenate([np.roll(vel, c, 0) for c in range(copies)])[:n]
+        cfg.box_hi = (copies * width, *cfg.box_hi[1:])
+        got = []
+        for calls in ([9], [1] * 9):
+            eng = sdlib.DEMEngine(cfg)
+            eng.add_spheres(pos, vel)
+            eng.prepare()
+            moved = []
+            for k in calls:
+                eng.step(dt, k)
+                moved.append(eng.stats()["moved_keys"])
+            assert min(moved) > 256
+            got.append(_state(eng))
+            eng.close()
+        assert all(np.array_equal(a, b) for a, b in zip(*got))
+    finally:
+        for k, v in old.items():
+            _abi.tune_set(k, v)
+
+
+def test_engines_in_runs_beside_each_other(sdlib):
+    """Two engines in runs of steps from two threads, each step a kernel whose
+    blocks meet: the states that each reaches alone."""
+    import threading
+    scenes = [moving_scene(60_000, 300, seed=3), moving_scene(20_000, 2_000, seed=4)]
+
+    def run(k, out):
+        pos, vel, cfg, dt = scenes[k]
+        eng = sdlib.DEMEngine(cfg)
+        eng.add_spheres(pos, vel)
+        eng.prepare()
+        for _ in range(10):
+            eng.step(dt, 16)
+        out[k] = _state(eng)
+        eng.close()
+
+    alone, beside = {}, {}
+    for k in (0, 1):
+        run(k, alone)
+    threads = [threading.Thread(target=run, args=(k, beside)) for k in (0, 1)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for k in (0, 1):
+        assert all(np.array_equal(a, b) for a, b in zip(alone[k], beside[k]))

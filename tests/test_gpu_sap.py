@@ -240,3 +240,62 @@ def test_workspaces_stay_enough(sdlib, orc, op, n):
         assert cnt.tolist() == [len(want), 0]
         assert np.array_equal(out.cpu().numpy().view(np.uint64)[:cap], want)
     assert (buf[ask.value:] == 0xA5).all()
+
+
+@pytest.mark.parametrize("n", [287, 288, 289, 543, 544, 545])
+def test_sweep_at_the_end_of_a_blocks_entries(sdlib, orc, n):
+    """One column that ends at, before and behind the 256 + 32 entries that a
+    block holds, and so for the second block; every box's window in x reaches
+    past them."""
+    import torch
+    rng = np.random.default_rng(n)
+    c = rng.uniform(0.0, 1.0, (n, 3)).astype(np.float32)
+    h = np.array([1.0, 0.02, 0.02], np.float32)
+    c[:, 1:] *= np.float32(0.03)
+    L = np.zeros((n, 4), np.float32)
+    H = np.zeros((n, 4), np.float32)
+    L[:, :3] = c - h
+    H[:, :3] = c + h
+    want = orc.aabb_pairs(L, H)
+    assert len(want) > 30 * n
+    got, cnt, err = sdlib.SweepAndPrune.pairs(torch.from_numpy(L).cuda(), torch.from_numpy(H).cuda(), len(want))
+    assert err == 0 and cnt == len(want)
+    assert np.array_equal(got.cpu().numpy().view(np.uint64), want)
+
+
+@pytest.mark.parametrize("op,n", [("sap", 50_001), ("lbvh", 5_001), ("lbvh", 70_001)])
+def test_pairs_captured(sdlib, orc, op, n):
+    """The operators in a caller's graph, where what a step clears is cleared
+    by memsets and the launches are plain ones: replayed on new boxes and over
+    a workspace that holds something else."""
+    import ctypes as C
+    import torch
+    from stardust_gb300 import _abi
+    rng = np.random.default_rng(n)
+    boxes = []
+    for _ in range(2):
+        L, H = np.zeros((n, 4), np.float32), np.zeros((n, 4), np.float32)
+        c = rng.uniform(0.0, 1.0, (n, 3))
+        h = rng.uniform(0.2, 1.0, (n, 1)) * n ** (-1 / 3)
+        L[:, :3], H[:, :3] = c - h, c + h
+        boxes.append((L, H, orc.aabb_pairs(L, H)))
+    cap = max(len(b[2]) for b in boxes)
+    size = C.c_uint64()
+    _abi.call(f"sd_{op}_scratch_bytes", n, cap, C.byref(size))
+    scratch = torch.zeros(size.value, dtype=torch.uint8, device="cuda")
+    lo, hi = (torch.zeros((n, 4), device="cuda") for _ in range(2))
+    out = torch.zeros(cap, dtype=torch.int64, device="cuda")
+    cnt = torch.zeros(2, dtype=torch.int32, device="cuda")
+    graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.graph(graph, stream=side):
+        _abi.call(f"sd_{op}_pairs", n, lo.data_ptr(), hi.data_ptr(), out.data_ptr(), cap, cnt.data_ptr(),
+                  scratch.data_ptr(), scratch.numel(), C.c_void_p(side.cuda_stream))
+    for fill, (L, H, want) in zip((0xAB, 0x01, 0xFF), (*boxes, boxes[0])):
+        lo.copy_(torch.from_numpy(L))
+        hi.copy_(torch.from_numpy(H))
+        scratch.fill_(fill)
+        cnt.fill_(7)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert cnt.tolist() == [len(want), 0]
+        assert np.array_equal(out.cpu().numpy().view(np.uint64)[:len(want)], want)
