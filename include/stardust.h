@@ -405,13 +405,14 @@ sd_status sd_engine_mlp_train(sd_engine* h, const float* d_feat16, const float* 
 /* ------------------------------------------------------ sweep and prune
  * (SAPCollision, src/engine/cuda/collisions/SAP/sap_detection.cu:135-706). */
 
-/* Device scratch for sd_sap_pairs (pair_cap pairs) and
- * sd_sap_process_collisions (pair_cap 0). */
+/* Device scratch for sd_sap_pairs (pair_cap pairs; the size does not depend
+ * on them) and sd_sap_process_collisions (pair_cap 0; takes less of it). */
 sd_status sd_sap_scratch_bytes(uint64_t n, uint64_t pair_cap, uint64_t* bytes);
 /* Exact broad phase: every pair (i < j) of overlapping closed boxes,
  * ascending u64 (i << 32 | j), by sorting the lower x extents (order-
  * preserving keys, negative coordinates allowed) and sweeping.  d_count[0] =
- * pairs, d_count[1] = device error bits. */
+ * pairs (0, and nothing is written, when there are more than cap), d_count[1] =
+ * device error bits (SD_DEVERR_PAIR_OVERFLOW then). */
 sd_status sd_sap_pairs(uint64_t n, const float* d_lo4, const float* d_hi4, uint64_t* d_pairs, uint64_t cap,
                        uint32_t* d_count, void* d_scratch, uint64_t scratch_bytes, void* stream);
 /* sweepAndPruneCUDA (sap_detection.cu:385-440) on given sorted inputs: per
@@ -435,9 +436,9 @@ sd_status sd_sap_process_collisions(uint64_t n, const float* d_pos4, const float
 /* Device scratch for sd_lbvh_pairs / sd_lbvh_morton. */
 sd_status sd_lbvh_scratch_bytes(uint64_t n, uint64_t pair_cap, uint64_t* bytes);
 /* Every pair (i < j) of overlapping closed boxes, ascending u64
- * (i << 32 | j).  d_count[0] = number of pairs (written up to cap),
- * d_count[1] = device error bits (SD_DEVERR_PAIR_OVERFLOW when there are
- * more than cap pairs). */
+ * (i << 32 | j).  d_count[0] = number of pairs (0, and nothing is written,
+ * when there are more than cap), d_count[1] = device error bits
+ * (SD_DEVERR_PAIR_OVERFLOW then). */
 sd_status sd_lbvh_pairs(uint64_t n, const float* d_lo4, const float* d_hi4, uint64_t* d_pairs, uint64_t cap,
                         uint32_t* d_count, void* d_scratch, uint64_t scratch_bytes, void* stream);
 /* The reference's 30-bit Morton code of each box centroid relative to the

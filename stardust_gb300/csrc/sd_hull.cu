@@ -8,12 +8,12 @@
 // case analysis; EPA (van den Bergen 2001) for the penetration depth,
 // normal and witness points, which the reference lacks.
 //
-// Work split: one thread per candidate ENTRY (self, other) of the per-body
-// partner lists built by the LBVH; each entry evaluates its pair as
-// (A, B) = (min, max), so the two entries of a pair compute identical
-// numbers and take opposite signs -- exact action = reaction with no
-// atomics.  One thread per body then sums its entries in list order (the
-// segmented reduction), adds walls and gravity and integrates.
+// Work split: a few lanes per unique pair (A, B) = (min, max) of the per-body
+// partner lists built by the LBVH (four for the first support, eight for the
+// rest of GJK, a warp for EPA); what they find goes to the pair's entry in
+// A's list and to its mirror in B's with the opposite sign -- exact action =
+// reaction with no atomics.  One thread per body then sums its entries in list
+// order (the segmented reduction), adds walls and gravity and integrates.
 //
 // Every float operation follows oracle/sd_oracle_hull.c in order
 // (-fmad=false), so results are bit-identical to the CPU restatement.
@@ -1152,9 +1152,8 @@ cudaError_t hull_seed_async(HullBuffers& H, uint32_t mode, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-// Each pair is evaluated once, by one thread, into both of its entries.
-// The grid covers the largest possible pair count (cap / 2); threads past
-// the step's count return at once.
+// A training step's samples (w = 1 in teach) gathered in entry order: flags,
+// their scan, the copies.  Threads past the step's entry count return at once.
 __global__ void hull_teach_flags_kernel(const float4* __restrict__ teach, const uint32_t* __restrict__ d_count,
                                         uint32_t cap, uint32_t* __restrict__ flags) {
     stream_wait();

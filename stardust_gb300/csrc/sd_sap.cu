@@ -27,7 +27,7 @@
 //    lower y-z corner, so every pair is found once, by the same tests as the
 //    unbinned sweep: the same pair set, listed by sd_pairs.cuh.
 //    Measured, 2,000,000 boxes of one size, 2.25 entries and two pairs each:
-//    442 us in all; six radix passes 157, sweep 149, gather into x order 37, list
+//    425 us in all (488 in some processes); six radix passes 157, sweep 149, gather into x order 37, list
 //    31, entries 22, bounds 23, scans 19.  It was 1412: four entries for every
 //    box whether used or not, boxes of 48 bytes gathered through two indices,
 //    and the sweep twice, once to count.
